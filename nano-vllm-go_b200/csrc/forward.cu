@@ -87,7 +87,7 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
   WS(w.chain_ctr, 256);
   if (h->n_mamba) {
     WS(w.m_xbc, (size_t)Tc * h->m_conv * 4);
-    WS(w.m_dt, (size_t)Tc * h->m_nh * 4);
+    WS(w.m_dt, (size_t)Tc * h->m_nh * 8);
     WS(w.m_y, (size_t)Tc * h->m_E * 4);
     WS(w.m_yn, (size_t)Tc * h->m_E * asz);
   }

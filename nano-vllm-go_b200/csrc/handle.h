@@ -159,7 +159,7 @@ struct Workspace {
   void* hbuf = nullptr;      // [T, F] or [T k, I]
   void* xn_last = nullptr;   // [n, H]
   float* m_xbc = nullptr;    // [T, conv_dim] Mamba2: conv + SiLU output (x | B | C)
-  float* m_dt = nullptr;     // [T, heads]    softplus(dt + bias)
+  float2* m_dt = nullptr;    // [T, heads]    {softplus(dt + bias), the head's decay}
   float* m_y = nullptr;      // [T, E] fp32 scan output
   void* m_yn = nullptr;      // [T, E] gated + normed, act dtype (out_proj input)
   // folded RMSNorm (forward.cu): bf16(x * g) of the residual stream (g = the next norm's weight), the

@@ -677,7 +677,7 @@ struct MambaArgs {
   size_t stride;
   const float *conv_w, *conv_b, *dt_bias, *a_log, *d_skip, *norm_w;
   float* xbc;          // [T, conv]  SiLU(conv1d(xBC))
-  float* dt;           // [T, nh]    softplus(dt + bias)
+  float2* dt;          // [T, nh]    {softplus(dt + bias), exp(-exp(A_log) of it)}
   float* y;            // [T, E]     scan output
   const int* cu_q;         // [n_seqs + 1] rows of each sequence
   const int* positions;    // [T]

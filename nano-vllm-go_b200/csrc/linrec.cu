@@ -345,25 +345,6 @@ cudaError_t launch_mlstm_prep(cudaStream_t st, const LinRecArgs& a) {
 // lanes that share them) for 8 CN state entries, and updates two rows with one packed fp32 instruction
 // (f32x2: two independent IEEE fp32 operations).  The row groups' partial read-outs are summed by shuffles that
 // scatter the columns over the lanes, the warps' in shared memory once per chunk of tokens.
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // DP: rows of the state, padded (RG * 8 * WR); TMIX: read before the update, with a bonus; SD: one decay per
 // (token, head) instead of one per row; NRM (with SD): mLSTM — keys are scaled by the token's input gate, and the CTAs of
 // the first column range carry the vector n beside the state (every column group of lanes holds its 8 entries)

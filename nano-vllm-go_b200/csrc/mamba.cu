@@ -1,18 +1,19 @@
 // mamba.cu — Mamba2 block of the Granite-4 hybrid (SURVEY.md §8f rank 4;
 // purego/tensor/mamba2.go:72-351), for a ragged batch of sequences.  The two projections are
 // ordinary GEMMs (forward.cu); this file holds what sits between them:
-//   mamba_conv_kernel   sum of the in_proj split-K slices, causal conv1d over the xBC columns
+//   mamba_conv_rows_kernel  sum of the in_proj split-K slices, causal conv1d over the xBC columns
 //                       (zero-padded at the start of every CALL, like causalConv1d :209-270 — the
-//                       reference never reads its ConvCache), SiLU, and dt = softplus(dt + bias)
-//   mamba_scan_kernel   the selective scan (:273-351), sequential over a sequence's new tokens,
-//                       one CTA per (sequence, head), one thread per head_dim row holding its
-//                       state_size states in registers; the SSM state lives per KV BLOCK
-//                       (handle.h) and is read / written through the block table
+//                       reference never reads its ConvCache), SiLU; dt = softplus(dt + bias) and the
+//                       head's decay exp(-exp(A_log) dt)
+//   mamba_scan_tile_kernel  the selective scan (:273-351), sequential over a sequence's new tokens;
+//                       the SSM state lives per KV BLOCK (handle.h) and is read / written through
+//                       the block table
 //   mamba_gate_norm_kernel  y * silu(gate), RMS norm over E with eps 1e-5, * Norm (:139-173)
-// Correctness-first kernels: HBM traffic is small next to the projections, and the scan's
-// token loop is latency-bound by construction (a chunked scan is the obvious next step).
+// mamba_conv_kernel and mamba_scan_kernel take the sizes the first two do not: taps other than 4,
+// rows or heads that are no multiples of 16 bytes, states other than 16 / 32 / 64 / 128.
 #include "common.cuh"
 #include "kernels.h"
+#include "mma.cuh"
 
 namespace nvllm {
 
@@ -32,6 +33,34 @@ __device__ __forceinline__ float sum_slices(const float* __restrict__ p, int S, 
   float acc = 0.f;
   for (int s = 0; s < S; s++) acc += p[(size_t)s * stride];
   return acc;
+}
+
+// 16-byte accesses of the row kernels: four neighbouring channels per thread
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 sum_slices4(const float* __restrict__ p, int S, size_t stride) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < S; s++) {
+    const float4 v = ld4(p + (size_t)s * stride);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  return acc;
+}
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void st4(bf16* p, float a, float b, float c, float d) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+  uint2 u;
+  u.x = *reinterpret_cast<uint32_t*>(&lo);
+  u.y = *reinterpret_cast<uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(p) = u;
+}
+
+// step size softplus(z) (mamba2.go:369-376) and decay exp(-exp(A_log) dt) of a (token, head), through double
+__device__ __forceinline__ void store_step(const MambaArgs& a, int t, int h, float z) {
+  const float dt = (float)log(1.0 + exp((double)z));
+  const float A = a.a_log ? -(float)exp((double)a.a_log[h]) : 0.f;
+  a.dt[(size_t)t * a.nh + h] = make_float2(dt, a.a_log ? (float)exp((double)(A * dt)) : 1.0f);
 }
 
 }  // namespace
@@ -61,7 +90,7 @@ mamba_conv_kernel(MambaArgs a, Trace tr) {
     const int h = threadIdx.x;
     float dt = sum_slices(a.proj + (size_t)t * a.P + a.E + a.conv + h, a.S, a.stride);
     if (a.dt_bias) dt += a.dt_bias[h];
-    a.dt[(size_t)t * a.nh + h] = (float)log(1.0 + exp((double)dt));  // Softplus, mamba2.go:369-376
+    store_step(a, t, h, dt);
   }
   TRACE_EXIT(tr);
 }
@@ -93,7 +122,6 @@ mamba_scan_kernel(MambaArgs a, Trace tr) {
   }
   int grp = h * a.G / a.nh;
   if (grp >= a.G) grp = a.G - 1;
-  const float A = a.a_log ? -(float)exp((double)a.a_log[h]) : 0.f;
   const float Dh = a.d_skip ? a.d_skip[h] : 0.f;
   for (int t = r0; t < r1; t++) {
     __syncthreads();  // the previous token's sB / sC have been consumed
@@ -103,8 +131,8 @@ mamba_scan_kernel(MambaArgs a, Trace tr) {
     }
     __syncthreads();
     if (d < a.hd) {
-      const float dt = a.dt[(size_t)t * a.nh + h];
-      const float abar = a.a_log ? (float)exp((double)(A * dt)) : 1.0f;
+      const float2 step = a.dt[(size_t)t * a.nh + h];
+      const float dt = step.x, abar = step.y;
       const float u = a.xbc[(size_t)t * a.conv + (size_t)h * a.hd + d];
       float sum = 0.f;
 #pragma unroll
@@ -128,28 +156,235 @@ mamba_scan_kernel(MambaArgs a, Trace tr) {
   TRACE_EXIT(tr);
 }
 
+// ------------------------------------------------------------------ block-pooled path, 16-byte rows
+// Rows, segments and split-K slices of the projection start on 16-byte boundaries (E is a multiple of 8).
+static bool mamba_rows_aligned(const MambaArgs& a) { return a.P % 4 == 0 && a.conv % 4 == 0 && a.stride % 4 == 0; }
+
+// Convolution of MC_ROWS neighbouring rows, four channels per thread: the K taps of a channel quad stay in
+// registers and every row of the projection is read once per window instead of once per tap (bound by memory:
+// one read of the xBC columns and one write).  blockIdx.y == 0 also makes the steps and decays of its rows.
+// 16 sequences of 256 to 512 tokens (6446 rows), 6144 channels: 131 us (2.4 TB/s), 465 us with one channel and token
+// per thread and K strided loads each.
+constexpr int MC_ROWS = 8;
+template <int K>
+__global__ void __launch_bounds__(256) mamba_conv_rows_kernel(MambaArgs a, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  const int t0 = blockIdx.x * MC_ROWS, t1 = min(a.T, t0 + MC_ROWS);
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  float wv[4][K], bias[4] = {0.f, 0.f, 0.f, 0.f};  // immutable: fetched before the dependency resolves
+  if (c < a.conv) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+#pragma unroll
+      for (int k = 0; k < K; k++) wv[q][k] = a.conv_w[(size_t)(c + q) * K + k];
+      if (a.conv_b) bias[q] = a.conv_b[c + q];
+    }
+  }
+  pdl_wait();
+  int s = seq_of_row(a.cu_q, a.n_seqs, t0);
+  int first = a.cu_q[s], last = a.cu_q[s + 1];  // rows of the sequence that the current row belongs to
+  if (c < a.conv) {
+    float4 u[K];  // the window: u[K - 1] is the current row's input
+#pragma unroll
+    for (int k = 0; k + 1 < K; k++) {
+      const int t = t0 - (K - 1) + k;
+      u[k + 1] = t >= first ? sum_slices4(a.proj + (size_t)t * a.P + a.E + c, a.S, a.stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int t = t0; t < t1; t++) {
+      while (t >= last) {
+        s++;
+        first = last;
+        last = a.cu_q[s + 1];
+      }
+#pragma unroll
+      for (int k = 0; k + 1 < K; k++) {
+        u[k] = u[k + 1];
+        if (t - (K - 1 - k) < first) u[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      u[K - 1] = sum_slices4(a.proj + (size_t)t * a.P + a.E + c, a.S, a.stride);
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        y[0] += u[k].x * wv[0][k]; y[1] += u[k].y * wv[1][k];
+        y[2] += u[k].z * wv[2][k]; y[3] += u[k].w * wv[3][k];
+      }
+      st4(a.xbc + (size_t)t * a.conv + c, silu(y[0] + bias[0]), silu(y[1] + bias[1]), silu(y[2] + bias[2]), silu(y[3] + bias[3]));
+    }
+  }
+  if (blockIdx.y == 0)
+    for (int i = threadIdx.x; i < (t1 - t0) * a.nh; i += blockDim.x) {
+      const int t = t0 + i / a.nh, h = i % a.nh;
+      const float z = sum_slices(a.proj + (size_t)t * a.P + a.E + a.conv + h, a.S, a.stride);
+      store_step(a, t, h, a.dt_bias ? z + a.dt_bias[h] : z);
+    }
+  TRACE_EXIT(tr);
+}
+
+// Selective scan.  Four lanes share R rows of a head's state (lane q holds entries 16 j + 4 q .. + 3 of each, as
+// packed pairs in registers), 4 hd / R threads make a head and HPC heads of one group a CTA.  Per token a lane reads
+// N / 4 entries of B and of C (64 contiguous bytes per quad, broadcast to the warp's other rows) for R N / 4 state
+// entries and spends three packed instructions per entry pair; the four partial read-outs of a row meet by shuffles.
+// B, C, u and the (step, decay) pairs of the next MS_TC tokens arrive by cp.async under the current ones.
+// Bound by fp32 issue, 3 operations per state entry and token.  The 6446 rows above, 64 heads of 64 x 128: 730 us; a
+// thread per row with scalar operations and the decay computed in every thread: 7405 us.  R = 2 keeps five CTAs
+// of 128 threads on an SM; R = 1 doubles the threads of a head when few (sequence, head) pairs are to be shared out.
+constexpr int MS_TC = 8;
+template <int R, int NJ>
+__global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int hpc, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  constexpr int N = 16 * NJ;
+  extern __shared__ __align__(16) float sm[];
+  const int s = blockIdx.x, h0 = blockIdx.y * hpc;
+  const int tid = threadIdx.x, nt = blockDim.x, tph = 4 * a.hd / R;
+  const int hl = tid / tph, ht = tid % tph, q = ht & 3, d0 = (ht >> 2) * R, h = h0 + hl;
+  const int uw = hpc * a.hd, row = 2 * N + uw + 2 * hpc;  // floats of a staged token: B | C | u | (step, decay)
+  const int rowp = (row + 3) & ~3;
+  pdl_wait();
+  const int r0 = a.cu_q[s], r1 = a.cu_q[s + 1];
+  if (r0 >= r1) return;
+  const int start = a.positions[r0];  // position of the first new token
+  const int* bt = a.block_tables + (size_t)s * a.max_blocks;
+  const size_t per_layer = (size_t)a.nh * a.hd * N;
+  const size_t per_block = (size_t)a.n_mamba * per_layer;
+  const size_t mine = (size_t)a.layer * per_layer + ((size_t)h * a.hd + d0) * N + 4 * q;
+  const int grp = h0 / (a.nh / a.G);
+  const float* base = a.xbc + a.E + (size_t)grp * N;
+  auto fetch = [&](int t0, int buf) {
+    const int n = min(MS_TC, r1 - t0);
+    float* dst = sm + buf * MS_TC * rowp;
+    for (int i = tid; i < n * (N / 2 + uw / 4); i += nt) {
+      const int t = i / (N / 2 + uw / 4), p = i % (N / 2 + uw / 4);
+      const float* x = a.xbc + (size_t)(t0 + t) * a.conv;
+      const float* src = p < N / 4 ? base + (size_t)(t0 + t) * a.conv + 4 * p
+                         : p < N / 2 ? base + (size_t)(t0 + t) * a.conv + (size_t)a.G * N + 4 * (p - N / 4)
+                                     : x + (size_t)h0 * a.hd + 4 * (p - N / 2);
+      cp_async16(smem_addr(dst + t * rowp + 4 * p), src, true);
+    }
+    for (int i = tid; i < n * hpc; i += nt) {
+      const int t = i / hpc, k = i % hpc;
+      *reinterpret_cast<float2*>(dst + t * rowp + 2 * N + uw + 2 * k) = a.dt[(size_t)(t0 + t) * a.nh + h0 + k];
+    }
+    cp_async_commit();
+  };
+  fetch(r0, 0);
+  unsigned long long st[R][2 * NJ];
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int j = 0; j < 2 * NJ; j++) st[r][j] = 0ull;
+  if (start > 0) {
+    // the state after position start - 1 sits in that position's block
+    const float* src = a.ssm_pool + (size_t)bt[(start - 1) / KV_BLOCK] * per_block + mine;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+      for (int j = 0; j < NJ; j++) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + (size_t)r * N + 16 * j);
+        st[r][2 * j] = v.x;
+        st[r][2 * j + 1] = v.y;
+      }
+  }
+  const float Dh = a.d_skip ? a.d_skip[h] : 0.f;
+  for (int t0 = r0, buf = 0; t0 < r1; t0 += MS_TC, buf ^= 1) {
+    cp_async_wait<0>();
+    __syncthreads();  // this chunk has arrived, and everybody is done with the other buffer
+    if (t0 + MS_TC < r1) fetch(t0 + MS_TC, buf ^ 1);
+    const int n = min(MS_TC, r1 - t0);
+    for (int t = 0; t < n; t++) {
+      const float* x = sm + (buf * MS_TC + t) * rowp;
+      const float2 step = *reinterpret_cast<const float2*>(x + 2 * N + uw + 2 * hl);
+      const float* u = x + 2 * N + hl * a.hd + d0;
+      const unsigned long long decay = pack2(step.y, step.y);
+      unsigned long long du[R], acc[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const float v = step.x * u[r];
+        du[r] = pack2(v, v);
+        acc[r] = 0ull;
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; j++) {
+        const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(x + 16 * j + 4 * q);
+        const ulonglong2 Cc = *reinterpret_cast<const ulonglong2*>(x + N + 16 * j + 4 * q);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          st[r][2 * j] = fma2(decay, st[r][2 * j], mul2(du[r], B.x));          // mamba2.go:325-331
+          acc[r] = fma2(Cc.x, st[r][2 * j], acc[r]);                            // :335-340
+          st[r][2 * j + 1] = fma2(decay, st[r][2 * j + 1], mul2(du[r], B.y));
+          acc[r] = fma2(Cc.y, st[r][2 * j + 1], acc[r]);
+        }
+      }
+      float y[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        float lo, hi;
+        unpack2(acc[r], lo, hi);
+        y[r] = lo + hi;
+      }
+      float out;  // lanes q < R end up with row d0 + q
+      if constexpr (R == 2) {
+        const float give = (q & 1) ? y[0] : y[1], keep = (q & 1) ? y[1] : y[0];
+        out = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+      } else {
+        out = y[0] + __shfl_xor_sync(0xffffffffu, y[0], 1);
+      }
+      out += __shfl_xor_sync(0xffffffffu, out, 2);
+      if (q < R) a.y[(size_t)(t0 + t) * a.E + (size_t)h * a.hd + d0 + q] = out + Dh * u[q];
+      const int pos = start + (t0 + t - r0);
+      if ((pos + 1) % KV_BLOCK == 0 || t0 + t == r1 - 1) {
+        // snapshot: the state after the last token written into this block
+        float* dst = a.ssm_pool + (size_t)bt[pos / KV_BLOCK] * per_block + mine;
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+          for (int j = 0; j < NJ; j++)
+            *reinterpret_cast<ulonglong2*>(dst + (size_t)r * N + 16 * j) = make_ulonglong2(st[r][2 * j], st[r][2 * j + 1]);
+      }
+    }
+  }
+  TRACE_EXIT(tr);
+}
+
 // one CTA per token row: y[t, :] * silu(gate[t, :]) -> RMS norm (eps 1e-5, mamba2.go:150-166)
-// -> * Norm -> act dtype (the out_proj GEMM's input)
-template <typename OT>
+// -> * Norm -> act dtype (the out_proj GEMM's input).  V = 4: 16-byte accesses (aligned rows): 68 us for 6446 rows
+// of 4096 (bound by memory: gates, scan outputs and results once), 129 us with 4-byte ones.
+template <typename OT, int V>
 __global__ void __launch_bounds__(256)
 mamba_gate_norm_kernel(MambaArgs a, OT* __restrict__ out, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
   pdl_wait();
-  extern __shared__ float row[];
+  extern __shared__ __align__(16) float row[];
   __shared__ float red[32];
   const int t = blockIdx.x;
   float lsq = 0.f;
-  for (int i = threadIdx.x; i < a.E; i += blockDim.x) {
-    const float g = sum_slices(a.proj + (size_t)t * a.P + i, a.S, a.stride);
-    const float v = a.y[(size_t)t * a.E + i] * silu(g);
-    row[i] = v;
-    lsq += v * v;
+  for (int i = threadIdx.x * V; i < a.E; i += blockDim.x * V) {
+    const float* g = a.proj + (size_t)t * a.P + i;
+    const float* y = a.y + (size_t)t * a.E + i;
+    if constexpr (V == 4) {
+      const float4 g4 = sum_slices4(g, a.S, a.stride), y4 = ld4(y);
+      const float4 v = make_float4(y4.x * silu(g4.x), y4.y * silu(g4.y), y4.z * silu(g4.z), y4.w * silu(g4.w));
+      st4(row + i, v.x, v.y, v.z, v.w);
+      lsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    } else {
+      const float v = *y * silu(sum_slices(g, a.S, a.stride));
+      row[i] = v;
+      lsq += v * v;
+    }
   }
   const float tot = block_sum(lsq, red);
   const float rms = 1.0f / sqrtf(tot / (float)a.E + 1e-5f);
-  for (int i = threadIdx.x; i < a.E; i += blockDim.x)
-    out[(size_t)t * a.E + i] = from_f32<OT>(row[i] * rms * (a.norm_w ? a.norm_w[i] : 1.f));
+  OT* o = out + (size_t)t * a.E;
+  for (int i = threadIdx.x * V; i < a.E; i += blockDim.x * V) {
+    if constexpr (V == 4) {
+      const float4 v = ld4(row + i), w = a.norm_w ? ld4(a.norm_w + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+      st4(o + i, v.x * rms * w.x, v.y * rms * w.y, v.z * rms * w.z, v.w * rms * w.w);
+    } else {
+      o[i] = from_f32<OT>(row[i] * rms * (a.norm_w ? a.norm_w[i] : 1.f));
+    }
+  }
   TRACE_EXIT(tr);
 }
 
@@ -163,26 +398,6 @@ mamba_gate_norm_kernel(MambaArgs a, OT* __restrict__ out, Trace tr) {
 //                            clamp), the head's decay exp(-exp(A_log) dt), and dt x (the scan's values)
 //   mamba2_slot_out_kernel   one CTA per token: y = read-out + D x, times silu(z), RMS norm in norm_groups
 //                            equal parts (eps of the model), times the weight -> act dtype
-// 16-byte accesses of the row kernels below: four neighbouring channels per thread
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 sum_slices4(const float* __restrict__ p, int S, size_t stride) {
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = 0; s < S; s++) {
-    const float4 v = ld4(p + (size_t)s * stride);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-  }
-  return acc;
-}
-__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
-  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-__device__ __forceinline__ void st4(bf16* p, float a, float b, float c, float d) {
-  __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
-  uint2 u;
-  u.x = *reinterpret_cast<uint32_t*>(&lo);
-  u.y = *reinterpret_cast<uint32_t*>(&hi);
-  *reinterpret_cast<uint2*>(p) = u;
-}
 // every row, segment and tail of the two kernels starts on a 16-byte boundary
 __device__ __forceinline__ bool m2_rows_aligned(const Mamba2SlotArgs& a) {
   const int inner = a.heads * a.vdim, gn = a.G * a.N;
@@ -496,14 +711,42 @@ cudaError_t launch_mamba2_slot_out(cudaStream_t st, int odt, const Mamba2SlotArg
 
 cudaError_t launch_mamba_conv(cudaStream_t st, const MambaArgs& a) {
   if (a.T <= 0) return cudaSuccess;
-  (void)launch_k(mamba_conv_kernel, dim3(a.T, ceil_div(a.conv, 256)), dim3(256), 0, st, a, next_trace(20));
+  if (a.K == 4 && mamba_rows_aligned(a)) {
+    const dim3 grid(ceil_div(a.T, MC_ROWS), ceil_div(a.conv, 1024));
+    (void)launch_k(mamba_conv_rows_kernel<4>, grid, dim3(256), 0, st, a, next_trace(20));
+  } else {
+    (void)launch_k(mamba_conv_kernel, dim3(a.T, ceil_div(a.conv, 256)), dim3(256), 0, st, a, next_trace(20));
+  }
   return cudaGetLastError();
 }
 
+// heads of a CTA of the tiled scan, 0 where it does not fit: whole warps, the heads of a CTA from one group
+static int mamba_scan_hpc(const MambaArgs& a, int R) {
+  if (!mamba_rows_aligned(a) || a.hd % 4 != 0) return 0;
+  if (a.N != 16 && a.N != 32 && a.N != 64 && a.N != 128) return 0;
+  const int tph = 4 * a.hd / R, per_group = a.nh / a.G;
+  int hpc = 1;
+  while (hpc * 2 * tph <= 128 && per_group % (hpc * 2) == 0) hpc *= 2;
+  return hpc * tph % 32 == 0 && hpc * tph <= 512 ? hpc : 0;
+}
+template <int R>
+static cudaError_t mamba_scan_tiles(cudaStream_t st, const MambaArgs& a, int hpc) {
+  const dim3 grid(a.n_seqs, a.nh / hpc), block(hpc * 4 * a.hd / R);
+  const size_t smem = (size_t)2 * MS_TC * ((2 * a.N + hpc * a.hd + 2 * hpc + 3) & ~3) * sizeof(float);
+  if (a.N == 16) return launch_k(mamba_scan_tile_kernel<R, 1>, grid, block, smem, st, a, hpc, next_trace(21));
+  if (a.N == 32) return launch_k(mamba_scan_tile_kernel<R, 2>, grid, block, smem, st, a, hpc, next_trace(21));
+  if (a.N == 64) return launch_k(mamba_scan_tile_kernel<R, 4>, grid, block, smem, st, a, hpc, next_trace(21));
+  return launch_k(mamba_scan_tile_kernel<R, 8>, grid, block, smem, st, a, hpc, next_trace(21));
+}
 cudaError_t launch_mamba_scan(cudaStream_t st, const MambaArgs& a) {
   if (a.n_seqs <= 0) return cudaSuccess;
   const int threads = max(32, ((a.hd + 31) / 32) * 32);
   if (threads > 128 || a.N > 128) return cudaErrorInvalidValue;
+  // R = 1 has twice the warps per head and half the state per lane: the shorter chain per token
+  // while the grid leaves schedulers idle (148 SMs x 4, two warps each at 4 hd / 64 warps a head)
+  const int one = mamba_scan_hpc(a, 1), two = mamba_scan_hpc(a, 2);
+  if (two && (!one || (long)a.n_seqs * a.nh * a.hd * 4 / 64 > 148 * 8)) return mamba_scan_tiles<2>(st, a, two);
+  if (one) return mamba_scan_tiles<1>(st, a, one);
   const dim3 grid(a.n_seqs, a.nh);
   if (a.N <= 16) (void)launch_k(mamba_scan_kernel<16>, grid, dim3(threads), 0, st, a, next_trace(21));
   else if (a.N <= 32) (void)launch_k(mamba_scan_kernel<32>, grid, dim3(threads), 0, st, a, next_trace(21));
@@ -512,14 +755,18 @@ cudaError_t launch_mamba_scan(cudaStream_t st, const MambaArgs& a) {
   return cudaGetLastError();
 }
 
+template <typename OT>
+static cudaError_t mamba_gate_norm(cudaStream_t st, const MambaArgs& a, OT* out) {
+  const size_t smem = (size_t)a.E * sizeof(float);
+  if (mamba_rows_aligned(a))
+    (void)launch_k(mamba_gate_norm_kernel<OT, 4>, dim3(a.T), dim3(256), smem, st, a, out, next_trace(22));
+  else
+    (void)launch_k(mamba_gate_norm_kernel<OT, 1>, dim3(a.T), dim3(256), smem, st, a, out, next_trace(22));
+  return cudaGetLastError();
+}
 cudaError_t launch_mamba_gate_norm(cudaStream_t st, const MambaArgs& a, int odt, void* out) {
   if (a.T <= 0) return cudaSuccess;
-  const size_t smem = (size_t)a.E * sizeof(float);
-  if (odt == DT_F32)
-    (void)launch_k(mamba_gate_norm_kernel<float>, dim3(a.T), dim3(256), smem, st, a, (float*)out, next_trace(22));
-  else
-    (void)launch_k(mamba_gate_norm_kernel<bf16>, dim3(a.T), dim3(256), smem, st, a, (bf16*)out, next_trace(22));
-  return cudaGetLastError();
+  return odt == DT_F32 ? mamba_gate_norm(st, a, (float*)out) : mamba_gate_norm(st, a, (bf16*)out);
 }
 
 }  // namespace nvllm

@@ -106,3 +106,20 @@ def test_hybrid_rejects_multi_token_prefill_on_a_cached_prefix():
         run.run_flat([p + [5]], True, [300], [[0, 1]], [0.0])  # decode-shaped: fine
     finally:
         run.close()
+
+
+@pytest.mark.parametrize("nh,hd,N,G,K", [
+    (8, 4, 16, 1, 4),     # smallest head of the tiled scan: two heads to a warp and more
+    (8, 64, 64, 2, 4),
+    (4, 128, 128, 4, 4),  # largest head and state, one head per group
+    (32, 128, 32, 8, 4),  # five sequences are enough warps for two rows per lane
+    (8, 32, 24, 2, 4),    # state that is no power of two: the scan without tiles
+    (6, 12, 16, 3, 4),    # rows that start off 16-byte boundaries
+    (8, 32, 16, 2, 3),    # other taps
+])
+def test_hybrid_prompts_at_the_edges_of_the_scan_tiles(nh, hd, N, G, K):
+    """Prompts of one token, around the scan's chunk of eight and over a block border, decoded on."""
+    cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=nh, mamba_head_dim=hd,
+                        mamba_state_size=N, mamba_n_groups=G, mamba_conv_kernel=K)
+    prompts = [W.random_prompt(cfg.vocab_size, n, 50 + i) for i, n in enumerate((1, 7, 8, 17, 258))]
+    _run(cfg, C.PREC_FP32, prompts, 3, [[0], [1], [2], [3], [4, 5]], 6)
