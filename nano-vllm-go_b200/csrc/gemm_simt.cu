@@ -4,14 +4,16 @@
 //    Weights [N,K] are read exactly once with 16-byte streaming loads (L1 no-allocate), one
 //    warp per R output rows, activations staged in shared memory as fp32, fp32 accumulate.
 //    HBM-bound: algorithmic bytes = N*K*sizeof(W).
-//  * gemm_simt_kernel: 64x64x16 register-tiled fp32-FMA GEMM.  This is the fp32 PARITY-mode
-//    engine (1e-4 gate: TF32/bf16 tensor cores are not accurate enough) and the grouped
-//    (MoE expert) GEMM with row gather.  The bf16 throughput path is gemm_tcgen05.cu.
+//  * gemm_f32_kernel: register-tiled packed-FMA GEMM.  This is the fp32 PARITY-mode
+//    engine (1e-4 gate: TF32/bf16 tensor cores are not accurate enough) and its grouped
+//    (MoE expert) GEMM with row gather.
+//  * gemm_simt_kernel: 64x64x16 fp32-FMA tiles on bf16 operands that the tcgen05 path cannot address.
 //
-// Both compute C[m,n] = alpha * sum_k A[m,k] * W[n,k]  (reference tensor.go:62-88 MatMul with
+// All compute C[m,n] = alpha * sum_k A[m,k] * W[n,k]  (reference tensor.go:62-88 MatMul with
 // the weight held [out,in]) and write fp32 split-K partials.
 #include "common.cuh"
 #include "kernels.h"
+#include "mma.cuh"
 
 namespace nvllm {
 
@@ -242,22 +244,13 @@ cudaError_t launch_gemv(cudaStream_t st, GemmArgs& g, const GemvPre* pre_in) {
 // ------------------------------------------------------------------ tiled SIMT GEMM
 constexpr int SBM = 64, SBN = 64, SBK = 16;
 
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, float (&v)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) {
-  float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-template <>
-__device__ __forceinline__ void load4<bf16>(const bf16* p, float (&v)[4]) {
+__device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
   uint2 r = *reinterpret_cast<const uint2*>(p);
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
   float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
-template <typename AT, typename WT>
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(GemmArgs g, Trace tr) {
   TRACE_ENTRY(tr);
@@ -266,7 +259,7 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
   __shared__ float As[2][SBK][SBM + 4];
   __shared__ float Ws[2][SBK][SBN + 4];
   int row0, rows_valid;
-  const WT* W = (const WT*)g.W;
+  const bf16* W = (const bf16*)g.W;
   if (g.tile_expert) {
     if ((int)blockIdx.x >= *g.n_tiles) return;
     row0 = g.tile_row0[blockIdx.x];
@@ -277,15 +270,15 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
     rows_valid = min(SBM, g.M - row0);
   }
   const int col0 = blockIdx.y * SBN;
-  const AT* A = (const AT*)g.A;
+  const bf16* A = (const bf16*)g.A;
   const int tid = threadIdx.x;
   // loader mapping: 64 rows x 16 k = 256 threads x 4 consecutive k
   const int lr = tid >> 2, lk = (tid & 3) * 4;
   int arow = -1;
   if (lr < rows_valid) arow = g.a_rows ? g.a_rows[row0 + lr] : row0 + lr;
   const int wrow = (col0 + lr < g.N) ? col0 + lr : -1;
-  const AT* ap = (arow >= 0) ? A + (size_t)arow * g.lda : nullptr;
-  const WT* wp = (wrow >= 0) ? W + (size_t)wrow * g.K : nullptr;
+  const bf16* ap = (arow >= 0) ? A + (size_t)arow * g.lda : nullptr;
+  const bf16* wp = (wrow >= 0) ? W + (size_t)wrow * g.K : nullptr;
   const int ty = tid >> 4, tx = tid & 15;
   float acc[4][4];
 #pragma unroll
@@ -298,8 +291,8 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
 #pragma unroll
     for (int j = 0; j < 4; j++) ra[j] = rw[j] = 0.f;
     if (k0 + lk < g.K) {  // K % 4 == 0 is guaranteed (K % 8 == 0)
-      if (ap) load4<AT>(ap + k0 + lk, ra);
-      if (wp) load4<WT>(wp + k0 + lk, rw);
+      if (ap) load4(ap + k0 + lk, ra);
+      if (wp) load4(wp + k0 + lk, rw);
     }
   };
   auto stash = [&](int buf) {
@@ -346,15 +339,153 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
   TRACE_EXIT(tr);
 }
 
+// ------------------------------------------------------------------ tiled fp32 GEMM
+// C tile of 8 MI x 64 by four warps, a lane holds MI x 4 sums, each as a packed pair: the even and the odd k of every
+// step of two, added at the end, so that the 16-byte pieces of A and W feed the packed FMA (f32x2, two IEEE
+// fp32 operations) as they lie in memory.  A and W go to shared memory in steps of 32 k by 16-byte cp.async, three
+// stages deep; rows are 36 floats apart, which puts the 8 (4) rows that a warp reads at once on different
+// banks: per 4 k a lane reads 4 + MI pieces for 8 MI packed FMAs, so at MI = 8 the fp32 pipe is the
+// bound and not shared memory.  k is split over CTAs (fp32 slices, summed by the consumer) until each SM has two.
+// MI = 2 / 4 keep tiles of 16 / 32 rows for small steps, which are bound by the weights.
+// GPT-2 small, four prompts of 50 to 100 tokens: the step's 48 matrix products 7.24 -> 2.5 ms against tiles of 64 x 64
+// x 16 with scalar FMAs, operands transposed through registers and one k range (60 to 240 CTAs of the chip's 296).
+constexpr int FG_BN = 64, FG_BK = 32, FG_PITCH = 36, FG_STAGES = 3, FG_THREADS = 128;
+
+template <int MI>
+__global__ void __launch_bounds__(FG_THREADS)
+gemm_f32_kernel(GemmArgs g, int kc, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  constexpr int BM = 8 * MI;
+  extern __shared__ __align__(16) float fsm[];  // [stage][BM + 64][pitch]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  int row0, rows_valid;
+  const float* W = (const float*)g.W;
+  if (g.tile_expert) {
+    if ((int)blockIdx.x >= *g.n_tiles) return;
+    row0 = g.tile_row0[blockIdx.x];
+    rows_valid = g.tile_rows[blockIdx.x];
+    W += (size_t)g.tile_expert[blockIdx.x] * g.expert_stride;
+  } else {
+    row0 = blockIdx.x * BM;
+    rows_valid = min(BM, g.M - row0);
+  }
+  const int col0 = blockIdx.y * FG_BN;
+  const int ks = blockIdx.z * kc, ke = min(g.K, ks + kc);
+  const int nk = (ke - ks + FG_BK - 1) / FG_BK;
+  // loader: 8 pieces of 16 bytes per row and step, 16 rows at a time
+  const int lr = tid >> 3, lp = (tid & 7) * 4;
+  constexpr int LA = (BM + 15) / 16;
+  const float* ap[LA];
+#pragma unroll
+  for (int i = 0; i < LA; i++) {
+    const int r = lr + 16 * i;
+    ap[i] = r < rows_valid ? (const float*)g.A + (size_t)(g.a_rows ? g.a_rows[row0 + r] : row0 + r) * g.lda + ks + lp : nullptr;
+  }
+  const float* wp[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int n = col0 + lr + 16 * i;
+    wp[i] = n < g.N ? W + (size_t)n * g.K + ks + lp : nullptr;
+  }
+  const float* any = (const float*)g.A;  // a valid address for pieces that are filled with zeros
+  auto fetch = [&](int kb) {
+    if (kb < nk) {
+      float* dst = fsm + (kb % FG_STAGES) * (BM + FG_BN) * FG_PITCH + lr * FG_PITCH + lp;
+      const int k = kb * FG_BK;
+      const bool in = ks + k + lp < ke;  // K and the k ranges are multiples of 4
+#pragma unroll
+      for (int i = 0; i < LA; i++)
+        if (lr + 16 * i < BM) cp_async16(smem_addr(dst + 16 * i * FG_PITCH), ap[i] && in ? ap[i] + k : any, ap[i] && in);
+#pragma unroll
+      for (int i = 0; i < 4; i++) cp_async16(smem_addr(dst + (BM + 16 * i) * FG_PITCH), wp[i] && in ? wp[i] + k : any, wp[i] && in);
+    }
+    cp_async_commit();
+  };
+  const int am = (warp >> 1) * 4 + (lane >> 3), wn = (warp & 1) * 8 + (lane & 7);
+  unsigned long long acc[MI][4];
+#pragma unroll
+  for (int i = 0; i < MI; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+#pragma unroll
+  for (int i = 0; i + 1 < FG_STAGES; i++) fetch(i);
+  for (int kb = 0; kb < nk; kb++) {
+    cp_async_wait<FG_STAGES - 2>();
+    __syncthreads();  // step kb has arrived, and step kb - 1's buffer is free
+    fetch(kb + FG_STAGES - 1);
+    const float* a_s = fsm + (kb % FG_STAGES) * (BM + FG_BN) * FG_PITCH + am * FG_PITCH;
+    const float* w_s = fsm + (kb % FG_STAGES) * (BM + FG_BN) * FG_PITCH + (BM + wn) * FG_PITCH;
+#pragma unroll
+    for (int k = 0; k < FG_BK; k += 4) {
+      ulonglong2 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + 16 * j * FG_PITCH + k);
+#pragma unroll
+      for (int i = 0; i < MI; i++) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + 8 * i * FG_PITCH + k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          acc[i][j] = fma2(a.x, w[j].x, acc[i][j]);
+          acc[i][j] = fma2(a.y, w[j].y, acc[i][j]);
+        }
+      }
+    }
+  }
+  float* out = g.out + (size_t)blockIdx.z * g.split_stride;
+#pragma unroll
+  for (int i = 0; i < MI; i++) {
+    const int r = 8 * i + am;
+    if (r >= rows_valid) continue;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int n = col0 + 16 * j + wn;
+      float lo, hi;
+      unpack2(acc[i][j], lo, hi);
+      if (n < g.N) out[(size_t)(row0 + r) * g.ldo + n] = g.alpha * (lo + hi);
+    }
+  }
+  TRACE_EXIT(tr);
+}
+
+template <int MI>
+static cudaError_t gemm_f32_launch(cudaStream_t st, const GemmArgs& g, dim3 grid, int kc) {
+  constexpr size_t smem = (size_t)FG_STAGES * (8 * MI + FG_BN) * FG_PITCH * sizeof(float);
+  if (smem > 48 * 1024) {  // (an attribute of the device's kernel: set on whichever device is current)
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<MI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_k(gemm_f32_kernel<MI>, grid, dim3(FG_THREADS), smem, st, g, kc, next_trace(12));
+}
+
+static cudaError_t launch_gemm_f32(cudaStream_t st, GemmArgs& g) {
+  const int mi = g.tile_expert || g.M > 32 ? 8 : g.M > 16 ? 4 : 2;
+  const int mt = g.tile_expert ? g.max_tiles : ceil_div(g.M, 8 * mi), nt = ceil_div(g.N, FG_BN);
+  g.S = 1;
+  if (mt == 0 || nt == 0) return cudaSuccess;
+  // slices: up to the eight that a consumer sums with one batch of loads, each at least 128 of k, as many as the
+  // buffer has room for, while two CTAs per SM are not reached (grouped tiles write one slice)
+  int S = 1;
+  if (!g.tile_expert && g.out_capacity)
+    while (S < 8 && (long)mt * nt * S < 2 * 148 && g.K / (S + 1) >= 128 &&
+           (size_t)(S + 1) * g.split_stride <= g.out_capacity) S++;
+  const int kc = ceil_div(ceil_div(g.K, FG_BK), S) * FG_BK;
+  g.S = ceil_div(g.K, kc);
+  const dim3 grid(mt, nt, g.S);
+  if (mi == 8) return gemm_f32_launch<8>(st, g, grid, kc);
+  if (mi == 4) return gemm_f32_launch<4>(st, g, grid, kc);
+  return gemm_f32_launch<2>(st, g, grid, kc);
+}
+
 cudaError_t launch_gemm_simt(cudaStream_t st, GemmArgs& g) {
   if ((g.K % 8) != 0) return cudaErrorInvalidValue;
+  if (g.adt == DT_F32 && g.wdt == DT_F32) return launch_gemm_f32(st, g);
   g.S = 1;
   dim3 grid(g.tile_expert ? g.max_tiles : ceil_div(g.M, SBM), ceil_div(g.N, SBN));
   if (grid.x == 0 || grid.y == 0) return cudaSuccess;
-  if (g.adt == DT_F32 && g.wdt == DT_F32) (void)launch_k(gemm_simt_kernel<float, float>, dim3(grid), dim3(256), 0, st, g, next_trace(12));
-  else if (g.adt == DT_F32 && g.wdt == DT_BF16) (void)launch_k(gemm_simt_kernel<float, bf16>, dim3(grid), dim3(256), 0, st, g, next_trace(12));
-  else if (g.adt == DT_BF16 && g.wdt == DT_BF16) (void)launch_k(gemm_simt_kernel<bf16, bf16>, dim3(grid), dim3(256), 0, st, g, next_trace(12));
-  else return cudaErrorInvalidValue;
+  if (g.adt != DT_BF16 || g.wdt != DT_BF16) return cudaErrorInvalidValue;
+  (void)launch_k(gemm_simt_kernel, dim3(grid), dim3(256), 0, st, g, next_trace(12));
   return cudaGetLastError();
 }
 
