@@ -347,9 +347,10 @@ int forward_step(nvllm_handle* h) {
   // read per step (not cached): the parity tests switch it between runs
   const char* chain_env = getenv("NVLLM_CHAIN");
   const bool chain_on = !(chain_env && atoi(chain_env) == 0);
-  // Steps of <= 8 rows (GEMV shapes): the FFN activation is built inside the W2 GEMV — one
-  // launch per layer less on a chain of ~100 dependent launches.  NVLLM_GEMV_PRE=0 keeps the
-  // stand-alone activation kernel (read per step: the parity tests switch it).
+  // Steps of <= 8 rows (GEMV shapes) whose W1 GEMV left slices (fp32 mode, one row in bf16 mode): the FFN
+  // activation is built inside the W2 GEMV — one launch per layer less on a chain of ~100 dependent
+  // launches.  NVLLM_GEMV_PRE=0 keeps the stand-alone activation kernel (read per step: the parity
+  // tests switch it).
   const char* gpre_env = getenv("NVLLM_GEMV_PRE");
   const bool gpre_act = !(gpre_env && atoi(gpre_env) == 0) && T <= 8 && !h->moe;
   int xb_parts = h->fold ? 1 : 0;

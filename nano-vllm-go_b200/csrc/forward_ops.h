@@ -108,8 +108,8 @@ struct RouterArgs {  // expert routing fused into the FFN norm of a MoE layer
 
 // C = A @ W^T into fp32 split-K partials at `out`
 // epi != 0 asks for the FFN activation to be fused into the GEMM epilogue (bf16 hidden state
-// written to epi_out); granted only on the tcgen05 path when the GEMM needs no split-K, in
-// which case res->S comes back 0 (no partials to reduce).
+// written to epi_out); granted in bf16 mode to steps of 2 .. 8 rows and, on the tcgen05 path, when the GEMM
+// needs no split-K: res->S then comes back 0 (no partials to reduce).
 static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int M, int N, int K,
                     float alpha, float* out, size_t cap, int ldo, Pending* res, int epi = 0,
                     void* epi_out = nullptr, int epi_ld = 0, const float* epi_bias = nullptr,
@@ -133,6 +133,19 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
     if (gp && gp->mode == 2) {
       pre_alg = (double)M * gp->hld * 4 - (double)M * K * dt_size(h->adt);
       pre_impl = (double)M * gp->hld * 4 * (gp->Sh - 1);
+    }
+    if (epi && h->adt == DT_BF16 && h->wdt == DT_BF16 && M >= GEMV_MMA_ROWS) {
+      // a CTA holds whole sums over k: the activation goes out directly, no slices and no activation kernel
+      GemvMmaArgs ga{};
+      ga.A = (const bf16*)A; ga.W = (const bf16*)W; ga.lda = lda; ga.M = M; ga.N = N; ga.K = K;
+      ga.alpha = alpha; ga.epi = epi; ga.epi_out = (bf16*)epi_out; ga.epi_ld = epi_ld; ga.epi_bias = epi_bias;
+      ga.glu_limit = h->glu_limit_cur;
+      const GemvMmaPlan mp = gemv_mma_plan(N, K, 1);
+      ga.KC = mp.KC;
+      ProfScope ps(h, NVLLM_K_GEMV, io, flops, a_in + (double)M * epi_ld * 2);
+      LAUNCH(h, launch_gemv_mma(h->stream, ga, mp));
+      res->S = 0;
+      return NVLLM_OK;
     }
     ProfScope ps(h, NVLLM_K_GEMV, io + pre_alg, flops, a_in + pre_impl + 4.0 * gemv_splits(M, N, K) * M * N);
     LAUNCH(h, launch_gemv(h->stream, g, gp));

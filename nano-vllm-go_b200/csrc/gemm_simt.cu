@@ -1,6 +1,6 @@
 // gemm_simt.cu — CUDA-core matrix kernels.
 //
-//  * gemv_kernel: skinny (M <= 8) weight-streaming split-K GEMV for single-sequence decode.
+//  * gemv_kernel: skinny weight-streaming split-K GEMV: M <= 8 in fp32 mode, one row in bf16 mode (more: gemv_mma.cu).
 //    Weights [N,K] are read exactly once with 16-byte streaming loads (L1 no-allocate), one
 //    warp per R output rows, activations staged in shared memory as fp32, fp32 accumulate.
 //    HBM-bound: algorithmic bytes = N*K*sizeof(W).
@@ -73,9 +73,9 @@ template <> struct Raw8<float> {
 // BEFORE griddepcontrol.wait, so the HBM stream of this GEMV runs under the tail of the kernel
 // in front of it (a single-sequence decode step is a chain of ~100 such dependent launches).
 constexpr int GEMV_PF = 2;
-template <typename AT, typename WT, int M, int R>
+template <typename T, int M, int R>
 __global__ void __launch_bounds__(256)
-gemv_kernel(const AT* __restrict__ A, int lda, const WT* __restrict__ W, int N, int K, int KC,
+gemv_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int N, int K, int KC,
             float* __restrict__ out, int ldo, size_t split_stride, float alpha, GemvPre pre, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
@@ -83,7 +83,7 @@ gemv_kernel(const AT* __restrict__ A, int lda, const WT* __restrict__ W, int N, 
   const int ks = blockIdx.y * KC;
   const int ke = min(K, ks + KC);
   const int klen = ke - ks;
-  Raw8<WT> wpre[GEMV_PF][R];
+  Raw8<T> wpre[GEMV_PF][R];
   {
     const int lane_ = threadIdx.x & 31, warp_ = threadIdx.x >> 5, nw_ = blockDim.x >> 5;
     const int n0_ = (blockIdx.x * nw_ + warp_) * R;
@@ -133,7 +133,7 @@ gemv_kernel(const AT* __restrict__ A, int lda, const WT* __restrict__ W, int N, 
           if (pre.hbias) hsum += pre.hbias[col];
           y = pre.swiglu == 2 ? relu2(hsum) : gelu_tanh(hsum);
         }
-        y = to_f32(from_f32<AT>(y));
+        y = to_f32(from_f32<T>(y));
       }
       a_s[i] = y;
     }
@@ -147,7 +147,7 @@ gemv_kernel(const AT* __restrict__ A, int lda, const WT* __restrict__ W, int N, 
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int m = 0; m < M; m++) acc[r][m] = 0.f;
-  const WT* wrow[R];
+  const T* wrow[R];
 #pragma unroll
   for (int r = 0; r < R; r++) wrow[r] = W + (size_t)min(n0 + r, N - 1) * K + ks;
 
@@ -198,13 +198,13 @@ gemv_kernel(const AT* __restrict__ A, int lda, const WT* __restrict__ W, int N, 
   TRACE_EXIT(tr);
 }
 
-template <typename AT, typename WT, int M>
+template <typename T, int M>
 static cudaError_t gemv_dispatch_r(cudaStream_t st, const GemmArgs& g, const GemvPlan& p, const GemvPre& pre) {
   dim3 grid(ceil_div(g.N, p.warps * p.R), p.S);
   size_t smem = (size_t)M * p.KC * sizeof(float);
 #define GV(RR)                                                                                     \
-  (void)launch_k(gemv_kernel<AT, WT, M, RR>, dim3(grid), dim3(p.warps * 32), smem, st,                                     \
-      (const AT*)g.A, g.lda, (const WT*)g.W, g.N, g.K, p.KC, g.out, g.ldo, g.split_stride, g.alpha, \
+  (void)launch_k(gemv_kernel<T, M, RR>, dim3(grid), dim3(p.warps * 32), smem, st,                                     \
+      (const T*)g.A, g.lda, (const T*)g.W, g.N, g.K, p.KC, g.out, g.ldo, g.split_stride, g.alpha, \
       pre, next_trace(11))
   if (p.R == 4) GV(4);
   else if (p.R == 2) GV(2);
@@ -212,17 +212,17 @@ static cudaError_t gemv_dispatch_r(cudaStream_t st, const GemmArgs& g, const Gem
 #undef GV
   return cudaGetLastError();
 }
-template <typename AT, typename WT>
+template <typename T>
 static cudaError_t gemv_dispatch_m(cudaStream_t st, const GemmArgs& g, const GemvPlan& p, const GemvPre& pre) {
   switch (g.M) {
-    case 1: return gemv_dispatch_r<AT, WT, 1>(st, g, p, pre);
-    case 2: return gemv_dispatch_r<AT, WT, 2>(st, g, p, pre);
-    case 3: return gemv_dispatch_r<AT, WT, 3>(st, g, p, pre);
-    case 4: return gemv_dispatch_r<AT, WT, 4>(st, g, p, pre);
-    case 5: return gemv_dispatch_r<AT, WT, 5>(st, g, p, pre);
-    case 6: return gemv_dispatch_r<AT, WT, 6>(st, g, p, pre);
-    case 7: return gemv_dispatch_r<AT, WT, 7>(st, g, p, pre);
-    case 8: return gemv_dispatch_r<AT, WT, 8>(st, g, p, pre);
+    case 1: return gemv_dispatch_r<T, 1>(st, g, p, pre);
+    case 2: return gemv_dispatch_r<T, 2>(st, g, p, pre);
+    case 3: return gemv_dispatch_r<T, 3>(st, g, p, pre);
+    case 4: return gemv_dispatch_r<T, 4>(st, g, p, pre);
+    case 5: return gemv_dispatch_r<T, 5>(st, g, p, pre);
+    case 6: return gemv_dispatch_r<T, 6>(st, g, p, pre);
+    case 7: return gemv_dispatch_r<T, 7>(st, g, p, pre);
+    case 8: return gemv_dispatch_r<T, 8>(st, g, p, pre);
   }
   return cudaErrorInvalidValue;
 }
@@ -235,9 +235,18 @@ cudaError_t launch_gemv(cudaStream_t st, GemmArgs& g, const GemvPre* pre_in) {
   GemvPlan p = gemv_plan(g.M, g.N, g.K);
   g.S = p.S;
   if (g.out_capacity && (size_t)p.S * g.split_stride > g.out_capacity) return cudaErrorInvalidValue;
-  if (g.adt == DT_F32 && g.wdt == DT_F32) return gemv_dispatch_m<float, float>(st, g, p, pre);
-  if (g.adt == DT_F32 && g.wdt == DT_BF16) return gemv_dispatch_m<float, bf16>(st, g, p, pre);
-  if (g.adt == DT_BF16 && g.wdt == DT_BF16) return gemv_dispatch_m<bf16, bf16>(st, g, p, pre);
+  if (g.adt == DT_F32 && g.wdt == DT_F32) return gemv_dispatch_m<float>(st, g, p, pre);
+  if (g.adt == DT_BF16 && g.wdt == DT_BF16) {
+    if (g.M < GEMV_MMA_ROWS) return gemv_dispatch_r<bf16, 1>(st, g, p, pre);
+    if (pre.mode != 0) return cudaErrorInvalidValue;
+    // gemv_mma_plan stays within the slices that the callers have room for
+    const GemvMmaPlan mp = gemv_mma_plan(g.N, g.K, p.S);
+    g.S = mp.S;
+    GemvMmaArgs a{};
+    a.A = (const bf16*)g.A; a.W = (const bf16*)g.W; a.lda = g.lda; a.M = g.M; a.N = g.N; a.K = g.K; a.KC = mp.KC;
+    a.out = g.out; a.ldo = g.ldo; a.split_stride = g.split_stride; a.alpha = g.alpha;
+    return launch_gemv_mma(st, a, mp);
+  }
   return cudaErrorInvalidValue;
 }
 

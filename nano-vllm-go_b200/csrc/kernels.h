@@ -10,6 +10,7 @@
 //    sum the S slices (deterministic, no atomics) and add the bias
 //  * KV pool of one layer: K and V each [num_blocks][n_kv][256][hd], dtype DT
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -242,7 +243,7 @@ struct GemmArgs {
 // Single-sequence decode (M <= 8) is a chain of ~100 dependent launches of ~3 us: the W2 GEMV
 // builds its own activation from the W1 GEMV's split-K slices instead of reading what an
 // activation kernel stored (one launch per layer less; every CTA only touches its own k-chunk,
-// so nothing is read twice).
+// so nothing is read twice).  In bf16 mode only at one row: from two on the W1 GEMV writes the activation (gemv_mma.cu).
 //  mode 2: A = act(sum_s hp[s] + hbias): SwiGLU over interleaved gate / up columns, or tanh-GELU,
 //          rounded to `adt` exactly like the stand-alone kernel rounds what it stores.
 // (The same trick for the norms — every CTA re-deriving the row statistics from x + the pending
@@ -257,10 +258,34 @@ struct GemvPre {
   int swiglu;          // 0 tanh-GELU, 1 gated unit, 2 squared ReLU
   float glu_limit;     // with swiglu: which gated unit (see launch_act)
 };
-// split-K slices a skinny GEMV will produce for (M,N,K); workspace must hold S*M*N floats
+// most split-K slices a skinny GEMV produces for (M,N,K); workspace must hold S*M*N floats
 int gemv_splits(int M, int N, int K);
 cudaError_t launch_gemv(cudaStream_t st, GemmArgs& g, const GemvPre* pre = nullptr);  // M <= 8
 cudaError_t launch_gemm_simt(cudaStream_t st, GemmArgs& g);  // any M (fp32 parity mode, MoE)
+
+// ---------------------------------------------------------------- gemv_mma.cu
+// bf16 activations and weights, 2 <= M <= 8 (launch_gemv takes this path by itself; run_gemm calls it with an epilogue)
+constexpr int GEMV_MMA_ROWS = 2;  // from this many rows on; one row: gemv_kernel (gemm_simt.cu)
+struct GemvMmaArgs {
+  const __nv_bfloat16* A;  // [M, lda], rows 16-byte aligned
+  const __nv_bfloat16* W;  // [N, K], K a multiple of 8
+  int lda, M, N, K, KC;    // KC: k range of a split-K slice, a multiple of 32
+  float* out;              // [S][M][ldo] (TC5_EPI_PARTIAL)
+  int ldo;
+  size_t split_stride;
+  float alpha;
+  // S == 1: the feed-forward's activation (TC5_EPI_SWIGLU / GELU / RELU2), bf16 to epi_out [M, epi_ld]
+  int epi;
+  __nv_bfloat16* epi_out;
+  int epi_ld;
+  const float* epi_bias;
+  float glu_limit;
+};
+struct GemvMmaPlan {
+  int mt, KC, S;  // 16-row tiles per warp, k range of a slice, slices
+};
+GemvMmaPlan gemv_mma_plan(int N, int K, int most);
+cudaError_t launch_gemv_mma(cudaStream_t st, const GemvMmaArgs& a, const GemvMmaPlan& p);
 
 // ---------------------------------------------------------------- gemm_tcgen05.cu
 struct TmaDesc {

@@ -28,3 +28,12 @@ def _product(M, N, K, prec, kernel):
 ])
 def test_fp32_tiles(M, N, K):
     assert _product(M, N, K, C.PREC_FP32, 2) <= 1.0
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (2, 1, 8), (3, 15, 72), (5, 17, 264), (8, 16, 64),   # rows, columns and k around one 16 x 64 chunk
+    (7, 100, 776), (8, 768, 3072), (2, 2304, 768),       # k ranges on several CTAs
+    (4, 9473, 520), (8, 9472, 4544),                     # the first column counts with 32-row tiles
+])
+def test_bf16_rows_on_mma(M, N, K):
+    assert _product(M, N, K, C.PREC_BF16, 1) <= 1.0
