@@ -1844,6 +1844,7 @@ extern "C" int nvllm_create_layered(const nvllm_layered_config* c, const nvllm_l
   g.tp_size = 1; g.device = c->device;
   h->dev = c->device;
   h->sm_count = prop.multiProcessorCount;
+  tc5_pair_init(c->device);
   h->wdt = h->adt = h->kvdt = (c->precision == NVLLM_PREC_BF16) ? DT_BF16 : DT_F32;
   h->H = c->hidden; h->V = c->vocab_size; h->L = c->num_layers;
   h->ldl = (int)up8(h->V); h->Vl = h->ldl; h->Vl_valid = h->V;

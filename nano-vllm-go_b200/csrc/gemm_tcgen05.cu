@@ -21,15 +21,10 @@
 #include <tuple>
 
 #include "common.cuh"
-#include "tma.cuh"
-#include "tc5.cuh"
+#include "gemm_tc5.cuh"
 #include "kernels.h"
 
 namespace nvllm {
-
-constexpr int TC_BN = 128;  // weight rows per CTA (UMMA M)
-constexpr int TC_BK = 64;   // k elements per stage = one 128-byte swizzle row of bf16
-constexpr int TC_THREADS = 192;
 
 // ------------------------------------------------------------------ kernel
 // Persistent: grid = min(units, #SM) CTAs, one per SM (the operand ring takes ~192 KB of
@@ -41,37 +36,7 @@ constexpr int TC_THREADS = 192;
 // on the previous kernel, so the producer issues them BEFORE griddepcontrol.wait — the HBM
 // stream of this GEMM starts while the elementwise kernel in front of it is still running.
 // Only the activation tiles (and every global store) wait for the dependency.
-struct Tc5Sched {
-  int units, n_tiles, S, kbps, nkb_total;
-  // grouped (mixture-of-experts) mode, g_expert != nullptr: token tile t covers rows
-  // [g_row0[t], g_row0[t] + g_rows[t]) of the expert-sorted activations and multiplies expert
-  // g_expert[t]'s [g_N, K] weight matrix (experts stacked row-wise in W); the tile list lives
-  // on the device (moe_sort_kernel), so units = *g_ntiles * n_tiles is read after the wait
-  const int* g_expert;
-  const int* g_row0;
-  const int* g_rows;
-  const int* g_ntiles;
-  int g_N;
-  // decode-sized grouped GEMMs: raw weight base / bytes per weight row / expert count for the
-  // speculative L2 prefetch before the dependency resolves (null = off)
-  const uint8_t* g_wbase;
-  int g_row_bytes, g_E;
-};
-// the RMSNorm-fold arguments of Tc5Args (kernels.h), as the kernel takes them
-struct Tc5Fuse {
-  const float* rs_ssq;
-  int rs_parts, rs_ld;
-  float rs_inv_h, rs_eps;
-  float* x;
-  bf16* xb;
-  float* ssq;
-  int ssq_ld;
-  const float* bias;
-  float m;
-  const float* g;  // weight of the norm that reads x next: xb = bf16(x * g); null = ones
-  int cl;          // > 1: the S k-splits of an output tile are one thread-block cluster of `cl` CTAs
-  float glu_limit; // != 0: the gated epilogue computes another unit than silu(g) u (common.cuh glu_unit)
-};
+//
 // A second GEMM chained behind the first inside ONE launch (the FFN pair of a decode step:
 // W1 + activation, then W2): every CTA runs its units of problem 1, then its units of problem 2.
 // Problem 2 reads what problem 1's epilogues wrote, so its activation tiles wait for
@@ -88,28 +53,10 @@ struct Tc5Chain {
   unsigned* ctr;
   int n_waiters;  // CTAs owning at least one unit of problem 2
 };
-__device__ __forceinline__ void named_bar(int id, int n) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-// thread-block cluster primitives (the fused-residual split-K epilogue)
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_arrive_release() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait_acquire() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
 }
 // bulk copy from this CTA's shared memory into a peer's (both 16-byte aligned, bytes % 16 == 0);
 // completion is signalled as `bytes` of transaction count on the PEER's mbarrier
@@ -128,56 +75,6 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
-// v[c] of every lane -> lane l gets sum over lanes of v[l]  (31 shuffles instead of 32 x 5)
-__device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < off; i++) {
-      const float send = up ? v[i] : v[i + off];
-      const float keep = up ? v[i + off] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  return v[0];
-}
-// rot: CTAs working on the same k range start at different k-blocks (and wrap), so that at any
-// instant they pull DIFFERENT activation tiles out of L2 — otherwise every CTA of a skinny
-// GEMM requests the same 8 KB A tile at the same time and the few L2 slices holding it pace
-// the whole kernel (measured: ~390 ns per k-block with W already in shared memory).
-struct Tc5Unit {
-  int n0;     // first output column (weight row inside the expert)
-  int wrow;   // first weight row in the stacked weight tensor (TMA coordinate)
-  int m0;     // first token row
-  int m_end;  // one past the last valid token row of this tile
-  int kb0, nkb, split, rot;
-};
-__device__ __forceinline__ Tc5Unit tc5_unit(const Tc5Sched& sc, int u, int BT, int M) {
-  Tc5Unit t;
-  t.split = u % sc.S;
-  const int r = u / sc.S;
-  const int nt = r % sc.n_tiles, mt = r / sc.n_tiles;
-  t.n0 = nt * TC_BN;
-  if (sc.g_expert) {
-    t.m0 = sc.g_row0[mt];
-    t.m_end = t.m0 + sc.g_rows[mt];
-    t.wrow = sc.g_expert[mt] * sc.g_N + t.n0;
-  } else {
-    t.m0 = mt * BT;
-    t.m_end = M;
-    t.wrow = t.n0;
-  }
-  t.kb0 = t.split * sc.kbps;
-  t.nkb = min(sc.kbps, sc.nkb_total - t.kb0);
-  t.rot = (nt + 5 * mt) % t.nkb;
-  return t;
-}
-__device__ __forceinline__ int tc5_kb(int kb0, int kb, int rot, int nkb) {
-  const int k = kb + rot;
-  return kb0 + (k >= nkb ? k - nkb : k);
-}
-
 template <int BT, int STAGES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
@@ -1115,6 +1012,10 @@ cudaError_t launch_gemm_tc5(cudaStream_t st, const Tc5Args& a, int* S_out) {
       case 64: return launch_bt<64, CL_STAGES_64, true>(st, a, tw, ta, S);
       default: return cudaErrorInvalidValue;
     }
+  }
+  if (tc5_pair_fits(a, bt, S)) {
+    const TmaDesc* half = cached_map(a.A, a.M, a.K, bt / 2);
+    return half ? launch_gemm_tc5_pair(st, a, tw, half) : cudaErrorInvalidValue;
   }
   switch (bt) {
     case 32: return launch_bt<32, 10>(st, a, tw, ta, S);

@@ -351,6 +351,13 @@ struct Tc5Args {
 };
 // TC5_EPI_RELU2: like TC5_EPI_GELU (bf16 activation written, no bias needed) with relu(h)^2
 enum { TC5_EPI_PARTIAL = 0, TC5_EPI_SWIGLU = 1, TC5_EPI_GELU = 2, TC5_EPI_RESID = 3, TC5_EPI_RELU2 = 4 };
+// gemm_tc5_pair.cu: the kernel for many token rows, two CTAs per tile.  init: once per device and outside any stream
+// capture (returns the resident pairs; without it the kernel is not used).  failed: a wait of the kernel ran out
+// since the last call.
+int tc5_pair_init(int dev);
+bool tc5_pair_failed();
+bool tc5_pair_fits(const Tc5Args& a, int bt, int S);
+cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDesc* tw, const TmaDesc* ta);
 // split-K slices for a TC5_EPI_RESID GEMM: like tc5_splits, but every unit must own an SM
 // (the CTAs of a tile wait for each other); 0 = the shape cannot take the fused epilogue
 int tc5_resid_splits(int M, int N, int K, int sm_count);

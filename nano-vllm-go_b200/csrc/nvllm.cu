@@ -148,6 +148,7 @@ int nvllm_create(const nvllm_config* c, const uint8_t* tp_id, nvllm_handle** out
   h->rank = rank;
   h->dev = c->device;
   h->sm_count = prop.multiProcessorCount;
+  tc5_pair_init(c->device);
   h->wdt = h->adt = h->kvdt = (c->precision == NVLLM_PREC_BF16) ? DT_BF16 : DT_F32;
   h->H = c->hidden;
   h->V = c->vocab_size;

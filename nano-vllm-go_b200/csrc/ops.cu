@@ -33,6 +33,7 @@ struct Scratch {  // frees everything on scope exit
 
 int op_begin(Scratch& s, int device) {
   OP_CHECK(cudaSetDevice(device));
+  tc5_pair_init(device);
   OP_CHECK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
   OP_CHECK(cudaEventCreate(&s.e0));
   OP_CHECK(cudaEventCreate(&s.e1));

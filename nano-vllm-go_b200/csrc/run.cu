@@ -234,6 +234,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
       cudaError_t e = cudaStreamSynchronize(st);
       if (e != cudaSuccess)
         return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
+      if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
       memcpy(out_tokens, h->h_out, (size_t)n * 4);
       h->run_lay = h->lay;
       h->run_lay_ok = true;
@@ -438,6 +439,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess)
     return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
+  if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
   memcpy(out_tokens, h->h_out, (size_t)n * 4);
   h->resident_ok = true;
   h->run_lay = L;
@@ -605,6 +607,7 @@ extern "C" int nvllm_sync(nvllm_handle* h, int32_t* out_tokens, int n, float* la
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess)
     return set_err(h, NVLLM_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
+  if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "stream failed: a wait inside a GEMM ran out");
   if (out_tokens && n > 0) {
     if (n > h->lay.n) n = h->lay.n;
     if (h->spec_pending)  // ws.out_tokens already holds the speculative step's tokens
