@@ -17,7 +17,7 @@
 //                      unit lengths; beta and g.  All fp32.
 //   delta_scan_kernel  one CTA per (sequence, head, block of value columns).  A value column of
 //                      the state is independent of the others: it lives in the registers of LPC
-//                      lanes (dim / LPC entries each), the two inner products of a token are
+//                      lanes (dim / LPC entries each), the inner products of a token are
 //                      reduced with shuffles inside that lane group.  Token inputs arrive in
 //                      double-buffered shared-memory tiles of 16 tokens (cp.async), so the loop
 //                      over tokens never waits for memory.  The state is read from the slot when
@@ -131,9 +131,121 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(DeltaArgs a, Trace tr) 
   TRACE_EXIT(tr);
 }
 
+// The same for steps of many rows, DP_ROWS neighbouring rows per CTA: a warp keeps the taps of its unit (a head of up to
+// 128 channels, or 128 value channels; four per lane) and slides a window of rows over them, so a row of the projection
+// is read once, 16 bytes at a time, instead of once per tap with a search for its sequence in front.  Bound by
+// memory (the projection's columns once, the results once): 18 k rows of 4096 channels 195 us, 950 us with a row per
+// CTA.  Fewer rows than 1024 keep that kernel, which spreads a row over several CTAs.
+constexpr int DP_ROWS = 8;
+__device__ __forceinline__ float4 sum_slices4(const float* __restrict__ p, int S, size_t stride) {
+  float4 acc = *reinterpret_cast<const float4*>(p);
+  for (int s = 1; s < S; s++) {
+    const float4 v = *reinterpret_cast<const float4*>(p + (size_t)s * stride);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  return acc;
+}
+template <int TAPS, bool FAST>
+__global__ void __launch_bounds__(256) delta_prep_rows_kernel(DeltaArgs a, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  const int t0 = blockIdx.x * DP_ROWS, t1 = min(a.T, t0 + DP_ROWS);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int u = blockIdx.y * 8 + warp;  // this warp's unit
+  const bool head = u < 2 * a.G;
+  const int c0 = head ? u * a.dim : a.n_q + a.n_k + (u - 2 * a.G) * 128;
+  const int cn = head ? a.dim : min(128, a.conv_ch - c0);
+  const bool on = 4 * lane < cn;  // heads and pieces are multiples of 4 channels; a unit past the last has none
+  const int c = c0 + 4 * lane;
+  float wv[4][TAPS];  // immutable: fetched before the dependency resolves
+#pragma unroll
+  for (int e = 0; e < 4; e++)
+#pragma unroll
+    for (int k = 0; k < TAPS; k++) wv[e][k] = on ? a.conv_w[(size_t)(c + e) * TAPS + k] : 0.f;
+  pdl_wait();
+  const float qmul = 1.0f / sqrtf((float)a.dim);
+  int s = seq_of_row(a.cu_q, a.n_seqs, t0);
+  int first = a.cu_q[s], last = a.cu_q[s + 1], pos0 = a.positions[first];
+  float4 win[TAPS];  // the last TAPS rows, the current one last
+  // the rows in front of row t: of the step, of the slot's tail, or zeros before the sequence's start
+  auto refill = [&](int t) {
+    const float* tail = a.state_pool + (size_t)a.state_slots[s] * a.slot_floats + a.tail_off;
+    const int li = t - first, pos = pos0 + li;
+#pragma unroll
+    for (int k = 0; k + 1 < TAPS; k++) {
+      const int back = TAPS - 1 - k;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on) {
+        if (li - back >= 0) v = sum_slices4(a.in_p + (size_t)(t - back) * a.in_ld + c, a.in_S, a.in_stride);
+        else if (pos - back >= 0) v = *reinterpret_cast<const float4*>(tail + (size_t)(TAPS - 1 + li - back) * a.conv_ch + c);
+      }
+      win[k + 1] = v;  // moves to k when row t enters
+    }
+  };
+  refill(t0);
+  for (int t = t0; t < t1; t++) {
+    if (t >= last) {  // the next sequence (every sequence of a step has rows)
+      s++;
+      first = last;
+      last = a.cu_q[s + 1];
+      pos0 = a.positions[first];
+      refill(t);
+    }
+#pragma unroll
+    for (int k = 0; k + 1 < TAPS; k++) win[k] = win[k + 1];
+    win[TAPS - 1] = on ? sum_slices4(a.in_p + (size_t)t * a.in_ld + c, a.in_S, a.in_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < TAPS; k++) {
+      y[0] = fmaf(win[k].x, wv[0][k], y[0]);
+      y[1] = fmaf(win[k].y, wv[1][k], y[1]);
+      y[2] = fmaf(win[k].z, wv[2][k], y[2]);
+      y[3] = fmaf(win[k].w, wv[3][k], y[3]);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      y[e] = silu_t<FAST>(y[e]);
+      ss += y[e] * y[e];
+    }
+    float mul = 1.f;
+    if (head) {  // unit length; the queries also carry 1 / sqrt(dim)
+      mul = 1.0f / sqrtf(warp_sum(on ? ss : 0.f) + 1e-6f);
+      if (u < a.G) mul *= qmul;
+    }
+    if (on)
+      *reinterpret_cast<float4*>(a.qkv + (size_t)t * a.conv_ch + c) = make_float4(y[0] * mul, y[1] * mul, y[2] * mul, y[3] * mul);
+  }
+  if (blockIdx.y == 0)
+    for (int i = threadIdx.x; i < (t1 - t0) * a.H; i += blockDim.x) {
+      const int t = t0 + i / a.H, h = i % a.H;
+      const float* q = a.in_p + (size_t)t * a.in_ld + a.conv_ch;
+      const float b = sum_slices(q + h, a.in_S, a.in_stride);
+      const float d = sum_slices(q + a.H + h, a.in_S, a.in_stride);
+      a.bg[(size_t)t * 2 * a.H + h] = 1.0f / (1.0f + expf(-b));
+      a.bg[(size_t)t * 2 * a.H + a.H + h] = expf(-expf(a.a_log[h]) * softplus(d + a.dt_bias[h]));
+    }
+  TRACE_EXIT(tr);
+}
+// rows, units and tails that start on 16-byte boundaries, heads of one warp, enough rows to fill the chip eight at a time
+static bool delta_prep_rows_fit(const DeltaArgs& a) {
+  return a.T >= 1024 && a.taps >= 2 && a.taps <= 4 && a.dim <= 128 && a.dim % 4 == 0 && a.n_v % 4 == 0 && a.in_ld % 4 == 0 &&
+         a.in_stride % 4 == 0 && a.tail_off % 4 == 0 && a.slot_floats % 4 == 0;
+}
+template <int TAPS>
+static cudaError_t delta_prep_rows(cudaStream_t st, const DeltaArgs& a) {
+  const dim3 grid(ceil_div(a.T, DP_ROWS), ceil_div(2 * a.G + ceil_div(a.n_v, 128), 8));
+  return a.fast_act ? launch_k(delta_prep_rows_kernel<TAPS, true>, grid, dim3(256), 0, st, a, next_trace(34))
+                    : launch_k(delta_prep_rows_kernel<TAPS, false>, grid, dim3(256), 0, st, a, next_trace(34));
+}
+
 cudaError_t launch_delta_prep(cudaStream_t st, const DeltaArgs& a) {
   if (a.T <= 0) return cudaSuccess;
   if (a.taps < 1 || a.taps > DELTA_MAX_TAPS || a.H > 256 || a.dim > 1024) return cudaErrorInvalidValue;
+  if (delta_prep_rows_fit(a)) {
+    if (a.taps == 4) return delta_prep_rows<4>(st, a);
+    return a.taps == 3 ? delta_prep_rows<3>(st, a) : delta_prep_rows<2>(st, a);
+  }
   const int maxv = a.dim <= 128 ? 4 : a.dim <= 256 ? 8 : 32;
   const int n_units = 2 * a.G + ceil_div(a.n_v, 32 * maxv);
   // few rows (decode): a row's units spread over several CTAs
@@ -283,17 +395,34 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a, int LPC, i
 }
 
 
-// The same scan with compile-time sizes, dim = R * LPC: lane p of a column holds the R
-// neighbouring rows p R .. p R + R - 1, the keys and queries of a token sit in shared memory as
-// LPC segments of R + 4 floats (the padding puts the lanes' 16-byte reads in different banks),
-// no bounds checks in the token loop, four partial sums per inner product; one column per
-// thread and two CTAs per SM, or two columns per thread (CC = 2) and one.
+// The same scan with compile-time sizes, dim = R * LPC, and packed operations.  Lane p of a column holds the R
+// neighbouring rows p R .. p R + R - 1 of CC neighbouring columns as packed pairs of rows; the keys and queries of a
+// token sit in shared memory as LPC segments of R + 4 floats (the padding puts the lanes' 16-byte reads in different
+// banks).  The inner products of the CC columns are summed by shuffles that scatter them over the lanes.  Three fp32 operations per state entry and token instead of four:
+//   * the state is kept as S / c with c the product of the decays since the last rescaling, so a token multiplies one
+//     number by g; S k and S q are taken in one pass over the old state, the update adds k (u / c)^T, and
+//     o = c (S / c) q + (k . q) u.  c starts at one in every tile of tokens (the state is multiplied by the previous
+//     tile's c), and whenever it falls below 1e-18 inside one, so u / c stays far from overflow.
+//   * k . q, c, 1 / c and the multipliers are made once per token and CTA when a tile has arrived.
+// Bound by fp32 issue and, about equally, by shared-memory reads: a 16-byte read costs its four quarter-warps a pass
+// each even where they read the same bytes, so eight lanes with four columns (28 reads and 12 shuffles for 96
+// packed operations) replace four lanes with two columns.  Four CTAs of 128 threads per SM.  16 sequences of 750 to
+// 1500 tokens, 16 heads of 128 x 128: 1502 us; four scalar operations, one inner product after the other: 1905 us.
+constexpr float DELTA_RESCALE = 1e-18f;
+// a read that is not merged with an earlier one of the same place
+__device__ __forceinline__ ulonglong2 lds_pairs(const float* p) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(smem_addr(p)));
+  return v;
+}
 template <int R, int LPC, int CC>
-__global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_fixed_kernel(DeltaArgs a, int VC, Trace tr) {
+__global__ void __launch_bounds__(128, 4) delta_scan_fixed_kernel(DeltaArgs a, int VC, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
+  __shared__ float4 tok_s[DELTA_TT];  // of a token: c, 1 / c, k . q, beta
+  __shared__ float mul_s[DELTA_TT];   // what multiplies the state before it
   constexpr int DIM = R * LPC, RP = R + 4, KL = LPC * RP;
   const int vdim = a.vdim;
   const int s = blockIdx.x, h = blockIdx.y, vbase = blockIdx.z * VC;
@@ -302,15 +431,11 @@ __global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_fixed_kernel(
   const int start = a.positions[r0];
   float* slot = a.state_pool + (size_t)a.state_slots[s] * a.slot_floats;
   const int tid = threadIdx.x;
-  const int p = tid % LPC, jl = tid / LPC;  // the thread's CC columns: vbase + jl + cc * (VC / CC)
-  const int VH = VC / CC;
-  bool col_ok[CC];
-  int col[CC];
-#pragma unroll
-  for (int cc = 0; cc < CC; cc++) {
-    col[cc] = vbase + jl + cc * VH;
-    col_ok[cc] = jl < VH && col[cc] < vdim;
-  }
+  const int p = tid % LPC, jl = tid / LPC;  // the thread's columns: vbase + CC jl + cc
+  // after the shuffles a lane holds one inner product: of column mc, with k (typ 0) or q (typ 1)
+  static_assert((CC == 2 || CC == 4) && 2 * CC <= LPC, "a lane for every inner product");
+  const int mc = p & (CC - 1), typ = (p / CC) & 1, lane0 = (tid & 31) - p;
+  const int vcn = min(VC, vdim - vbase);
   const int kvh = h / (a.H / a.G);
 
   if (a.taps > 1) {  // roll the convolution tail forward (see the generic kernel)
@@ -333,18 +458,21 @@ __global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_fixed_kernel(
     }
   }
 
-  float* S_g = slot + a.state_off + (size_t)h * DIM * vdim;
-  float S[CC][R];
+  float* S_g = slot + a.state_off + (size_t)h * DIM * vdim + vbase;
+  unsigned long long S[CC][R / 2];
 #pragma unroll
   for (int cc = 0; cc < CC; cc++)
 #pragma unroll
-    for (int r = 0; r < R; r++) S[cc][r] = (start > 0 && col_ok[cc]) ? S_g[(size_t)(p * R + r) * vdim + col[cc]] : 0.f;
+    for (int r = 0; r < R; r += 2) {
+      const bool ok = start > 0 && CC * jl + cc < vcn;
+      const float* src = S_g + (size_t)(p * R + r) * vdim + CC * jl + cc;
+      S[cc][r / 2] = ok ? pack2(src[0], src[vdim]) : 0ull;
+    }
   // tile of DELTA_TT tokens: q [TT][KL], k [TT][KL], v [TT][VC], beta [TT], g [TT]
   const int tile_floats = DELTA_TT * (2 * KL + VC + 2);
   const float* qg = a.qkv + (size_t)kvh * DIM;
   const float* kg = a.qkv + a.n_q + (size_t)kvh * DIM;
   const float* vg = a.qkv + a.n_q + a.n_k + (size_t)h * vdim + vbase;
-  const int vcn = min(VC, vdim - vbase);
   auto issue = [&](int t0, int buf) {
     float* b = sm + buf * tile_floats;
     const int nt = min(DELTA_TT, n_new - t0);
@@ -369,7 +497,8 @@ __global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_fixed_kernel(
   issue(0, 0);
   cp_async_commit();
   const int HV = a.H * vdim;
-  float* og = a.o + (size_t)h * vdim;
+  float* og = a.o + (size_t)h * vdim + vbase;
+  float c_end = 1.f;  // (last warp) c after the previous tile
   for (int t0 = 0, it = 0; t0 < n_new; t0 += DELTA_TT, it++) {
     const int buf = it & 1;
     if (t0 + DELTA_TT < n_new) issue(t0 + DELTA_TT, buf ^ 1);
@@ -382,88 +511,175 @@ __global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_fixed_kernel(
     const float* vs = b + 2 * DELTA_TT * KL;
     const float* bs = b + DELTA_TT * (2 * KL + VC);
     const int nt = min(DELTA_TT, n_new - t0);
-    for (int tt = 0; tt < nt; tt++) {
-      const float beta = bs[tt], g = bs[DELTA_TT + tt];
-      float v[CC], dot[CC], out[CC];
+    for (int i0 = 0; i0 < DELTA_TT * LPC; i0 += blockDim.x) {  // k . q: LPC neighbouring lanes share a token
+      const int i = i0 + tid, tt = i / LPC;
+      float dot = 0.f;
+      if (tt < nt) {
+        const float* kk = b + DELTA_TT * KL + tt * KL + (i % LPC) * RP;
+        const float* qq = b + tt * KL + (i % LPC) * RP;
+        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int cc = 0; cc < CC; cc++) v[cc] = col_ok[cc] ? vs[tt * VC + jl + cc * VH] : 0.f;
-      float kr[R];
-      float d4[CC][4];
+        for (int r = 0; r < R; r += 4) {
+          const float4 k4 = *reinterpret_cast<const float4*>(kk + r), q4 = *reinterpret_cast<const float4*>(qq + r);
+          d.x = fmaf(k4.x, q4.x, d.x); d.y = fmaf(k4.y, q4.y, d.y);
+          d.z = fmaf(k4.z, q4.z, d.z); d.w = fmaf(k4.w, q4.w, d.w);
+        }
+        dot = (d.x + d.y) + (d.z + d.w);
+      }
 #pragma unroll
-      for (int cc = 0; cc < CC; cc++) d4[cc][0] = d4[cc][1] = d4[cc][2] = d4[cc][3] = 0.f;
+      for (int o = 1; o < LPC; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      if (i % LPC == 0 && tt < nt) tok_s[tt].z = dot;
+    }
+    if (tid >= (int)blockDim.x - 32) {  // the last warp: lane tt makes c of token tt, the product of the decays up to it
+      const int tt = tid & 31;
+      float c = tt < nt ? bs[DELTA_TT + tt] : 1.f;
 #pragma unroll
-      for (int r = 0; r < R; r += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(ks + tt * KL + r);
-        kr[r] = k4.x; kr[r + 1] = k4.y; kr[r + 2] = k4.z; kr[r + 3] = k4.w;
-#pragma unroll
-        for (int cc = 0; cc < CC; cc++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            S[cc][r + e] *= g;
-            d4[cc][e] = fmaf(S[cc][r + e], kr[r + e], d4[cc][e]);
+      for (int o = 1; o < DELTA_TT; o <<= 1) {
+        const float before = __shfl_up_sync(0xffffffffu, c, o);
+        if (tt >= o) c *= before;
+      }
+      const float last = __shfl_sync(0xffffffffu, c, nt - 1);
+      if (last >= DELTA_RESCALE) {
+        if (tt < nt) {
+          tok_s[tt].x = c;
+          tok_s[tt].y = 1.0f / c;
+          tok_s[tt].w = bs[tt];
+          mul_s[tt] = tt == 0 ? c_end : 1.f;
+        }
+        c_end = last;
+      } else {  // strong decays: one lane goes through the tokens and rescales where it has to
+        float cc = 1.f;
+        for (int j = 0; j < nt; j++) {
+          cc *= bs[DELTA_TT + j];
+          float m = j == 0 ? c_end : 1.f;
+          if (cc < DELTA_RESCALE) {
+            m *= cc;
+            cc = 1.f;
           }
-      }
-#pragma unroll
-      for (int cc = 0; cc < CC; cc++) {
-        dot[cc] = (d4[cc][0] + d4[cc][1]) + (d4[cc][2] + d4[cc][3]);
-#pragma unroll
-        for (int o = 1; o < LPC; o <<= 1) dot[cc] += __shfl_xor_sync(0xffffffffu, dot[cc], o);
-        dot[cc] = beta * (v[cc] - dot[cc]);  // u: what the token writes into the column
-        d4[cc][0] = d4[cc][1] = d4[cc][2] = d4[cc][3] = 0.f;
-      }
-#pragma unroll
-      for (int r = 0; r < R; r += 4) {
-        const float4 q4 = *reinterpret_cast<const float4*>(qs + tt * KL + r);
-        const float qv[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-        for (int cc = 0; cc < CC; cc++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            S[cc][r + e] = fmaf(kr[r + e], dot[cc], S[cc][r + e]);
-            d4[cc][e] = fmaf(S[cc][r + e], qv[e], d4[cc][e]);
+          if (tt == 0) {
+            mul_s[j] = m;
+            tok_s[j].x = cc;
+            tok_s[j].y = 1.0f / cc;
+            tok_s[j].w = bs[j];
           }
-      }
-#pragma unroll
-      for (int cc = 0; cc < CC; cc++) {
-        out[cc] = (d4[cc][0] + d4[cc][1]) + (d4[cc][2] + d4[cc][3]);
-#pragma unroll
-        for (int o = 1; o < LPC; o <<= 1) out[cc] += __shfl_xor_sync(0xffffffffu, out[cc], o);
-        if (p == 0 && col_ok[cc]) og[(size_t)(r0 + t0 + tt) * HV + col[cc]] = out[cc];
+        }
+        c_end = cc;
       }
     }
-    __syncthreads();  // the buffer may be refilled
+    __syncthreads();
+    for (int tt = 0; tt < nt; tt++) {
+      const float4 tk = tok_s[tt];
+      const float m = mul_s[tt];
+      if (m != 1.f) {
+        const unsigned long long mm = pack2(m, m);
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++)
+#pragma unroll
+          for (int r = 0; r < R / 2; r++) S[cc][r] = mul2(S[cc][r], mm);
+      }
+      const float v = CC * jl + mc < vcn ? vs[tt * VC + CC * jl + mc] : 0.f;
+      constexpr bool KEEP = R <= 16;  // keys kept in registers for the update, or read again
+      unsigned long long kr[KEEP ? R / 2 : 1], dk[CC], dq[CC];
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) dk[cc] = dq[cc] = 0ull;
+#pragma unroll
+      for (int r = 0; r < R / 2; r += 2) {
+        const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(ks + tt * KL + 2 * r);
+        const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qs + tt * KL + 2 * r);
+        if constexpr (KEEP) {
+          kr[r] = k2.x;
+          kr[r + 1] = k2.y;
+        }
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++) {
+          dk[cc] = fma2(S[cc][r], k2.x, dk[cc]);
+          dq[cc] = fma2(S[cc][r], q2.x, dq[cc]);
+        }
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++) {
+          dk[cc] = fma2(S[cc][r + 1], k2.y, dk[cc]);
+          dq[cc] = fma2(S[cc][r + 1], q2.y, dq[cc]);
+        }
+      }
+      float w[2][CC];  // [k / q][column]
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) {
+        float x0, x1;
+        unpack2(dk[cc], x0, x1);
+        w[0][cc] = x0 + x1;
+        unpack2(dq[cc], x0, x1);
+        w[1][cc] = x0 + x1;
+      }
+      // halve the columns, then the two kinds, over the lanes; lanes beyond those bits add up
+#pragma unroll
+      for (int o = 1; o < CC; o <<= 1) {
+        const bool up = (p & o) != 0;
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+          for (int cc = 0; cc < CC / 2 / o; cc++) {
+            const float give = up ? w[t][2 * cc] : w[t][2 * cc + 1], keep = up ? w[t][2 * cc + 1] : w[t][2 * cc];
+            w[t][cc] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+      }
+      float e = (typ ? w[1][0] : w[0][0]) + __shfl_xor_sync(0xffffffffu, typ ? w[0][0] : w[1][0], CC);
+#pragma unroll
+      for (int o = 2 * CC; o < LPC; o <<= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+      e *= tk.x;
+      const float mine = tk.w * (v - e);  // u on the lanes of typ 0
+      const float u = __shfl_sync(0xffffffffu, mine, lane0 + mc);
+      if (p >= CC && p < 2 * CC && CC * jl + mc < vcn) og[(size_t)(r0 + t0 + tt) * HV + CC * jl + mc] = fmaf(tk.z, u, e);
+      unsigned long long wu[CC];
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) {
+        const float x = __shfl_sync(0xffffffffu, mine, lane0 + cc) * tk.y;
+        wu[cc] = pack2(x, x);
+      }
+#pragma unroll
+      for (int r = 0; r < R / 2; r += 2) {
+        ulonglong2 k2;
+        if constexpr (KEEP) k2 = make_ulonglong2(kr[r], kr[r + 1]);
+        else k2 = lds_pairs(ks + tt * KL + 2 * r);
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++) {
+          S[cc][r] = fma2(k2.x, wu[cc], S[cc][r]);
+          S[cc][r + 1] = fma2(k2.y, wu[cc], S[cc][r + 1]);
+        }
+      }
+    }
+    __syncthreads();  // the buffer and the token values may be refilled
   }
   cp_async_wait<0>();
+  if (tid == (int)blockDim.x - 1) mul_s[0] = c_end;
+  __syncthreads();
+  const float c = mul_s[0];
 #pragma unroll
   for (int cc = 0; cc < CC; cc++)
-    if (col_ok[cc]) {
+    if (CC * jl + cc < vcn) {
 #pragma unroll
-      for (int r = 0; r < R; r++) S_g[(size_t)(p * R + r) * vdim + col[cc]] = S[cc][r];
+      for (int r = 0; r < R; r += 2) {
+        float lo, hi;
+        unpack2(S[cc][r / 2], lo, hi);
+        float* dst = S_g + (size_t)(p * R + r) * vdim + CC * jl + cc;
+        dst[0] = c * lo;
+        dst[vdim] = c * hi;
+      }
     }
   TRACE_EXIT(tr);
 }
 
-template <int R, int LPC>
+template <int R, int LPC, int CC>
 static cudaError_t delta_scan_fixed_launch(cudaStream_t st, const DeltaArgs& a) {
-  // two columns per thread (the key / query reads from shared memory, which bound the one-column
-  // form, serve both) when the head has the columns for it
-  static const bool cc2_on = !(getenv("NVLLM_DELTA_CC2") && atoi(getenv("NVLLM_DELTA_CC2")) == 0);
-  const bool cc2 = cc2_on && a.vdim >= 2 * (256 / LPC);
-  int VC = (cc2 ? 2 : 1) * (256 / LPC);
-  if (VC > a.vdim) VC = a.vdim;
-  const int threads = cc2 ? 256 : (VC * LPC + 31) / 32 * 32;
+  constexpr int MOST = CC * 128 / LPC;  // columns of 128 threads
+  const int VC = std::min(MOST, (a.vdim + CC - 1) / CC * CC);
+  const int threads = (VC / CC * LPC + 31) / 32 * 32;
   const dim3 grid(a.n_seqs, a.H, ceil_div(a.vdim, VC));
   const size_t smem = (size_t)2 * DELTA_TT * (2 * LPC * (R + 4) + VC + 2) * sizeof(float);
-  if (cc2) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(delta_scan_fixed_kernel<R, LPC, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    (void)launch_k(delta_scan_fixed_kernel<R, LPC, 2>, grid, dim3(threads), smem, st, a, VC, next_trace(35));
-  } else {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(delta_scan_fixed_kernel<R, LPC, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    (void)launch_k(delta_scan_fixed_kernel<R, LPC, 1>, grid, dim3(threads), smem, st, a, VC, next_trace(35));
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(delta_scan_fixed_kernel<R, LPC, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  return launch_k(delta_scan_fixed_kernel<R, LPC, CC>, grid, dim3(threads), smem, st, a, VC, next_trace(35));
 }
 
 cudaError_t launch_delta_scan(cudaStream_t st, const DeltaArgs& a) {
@@ -473,13 +689,13 @@ cudaError_t launch_delta_scan(cudaStream_t st, const DeltaArgs& a) {
   static const bool fixed_on = !(getenv("NVLLM_DELTA_FIXED") && atoi(getenv("NVLLM_DELTA_FIXED")) == 0);
   if (fixed_on && a.conv_ch % 4 == 0 && a.n_q % 4 == 0 && a.n_k % 4 == 0) {
     switch (a.dim) {
-      case 16: return delta_scan_fixed_launch<4, 4>(st, a);
-      case 32: return delta_scan_fixed_launch<8, 4>(st, a);
-      case 48: return delta_scan_fixed_launch<12, 4>(st, a);
-      case 64: return delta_scan_fixed_launch<16, 4>(st, a);
-      case 96: return delta_scan_fixed_launch<24, 4>(st, a);
-      case 128: return delta_scan_fixed_launch<32, 4>(st, a);
-      case 256: return delta_scan_fixed_launch<32, 8>(st, a);
+      case 16: return delta_scan_fixed_launch<4, 4, 2>(st, a);
+      case 32: return delta_scan_fixed_launch<4, 8, 4>(st, a);
+      case 48: return delta_scan_fixed_launch<12, 4, 2>(st, a);
+      case 64: return delta_scan_fixed_launch<8, 8, 4>(st, a);
+      case 96: return delta_scan_fixed_launch<12, 8, 4>(st, a);
+      case 128: return delta_scan_fixed_launch<16, 8, 4>(st, a);
+      case 256: return delta_scan_fixed_launch<32, 8, 2>(st, a);
     }
   }
   // registers per thread R and lanes per column LPC (a power of two): R * LPC >= dim
@@ -508,6 +724,35 @@ cudaError_t launch_delta_scan(cudaStream_t st, const DeltaArgs& a) {
 }
 
 // ------------------------------------------------------------------ gated norm of the read-out
+// heads of up to 128 columns that start on 16-byte boundaries: four columns per lane (bound by memory; 18 k rows of 16
+// heads of 128: 83 us, 215 us with 4-byte accesses)
+template <typename OT>
+__global__ void __launch_bounds__(256) delta_out_vec_kernel(DeltaArgs a, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  constexpr bool FAST = sizeof(OT) == 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int t = blockIdx.x, vdim = a.vdim;
+  const bool on = 4 * lane < vdim;
+  const float4 w = on ? *reinterpret_cast<const float4*>(a.onorm_w + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+  pdl_wait();
+  OT* out = (OT*)a.out + (size_t)t * a.o_ld;
+  const float* gate = a.in_p + (size_t)t * a.in_ld + a.conv_ch + 2 * a.H + 4 * lane;
+  const float* o = a.o + (size_t)t * a.H * vdim + 4 * lane;
+  for (int h = blockIdx.y * nw + warp; h < a.H; h += gridDim.y * nw) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 v = on ? *reinterpret_cast<const float4*>(o + (size_t)h * vdim) : zero;
+    const float4 g = on ? sum_slices4(gate + (size_t)h * vdim, a.in_S, a.in_stride) : zero;
+    const float inv = 1.0f / sqrtf(warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) / (float)vdim + a.eps);
+    const float r[4] = {v.x * inv * w.x * silu_t<FAST>(g.x), v.y * inv * w.y * silu_t<FAST>(g.y),
+                        v.z * inv * w.z * silu_t<FAST>(g.z), v.w * inv * w.w * silu_t<FAST>(g.w)};
+    if (on) store4(out + h * vdim + 4 * lane, r);
+  }
+  if (blockIdx.y == 0)
+    for (int c = a.H * vdim + threadIdx.x; c < a.o_ld; c += blockDim.x) out[c] = from_f32<OT>(0.f);
+  TRACE_EXIT(tr);
+}
+
 template <typename OT, int MV>
 __global__ void __launch_bounds__(256) delta_out_kernel(DeltaArgs a, Trace tr) {
   TRACE_ENTRY(tr);
@@ -557,6 +802,10 @@ __global__ void __launch_bounds__(256) delta_out_kernel(DeltaArgs a, Trace tr) {
 cudaError_t launch_delta_out(cudaStream_t st, int odt, const DeltaArgs& a) {
   if (a.T <= 0) return cudaSuccess;
   const dim3 grid(a.T, a.T >= 1024 ? 1 : ceil_div(a.H, 8));  // few rows (decode): a row's heads spread over several CTAs
+  // (the gates' columns start behind 2 H entries of the projection)
+  if (a.vdim <= 128 && a.vdim % 4 == 0 && (a.conv_ch + 2 * a.H) % 4 == 0 && a.in_ld % 4 == 0 && a.in_stride % 4 == 0 && a.o_ld % 4 == 0)
+    return odt == DT_F32 ? launch_k(delta_out_vec_kernel<float>, grid, dim3(256), 0, st, a, next_trace(36))
+                         : launch_k(delta_out_vec_kernel<bf16>, grid, dim3(256), 0, st, a, next_trace(36));
   if (odt == DT_F32) (void)launch_k(delta_out_kernel<float, 8>, grid, dim3(256), 0, st, a, next_trace(36));
   else if (a.vdim <= 128) (void)launch_k(delta_out_kernel<bf16, 4>, grid, dim3(256), 0, st, a, next_trace(36));
   else (void)launch_k(delta_out_kernel<bf16, 8>, grid, dim3(256), 0, st, a, next_trace(36));

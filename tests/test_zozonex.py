@@ -428,6 +428,50 @@ def test_long_decoding_stays_on_the_reference():
         eng.close()
 
 
+@gpu
+@pytest.mark.parametrize("dim,vdim", [(16, 17), (32, 64), (48, 130), (64, 66), (96, 9), (128, 128), (256, 34)])
+def test_delta_rule_decays_of_every_strength(dim, vdim):
+    """The compile-time scan keeps the state divided by the product of its decays: heads whose decays are near one, small
+    enough that the product leaves fp32's range several times in a tile of tokens, and zero."""
+    j = model([layer(delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=2))])
+    cfg, w = random_weights(j, 11)
+    w["l0.mix.A_log"] = np.array([-8.0, 1.0, 2.5, 6.0], dtype=np.float32)
+    eng = Engine(cfg, w, C.PREC_FP32)
+    try:
+        toks = prompt(j, 75, 12)
+        want = ref.forward(j, w, toks)
+        got, _ = eng.step([("s", toks[:50], list(range(50)))])
+        check(got, want[:50], C.PREC_FP32, "prompt")
+        rows = [eng.step([("s", [toks[t]], [0])], decode=True)[0][0] for t in range(50, 75)]
+        check(np.stack(rows), want[50:], C.PREC_FP32, "decoded")
+    finally:
+        eng.close()
+
+
+@gpu
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("dim,vdim,conv", [(128, 128, 4), (64, 36, 2), (20, 12, 3)])
+def test_delta_rule_prompts_of_many_rows(dim, vdim, conv, prec):
+    """Steps of more than a thousand rows slide windows of eight rows over the sequences: sequences shorter than the
+    convolution between longer ones, borders inside a window, and a second portion that starts from the slots' tails."""
+    j = model([layer(delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=conv))])
+    cfg, w, eng = setup(j, prec, num_blocks=16, slots=6)
+    try:
+        lens = {"a": (520, 513), "b": (1, 2), "c": (2, 1), "d": (505, 508), "e": (3, 9)}
+        toks = {k: prompt(j, sum(n), 50 + i) for i, (k, n) in enumerate(lens.items())}
+        want = {k: ref.forward(j, w, t) for k, t in toks.items()}
+        for part in range(2):
+            entries, rows = [], []
+            for k, n in lens.items():
+                lo = sum(n[:part])
+                entries.append((k, toks[k][lo:lo + n[part]], list(range(n[part]))))
+                rows.append(want[k][lo:lo + n[part]])
+            got, _ = eng.step(entries)
+            check(got, np.concatenate(rows), prec, f"portion {part}")
+    finally:
+        eng.close()
+
+
 # ------------------------------------------------------------------ GPU: entry points
 @gpu
 def test_greedy_generation_through_the_engine_and_its_scheduler():
