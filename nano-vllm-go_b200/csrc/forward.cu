@@ -51,7 +51,7 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
   w.T_cap = Tc;
   w.n_cap = nc;
   const size_t H = h->H, asz = dt_size(h->adt);
-  // room for split-K slices of skinny GEMMs; the fp32 GEMM splits up to eight ways until two CTAs per SM
+  // room for split-K slices of skinny GEMMs; the fp32 GEMM splits up to eight ways to fill the SMs evenly
   const size_t rows = std::max(std::max(Tc, 512), h->adt == DT_F32 ? std::min(8 * Tc, 2048) : 0);
   uint64_t* acc = &h->ws_bytes;
   auto A = [&](void** p, size_t bytes) -> cudaError_t {

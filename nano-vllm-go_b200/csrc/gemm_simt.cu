@@ -354,10 +354,12 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
 // fp32 operations) as they lie in memory.  A and W go to shared memory in steps of 32 k by 16-byte cp.async, three
 // stages deep; rows are 36 floats apart, which puts the 8 (4) rows that a warp reads at once on different
 // banks: per 4 k a lane reads 4 + MI pieces for 8 MI packed FMAs, so at MI = 8 the fp32 pipe is the
-// bound and not shared memory.  k is split over CTAs (fp32 slices, summed by the consumer) until each SM has two.
+// bound and not shared memory.  k is split over CTAs (fp32 slices, summed by the consumer) so that the SMs get equal
+// shares.
 // MI = 2 / 4 keep tiles of 16 / 32 rows for small steps, which are bound by the weights.
-// GPT-2 small, four prompts of 50 to 100 tokens: the step's 48 matrix products 7.24 -> 2.5 ms against tiles of 64 x 64
-// x 16 with scalar FMAs, operands transposed through registers and one k range (60 to 240 CTAs of the chip's 296).
+// GPT-2 small, four prompts of 50 to 100 tokens: the step's 48 matrix products 7.24 -> 2.04 ms against tiles of 64 x 64
+// x 16 with scalar FMAs, operands transposed through registers and one k range (60 to 240 CTAs of the chip's 296); 32
+// TFLOP/s in the widest, three CTAs per SM (four at 128 registers each: 2.50 ms).
 constexpr int FG_BN = 64, FG_BK = 32, FG_PITCH = 36, FG_STAGES = 3, FG_THREADS = 128;
 
 template <int MI>
@@ -435,10 +437,9 @@ gemm_f32_kernel(GemmArgs g, int kc, Trace tr) {
       for (int i = 0; i < MI; i++) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + 8 * i * FG_PITCH + k);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          acc[i][j] = fma2(a.x, w[j].x, acc[i][j]);
-          acc[i][j] = fma2(a.y, w[j].y, acc[i][j]);
-        }
+        for (int j = 0; j < 4; j++) acc[i][j] = fma2(a.x, w[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fma2(a.y, w[j].y, acc[i][j]);
       }
     }
   }
@@ -473,12 +474,21 @@ static cudaError_t launch_gemm_f32(cudaStream_t st, GemmArgs& g) {
   const int mt = g.tile_expert ? g.max_tiles : ceil_div(g.M, 8 * mi), nt = ceil_div(g.N, FG_BN);
   g.S = 1;
   if (mt == 0 || nt == 0) return cudaSuccess;
-  // slices: up to the eight that a consumer sums with one batch of loads, each at least 128 of k, as many as the
-  // buffer has room for, while two CTAs per SM are not reached (grouped tiles write one slice)
+  // slices: up to the eight that a consumer sums with one batch of loads, each at least 128 of k, as many as the buffer
+  // has room for (grouped tiles write one slice): the count with the least work on the fullest SM, in steps of 32 k
+  // plus two for a CTA's fill and its results; an SM with fewer than three CTAs runs them at a lower rate
   int S = 1;
-  if (!g.tile_expert && g.out_capacity)
-    while (S < 8 && (long)mt * nt * S < 2 * 148 && g.K / (S + 1) >= 128 &&
-           (size_t)(S + 1) * g.split_stride <= g.out_capacity) S++;
+  if (!g.tile_expert && g.out_capacity) {
+    double best = 1e30;
+    for (int s = 1; s <= 8 && (s == 1 || g.K / s >= 128) && (s == 1 || (size_t)s * g.split_stride <= g.out_capacity); s++) {
+      const int per_sm = ceil_div(mt * nt * s, 148), steps = ceil_div(ceil_div(g.K, FG_BK), s);
+      const double cost = (per_sm >= 3 ? per_sm : per_sm == 2 ? 2.4 : 1.8) * (steps + 2.0) + 0.3 * s;
+      if (cost < best) {
+        best = cost;
+        S = s;
+      }
+    }
+  }
   const int kc = ceil_div(ceil_div(g.K, FG_BK), S) * FG_BK;
   g.S = ceil_div(g.K, kc);
   const dim3 grid(mt, nt, g.S);
