@@ -221,24 +221,33 @@ __global__ void __launch_bounds__(256) mamba_conv_rows_kernel(MambaArgs a, Trace
   TRACE_EXIT(tr);
 }
 
-// Selective scan.  Four lanes share R rows of a head's state (lane q holds entries 16 j + 4 q .. + 3 of each, as
-// packed pairs in registers), 4 hd / R threads make a head and HPC heads of one group a CTA.  Per token a lane reads
-// N / 4 entries of B and of C (64 contiguous bytes per quad, broadcast to the warp's other rows) for R N / 4 state
-// entries and spends three packed instructions per entry pair; the four partial read-outs of a row meet by shuffles.
-// B, C, u and the (step, decay) pairs of the next MS_TC tokens arrive by cp.async under the current ones.
-// Bound by fp32 issue, 3 operations per state entry and token.  The 6446 rows above, 64 heads of 64 x 128: 730 us; a
-// thread per row with scalar operations and the decay computed in every thread: 7405 us.  R = 2 keeps five CTAs
-// of 128 threads on an SM; R = 1 doubles the threads of a head when few (sequence, head) pairs are to be shared out.
-constexpr int MS_TC = 8;
-template <int R, int NJ>
+// Selective scan.  L lanes share R rows of a head's state (lane q holds entries 4 L j + 4 q .. + 3 of each, as packed
+// pairs in registers), L hd / R threads make a head and HPC heads of one group a CTA.  Per token a lane reads N / L
+// entries of B and of C for R N / L state entries and spends three packed instructions per entry pair; the L partial
+// read-outs of a row meet by shuffles that scatter the rows over the lanes.  B, C, u and the (step, decay) pairs of the
+// next MS_TC tokens arrive by cp.async under the current ones.
+// Two fp32 operations per state entry and token: the state is kept as S / c, c the product of the decays since the chunk
+// of tokens began, so a token adds (dt u / c) B and reads c (S / c) C; the state is multiplied by the last chunk's c when
+// the next one begins, and by c inside one whenever that falls below 1e-18 (nothing leaves fp32's range).  c and
+// dt / c are made once per token and head.
+// Bound by instruction issue, half of it those operations; a 16-byte read of shared memory brings eight different pieces
+// to eight lanes (four lanes per row where the state has only 16 entries).  6446 rows in 16 sequences, 64 heads of
+// 64 x 128: 683 us; 730 us with four lanes and three operations per entry, 7405 us with a thread per row, scalar
+// operations and the decay computed in every thread.  Half the rows per lane doubles the threads of a head when few
+// (sequence, head) pairs are to be shared out.
+constexpr int MS_TC = 16;
+constexpr float MS_RESCALE = 1e-18f;
+constexpr int MS_MAX_HPC = 16;  // heads of a CTA
+template <int R, int L, int NJ>
 __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int hpc, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
-  constexpr int N = 16 * NJ;
+  constexpr int N = 4 * L * NJ;
   extern __shared__ __align__(16) float sm[];
+  __shared__ float4 tok_s[2 * MS_TC * MS_MAX_HPC];  // [half][token][head]: c, dt / c, what multiplies the state before it
   const int s = blockIdx.x, h0 = blockIdx.y * hpc;
-  const int tid = threadIdx.x, nt = blockDim.x, tph = 4 * a.hd / R;
-  const int hl = tid / tph, ht = tid % tph, q = ht & 3, d0 = (ht >> 2) * R, h = h0 + hl;
+  const int tid = threadIdx.x, nt = blockDim.x, tph = L * a.hd / R;
+  const int hl = tid / tph, ht = tid % tph, q = ht % L, d0 = ht / L * R, h = h0 + hl;
   const int uw = hpc * a.hd, row = 2 * N + uw + 2 * hpc;  // floats of a staged token: B | C | u | (step, decay)
   const int rowp = (row + 3) & ~3;
   pdl_wait();
@@ -281,38 +290,63 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
     for (int r = 0; r < R; r++)
 #pragma unroll
       for (int j = 0; j < NJ; j++) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + (size_t)r * N + 16 * j);
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + (size_t)r * N + 4 * L * j);
         st[r][2 * j] = v.x;
         st[r][2 * j + 1] = v.y;
       }
   }
   const float Dh = a.d_skip ? a.d_skip[h] : 0.f;
+  auto scale = [&](float m) {
+    const unsigned long long mm = pack2(m, m);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+      for (int j = 0; j < 2 * NJ; j++) st[r][j] = mul2(st[r][j], mm);
+  };
+  float c_end = 1.f;  // c after the last token
   for (int t0 = r0, buf = 0; t0 < r1; t0 += MS_TC, buf ^= 1) {
     cp_async_wait<0>();
     __syncthreads();  // this chunk has arrived, and everybody is done with the other buffer
-    if (t0 + MS_TC < r1) fetch(t0 + MS_TC, buf ^ 1);
     const int n = min(MS_TC, r1 - t0);
+    for (int i = tid; i < n * hpc; i += nt) {  // token t of head k: the decays up to it
+      const int t = i / hpc, k = i % hpc;
+      const float* w = sm + buf * MS_TC * rowp + 2 * N + uw + 2 * k;
+      float c = 1.f, m = 1.f;
+      for (int j = 0; j <= t; j++) {
+        c *= w[j * rowp + 1];
+        m = 1.f;
+        if (c < MS_RESCALE) {
+          m = c;
+          c = 1.f;
+        }
+      }
+      tok_s[(buf * MS_TC + t) * MS_MAX_HPC + k] = make_float4(c, w[t * rowp] / c, m, 0.f);
+    }
+    if (t0 + MS_TC < r1) fetch(t0 + MS_TC, buf ^ 1);
+    __syncthreads();
+    if (c_end != 1.f) scale(c_end);
     for (int t = 0; t < n; t++) {
       const float* x = sm + (buf * MS_TC + t) * rowp;
-      const float2 step = *reinterpret_cast<const float2*>(x + 2 * N + uw + 2 * hl);
+      const float4 tk = tok_s[(buf * MS_TC + t) * MS_MAX_HPC + hl];
       const float* u = x + 2 * N + hl * a.hd + d0;
-      const unsigned long long decay = pack2(step.y, step.y);
+      if (tk.z != 1.f) scale(tk.z);
+      c_end = tk.x;
       unsigned long long du[R], acc[R];
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        const float v = step.x * u[r];
+        const float v = tk.y * u[r];
         du[r] = pack2(v, v);
         acc[r] = 0ull;
       }
 #pragma unroll
       for (int j = 0; j < NJ; j++) {
-        const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(x + 16 * j + 4 * q);
-        const ulonglong2 Cc = *reinterpret_cast<const ulonglong2*>(x + N + 16 * j + 4 * q);
+        const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(x + 4 * L * j + 4 * q);
+        const ulonglong2 Cc = *reinterpret_cast<const ulonglong2*>(x + N + 4 * L * j + 4 * q);
 #pragma unroll
         for (int r = 0; r < R; r++) {
-          st[r][2 * j] = fma2(decay, st[r][2 * j], mul2(du[r], B.x));          // mamba2.go:325-331
-          acc[r] = fma2(Cc.x, st[r][2 * j], acc[r]);                            // :335-340
-          st[r][2 * j + 1] = fma2(decay, st[r][2 * j + 1], mul2(du[r], B.y));
+          st[r][2 * j] = fma2(du[r], B.x, st[r][2 * j]);  // mamba2.go:325-331
+          st[r][2 * j + 1] = fma2(du[r], B.y, st[r][2 * j + 1]);
+          acc[r] = fma2(Cc.x, st[r][2 * j], acc[r]);      // :335-340
           acc[r] = fma2(Cc.y, st[r][2 * j + 1], acc[r]);
         }
       }
@@ -323,24 +357,31 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
         unpack2(acc[r], lo, hi);
         y[r] = lo + hi;
       }
-      float out;  // lanes q < R end up with row d0 + q
-      if constexpr (R == 2) {
-        const float give = (q & 1) ? y[0] : y[1], keep = (q & 1) ? y[1] : y[0];
-        out = keep + __shfl_xor_sync(0xffffffffu, give, 1);
-      } else {
-        out = y[0] + __shfl_xor_sync(0xffffffffu, y[0], 1);
+      // lanes q < R end up with row d0 + q
+#pragma unroll
+      for (int o = 1; o < R; o <<= 1) {
+        const bool up = (q & o) != 0;
+#pragma unroll
+        for (int r = 0; r < R / 2 / o; r++) {
+          const float give = up ? y[2 * r] : y[2 * r + 1], keep = up ? y[2 * r + 1] : y[2 * r];
+          y[r] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
       }
-      out += __shfl_xor_sync(0xffffffffu, out, 2);
-      if (q < R) a.y[(size_t)(t0 + t) * a.E + (size_t)h * a.hd + d0 + q] = out + Dh * u[q];
+      float out = y[0];
+#pragma unroll
+      for (int o = R; o < L; o <<= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
+      if (q < R) a.y[(size_t)(t0 + t) * a.E + (size_t)h * a.hd + d0 + q] = tk.x * out + Dh * u[q];
       const int pos = start + (t0 + t - r0);
       if ((pos + 1) % KV_BLOCK == 0 || t0 + t == r1 - 1) {
         // snapshot: the state after the last token written into this block
         float* dst = a.ssm_pool + (size_t)bt[pos / KV_BLOCK] * per_block + mine;
+        const unsigned long long cc = pack2(tk.x, tk.x);
 #pragma unroll
         for (int r = 0; r < R; r++)
 #pragma unroll
           for (int j = 0; j < NJ; j++)
-            *reinterpret_cast<ulonglong2*>(dst + (size_t)r * N + 16 * j) = make_ulonglong2(st[r][2 * j], st[r][2 * j + 1]);
+            *reinterpret_cast<ulonglong2*>(dst + (size_t)r * N + 4 * L * j) =
+                make_ulonglong2(mul2(st[r][2 * j], cc), mul2(st[r][2 * j + 1], cc));
       }
     }
   }
@@ -721,32 +762,42 @@ cudaError_t launch_mamba_conv(cudaStream_t st, const MambaArgs& a) {
 }
 
 // heads of a CTA of the tiled scan, 0 where it does not fit: whole warps, the heads of a CTA from one group
-static int mamba_scan_hpc(const MambaArgs& a, int R) {
+static int mamba_scan_hpc(const MambaArgs& a, int R, int L) {
   if (!mamba_rows_aligned(a) || a.hd % 4 != 0) return 0;
   if (a.N != 16 && a.N != 32 && a.N != 64 && a.N != 128) return 0;
-  const int tph = 4 * a.hd / R, per_group = a.nh / a.G;
+  const int tph = L * a.hd / R, per_group = a.nh / a.G;
   int hpc = 1;
   while (hpc * 2 * tph <= 128 && per_group % (hpc * 2) == 0) hpc *= 2;
-  return hpc * tph % 32 == 0 && hpc * tph <= 512 ? hpc : 0;
+  return hpc * tph % 32 == 0 && hpc * tph <= 512 && hpc <= MS_MAX_HPC ? hpc : 0;
 }
-template <int R>
+template <int R, int L, int NJ>
 static cudaError_t mamba_scan_tiles(cudaStream_t st, const MambaArgs& a, int hpc) {
-  const dim3 grid(a.n_seqs, a.nh / hpc), block(hpc * 4 * a.hd / R);
+  const dim3 grid(a.n_seqs, a.nh / hpc), block(hpc * L * a.hd / R);
   const size_t smem = (size_t)2 * MS_TC * ((2 * a.N + hpc * a.hd + 2 * hpc + 3) & ~3) * sizeof(float);
-  if (a.N == 16) return launch_k(mamba_scan_tile_kernel<R, 1>, grid, block, smem, st, a, hpc, next_trace(21));
-  if (a.N == 32) return launch_k(mamba_scan_tile_kernel<R, 2>, grid, block, smem, st, a, hpc, next_trace(21));
-  if (a.N == 64) return launch_k(mamba_scan_tile_kernel<R, 4>, grid, block, smem, st, a, hpc, next_trace(21));
-  return launch_k(mamba_scan_tile_kernel<R, 8>, grid, block, smem, st, a, hpc, next_trace(21));
+  if (smem > 32 * 1024) {  // (beside the kernel's own 8 KB the default limit is 40 KB)
+    const cudaError_t e = cudaFuncSetAttribute(mamba_scan_tile_kernel<R, L, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_k(mamba_scan_tile_kernel<R, L, NJ>, grid, block, smem, st, a, hpc, next_trace(21));
+}
+// R rows per lane, or half as many: twice the warps per head and half the state per lane, the shorter chain per token
+// while the grid leaves schedulers idle (148 SMs x 4, two warps each)
+template <int R, int L, int NJ>
+static bool mamba_scan_try(cudaStream_t st, const MambaArgs& a, cudaError_t* e) {
+  const int half = mamba_scan_hpc(a, R / 2, L), whole = mamba_scan_hpc(a, R, L);
+  if (whole && (!half || (long)a.n_seqs * a.nh * (L * a.hd / R) / 32 > 148 * 8)) *e = mamba_scan_tiles<R, L, NJ>(st, a, whole);
+  else if (half) *e = mamba_scan_tiles<R / 2, L, NJ>(st, a, half);
+  else return false;
+  return true;
 }
 cudaError_t launch_mamba_scan(cudaStream_t st, const MambaArgs& a) {
   if (a.n_seqs <= 0) return cudaSuccess;
   const int threads = max(32, ((a.hd + 31) / 32) * 32);
   if (threads > 128 || a.N > 128) return cudaErrorInvalidValue;
-  // R = 1 has twice the warps per head and half the state per lane: the shorter chain per token
-  // while the grid leaves schedulers idle (148 SMs x 4, two warps each at 4 hd / 64 warps a head)
-  const int one = mamba_scan_hpc(a, 1), two = mamba_scan_hpc(a, 2);
-  if (two && (!one || (long)a.n_seqs * a.nh * a.hd * 4 / 64 > 148 * 8)) return mamba_scan_tiles<2>(st, a, two);
-  if (one) return mamba_scan_tiles<1>(st, a, one);
+  cudaError_t e = cudaSuccess;
+  if (a.N == 16 ? mamba_scan_try<2, 4, 1>(st, a, &e) : a.N == 32 ? mamba_scan_try<4, 8, 1>(st, a, &e)
+      : a.N == 64 ? mamba_scan_try<4, 8, 2>(st, a, &e) : a.N == 128 && mamba_scan_try<4, 8, 4>(st, a, &e))
+    return e;
   const dim3 grid(a.n_seqs, a.nh);
   if (a.N <= 16) (void)launch_k(mamba_scan_kernel<16>, grid, dim3(threads), 0, st, a, next_trace(21));
   else if (a.N <= 32) (void)launch_k(mamba_scan_kernel<32>, grid, dim3(threads), 0, st, a, next_trace(21));

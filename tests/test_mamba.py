@@ -123,3 +123,29 @@ def test_hybrid_prompts_at_the_edges_of_the_scan_tiles(nh, hd, N, G, K):
                         mamba_state_size=N, mamba_n_groups=G, mamba_conv_kernel=K)
     prompts = [W.random_prompt(cfg.vocab_size, n, 50 + i) for i, n in enumerate((1, 7, 8, 17, 258))]
     _run(cfg, C.PREC_FP32, prompts, 3, [[0], [1], [2], [3], [4, 5]], 6)
+
+
+@pytest.mark.parametrize("N,hd", [(16, 8), (32, 32), (64, 16), (128, 64)])
+def test_hybrid_decays_of_every_strength(N, hd):
+    """The tiled scan keeps the state divided by the product of its decays: heads whose decays are near one, small
+    enough that the product leaves fp32's range inside a chunk of tokens, and zero."""
+    R = nvllm_pkg.sub("runner")
+    cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=8, mamba_head_dim=hd,
+                        mamba_state_size=N, mamba_n_groups=2, mamba_conv_kernel=4)
+    a_log = np.array([-6.0, 0.0, 1.0, 2.0, 3.0, 4.5, 6.0, -1.0], dtype=np.float32)
+
+    def weights():
+        for wid, layer, w in W.random_weights(cfg, 1234):
+            yield wid, layer, a_log if wid == C.W_MAMBA_A_LOG else w
+
+    prompt = [int(t) for t in W.random_prompt(cfg.vocab_size, 70, 9)]
+    ref = oracle_mod().OracleModel(cfg, weights())
+    want = ref.greedy(prompt, 2)
+    run = R.CudaModelRunner(cfg, weights(), precision=C.PREC_FP32, num_kv_blocks=1, sampling=None)
+    try:
+        _, logits = run.run_flat([prompt], True, [0], [[0]], [0.0], want_logits=True)
+        assert rel_err(logits[0], want[1][0]) <= 1e-4
+        _, logits = run.run_flat([prompt + [int(want[0][0])]], False, None, [[0]], [0.0], want_logits=True)
+        assert rel_err(logits[0], want[1][1]) <= 1e-4
+    finally:
+        run.close()
