@@ -440,9 +440,151 @@ __global__ void __launch_bounds__(512) norm_kernel(NormArgs a, Trace tr) {
     trace_rec(tr, t_entry, t_wait, ((t_loads - t_wait) << 32) | (t_red - t_wait));
 }
 
+// The same for many rows whose addends need no summing over slices (prompts): a row stays in registers, four entries per
+// thread and vector, V vectors; all loads of a row, the expert rows of a combine included, are in flight at
+// once.  Bound by memory.  norm_kernel keeps eight entries per thread, sums up to eight slices, stages the row in shared
+// memory and needs 128 registers for all its options, too many for enough loads in flight.  Per launch inside whole
+// steps: 6446 rows of 2048 with one addend 55 -> 31 us (5.9 TB/s); 18 k rows of 2048, norm on the addend 148 -> 86 us;
+// 2048 rows of 4544, LayerNorm and two addends 54 -> 24 us; 18.7 k rows of 1024 through combines of eight expert rows and
+// routing 161 -> 140 us.  From 512 rows on (every SM has more than three); fewer keep norm_kernel, whose CTAs start
+// their weights' loads before the dependency resolves.
+constexpr int NR_MAX_V = 4, NR_THREADS = 512;
+template <typename YT, int V, int COMB>
+__global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Trace tr) {
+  const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
+  pdl_launch_dependents();
+  __shared__ float red[32];
+  const int H = a.H, r = blockIdx.x;
+  pdl_wait();
+  const unsigned long long t_wait = trace_on(tr) ? gtime() : 0ull;
+  float* xr = a.x + (size_t)r * H;
+  float v[V][4], acc[V][4];
+  int prow[COMB ? COMB : 1];
+  float cw[COMB ? COMB : 1];
+  if constexpr (COMB > 0) {
+#pragma unroll
+    for (int q = 0; q < COMB; q++) {
+      prow[q] = q < a.comb_k ? a.comb_rows[(size_t)r * a.comb_k + q] : -1;
+      cw[q] = q < a.comb_k ? a.comb_w[(size_t)r * a.comb_k + q] : 0.f;
+    }
+  }
+  auto get = [](const float* p, float (&o)[4]) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
+  };
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = ((int)threadIdx.x + k * (int)blockDim.x) * 4;
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[k][j] = acc[k][j] = 0.f;
+    if (i >= H) continue;
+    get(xr + i, v[k]);
+    if constexpr (COMB > 0) {
+      float pv[COMB][4];
+#pragma unroll
+      for (int q = 0; q < COMB; q++)
+        if (prow[q] >= 0) get(a.p1 + (size_t)prow[q] * H + i, pv[q]);
+#pragma unroll
+      for (int q = 0; q < COMB; q++)  // slot order (moe.go:116-118)
+        if (prow[q] >= 0) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[k][j] += cw[q] * pv[q][j];
+        }
+    } else if (a.p1) {
+      get(a.p1 + (size_t)r * H + i, acc[k]);
+    }
+    if (a.post) continue;
+    float p2[4] = {0.f, 0.f, 0.f, 0.f}, b[4];
+    if (a.p2) get(a.p2 + (size_t)r * H + i, p2);
+    if (a.p1 && a.bias1) {
+      get(a.bias1 + i, b);
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[k][j] += b[j];
+    }
+    if (a.p2 && a.bias2) {
+      get(a.bias2 + i, b);
+#pragma unroll
+      for (int j = 0; j < 4; j++) p2[j] += b[j];
+    }
+    if (a.p1)
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[k][j] = v[k][j] + a.m1 * acc[k][j];
+    if (a.p2)
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[k][j] = v[k][j] + a.m2 * p2[j];
+    if (a.p1 || a.p2) store4(xr + i, v[k]);
+  }
+  if (a.y || a.y_f32 || a.post) {
+    const bool ln = a.b != nullptr || a.centered != 0;
+    float part = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; k++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) part += a.post ? acc[k][j] * acc[k][j] : ln ? v[k][j] : v[k][j] * v[k][j];  // (zeros past the row)
+    const float tot = block_sum(part, red);
+    float mean = 0.f, inv;
+    if (ln && !a.post) {
+      mean = tot / (float)H;
+      float lv = 0.f;
+#pragma unroll
+      for (int k = 0; k < V; k++)
+        if (((int)threadIdx.x + k * (int)blockDim.x) * 4 < H) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float d = v[k][j] - mean;
+            lv += d * d;
+          }
+        }
+      inv = 1.0f / sqrtf(block_sum(lv, red) / (float)H + a.eps);
+    } else {
+      inv = 1.0f / sqrtf(tot / (float)H + a.eps);
+    }
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const int i = ((int)threadIdx.x + k * (int)blockDim.x) * 4;
+      if (i >= H) continue;
+      float w[4] = {1.f, 1.f, 1.f, 1.f}, b[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
+      if (a.w) get(a.w + i, w);
+      if (a.b) get(a.b + i, b);
+      if (a.post) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = fmaf(acc[k][j] * inv, w[j], v[k][j]);
+        store4(xr + i, o);
+      } else if (ln) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = (v[k][j] - mean) * inv * w[j] + b[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = v[k][j] * inv * w[j];
+      }
+      if (a.y) store4((YT*)a.y + (size_t)r * H + i, o);
+      if (a.y_f32 && !a.post) store4(a.y_f32 + (size_t)r * H + i, o);
+    }
+  }
+  if (threadIdx.x == 0 && trace_on(tr)) trace_rec(tr, t_entry, t_wait, 0ull);
+}
+// many rows, no option of norm_kernel that these kernels lack, at most one slice (or eight expert rows) per addend
+static bool norm_rows_fit(const NormArgs& a) {
+  return a.n_rows >= 512 && a.H % 8 == 0 && a.H <= NR_MAX_V * NR_THREADS * 4 && !a.row_idx && !a.router && !a.gate_w && !a.plain &&
+         a.groups <= 1 && !a.xadd && !a.xadd_table && !a.row_m2 && !a.conv_taps && !a.p1_bf16 &&
+         (!a.p1 || (a.comb_rows ? a.comb_k <= 8 : a.S1 == 1)) && (!a.p2 || a.S2 == 1) &&
+         (!a.post || (a.p1 && a.w && !a.comb_rows && !a.p2));
+}
+template <typename YT>
+static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
+  const int V = ceil_div(a.H, NR_THREADS * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
+  const bool comb = a.p1 && a.comb_rows;
+#define NR(V_)                                                                                                       \
+  (comb ? launch_k(norm_rows_kernel<YT, V_, 8>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(2))              \
+        : launch_k(norm_rows_kernel<YT, V_, 0>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(2)))
+  return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
+#undef NR
+}
+
 cudaError_t launch_norm(cudaStream_t st, const NormArgs& a) {
   if (a.n_rows <= 0) return cudaSuccess;
   if (a.groups > 64 || (a.groups > 1 && a.H % a.groups) || (a.plain && !a.y)) return cudaErrorInvalidValue;
+  if (norm_rows_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float>(st, a) : launch_norm_rows<bf16>(st, a);
   int threads = min(512, max(64, ((a.H / 8 + 31) / 32) * 32));
   // fused router, decode-sized batches (latency-bound: fewer row CTAs than two waves): 16 warps
   // so that each takes two experts of a 32-expert layer in one pass; prefill keeps the

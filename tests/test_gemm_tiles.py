@@ -37,3 +37,17 @@ def test_fp32_tiles(M, N, K):
 ])
 def test_bf16_rows_on_mma(M, N, K):
     assert _product(M, N, K, C.PREC_BF16, 1) <= 1.0
+
+
+@pytest.mark.parametrize("H", [8, 72, 1024, 2048, 2056, 4544, 8192])
+@pytest.mark.parametrize("layer_norm", [False, True])
+def test_norm_of_many_rows(H, layer_norm):
+    """512 rows take the kernel that keeps a row in registers (one to four vectors per thread)."""
+    L = nvllm_pkg.sub("lib")
+    g = torch.Generator().manual_seed(H)
+    x, w, b = torch.randn(512, H, generator=g) * 3 + 1, torch.randn(H, generator=g), torch.randn(H, generator=g)
+    y, _ = L.op_norm(x.numpy(), w.numpy(), b.numpy() if layer_norm else None, eps=1e-5)
+    xd = x.double() - (x.double().mean(-1, keepdim=True) if layer_norm else 0.0)
+    ref = xd / torch.sqrt(xd.square().mean(-1, keepdim=True) + 1e-5) * w.double() + (b.double() if layer_norm else 0.0)
+    # a few fp32 roundings of numbers up to ~10 times a weight, and a sum of H terms: 2^-24 (H / 256 + 16) of the largest
+    assert float((torch.from_numpy(y).double() - ref).abs().max()) <= 2.0 ** -24 * (H / 256 + 16) * float(ref.abs().max())
