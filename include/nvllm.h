@@ -521,6 +521,11 @@ int nvllm_get_profile(nvllm_handle* h, nvllm_profile_entry* out);
 int nvllm_trace_begin(nvllm_handle* h, int capacity);
 int nvllm_trace_end(nvllm_handle* h, uint64_t* out, int max_records, int* n_records);
 
+/* Tests of the error path: does on the host what a kernel does on the device when one of its bounded waits runs out.  The
+ * handle's next call that synchronises and hands out results (nvllm_run, nvllm_sync) fails with NVLLM_ERR_CUDA, and the
+ * resident state is dropped.  h == NULL: the calling thread's next nvllm_op_matmul instead. */
+int nvllm_inject_wait_failure(nvllm_handle* h);
+
 /* Wait for the resident steps issued so far; optionally read back the last sampled tokens
  * (n <= n_seqs of the last nvllm_run) and the device time of the last step. */
 int nvllm_sync(nvllm_handle* h, int32_t* out_tokens, int n, float* last_step_ms);

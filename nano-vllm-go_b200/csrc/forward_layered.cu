@@ -1882,6 +1882,7 @@ extern "C" int nvllm_create_layered(const nvllm_layered_config* c, const nvllm_l
   if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "cudaStreamCreate");
   if ((e = cudaEventCreate(&h->ev0)) != cudaSuccess) return fail(e, "cudaEventCreate");
   if ((e = cudaEventCreate(&h->ev1)) != cudaSuccess) return fail(e, "cudaEventCreate");
+  if ((e = h->waits.create()) != cudaSuccess) return fail(e, "cudaHostAlloc");
   const int W = h->H;
   const size_t wsz = dt_size(h->wdt);
   // zero-filled: inner extents are padded to 8 and the padding must stay zero

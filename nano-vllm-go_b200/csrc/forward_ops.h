@@ -158,6 +158,7 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
     t.split_stride = res->stride; t.alpha = alpha; t.out_capacity = cap;
     t.S = tc5_splits(M, N, K, h->sm_count);
     t.max_ctas = h->gemm_max_ctas;
+    t.wait_flag = h->waits.dev;
     if (rs && rs->ssq) {
       t.rs_ssq = rs->ssq; t.rs_parts = rs->parts; t.rs_ld = h->ws.T_cap;
       t.rs_inv_h = 1.0f / (float)h->H; t.rs_eps = h->cfg.norm_eps;
@@ -321,6 +322,7 @@ static int run_moe_ffn(nvllm_handle* h, int T, const void* xn, int E, int k, int
     t.g_experts = E; t.g_tile = tile; t.g_max_tiles = w.max_tiles;
     t.g_tile_expert = w.sort.tile_expert; t.g_tile_row0 = w.sort.tile_row0;
     t.g_tile_rows = w.sort.tile_rows; t.g_n_tiles = w.sort.n_tiles;
+    t.wait_flag = h->waits.dev;
     {
       ProfScope ps(h, NVLLM_K_MOE_GEMM, (double)e_touched * N1 * H * wsz, 2.0 * P * N1 * H,
                    (double)P * H * asz + (double)P * I * asz);

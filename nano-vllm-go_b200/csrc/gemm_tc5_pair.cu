@@ -20,8 +20,9 @@
 // epilogue took longer than its products.  What bounds it now is the clock under the power limit (tensor pipe 92 %
 // busy at 1.3 GHz in the widest product) and, below 2048 of k, the epilogue.
 //
-// Every wait on a barrier has a limit: past it the kernel sets a flag in host memory, leaves its loops, gives the copies
-// in flight time to land, frees its tensor memory and returns; the host reports the step as failed.
+// The waits of the loading, MMA and epilogue loops have a limit: past it the kernel sets its launch's flag in host memory
+// (WaitFlag), leaves its loops, gives the copies in flight time to land, frees its tensor memory and returns; the host
+// reports the step as failed.
 #include <cuda.h>
 
 #include <mutex>
@@ -438,23 +439,34 @@ struct PairDevice {
 };
 std::mutex g_pair_mu;
 PairDevice g_pair_dev[64];
-int* g_pair_flag = nullptr;       // pinned, mapped on every device
 }  // namespace
 
-// Once per device, outside any stream capture (handle creation): kernel attributes, resident pairs, the flag
+cudaError_t WaitFlag::create() {
+  cudaError_t e = cudaHostAlloc((void**)&host, sizeof(int), cudaHostAllocMapped);
+  if (e != cudaSuccess) {
+    host = nullptr;
+    return e;
+  }
+  *host = 0;
+  e = cudaHostGetDevicePointer((void**)&dev, host, 0);
+  if (e != cudaSuccess) destroy();
+  return e;
+}
+void WaitFlag::destroy() {
+  if (host) cudaFreeHost(host);
+  host = dev = nullptr;
+}
+void WaitFlag::raise() {
+  if (host) __atomic_store_n(host, 1, __ATOMIC_RELEASE);
+}
+bool WaitFlag::take() { return host && __atomic_exchange_n(host, 0, __ATOMIC_ACQ_REL) != 0; }
+
+// Once per device, outside any stream capture (handle creation): kernel attributes, resident pairs
 int tc5_pair_init(int dev) {
   std::lock_guard<std::mutex> g(g_pair_mu);
   if (dev < 0 || dev >= 64) return 0;
   PairDevice& d = g_pair_dev[dev];
   if (d.known) return d.pairs;
-  if (!g_pair_flag) {
-    if (cudaHostAlloc((void**)&g_pair_flag, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-      g_pair_flag = nullptr;
-      (void)cudaGetLastError();
-      return 0;
-    }
-    *g_pair_flag = 0;
-  }
   int n = 0;
   if (cudaFuncSetAttribute(gemm_tc5_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PR_SMEM) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
@@ -475,21 +487,13 @@ int tc5_pair_init(int dev) {
   d.known = true;
   return n;
 }
-// did a wait of a pair kernel run out since the last call?
-bool tc5_pair_failed() {
-  volatile int* f = g_pair_flag;
-  if (!f || !*f) return false;
-  *f = 0;
-  return true;
-}
-
 // Token tiles of 256 rows and one k range per tile are taken over, unless rounding the weight tiles up to 256 rows costs
 // more rounds of the persistent schedule than the pair gains (1.15: the smallest gain above at equal rounds).
 bool tc5_pair_fits(const Tc5Args& a, int bt, int S) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   const int pairs = g_pair_dev[dev].pairs, sms = g_pair_dev[dev].sms;
-  if (pairs <= 0 || bt != PR_BT || S != 1 || a.N <= TC_BN) return false;
+  if (pairs <= 0 || !a.wait_flag || bt != PR_BT || S != 1 || a.N <= TC_BN) return false;
   const long mt = a.g_experts > 0 ? a.M / PR_BT + a.g_experts : ceil_div(a.M, PR_BT);
   const long one = (mt * ceil_div(a.N, TC_BN) + sms - 1) / sms;
   const long two = (mt * ceil_div(a.N, 2 * TC_BN) + pairs - 1) / pairs;
@@ -500,11 +504,8 @@ cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDes
   int dev = 0;
   cudaGetDevice(&dev);
   const int pairs = g_pair_dev[dev].pairs;
-  if (pairs <= 0 || !g_pair_flag) return cudaErrorInvalidValue;
+  if (pairs <= 0 || !a.wait_flag) return cudaErrorInvalidValue;
   if (a.epi == TC5_EPI_RESID && (!a.res_x || !a.res_xb || !a.res_ssq || a.g_experts > 0)) return cudaErrorInvalidValue;
-  int* flag = nullptr;
-  cudaError_t e = cudaHostGetDevicePointer((void**)&flag, g_pair_flag, 0);
-  if (e != cudaSuccess) return e;
   Tc5Sched sc{};
   sc.nkb_total = sc.kbps = ceil_div(a.K, TC_BK);
   sc.S = 1;
@@ -526,7 +527,7 @@ cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDes
                    a.res_ssq_ld, a.res_bias, a.res_m, a.res_g, 0, a.glu_limit};
   return launch_k_cluster(gemm_tc5_pair_kernel, dim3(2 * n), dim3(PR_THREADS), PR_SMEM, st, 2,
                           *reinterpret_cast<const CUtensorMap*>(tw), *reinterpret_cast<const CUtensorMap*>(ta), a.M, a.N, sc,
-                          a.out, a.ldo, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias, fz, flag,
+                          a.out, a.ldo, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias, fz, a.wait_flag,
                           next_trace(1));
 }
 

@@ -219,6 +219,7 @@ struct nvllm_handle {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t tm0 = nullptr, tm1 = nullptr;  // nvllm_timer_record
+  nvllm::WaitFlag waits;                     // of the kernels launched for this handle
   std::string err;
   bool finalized = false;
   int wdt = 0, adt = 0, kvdt = 0;

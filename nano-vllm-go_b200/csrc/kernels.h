@@ -296,6 +296,16 @@ int make_tma_2d_bf16(TmaDesc* out, const void* base, uint64_t rows, uint64_t col
                      uint64_t row_stride_elems, uint32_t box_rows, std::string* err);
 // memoised tensor map (pure function of pointer, shape, box); null on failure
 const TmaDesc* tma_map_cached(const void* base, int rows, int cols, int box_rows);
+// Where a kernel reports that one of its bounded waits ran out: an int in host memory, mapped on the device.  Every handle
+// and every single-operator call has its own, so nobody takes another's failure.
+struct WaitFlag {
+  int* host = nullptr;
+  int* dev = nullptr;  // what the kernels write
+  cudaError_t create();  // on the current device
+  void destroy();
+  void raise();  // from the host (tests of the error path)
+  bool take();   // after a synchronise: did a wait run out since the last call?
+};
 struct Tc5Args {
   const void* A;  // activations [M, K] bf16, K contiguous
   const void* W;  // weights     [N, K] bf16, K contiguous
@@ -348,14 +358,13 @@ struct Tc5Args {
   const int* g_tile_row0;
   const int* g_tile_rows;
   const int* g_n_tiles;  // [1] on the device
+  int* wait_flag;        // WaitFlag::dev; null: kernels with bounded waits are not used
 };
 // TC5_EPI_RELU2: like TC5_EPI_GELU (bf16 activation written, no bias needed) with relu(h)^2
 enum { TC5_EPI_PARTIAL = 0, TC5_EPI_SWIGLU = 1, TC5_EPI_GELU = 2, TC5_EPI_RESID = 3, TC5_EPI_RELU2 = 4 };
 // gemm_tc5_pair.cu: the kernel for many token rows, two CTAs per tile.  init: once per device and outside any stream
-// capture (returns the resident pairs; without it the kernel is not used).  failed: a wait of the kernel ran out
-// since the last call.
+// capture (returns the resident pairs; without it the kernel is not used).
 int tc5_pair_init(int dev);
-bool tc5_pair_failed();
 bool tc5_pair_fits(const Tc5Args& a, int bt, int S);
 cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDesc* tw, const TmaDesc* ta);
 // split-K slices for a TC5_EPI_RESID GEMM: like tc5_splits, but every unit must own an SM

@@ -195,6 +195,7 @@ int nvllm_create(const nvllm_config* c, const uint8_t* tp_id, nvllm_handle** out
     return fail(e, "cudaStreamCreate");
   if ((e = cudaEventCreate(&h->ev0)) != cudaSuccess) return fail(e, "cudaEventCreate");
   if ((e = cudaEventCreate(&h->ev1)) != cudaSuccess) return fail(e, "cudaEventCreate");
+  if ((e = h->waits.create()) != cudaSuccess) return fail(e, "cudaHostAlloc");
 
   // ---- weights (device layouts; see handle.h) ----
   uint64_t* wb = &h->weight_bytes;
@@ -343,6 +344,7 @@ int nvllm_destroy(nvllm_handle* h) {
   nvllm::tp_destroy(h);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
+  h->waits.destroy();
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return NVLLM_OK;

@@ -12,7 +12,9 @@ struct Scratch {  // frees everything on scope exit
   std::vector<void*> ptrs;
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
+  WaitFlag waits;
   ~Scratch() {
+    waits.destroy();
     for (void* p : ptrs) cudaFree(p);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -37,8 +39,10 @@ int op_begin(Scratch& s, int device) {
   OP_CHECK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
   OP_CHECK(cudaEventCreate(&s.e0));
   OP_CHECK(cudaEventCreate(&s.e1));
+  OP_CHECK(s.waits.create());
   return 0;
 }
+thread_local bool t_fail_next_matmul = false;  // nvllm_inject_wait_failure(NULL)
 constexpr size_t FLUSH_FLOATS = (size_t)64 << 20;  // 256 MB > 126 MB L2
 }  // namespace
 
@@ -76,6 +80,7 @@ extern "C" int nvllm_op_matmul(int device, int prec, int kernel, int M, int N, i
       Tc5Args t{};
       t.A = dA; t.W = dWt; t.M = M; t.N = N; t.K = K; t.out = dOut; t.ldo = ldo;
       t.split_stride = (size_t)M * ldo; t.alpha = 1.f; t.out_capacity = cap;
+      t.wait_flag = s.waits.dev;
       t.S = tc5_splits(M, N, K, 148);
       while (t.S > 1 && (size_t)t.S * M * ldo > cap) t.S--;
       return launch_gemm_tc5(s.st, t, &S);
@@ -105,10 +110,19 @@ extern "C" int nvllm_op_matmul(int device, int prec, int kernel, int M, int N, i
   // sum the split-K slices and add the bias the way the consumer kernels do
   OP_CHECK(launch_reduce_partials(s.st, dOut, S, (size_t)M * ldo, (size_t)M * ldo, dC));
   OP_CHECK(cudaStreamSynchronize(s.st));
+  if (t_fail_next_matmul) s.waits.raise();
+  t_fail_next_matmul = false;
+  if (s.waits.take()) return set_err(nullptr, NVLLM_ERR_CUDA, "op_matmul: a wait inside the GEMM ran out");
   std::vector<float> hc((size_t)M * ldo);
   OP_CHECK(cudaMemcpy(hc.data(), dC, hc.size() * 4, cudaMemcpyDeviceToHost));
   for (int m = 0; m < M; m++)
     for (int n = 0; n < N; n++) C[(size_t)m * N + n] = hc[(size_t)m * ldo + n] + (bias ? bias[n] : 0.f);
+  return NVLLM_OK;
+}
+
+extern "C" int nvllm_inject_wait_failure(nvllm_handle* h) {
+  if (h) h->waits.raise();
+  else t_fail_next_matmul = true;
   return NVLLM_OK;
 }
 

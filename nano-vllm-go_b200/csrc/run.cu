@@ -149,6 +149,14 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
 // A speculative step that is thrown away has only written K/V at the next position of each
 // sequence, a slot nothing reads before its owner writes it.
 static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_graph = nullptr);
+// After a synchronise: did a bounded wait of this handle's kernels run out?  Then neither the results nor the device state
+// that a resident, speculative or repeated step would start from are used.
+static int check_waits(nvllm_handle* h) {
+  if (!h->waits.take()) return NVLLM_OK;
+  h->resident_ok = h->run_lay_ok = h->spec_pending = false;
+  h->fetched_rows = 0;
+  return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
+}
 static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, const int32_t* block_tables,
                           const int32_t* cu_blocks) {
   h->spec_len.resize(n);
@@ -234,7 +242,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
       cudaError_t e = cudaStreamSynchronize(st);
       if (e != cudaSuccess)
         return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
-      if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
+      if (const int rc = check_waits(h)) return rc;
       memcpy(out_tokens, h->h_out, (size_t)n * 4);
       h->run_lay = h->lay;
       h->run_lay_ok = true;
@@ -439,7 +447,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess)
     return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
-  if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
+  if ((rc = check_waits(h))) return rc;
   memcpy(out_tokens, h->h_out, (size_t)n * 4);
   h->resident_ok = true;
   h->run_lay = L;
@@ -607,7 +615,7 @@ extern "C" int nvllm_sync(nvllm_handle* h, int32_t* out_tokens, int n, float* la
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess)
     return set_err(h, NVLLM_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
-  if (tc5_pair_failed()) return set_err(h, NVLLM_ERR_CUDA, "stream failed: a wait inside a GEMM ran out");
+  if (const int rc = check_waits(h)) return rc;
   if (out_tokens && n > 0) {
     if (n > h->lay.n) n = h->lay.n;
     if (h->spec_pending)  // ws.out_tokens already holds the speculative step's tokens

@@ -68,6 +68,7 @@ SIGNATURES = {
                                  _i32p, _i32p, _f32p, _f32p, _i32p, _f32p,
                                  ctypes.POINTER(RunStats)]),
     "nvllm_run_resident": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(RunStats)]),
+    "nvllm_inject_wait_failure": (ctypes.c_int, [ctypes.c_void_p]),
     "nvllm_sync": (ctypes.c_int, [ctypes.c_void_p, _i32p, ctypes.c_int, _f32p]),
     "nvllm_rerun": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(RunStats)]),
     "nvllm_set_profile": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
