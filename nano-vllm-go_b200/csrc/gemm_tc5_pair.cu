@@ -227,7 +227,9 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       // fp32 accumulate, bf16 x bf16, both K-major, N = 256, M = 256 over the two CTAs
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PR_BT >> 3) << 17) |
                                  ((uint32_t)((2 * TC_BN) >> 4) << 24);
-      if (grouped) pdl_wait();  // the tile list is the previous kernel's output
+      // the tile list is the previous kernel's output; and the limit of the waits below counts from here, not from
+      // this CTA's start: the kernels in front may take longer than it (an all-reduce waits up to 5 s for a late peer)
+      pdl_wait();
       const int units = grouped ? *sc.g_ntiles * sc.n_tiles : sc.units;
       int i = 0, lu = 0;
       bool ok = true;

@@ -1,14 +1,16 @@
 """A bounded wait inside a kernel that runs out is reported to the caller whose launch it was, and to nobody else.  The
 failure is made on the host (nvllm_inject_wait_failure does there what the kernel does); no wait runs out on the device."""
+import os
+import re
 import threading
 
 import numpy as np
 import pytest
 
-from helpers import C, W
+from helpers import C, ROOT, W
 import nvllm_pkg
 
-pytestmark = pytest.mark.gpu
+gpu = pytest.mark.gpu
 
 
 def _runner(seed):
@@ -17,6 +19,19 @@ def _runner(seed):
     return R.CudaModelRunner(cfg, W.random_weights(cfg, seed, round_bf16=True), precision=C.PREC_BF16, num_kv_blocks=4, sampling=None)
 
 
+def test_limits_count_from_the_launch_dependency():
+    """Under programmatic launch a CTA may start long before the kernels in front are done: each role of the pair kernel
+    waits for them, in dense and grouped products alike, before its first wait with a limit."""
+    with open(os.path.join(ROOT, "nano-vllm-go_b200", "csrc", "gemm_tc5_pair.cu")) as f:
+        kernel = f.read().split("\ngemm_tc5_pair_kernel(", 1)[1].split("\n}\n", 1)[0]
+    roles = re.split(r"\n  (?:if \(warp == 0\) \{\n    uint64_t|\} else if \(warp == 1\) \{|\} else \{)", kernel)[1:]
+    assert len(roles) == 3
+    for role in roles:
+        dependency = re.search(r"^ +pdl_wait\(\);", role, re.M)
+        assert dependency and dependency.start() < role.index("wait_limited(")
+
+
+@gpu
 def test_only_the_handle_whose_wait_ran_out_fails():
     L = nvllm_pkg.sub("lib")
     a, b = _runner(1), _runner(2)
@@ -48,6 +63,7 @@ def test_only_the_handle_whose_wait_ran_out_fails():
         b.close()
 
 
+@gpu
 def test_a_matrix_product_whose_wait_ran_out_fails_and_no_later_call():
     L = nvllm_pkg.sub("lib")
     x, w = np.ones((300, 64), np.float32), np.ones((64, 512), np.float32)
