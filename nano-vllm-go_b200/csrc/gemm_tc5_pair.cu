@@ -293,6 +293,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       if (!epilogue_agrees(wait_limited(bar_tfull + 8 * buf, (lu >> 1) & 1, dead, flag))) break;
       tc_fence_after();
       auto load_acc = [&](int c0, uint32_t (&r)[32]) {
+        __syncwarp();  // the load is the whole warp's: lanes past the last column have skipped the previous chunk's stores
         tmem_ld_32x32(lanes + (uint32_t)c0, r);
         if (rs) {
 #pragma unroll

@@ -18,6 +18,7 @@ pytestmark = pytest.mark.gpu
     (512, 20000, 200),   # k tail, N off the tiles
     (520, 12928, 136),   # the last pair's second half lies outside W
     (1000, 10240, 456),  # more k blocks than stages
+    (300, 37901, 72),    # the last columns fill 13 lanes of a warp
 ])
 def test_pair_product(M, N, K):
     assert _product(M, N, K, C.PREC_BF16, 3) <= 1.0
