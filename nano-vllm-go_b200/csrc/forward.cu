@@ -42,6 +42,31 @@ void free_workspace(nvllm_handle* h) {
   h->ws_bytes = 0;
 }
 
+// Floats of the buffers for split-K slices in a workspace of T tokens and n rows of logits
+struct SplitRoom {
+  size_t a, b, head;
+};
+static SplitRoom split_room(const nvllm_handle* h, int T, int n) {
+  // room for split-K slices of skinny GEMMs; the fp32 GEMM splits up to eight ways to fill the SMs evenly
+  const size_t rows = std::max(std::max(T, 512), h->adt == DT_F32 ? std::min(8 * T, 2048) : 0);
+  size_t a_cols = std::max(h->qkv_cols, h->moe ? 0 : h->w1_cols);
+  if (h->n_mamba) a_cols = std::max(a_cols, (size_t)h->m_P);
+  SplitRoom r{rows * a_cols, rows * h->H, 0};
+  if (h->moe) r.a = std::max(r.a, (size_t)T * h->topk * 2 * h->F);
+  // tp > 1: this rank's LM-head slice is Vl wide and the gathered logits are [tp][n][Vl]
+  r.head = (size_t)std::max(n, 64) * (h->tp > 1 ? (size_t)h->Vl : (size_t)h->ldl);
+  return r;
+}
+// The fp32 GEMM takes as many slices as there is room for: a step gets the room that a workspace made for it alone has,
+// so that its sums, which fp32 mode is compared by, don't depend on the steps before it.
+static void fit_split_room(nvllm_handle* h) {
+  if (h->adt != DT_F32) return;
+  const SplitRoom r = split_room(h, h->lay.T, std::max(h->lay.n, h->lay.n_out));
+  h->ws.ws_a_floats = r.a;
+  h->ws.ws_b_floats = r.b;
+  h->ws.logits_p_floats = r.head;
+}
+
 int ensure_workspace(nvllm_handle* h, int T, int n) {
   Workspace& w = h->ws;
   if (T <= w.T_cap && n <= w.n_cap) return NVLLM_OK;
@@ -51,8 +76,7 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
   w.T_cap = Tc;
   w.n_cap = nc;
   const size_t H = h->H, asz = dt_size(h->adt);
-  // room for split-K slices of skinny GEMMs; the fp32 GEMM splits up to eight ways to fill the SMs evenly
-  const size_t rows = std::max(std::max(Tc, 512), h->adt == DT_F32 ? std::min(8 * Tc, 2048) : 0);
+  const SplitRoom room = split_room(h, Tc, nc);
   uint64_t* acc = &h->ws_bytes;
   auto A = [&](void** p, size_t bytes) -> cudaError_t {
     *p = nullptr;
@@ -73,11 +97,8 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
   }
   WS(w.x, Tc * H * 4);
   WS(w.xn, Tc * H * asz);
-  size_t a_cols = std::max(h->qkv_cols, h->moe ? 0 : h->w1_cols);
-  if (h->n_mamba) a_cols = std::max(a_cols, (size_t)h->m_P);
-  w.ws_a_floats = rows * a_cols;
-  if (h->moe) w.ws_a_floats = std::max(w.ws_a_floats, (size_t)Tc * h->topk * 2 * h->F);
-  w.ws_b_floats = rows * H;
+  w.ws_a_floats = room.a;
+  w.ws_b_floats = room.b;
   WS(w.ws_a, w.ws_a_floats * 4);
   WS(w.ws_b, w.ws_b_floats * 4);
   if (h->parallel) WS(w.ws_c, w.ws_b_floats * 4);
@@ -174,9 +195,8 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
     }
   }
   if (h->tp > 1) WS(w.tp_buf, Tc * H * 4);
-  // tp > 1: this rank's LM-head slice is Vl wide and the gathered logits are [tp][n][Vl]
   const size_t lcols = h->tp > 1 ? (size_t)h->Vl : (size_t)h->ldl;
-  w.logits_p_floats = (size_t)std::max(nc, 64) * lcols;
+  w.logits_p_floats = room.head;
   WS(w.logits_p, w.logits_p_floats * 4);
   WS(w.logits, (size_t)nc * lcols * h->tp * 4);
   w.attn_ws_floats = (size_t)nc * h->nh * 32 * (h->hd + 2);
@@ -318,6 +338,7 @@ static int tp_reduce_pending(nvllm_handle* h, Pending* p1, Pending* p2, int T) {
 // ------------------------------------------------------------------ forward pass
 // Inputs are the device arrays of h->lay (already on the device).
 int forward_step(nvllm_handle* h) {
+  if (h->view_T == 0) fit_split_room(h);  // (a chunk of a step has its half of the step's room)
   if (h->layered) return forward_step_layered(h);
   const StepLayout& L = h->lay;
   Workspace& w = h->ws;
@@ -650,6 +671,7 @@ int forward_step_auto(nvllm_handle* h) {
   if (!(h->tp > 1 && h->nccl2 && L.prefill && L.n == 1 && !h->profile && !h->moe && L.T >= min_T &&
         ts >= 1 && r0 < L.T && (r0 % 8) == 0))
     return forward_step(h);
+  fit_split_room(h);
   const Workspace W0 = h->ws;
   cudaStream_t s0 = h->stream;
   static bool said = false;

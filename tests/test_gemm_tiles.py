@@ -39,6 +39,27 @@ def test_bf16_rows_on_mma(M, N, K):
     assert _product(M, N, K, C.PREC_BF16, 1) <= 1.0
 
 
+@pytest.mark.parametrize("lens", [[600], [10] * 40])  # slices of the layers' products; of the head's
+def test_fp32_step_does_not_depend_on_the_steps_before_it(lens):
+    """How many k ranges the fp32 products take is decided by the step, not by the room that a larger step left behind."""
+    from helpers import W
+    R = nvllm_pkg.sub("runner")
+    cfg = C.tiny_gpt2(hidden=512, num_heads=8, num_kv_heads=8, head_dim=64, ffn_dim=2048)
+    run = R.CudaModelRunner(cfg, W.random_weights(cfg, 5), precision=C.PREC_FP32, num_kv_blocks=200, sampling=None)
+
+    def step(lens):
+        prompts = [W.random_prompt(cfg.vocab_size, k, 60 + i) for i, k in enumerate(lens)]
+        return run.run_flat(prompts, True, [0] * len(lens), [[5 * i, 5 * i + 1, 5 * i + 2] if k > 256 else [i] for i, k in enumerate(lens)],
+                            [0.0] * len(lens), want_logits=True)[1]
+
+    try:
+        first = step(lens)
+        step([20] * 200)
+        assert np.array_equal(step(lens), first)
+    finally:
+        run.close()
+
+
 @pytest.mark.parametrize("H", [8, 72, 1024, 2048, 2056, 4544, 8192])
 @pytest.mark.parametrize("layer_norm", [False, True])
 def test_norm_of_many_rows(H, layer_norm):
