@@ -561,7 +561,8 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
       if (a.y_f32 && !a.post) store4(a.y_f32 + (size_t)r * H + i, o);
     }
   }
-  if (threadIdx.x == 0 && trace_on(tr)) trace_rec(tr, t_entry, t_wait, 0ull);
+  if (threadIdx.x == 0 && trace_on(tr))  // what the row took in: 1 an addend (2: expert rows), 4 a second one, 8 normed on it
+    trace_rec(tr, t_entry, t_wait, (a.p1 ? 1ull : 0ull) | (COMB ? 2ull : 0ull) | (a.p2 ? 4ull : 0ull) | (a.post ? 8ull : 0ull));
 }
 // many rows, no option of norm_kernel that these kernels lack, at most one slice (or eight expert rows) per addend
 static bool norm_rows_fit(const NormArgs& a) {
@@ -575,8 +576,8 @@ static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
   const int V = ceil_div(a.H, NR_THREADS * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
   const bool comb = a.p1 && a.comb_rows;
 #define NR(V_)                                                                                                       \
-  (comb ? launch_k(norm_rows_kernel<YT, V_, 8>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(2))              \
-        : launch_k(norm_rows_kernel<YT, V_, 0>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(2)))
+  (comb ? launch_k(norm_rows_kernel<YT, V_, 8>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47))             \
+        : launch_k(norm_rows_kernel<YT, V_, 0>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47)))
   return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
 #undef NR
 }

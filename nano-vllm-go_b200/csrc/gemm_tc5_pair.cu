@@ -428,7 +428,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   __syncthreads();
   cluster_arrive_release();  // the leader's MMAs read the peer's shared memory, the peer's warps arrive on the leader's barriers
   cluster_wait_acquire();
-  if (threadIdx.x == 0 && trace_on(tr)) trace_rec(tr, t_entry, t_wait, 0ull);
+  if (threadIdx.x == 0 && trace_on(tr)) trace_rec(tr, t_entry, t_wait, (unsigned long long)epi);
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * PR_BT)) : "memory");
 }
@@ -531,7 +531,7 @@ cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDes
   return launch_k_cluster(gemm_tc5_pair_kernel, dim3(2 * n), dim3(PR_THREADS), PR_SMEM, st, 2,
                           *reinterpret_cast<const CUtensorMap*>(tw), *reinterpret_cast<const CUtensorMap*>(ta), a.M, a.N, sc,
                           a.out, a.ldo, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias, fz, a.wait_flag,
-                          next_trace(1));
+                          next_trace(46));
 }
 
 }  // namespace nvllm

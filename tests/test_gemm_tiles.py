@@ -3,8 +3,9 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import C
+from helpers import C, W, rel_err
 import nvllm_pkg
+import test_zozonex as zozonex
 
 pytestmark = pytest.mark.gpu
 
@@ -42,7 +43,6 @@ def test_bf16_rows_on_mma(M, N, K):
 @pytest.mark.parametrize("lens", [[600], [10] * 40])  # slices of the layers' products; of the head's
 def test_fp32_step_does_not_depend_on_the_steps_before_it(lens):
     """How many k ranges the fp32 products take is decided by the step, not by the room that a larger step left behind."""
-    from helpers import W
     R = nvllm_pkg.sub("runner")
     cfg = C.tiny_gpt2(hidden=512, num_heads=8, num_kv_heads=8, head_dim=64, ffn_dim=2048)
     run = R.CudaModelRunner(cfg, W.random_weights(cfg, 5), precision=C.PREC_FP32, num_kv_blocks=200, sampling=None)
@@ -72,3 +72,42 @@ def test_norm_of_many_rows(H, layer_norm):
     ref = xd / torch.sqrt(xd.square().mean(-1, keepdim=True) + 1e-5) * w.double() + (b.double() if layer_norm else 0.0)
     # a few fp32 roundings of numbers up to ~10 times a weight, and a sum of H terms: 2^-24 (H / 256 + 16) of the largest
     assert float((torch.from_numpy(y).double() - ref).abs().max()) <= 2.0 ** -24 * (H / 256 + 16) * float(ref.abs().max())
+
+
+NORM_ROWS_KERNEL = 47  # its id in the timeline; a record's last word says what the row took in before its norm
+ADDEND, EXPERT_ROWS, SECOND_ADDEND, ON_THE_ADDEND = 1, 2, 4, 8
+
+
+@pytest.mark.parametrize("family", ["llama", "falcon", "moe", "zozonex"])
+def test_norm_of_many_rows_with_addends(family):
+    """One pending product, two of them and a LayerNorm, the expert rows of a combine, a norm on the addend: float32 prompts
+    as one batch, whose norms take the kernel for many rows, against the same prompts one at a time."""
+    R = nvllm_pkg.sub("runner")
+    if family == "zozonex":
+        cfg, w = zozonex.random_weights(zozonex.model([zozonex.layer(zozonex.attn(), 96)] * 2, width=264), 3)
+        weights, form = w.items(), ON_THE_ADDEND | ADDEND
+    else:
+        cfg, form = {"llama": (C.tiny_llama(hidden=264), ADDEND), "falcon": (C.tiny_falcon(), ADDEND | SECOND_ADDEND),
+                     "moe": (C.tiny_granite(hidden=264), ADDEND | EXPERT_ROWS)}[family]
+        weights = W.random_weights(cfg, 3)
+    n = 24
+    prompts = [W.random_prompt(cfg.vocab_size, 80 + (7 * i) % 23, 60 + i) for i in range(n)]  # 2199 rows: products in one slice
+    run = R.CudaModelRunner(cfg, weights, precision=C.PREC_FP32, num_kv_blocks=n, sampling=None)
+
+    def step(which):
+        run.trace_begin(1 << 18)
+        _, logits = run.run_flat([prompts[i] for i in which], True, [0] * len(which), [[i] for i in which], [0.0] * len(which),
+                                 want_logits=True)
+        rec = run.trace_end(1 << 18)
+        assert 0 < len(rec) < 1 << 18
+        return logits, set(rec[rec[:, 1] == NORM_ROWS_KERNEL, 7].tolist())
+
+    try:
+        batch, forms = step(range(n))
+        assert form in forms
+        for i in range(n):
+            one, forms = step([i])
+            assert not forms
+            assert rel_err(batch[i], one[0]) <= 1e-4  # what the fp32 mode is held to against the reference
+    finally:
+        run.close()

@@ -112,21 +112,32 @@ def test_hybrid_rejects_multi_token_prefill_on_a_cached_prefix():
     (8, 4, 16, 1, 4),     # smallest head of the tiled scan: two heads to a warp and more
     (8, 64, 64, 2, 4),
     (4, 128, 128, 4, 4),  # largest head and state, one head per group
-    (32, 128, 32, 8, 4),  # five sequences are enough warps for two rows per lane
+    (32, 128, 16, 8, 4),  # eight sequences of that many heads are enough warps for twice the rows per lane
+    (32, 128, 32, 8, 4),
+    (32, 128, 64, 8, 4),
+    (32, 128, 128, 8, 4),
     (8, 32, 24, 2, 4),    # state that is no power of two: the scan without tiles
     (6, 12, 16, 3, 4),    # rows that start off 16-byte boundaries
     (8, 32, 16, 2, 3),    # other taps
 ])
 def test_hybrid_prompts_at_the_edges_of_the_scan_tiles(nh, hd, N, G, K):
-    """Prompts of one token, around the scan's chunk of eight and over a block border, decoded on."""
+    """Prompts of one token, around the scan's chunk of sixteen and over a block border, decoded on."""
     cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=nh, mamba_head_dim=hd,
                         mamba_state_size=N, mamba_n_groups=G, mamba_conv_kernel=K)
-    prompts = [W.random_prompt(cfg.vocab_size, n, 50 + i) for i, n in enumerate((1, 7, 8, 17, 258))]
-    _run(cfg, C.PREC_FP32, prompts, 3, [[0], [1], [2], [3], [4, 5]], 6)
+    prompts = [W.random_prompt(cfg.vocab_size, n, 50 + i) for i, n in enumerate((1, 7, 15, 16, 17, 32, 33, 258))]
+    _run(cfg, C.PREC_FP32, prompts, 3, [[i] for i in range(7)] + [[7, 8]], 9)
 
 
-@pytest.mark.parametrize("N,hd", [(16, 8), (32, 32), (64, 16), (128, 64)])
-def test_hybrid_decays_of_every_strength(N, hd):
+def test_hybrid_scan_with_sixteen_heads_to_a_cta():
+    """The smallest heads, one group, and so many short prompts that a lane holds two rows of a head: 16 heads per CTA."""
+    cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=64, mamba_head_dim=4,
+                        mamba_state_size=16, mamba_n_groups=1, mamba_conv_kernel=4)
+    prompts = [W.random_prompt(cfg.vocab_size, 1 + i % 19, 50 + i) for i in range(75)]
+    _run(cfg, C.PREC_FP32, prompts, 3, [[i] for i in range(75)], 75)
+
+
+@pytest.mark.parametrize("N,hd,n", [(16, 8, 1), (32, 32, 1), (64, 16, 1), (128, 64, 1), (128, 128, 20)])  # (the last: 1280 warps)
+def test_hybrid_decays_of_every_strength(N, hd, n):
     """The tiled scan keeps the state divided by the product of its decays: heads whose decays are near one, small
     enough that the product leaves fp32's range inside a chunk of tokens, and zero."""
     R = nvllm_pkg.sub("runner")
@@ -141,11 +152,12 @@ def test_hybrid_decays_of_every_strength(N, hd):
     prompt = [int(t) for t in W.random_prompt(cfg.vocab_size, 70, 9)]
     ref = oracle_mod().OracleModel(cfg, weights())
     want = ref.greedy(prompt, 2)
-    run = R.CudaModelRunner(cfg, weights(), precision=C.PREC_FP32, num_kv_blocks=1, sampling=None)
+    run = R.CudaModelRunner(cfg, weights(), precision=C.PREC_FP32, num_kv_blocks=n, sampling=None)
+    tables, zeros = [[i] for i in range(n)], [0] * n
     try:
-        _, logits = run.run_flat([prompt], True, [0], [[0]], [0.0], want_logits=True)
-        assert rel_err(logits[0], want[1][0]) <= 1e-4
-        _, logits = run.run_flat([prompt + [int(want[0][0])]], False, None, [[0]], [0.0], want_logits=True)
-        assert rel_err(logits[0], want[1][1]) <= 1e-4
+        _, logits = run.run_flat([prompt] * n, True, zeros, tables, zeros, want_logits=True)
+        assert max(rel_err(row, want[1][0]) for row in logits) <= 1e-4
+        _, logits = run.run_flat([prompt + [int(want[0][0])]] * n, False, None, tables, zeros, want_logits=True)
+        assert max(rel_err(row, want[1][1]) for row in logits) <= 1e-4
     finally:
         run.close()

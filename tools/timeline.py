@@ -27,7 +27,7 @@ run.trace_begin(1 << 17)
 for _ in range(2):
     run.run_resident()
 rec = run.trace_end(1 << 17)
-names = {1: "gemm", 2: "norm", 3: "rope_kv", 4: "attn_dec"}
+names = {1: "gemm", 2: "norm", 3: "rope_kv", 4: "attn_dec", 46: "gemm_pair", 47: "norm_rows"}
 aux = rec[rec[:, 1] == 9]
 rec = rec[rec[:, 1] != 9]
 seqs = sorted(set(int(x) for x in rec[:, 0]))
