@@ -4,10 +4,12 @@
 //
 // Bound by the HBM stream of W (N K 2 bytes); at eight rows the arithmetic on the CUDA cores took four times as long
 // as that stream (a conversion per weight and 8 FMAs), so the products run on mma.sync m16n8k16: 16 weight rows are
-// the M side, the <= 8 activation rows the N side.  Each pair of mma's starts from zero and is added to fp32 sums, so
-// the long sum over k is ordinary fp32 addition.  The order of k inside a product is free as long as both operands
-// agree: a lane reads 16 contiguous bytes of a weight row and the same 16 of its activation row and feeds their
-// four 2-element pieces to two mma's.
+// the M side, the <= 8 activation rows the N side.  Each mma starts from zero, and the four of a chunk are added to four
+// fp32 sums that meet in pairs at the end, as the warps' do: 16 products are added inside the tensor core, which drops
+// bits, all else is short chains of ordinary fp32 addition.  Against float64, relative to chains of FMAs on the CUDA
+// cores: 0.93 to 1.06 times their error from 768 of k on (1.11 to 1.29 times with two mma's in a row and one sum).
+// The order of k inside a product is free as long as both operands agree: a lane reads 16 contiguous bytes of a weight
+// row and the same 16 of its activation row and feeds their four 2-element pieces to two mma's.
 //
 // The warps of a CTA share its k range in chunks of 64 and work alone: each has a ring of chunks (its 16 MT weight
 // rows and the activation rows) in shared memory that it fills by cp.async, 128 contiguous bytes of a row to eight
@@ -81,11 +83,7 @@ gemv_mma_kernel(GemvMmaArgs a, Trace tr) {
     if (i < mine) fetch_a(i);
     cp_async_commit();
   }
-  float acc[MT][4];
-#pragma unroll
-  for (int i = 0; i < MT; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+  float acc[4][MT][4] = {};  // [mma of a chunk]
   for (int i = 0; i < mine; i++) {
     cp_async_wait<NS - 2>();
     __syncwarp();  // chunk i has arrived for every lane, and every lane is done with the stage that is filled next
@@ -101,11 +99,14 @@ gemv_mma_kernel(GemvMmaArgs a, Trace tr) {
 #pragma unroll
       for (int t = 0; t < MT; t++) {
         const uint4 lo = ld_shared16(st + gm_at(16 * t + g, 4 * j + q)), hi = ld_shared16(st + gm_at(16 * t + g + 8, 4 * j + q));
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        mma16816(d, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
-        mma16816(d, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
+        float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816(d0, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
+        mma16816(d1, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[t][e] += d[e];
+        for (int e = 0; e < 4; e++) {
+          acc[2 * j][t][e] += d0[e];
+          acc[2 * j + 1][t][e] += d1[e];
+        }
       }
     }
   }
@@ -114,18 +115,25 @@ gemv_mma_kernel(GemvMmaArgs a, Trace tr) {
   float (*red)[8][16 * MT] = reinterpret_cast<float (*)[8][16 * MT]>(ring);
 #pragma unroll
   for (int i = 0; i < MT; i++) {  // fragment: weight rows g and g + 8, activation rows 2 q and 2 q + 1
-    red[warp][2 * q][16 * i + g] = acc[i][0];
-    red[warp][2 * q + 1][16 * i + g] = acc[i][1];
-    red[warp][2 * q][16 * i + g + 8] = acc[i][2];
-    red[warp][2 * q + 1][16 * i + g + 8] = acc[i][3];
+    float s[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) s[e] = (acc[0][i][e] + acc[1][i][e]) + (acc[2][i][e] + acc[3][i][e]);
+    red[warp][2 * q][16 * i + g] = s[0];
+    red[warp][2 * q + 1][16 * i + g] = s[1];
+    red[warp][2 * q][16 * i + g + 8] = s[2];
+    red[warp][2 * q + 1][16 * i + g + 8] = s[3];
   }
   __syncthreads();
   for (int e = tid; e < a.M * 16 * MT; e += NW * 32) {
     const int m = e / (16 * MT), r = e % (16 * MT), n = n0 + r;
-    float v = 0.f;
+    float p[NW];
 #pragma unroll
-    for (int w = 0; w < NW; w++) v += red[w][m][r];
-    v *= a.alpha;
+    for (int w = 0; w < NW; w++) p[w] = red[w][m][r];
+#pragma unroll
+    for (int o = 1; o < NW; o <<= 1)
+#pragma unroll
+      for (int w = 0; w < NW; w += 2 * o) p[w] += p[w + o];
+    float v = a.alpha * p[0];
     if (a.epi == TC5_EPI_PARTIAL) {
       if (n < a.N) a.out[(size_t)blockIdx.y * a.split_stride + (size_t)m * a.ldo + n] = v;
     } else if (a.epi == TC5_EPI_SWIGLU) {

@@ -40,6 +40,22 @@ def test_bf16_rows_on_mma(M, N, K):
     assert _product(M, N, K, C.PREC_BF16, 1) <= 1.0
 
 
+@pytest.mark.parametrize("N,K", [(2048, 2048), (16384, 2048), (4672, 4544)])
+def test_bf16_rows_on_mma_sum_as_exactly_as_single_rows(N, K):
+    """The tensor core adds 16 products at a time; the error of the whole sum stays that of the CUDA-core kernel's chains of
+    FMAs, which a single row takes (each side's 2-norm over some 10^4 outputs: known to a few percent)."""
+    L = nvllm_pkg.sub("lib")
+    g = torch.Generator().manual_seed(N + K)
+    A, B = (torch.randn(*s, generator=g).to(torch.bfloat16).float() for s in ((4, K), (K, N)))
+    ref = A.double() @ B.double()
+
+    def error(rows):
+        out = np.concatenate([L.op_matmul(A[r].numpy(), B.numpy(), prec=C.PREC_BF16, kernel=1)[0] for r in rows])
+        return float((torch.from_numpy(out).double() - ref).norm())
+
+    assert error([slice(0, 4)]) <= 1.1 * error([slice(i, i + 1) for i in range(4)])
+
+
 @pytest.mark.parametrize("lens", [[600], [10] * 40])  # slices of the layers' products; of the head's
 def test_fp32_step_does_not_depend_on_the_steps_before_it(lens):
     """How many k ranges the fp32 products take is decided by the step, not by the room that a larger step left behind."""
