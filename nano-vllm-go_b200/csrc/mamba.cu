@@ -9,8 +9,8 @@
 //                       the SSM state lives per KV BLOCK (handle.h) and is read / written through
 //                       the block table
 //   mamba_gate_norm_kernel  y * silu(gate), RMS norm over E with eps 1e-5, * Norm (:139-173)
-// mamba_conv_kernel and mamba_scan_kernel take the sizes the first two do not: taps other than 4,
-// rows or heads that are no multiples of 16 bytes, states other than 16 / 32 / 64 / 128.
+// mamba_conv_kernel and mamba_scan_kernel take what the first two do not: decode and other short steps (the
+// convolution), taps other than 4, rows or heads that are no multiples of 16 bytes, states other than 16 / 32 / 64 / 128.
 #include "common.cuh"
 #include "kernels.h"
 #include "mma.cuh"
@@ -750,9 +750,17 @@ cudaError_t launch_mamba2_slot_out(cudaStream_t st, int odt, const Mamba2SlotArg
   return cudaGetLastError();
 }
 
+// Windows of rows pay where sequences have several rows and there are some 100 CTAs of them.  Convolution, scan and norm
+// of a step, with a row per CTA against windows, us: decode of 16 / 64 / 128 sequences, 6144 channels, 14.6 / 79 / 137.7
+// against 18.6 / 86 / 139.9, 2304 channels and 64 / 256 sequences 18.6 / 41.8 against 26.9 / 47.5; one prompt of 16 / 64
+// tokens 13.1 / 31.0 against 17.5 / 32.8; from there on windows are ahead (96 CTAs: 128 tokens 53.3 against 52.2, 2304
+// channels and 256 tokens 62.6 against 57; 2048 tokens 709 against 508).
+static bool mamba_conv_rows_fit(const MambaArgs& a) {
+  return a.K == 4 && mamba_rows_aligned(a) && a.T >= 2 * a.n_seqs && ceil_div(a.T, MC_ROWS) * ceil_div(a.conv, 1024) >= 96;
+}
 cudaError_t launch_mamba_conv(cudaStream_t st, const MambaArgs& a) {
   if (a.T <= 0) return cudaSuccess;
-  if (a.K == 4 && mamba_rows_aligned(a)) {
+  if (mamba_conv_rows_fit(a)) {
     const dim3 grid(ceil_div(a.T, MC_ROWS), ceil_div(a.conv, 1024));
     (void)launch_k(mamba_conv_rows_kernel<4>, grid, dim3(256), 0, st, a, next_trace(20));
   } else {

@@ -129,10 +129,11 @@ def test_hybrid_prompts_at_the_edges_of_the_scan_tiles(nh, hd, N, G, K):
 
 
 def test_hybrid_scan_with_sixteen_heads_to_a_cta():
-    """The smallest heads, one group, and so many short prompts that a lane holds two rows of a head: 16 heads per CTA."""
+    """The smallest heads, one group, and so many short prompts that a lane holds two rows of a head: 16 heads per CTA.
+    (771 rows: also enough for the convolution's windows, with several sequences in each.)"""
     cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=64, mamba_head_dim=4,
                         mamba_state_size=16, mamba_n_groups=1, mamba_conv_kernel=4)
-    prompts = [W.random_prompt(cfg.vocab_size, 1 + i % 19, 50 + i) for i in range(75)]
+    prompts = [W.random_prompt(cfg.vocab_size, 1 + i % 21, 50 + i) for i in range(75)]
     _run(cfg, C.PREC_FP32, prompts, 3, [[i] for i in range(75)], 75)
 
 
