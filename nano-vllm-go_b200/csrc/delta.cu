@@ -22,7 +22,8 @@
 //                      double-buffered shared-memory tiles of 16 tokens (cp.async), so the loop
 //                      over tokens never waits for memory.  The state is read from the slot when
 //                      the sequence has earlier tokens (zero otherwise) and written back at the
-//                      end; the sequence's CTAs also roll the convolution tail forward.
+//                      end; the sequence's CTAs also roll the convolution tail forward.  Compile-time sizes:
+//                      delta_scan_columns_kernel, and delta_scan_packed_kernel for many columns.
 //   delta_out_kernel   one CTA per token, a warp per head: RMS over vdim, weight, gate -> act dtype.
 #include <stdlib.h>
 
@@ -395,7 +396,167 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a, int LPC, i
 }
 
 
-// The same scan with compile-time sizes, dim = R * LPC, and packed operations.  Lane p of a column holds the R
+// The same scan with compile-time sizes, dim = R * LPC: lane p of a column holds the R
+// neighbouring rows p R .. p R + R - 1, the keys and queries of a token sit in shared memory as
+// LPC segments of R + 4 floats (the padding puts the lanes' 16-byte reads in different banks),
+// no bounds checks in the token loop, four partial sums per inner product; one column per
+// thread and two CTAs per SM, or two columns per thread (CC = 2) and one.
+template <int R, int LPC, int CC>
+__global__ void __launch_bounds__(256, CC == 1 ? 2 : 1) delta_scan_columns_kernel(DeltaArgs a, int VC, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  constexpr int DIM = R * LPC, RP = R + 4, KL = LPC * RP;
+  const int vdim = a.vdim;
+  const int s = blockIdx.x, h = blockIdx.y, vbase = blockIdx.z * VC;
+  const int r0 = a.cu_q[s], r1 = a.cu_q[s + 1];
+  const int n_new = r1 - r0;
+  const int start = a.positions[r0];
+  float* slot = a.state_pool + (size_t)a.state_slots[s] * a.slot_floats;
+  const int tid = threadIdx.x;
+  const int p = tid % LPC, jl = tid / LPC;  // the thread's CC columns: vbase + jl + cc * (VC / CC)
+  const int VH = VC / CC;
+  bool col_ok[CC];
+  int col[CC];
+#pragma unroll
+  for (int cc = 0; cc < CC; cc++) {
+    col[cc] = vbase + jl + cc * VH;
+    col_ok[cc] = jl < VH && col[cc] < vdim;
+  }
+  const int kvh = h / (a.H / a.G);
+
+  if (a.taps > 1) {  // roll the convolution tail forward (see the generic kernel)
+    float* tail = slot + a.tail_off;
+    const int part = h * gridDim.z + blockIdx.z, parts = a.H * gridDim.z;
+    for (int c = part * blockDim.x + tid; c < a.conv_ch; c += parts * blockDim.x) {
+      float nv[DELTA_MAX_TAPS];
+#pragma unroll
+      for (int j = 0; j < DELTA_MAX_TAPS - 1; j++) {
+        if (j >= a.taps - 1) break;
+        const int q = n_new - (a.taps - 1) + j;
+        if (q >= 0) nv[j] = sum_slices(a.in_p + (size_t)(r0 + q) * a.in_ld + c, a.in_S, a.in_stride);
+        else nv[j] = (start + q >= 0) ? tail[(size_t)(j + n_new) * a.conv_ch + c] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < DELTA_MAX_TAPS - 1; j++) {
+        if (j >= a.taps - 1) break;
+        tail[(size_t)j * a.conv_ch + c] = nv[j];
+      }
+    }
+  }
+
+  float* S_g = slot + a.state_off + (size_t)h * DIM * vdim;
+  float S[CC][R];
+#pragma unroll
+  for (int cc = 0; cc < CC; cc++)
+#pragma unroll
+    for (int r = 0; r < R; r++) S[cc][r] = (start > 0 && col_ok[cc]) ? S_g[(size_t)(p * R + r) * vdim + col[cc]] : 0.f;
+  // tile of DELTA_TT tokens: q [TT][KL], k [TT][KL], v [TT][VC], beta [TT], g [TT]
+  const int tile_floats = DELTA_TT * (2 * KL + VC + 2);
+  const float* qg = a.qkv + (size_t)kvh * DIM;
+  const float* kg = a.qkv + a.n_q + (size_t)kvh * DIM;
+  const float* vg = a.qkv + a.n_q + a.n_k + (size_t)h * vdim + vbase;
+  const int vcn = min(VC, vdim - vbase);
+  auto issue = [&](int t0, int buf) {
+    float* b = sm + buf * tile_floats;
+    const int nt = min(DELTA_TT, n_new - t0);
+    const uint32_t qb = smem_addr(b), kb = smem_addr(b + DELTA_TT * KL), vb = smem_addr(b + 2 * DELTA_TT * KL),
+                   bb = smem_addr(b + DELTA_TT * (2 * KL + VC));
+    for (int i = tid; i < nt * (DIM / 4); i += blockDim.x) {  // 16 bytes at a time: rows and segments are 16-byte aligned
+      const int tt = i / (DIM / 4), d = (i % (DIM / 4)) * 4;
+      const size_t rowo = (size_t)(r0 + t0 + tt) * a.conv_ch;
+      const int so = tt * KL + (d / R) * RP + d % R;
+      cp_async16(qb + 4 * so, qg + rowo + d, true);
+      cp_async16(kb + 4 * so, kg + rowo + d, true);
+    }
+    for (int i = tid; i < nt * vcn; i += blockDim.x) {
+      const int tt = i / vcn, j = i % vcn;
+      cp_async4(vb + 4 * (tt * VC + j), vg + (size_t)(r0 + t0 + tt) * a.conv_ch + j);
+    }
+    for (int i = tid; i < nt * 2; i += blockDim.x) {
+      const int tt = i >> 1, w = i & 1;
+      cp_async4(bb + 4 * (w * DELTA_TT + tt), a.bg + (size_t)(r0 + t0 + tt) * 2 * a.H + w * a.H + h);
+    }
+  };
+  issue(0, 0);
+  cp_async_commit();
+  const int HV = a.H * vdim;
+  float* og = a.o + (size_t)h * vdim;
+  for (int t0 = 0, it = 0; t0 < n_new; t0 += DELTA_TT, it++) {
+    const int buf = it & 1;
+    if (t0 + DELTA_TT < n_new) issue(t0 + DELTA_TT, buf ^ 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    const float* b = sm + buf * tile_floats;
+    const float* qs = b + p * RP;
+    const float* ks = b + DELTA_TT * KL + p * RP;
+    const float* vs = b + 2 * DELTA_TT * KL;
+    const float* bs = b + DELTA_TT * (2 * KL + VC);
+    const int nt = min(DELTA_TT, n_new - t0);
+    for (int tt = 0; tt < nt; tt++) {
+      const float beta = bs[tt], g = bs[DELTA_TT + tt];
+      float v[CC], dot[CC], out[CC];
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) v[cc] = col_ok[cc] ? vs[tt * VC + jl + cc * VH] : 0.f;
+      float kr[R];
+      float d4[CC][4];
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) d4[cc][0] = d4[cc][1] = d4[cc][2] = d4[cc][3] = 0.f;
+#pragma unroll
+      for (int r = 0; r < R; r += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(ks + tt * KL + r);
+        kr[r] = k4.x; kr[r + 1] = k4.y; kr[r + 2] = k4.z; kr[r + 3] = k4.w;
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            S[cc][r + e] *= g;
+            d4[cc][e] = fmaf(S[cc][r + e], kr[r + e], d4[cc][e]);
+          }
+      }
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) {
+        dot[cc] = (d4[cc][0] + d4[cc][1]) + (d4[cc][2] + d4[cc][3]);
+#pragma unroll
+        for (int o = 1; o < LPC; o <<= 1) dot[cc] += __shfl_xor_sync(0xffffffffu, dot[cc], o);
+        dot[cc] = beta * (v[cc] - dot[cc]);  // u: what the token writes into the column
+        d4[cc][0] = d4[cc][1] = d4[cc][2] = d4[cc][3] = 0.f;
+      }
+#pragma unroll
+      for (int r = 0; r < R; r += 4) {
+        const float4 q4 = *reinterpret_cast<const float4*>(qs + tt * KL + r);
+        const float qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int cc = 0; cc < CC; cc++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            S[cc][r + e] = fmaf(kr[r + e], dot[cc], S[cc][r + e]);
+            d4[cc][e] = fmaf(S[cc][r + e], qv[e], d4[cc][e]);
+          }
+      }
+#pragma unroll
+      for (int cc = 0; cc < CC; cc++) {
+        out[cc] = (d4[cc][0] + d4[cc][1]) + (d4[cc][2] + d4[cc][3]);
+#pragma unroll
+        for (int o = 1; o < LPC; o <<= 1) out[cc] += __shfl_xor_sync(0xffffffffu, out[cc], o);
+        if (p == 0 && col_ok[cc]) og[(size_t)(r0 + t0 + tt) * HV + col[cc]] = out[cc];
+      }
+    }
+    __syncthreads();  // the buffer may be refilled
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int cc = 0; cc < CC; cc++)
+    if (col_ok[cc]) {
+#pragma unroll
+      for (int r = 0; r < R; r++) S_g[(size_t)(p * R + r) * vdim + col[cc]] = S[cc][r];
+    }
+  TRACE_EXIT(tr);
+}
+
+// The same for many columns (delta_packed_fits) with packed operations, dim = R * LPC.  Lane p of a column holds the R
 // neighbouring rows p R .. p R + R - 1 of CC neighbouring columns as packed pairs of rows; the keys and queries of a
 // token sit in shared memory as LPC segments of R + 4 floats (the padding puts the lanes' 16-byte reads in different
 // banks).  The inner products of the CC columns are summed by shuffles that scatter them over the lanes.  Three fp32 operations per state entry and token instead of four:
@@ -407,16 +568,10 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a, int LPC, i
 // Bound by fp32 issue and, about equally, by shared-memory reads: a 16-byte read costs its four quarter-warps a pass
 // each even where they read the same bytes, so eight lanes with four columns (28 reads and 12 shuffles for 96
 // packed operations) replace four lanes with two columns.  Four CTAs of 128 threads per SM.  16 sequences of 750 to
-// 1500 tokens, 16 heads of 128 x 128: 1502 us; four scalar operations, one inner product after the other: 1905 us.
+// 1500 tokens, 16 heads of 128 x 128: 1502 us; delta_scan_columns_kernel 1905 us.
 constexpr float DELTA_RESCALE = 1e-18f;
-// a read that is not merged with an earlier one of the same place
-__device__ __forceinline__ ulonglong2 lds_pairs(const float* p) {
-  ulonglong2 v;
-  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(smem_addr(p)));
-  return v;
-}
 template <int R, int LPC, int CC>
-__global__ void __launch_bounds__(128, 4) delta_scan_fixed_kernel(DeltaArgs a, int VC, Trace tr) {
+__global__ void __launch_bounds__(128, 4) delta_scan_packed_kernel(DeltaArgs a, int VC, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
   pdl_wait();
@@ -578,18 +733,15 @@ __global__ void __launch_bounds__(128, 4) delta_scan_fixed_kernel(DeltaArgs a, i
           for (int r = 0; r < R / 2; r++) S[cc][r] = mul2(S[cc][r], mm);
       }
       const float v = CC * jl + mc < vcn ? vs[tt * VC + CC * jl + mc] : 0.f;
-      constexpr bool KEEP = R <= 16;  // keys kept in registers for the update, or read again
-      unsigned long long kr[KEEP ? R / 2 : 1], dk[CC], dq[CC];
+      unsigned long long kr[R / 2], dk[CC], dq[CC];
 #pragma unroll
       for (int cc = 0; cc < CC; cc++) dk[cc] = dq[cc] = 0ull;
 #pragma unroll
       for (int r = 0; r < R / 2; r += 2) {
         const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(ks + tt * KL + 2 * r);
         const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qs + tt * KL + 2 * r);
-        if constexpr (KEEP) {
-          kr[r] = k2.x;
-          kr[r + 1] = k2.y;
-        }
+        kr[r] = k2.x;
+        kr[r + 1] = k2.y;
 #pragma unroll
         for (int cc = 0; cc < CC; cc++) {
           dk[cc] = fma2(S[cc][r], k2.x, dk[cc]);
@@ -636,16 +788,12 @@ __global__ void __launch_bounds__(128, 4) delta_scan_fixed_kernel(DeltaArgs a, i
         wu[cc] = pack2(x, x);
       }
 #pragma unroll
-      for (int r = 0; r < R / 2; r += 2) {
-        ulonglong2 k2;
-        if constexpr (KEEP) k2 = make_ulonglong2(kr[r], kr[r + 1]);
-        else k2 = lds_pairs(ks + tt * KL + 2 * r);
+      for (int r = 0; r < R / 2; r += 2)
 #pragma unroll
         for (int cc = 0; cc < CC; cc++) {
-          S[cc][r] = fma2(k2.x, wu[cc], S[cc][r]);
-          S[cc][r + 1] = fma2(k2.y, wu[cc], S[cc][r + 1]);
+          S[cc][r] = fma2(kr[r], wu[cc], S[cc][r]);
+          S[cc][r + 1] = fma2(kr[r + 1], wu[cc], S[cc][r + 1]);
         }
-      }
     }
     __syncthreads();  // the buffer and the token values may be refilled
   }
@@ -669,33 +817,68 @@ __global__ void __launch_bounds__(128, 4) delta_scan_fixed_kernel(DeltaArgs a, i
 }
 
 template <int R, int LPC, int CC>
-static cudaError_t delta_scan_fixed_launch(cudaStream_t st, const DeltaArgs& a) {
+static cudaError_t delta_scan_packed_launch(cudaStream_t st, const DeltaArgs& a) {
   constexpr int MOST = CC * 128 / LPC;  // columns of 128 threads
   const int VC = std::min(MOST, (a.vdim + CC - 1) / CC * CC);
   const int threads = (VC / CC * LPC + 31) / 32 * 32;
   const dim3 grid(a.n_seqs, a.H, ceil_div(a.vdim, VC));
   const size_t smem = (size_t)2 * DELTA_TT * (2 * LPC * (R + 4) + VC + 2) * sizeof(float);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(delta_scan_fixed_kernel<R, LPC, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(delta_scan_packed_kernel<R, LPC, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(delta_scan_fixed_kernel<R, LPC, CC>, grid, dim3(threads), smem, st, a, VC, next_trace(35));
+  return launch_k(delta_scan_packed_kernel<R, LPC, CC>, grid, dim3(threads), smem, st, a, VC, next_trace(48));
 }
 
+template <int R, int LPC>
+static cudaError_t delta_scan_columns_launch(cudaStream_t st, const DeltaArgs& a) {
+  // two columns per thread (the key / query reads from shared memory, which bound the one-column
+  // form, serve both) when the head has the columns for it
+  const bool cc2 = a.vdim >= 2 * (256 / LPC);
+  const int VC = std::min((cc2 ? 2 : 1) * (256 / LPC), a.vdim);
+  const int threads = cc2 ? 256 : (VC * LPC + 31) / 32 * 32;
+  const dim3 grid(a.n_seqs, a.H, ceil_div(a.vdim, VC));
+  const size_t smem = (size_t)2 * DELTA_TT * (2 * LPC * (R + 4) + VC + 2) * sizeof(float);
+  auto run = [&](auto kernel) -> cudaError_t {
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_k(kernel, grid, dim3(threads), smem, st, a, VC, next_trace(35));
+  };
+  return cc2 ? run(delta_scan_columns_kernel<R, LPC, 2>) : run(delta_scan_columns_kernel<R, LPC, 1>);
+}
+
+// The packed kernel does less work per token, but its chain from one token to the next is longer (two exchanges between
+// lanes more, the multipliers' reads) and several of its small CTAs share an SM even where others are empty: it pays where
+// the columns kernel needs a second wave (one CTA of two columns a thread per SM, two of one column) and the sequences
+// have some tokens.  16 heads, convolution + scan + norm of a layer, us, columns against packed: 128 x 128, 16 sequences
+// of 16 / 64 / 300 tokens 65 / 116 / 504 against 62 / 101 / 427, 32 of 300 994 against 748, but 8 of 300 256 against 321, one
+// of 1100 788 against 1190 (the scan alone), decode of 32 48 against 55; 64 x 64, 32 of 64 / 300 85 / 370 against 79 / 331,
+// 24 of 300 295 against 300, 16 of 300 187 against 232; 48 x 48, 32 of 300 352 against 330.  Heads of 16, 32, 96 and
+// 256 are slower in it at every size (one sequence of 300: 56 against 95, 72 against 134, 133 against 210, 297 against
+// 352; 32 of 300: 138 against 181, 181 against 242, 728 against 842, 4700 against 5550).
+static bool delta_packed_fits(const DeltaArgs& a) {
+  if (a.dim != 48 && a.dim != 64 && a.dim != 128) return false;
+  const bool cc2 = a.vdim >= 128;  // two columns per thread in delta_scan_columns_kernel
+  const long ctas = (long)a.n_seqs * a.H * ceil_div(a.vdim, cc2 ? 128 : 64);
+  return ctas > (cc2 ? 148 : 440) && a.T >= 16 * a.n_seqs;
+}
 cudaError_t launch_delta_scan(cudaStream_t st, const DeltaArgs& a) {
   if (a.n_seqs <= 0) return cudaSuccess;
   if (a.dim > 1024 || a.H % a.G) return cudaErrorInvalidValue;
   // compile-time sizes for the usual head widths (rows of the step's inputs must be 16-byte aligned)
   static const bool fixed_on = !(getenv("NVLLM_DELTA_FIXED") && atoi(getenv("NVLLM_DELTA_FIXED")) == 0);
   if (fixed_on && a.conv_ch % 4 == 0 && a.n_q % 4 == 0 && a.n_k % 4 == 0) {
+    const bool packed = delta_packed_fits(a);
     switch (a.dim) {
-      case 16: return delta_scan_fixed_launch<4, 4, 2>(st, a);
-      case 32: return delta_scan_fixed_launch<4, 8, 4>(st, a);
-      case 48: return delta_scan_fixed_launch<12, 4, 2>(st, a);
-      case 64: return delta_scan_fixed_launch<8, 8, 4>(st, a);
-      case 96: return delta_scan_fixed_launch<12, 8, 4>(st, a);
-      case 128: return delta_scan_fixed_launch<16, 8, 4>(st, a);
-      case 256: return delta_scan_fixed_launch<32, 8, 2>(st, a);
+      case 16: return delta_scan_columns_launch<4, 4>(st, a);
+      case 32: return delta_scan_columns_launch<8, 4>(st, a);
+      case 48: return packed ? delta_scan_packed_launch<12, 4, 2>(st, a) : delta_scan_columns_launch<12, 4>(st, a);
+      case 64: return packed ? delta_scan_packed_launch<8, 8, 4>(st, a) : delta_scan_columns_launch<16, 4>(st, a);
+      case 96: return delta_scan_columns_launch<24, 4>(st, a);
+      case 128: return packed ? delta_scan_packed_launch<16, 8, 4>(st, a) : delta_scan_columns_launch<32, 4>(st, a);
+      case 256: return delta_scan_columns_launch<32, 8>(st, a);
     }
   }
   // registers per thread R and lanes per column LPC (a power of two): R * LPC >= dim

@@ -431,8 +431,8 @@ def test_long_decoding_stays_on_the_reference():
 @gpu
 @pytest.mark.parametrize("dim,vdim", [(16, 17), (32, 64), (48, 130), (64, 66), (96, 9), (128, 128), (256, 34)])
 def test_delta_rule_decays_of_every_strength(dim, vdim):
-    """The compile-time scan keeps the state divided by the product of its decays: heads whose decays are near one, small
-    enough that the product leaves fp32's range several times in a tile of tokens, and zero."""
+    """Heads whose decays are near one, small enough that their product leaves fp32's range several times in a tile of
+    tokens, and zero."""
     j = model([layer(delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=2))])
     cfg, w = random_weights(j, 11)
     w["l0.mix.A_log"] = np.array([-8.0, 1.0, 2.5, 6.0], dtype=np.float32)
@@ -444,6 +444,37 @@ def test_delta_rule_decays_of_every_strength(dim, vdim):
         check(got, want[:50], C.PREC_FP32, "prompt")
         rows = [eng.step([("s", [toks[t]], [0])], decode=True)[0][0] for t in range(50, 75)]
         check(np.stack(rows), want[50:], C.PREC_FP32, "decoded")
+    finally:
+        eng.close()
+
+
+PACKED_SCAN = 48  # its id in the device timeline
+
+
+@gpu
+@pytest.mark.parametrize("dim,vdim,heads", [(48, 130, 12), (48, 3, 36), (64, 66, 18), (64, 128, 12), (128, 9, 36), (128, 128, 12)])
+def test_delta_rule_scan_of_many_columns(dim, vdim, heads):
+    """Enough sequences and heads for the packed scan, which keeps the state divided by the product of its decays: decays as
+    above, sequences around its tile of 16 tokens, column counts off its blocks, a second portion that starts from the
+    slots, and decoding, which another kernel does, on the states that it left."""
+    n, vocab = 13, 211
+    j = model([layer(delta(heads=heads, kv_heads=heads // 3, dim=dim, vdim=vdim, conv=2))], vocab=vocab)
+    cfg, w = random_weights(j, 11)
+    w["l0.mix.A_log"] = np.resize(np.array([-8.0, 1.0, 2.5, 6.0, 0.0], dtype=np.float32), heads)
+    eng = Engine(cfg, w, C.PREC_FP32, num_blocks=n, slots=n)
+    try:
+        toks = prompt(j, 100, 12)
+        want = ref.forward(j, w, toks)  # every sequence is a part of this one
+        lens = [(50, 1, 16, 17, 33, 15, 48, 31, 32, 2, 49, 47, 40)[i] for i in range(n)]
+        for lo, hi in (([0] * n, lens), (lens, [a + 17 + i for i, a in enumerate(lens)])):
+            eng.run.trace_begin(1 << 18)
+            got, _ = eng.step([(str(i), toks[a:b], list(range(b - a))) for i, (a, b) in enumerate(zip(lo, hi))])
+            rec = eng.run.trace_end(1 << 18)
+            assert 0 < len(rec) < 1 << 18 and np.any(rec[:, 1] == PACKED_SCAN)
+            check(got, np.concatenate([want[a:b] for a, b in zip(lo, hi)]), C.PREC_FP32, "prompts")
+        for k in range(3):
+            got, _ = eng.step([(str(i), [toks[b + k]], [0]) for i, b in enumerate(hi)], decode=True)
+            check(got, np.stack([want[b + k] for b in hi]), C.PREC_FP32, "decoded")
     finally:
         eng.close()
 
