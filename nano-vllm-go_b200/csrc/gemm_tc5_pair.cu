@@ -490,8 +490,20 @@ int tc5_pair_init(int dev) {
   d.known = true;
   return n;
 }
-// Token tiles of 256 rows and one k range per tile are taken over, unless rounding the weight tiles up to 256 rows costs
-// more rounds of the persistent schedule than the pair gains (1.15: the smallest gain above at equal rounds).
+// Products of 256-row token tiles with one k range are taken over, where rounding the weight tiles up to 256 rows does not
+// cost more rounds of the persistent schedule than the pair gains:
+//  * epilogues that work on the accumulator (activation, residual, the row scales of a folded norm), for which the pair has
+//    twice the warps: up to 1.15 times the rounds.  All products of a step's layers with these on pairs against
+//    not, 384 to 4544 wide, 520 to 20000 rows: activations 1.06 to 1.6 times as fast, residuals 1.0 to 1.08.  (With more
+//    rounds they lose: Falcon-7B layers, 780 rows 627 us against 590, 2040 rows 1252 against 1220.)
+//  * plain fp32 results: up to 1.1 times the rounds; from 768 of k on, a single round from 3072 of k on.  Time of the
+//    one-CTA kernel over that of pairs, alone with a cold L2, 156 shapes:
+//      k                        512        640        768        1024       2048       4096       8192
+//      one round             .89- .93   .90- .94   .97-1.04   .92-1.00   .97-1.04     1.07
+//      two                   .98-1.02   .99-1.00  1.01-1.03  1.00-1.07  1.02-1.09  1.09-1.10     1.15
+//      three to seven        .92- .99   .93-1.05  1.00-1.06  1.01-1.08  1.05-1.09  1.06-1.09  1.10-1.15
+//      13 rounds for 12      .96- .97                        1.06-1.09  1.04-1.05  1.04-1.06
+//      8 for 7, 9 for 8      .94- .96                        1.03-1.06  1.00-1.04   .98-1.00     1.02
 bool tc5_pair_fits(const Tc5Args& a, int bt, int S) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
@@ -500,6 +512,8 @@ bool tc5_pair_fits(const Tc5Args& a, int bt, int S) {
   const long mt = a.g_experts > 0 ? a.M / PR_BT + a.g_experts : ceil_div(a.M, PR_BT);
   const long one = (mt * ceil_div(a.N, TC_BN) + sms - 1) / sms;
   const long two = (mt * ceil_div(a.N, 2 * TC_BN) + pairs - 1) / pairs;
+  const bool plain = a.epi == TC5_EPI_PARTIAL && !a.rs_ssq;
+  if (plain) return two * 10 <= one * 11 && a.K >= (one > 1 ? 768 : 3072);
   return two * 20 <= one * 23;
 }
 
