@@ -1,7 +1,7 @@
 #!/usr/bin/env python
-"""bench.py — the hot path's headline benchmark (driver contract: see DESIGN.md "Measurement").
+"""bench.py — the hot path's headline benchmark (one JSON line on standard output).
 
-Workload at N=1 (BASELINE.json configs[1]): Llama-3.2-1B (GQA, bf16 weights, fp32 accumulate),
+Workload at N=1: Llama-3.2-1B (GQA, bf16 weights, fp32 accumulate),
 random-init weights, 64 sequences continuously batched: one 64 x 512-token prefill step, then
 256 greedy decode steps.  One bench "step" = that whole job (49152 tokens).  N>1: one replica
 per GPU over disjoint request batches (weak scaling, no data-path collective).
@@ -11,7 +11,7 @@ per GPU over disjoint request batches (weak scaling, no data-path collective).
   e2e    the same job through the C-ABI call nvllm_run with HOST buffers every step
          (token ids / block tables in, sampled tokens out; copies inside the timed region)
   roofline / kernels  per-kernel-class device time from a separate profiled pass of the
-         same job (events around every launch), algorithmic bytes / flops per DESIGN.md
+         same job (events around every launch), algorithmic bytes / flops
   cpu_baseline  the CPU oracle (restated reference, 1 thread) on a bounded sample
 
 `--impl reference` times the reference's CPU algorithm (oracle port; the Go reference cannot be
@@ -48,7 +48,7 @@ def load_peaks():
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons during the timed region (B200_PROFILING.md)."""
+    """nvidia-smi clocks / throttle reasons during the timed region."""
 
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
          "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -102,7 +102,7 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
-# BASELINE.json configs[0..4] (SURVEY.md §8d "Prompts")
+# the five workloads that --config selects
 CONFIGS = {
     1: dict(model="gpt2", batch=1, prompt_len=32, decode_steps=64, shared_prefix=0, tp=False,
             label="configs[0]: 1 sequence, 32-token prompt + 64 greedy decode steps"),
@@ -310,7 +310,7 @@ def gpu_parity(run, ref):
     full model size), last-token logits of every step against the oracle's.  Teacher-forced with
     the ORACLE's greedy tokens, so a near-tie flip (random-init logits are nearly flat) does not
     make the later steps incomparable; every flip is reported with the oracle's own margin
-    between the two tokens.  Gate (BASELINE.json north_star, bf16 mode): max|dlogit| /
+    between the two tokens.  Gate (bf16 mode): max|dlogit| /
     max|logit| <= 2e-2 per step and identical greedy tokens."""
     toks = list(ref["prompt"])
     steps = len(ref["greedy"])
@@ -333,7 +333,7 @@ def gpu_parity(run, ref):
 
 
 def tp_leg(dist, rank, world, device, steps, warmup, barrier):
-    """BASELINE.json configs[3] on ALL ranks of this launch as ONE tensor-parallel group (tp =
+    """Falcon-7B on ALL ranks of this launch as ONE tensor-parallel group (tp =
     world; tp = 1 is the anchor of the strong-scaling curve): Falcon-7B bf16, full depth, one
     2048-token prompt + 32 greedy decode steps, random-init weights drawn on the device.  Then
     the parity check the single-GPU test-suite cannot run at tp > 1: a 2-layer full-width
@@ -949,7 +949,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--config", type=int, default=2, choices=sorted(CONFIGS),
-                    help="BASELINE.json configs[N-1]; the default (2) is the config the metric is quoted on")
+                    help="which of the five workloads; the default (2) is the config the metric is quoted on")
     ap.add_argument("--model", default=None, choices=sorted(C.PRESETS))
     ap.add_argument("--batch", type=int, default=None)
     ap.add_argument("--prompt-len", type=int, default=None)
@@ -1133,7 +1133,7 @@ def main():
                   "prefix_cached_tokens": int(job.num_cached.sum()),
                   "decode_tok_s": job.n * job.D / (t_decode / 1e3) if job.D else None,
                   "decode_us_per_step": 1e3 * t_decode / job.D if job.D else None,
-                  # whole-phase roofline fractions on ALGORITHMIC work (SURVEY.md 8d): prefill
+                  # whole-phase roofline fractions on ALGORITHMIC work: prefill
                   # flops against the sustained bf16 tensor peak, decode bytes (weights + K/V +
                   # logits + one pass over each activation) against the measured HBM peak
                   "prefill_frac_of_tensor_peak":

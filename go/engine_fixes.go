@@ -1,5 +1,5 @@
 // Package nanovllm — engine-side fixes that let the CUDA runner be used at its batch
-// efficiency (SURVEY.md §8f rank 3).  Drop this file next to scheduler.go / llm_engine.go.
+// efficiency.  Drop this file next to scheduler.go / llm_engine.go.
 // Like cuda_model_runner.go it is shipped UNCOMPILED (no Go toolchain in the build image);
 // harness/engine_fixes.py is the same logic in Python, exercised by tests/test_engine_fixes.py
 // (scripted runner on the CPU, the real library on the GPU), and tests/test_go_shim.py checks

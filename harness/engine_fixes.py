@@ -1,4 +1,4 @@
-"""SURVEY.md §8f rank 3 — the engine-side fixes that limit batch efficiency, restated on top of
+"""The engine-side fixes that limit batch efficiency, restated on top of
 the Go bookkeeping of harness/go_engine.py (the Go versions are go/engine_fixes.go; this image
 has no Go toolchain, so the Python mirror is what the GPU tests drive):
 

@@ -6,7 +6,7 @@ toolchain in this image, so to drive the C-ABI library with exactly the inputs
 the Go engine would produce (block tables, NumCachedTokens, prefill-first
 batches, preemption) this module restates that bookkeeping in Python:
 
-  Sequence        /root/reference nanovllm/sequence.go:15-114
+  Sequence        nanovllm/sequence.go:15-114
   SamplingParams  nanovllm/sampling_params.go
   EngineConfig    nanovllm/config.go:9-70
   BlockManager    nanovllm/block_manager.go  (xxhash64 prefix cache, ref-counts)

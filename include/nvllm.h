@@ -10,7 +10,7 @@
  * (go/cuda_model_runner.go) or the ctypes mirror in
  * nano-vllm-go_b200/runner.py binds exactly these symbols.
  *
- * Rules of the boundary (SURVEY.md §8b):
+ * Rules of the boundary:
  *  - the caller owns every host buffer; the library copies what it needs
  *    before returning and retains no caller pointer (cgo rule);
  *  - the library owns device memory, streams, CUDA graphs, NCCL comms;
@@ -54,7 +54,7 @@ enum nvllm_position_type { NVLLM_POS_LEARNED = 0, NVLLM_POS_ROPE = 1, NVLLM_POS_
 enum nvllm_activation_type { NVLLM_ACT_GELU = 0, NVLLM_ACT_SWIGLU = 1 };
 enum nvllm_block_style { NVLLM_BLOCK_SEQUENTIAL = 0, NVLLM_BLOCK_PARALLEL = 1 };
 
-/* Arithmetic mode of the whole forward pass (BASELINE.json north_star):
+/* Arithmetic mode of the whole forward pass:
  *  FP32: fp32 weights / activations / KV, fp32 FMA everywhere. Parity gate
  *        1e-4 relative on logits against the reference's fp32 path.
  *  BF16: bf16 weights and KV cache, fp32 accumulate, fp32 residual stream;
@@ -482,7 +482,7 @@ int nvllm_rerun(nvllm_handle* h, nvllm_run_stats* stats);
  * predecessor's last exit to its own, so the classes add up to the window's device time (CUDA
  * graph replay is off while profiling; up to 2^18 launches per window).  mode 0: off.
  * `bytes` / `flops` are the ALGORITHMIC figures of each launch, `impl_bytes` what this
- * implementation moves on top (DESIGN.md).  nvllm_set_profile resets the counters;
+ * implementation moves on top.  nvllm_set_profile resets the counters;
  * nvllm_get_profile synchronises and fills out[NVLLM_K_COUNT]. */
 enum nvllm_kernel_class {
   NVLLM_K_EMBED = 0,

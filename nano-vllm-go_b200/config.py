@@ -1,6 +1,6 @@
 """Model configuration mirror of the reference's ``tensor.ModelConfig``.
 
-Field meaning follows /root/reference purego/tensor/config.go:58-122; the
+Field meaning follows purego/tensor/config.go:58-122; the
 presets follow config.go:125-148 (GPT-2), :151-193 (Falcon), :330-376
 (Granite-MoE, muP scalars from docs/ARCHITECTURE_GUIDE.md:1773-1776).  The
 Llama-3.2 shapes are the HF config.json values the reference reads at load
@@ -116,7 +116,7 @@ class ModelConfig:
     attention_multiplier: float = 0.0
     residual_multiplier: float = 0.0
     logits_scaling: float = 0.0
-    has_ffn_bias: bool = False  # GPT-2 c_fc/c_proj biases; optional at the boundary (SURVEY §8a quirks)
+    has_ffn_bias: bool = False  # GPT-2 c_fc/c_proj biases; optional at the boundary
     eos_token_id: int = -1
     # Granite-4 hybrid (purego/tensor/config.go:100-115): hybrid_layers[l] = True -> Mamba2 block
     mamba_num_heads: int = 0
@@ -143,7 +143,7 @@ class ModelConfig:
         return self.num_kv_heads
 
     def matmul_params(self) -> int:
-        """Parameters of every matmul touched once per decode step (SURVEY §8 table)."""
+        """Parameters of every matmul touched once per decode step."""
         H, F, L = self.hidden, self.ffn_dim, self.num_layers
         q = self.num_heads * self.head_dim
         kv = self.kv_heads() * self.head_dim

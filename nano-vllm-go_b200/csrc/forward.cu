@@ -659,7 +659,7 @@ int forward_step(nvllm_handle* h) {
 // the duplicate communicator.  Each chunk is a complete forward pass over its rows — causal
 // attention only needs the earlier chunk's K / V of the same layer, handed over by one event
 // per layer — so B's GEMMs run while A's per-layer all-reduce is on the wire and vice versa
-// (SURVEY.md 8e / hard part 3: "token-chunk pipelining").  The persistent GEMM grids leave 16
+// (token-chunk pipelining).  The persistent GEMM grids leave 16
 // SMs to the collective kernels.  Only B holds the sequence's last token: A skips the head.
 // Opt-in: NVLLM_TP_PIPE=1 (read at tp_init; measured slower at tp 2, see tp.cu), threshold
 // NVLLM_TP_PIPE_MIN_T.

@@ -218,7 +218,7 @@ static bool resid_gemm_ok(const nvllm_handle* h, int M, int N, int K, int lda) {
   // Split-K shapes (decode batches) can run the k-splits of an output tile as one thread-block
   // cluster that reduces through distributed shared memory and finishes the residual update
   // itself (gemm_tcgen05.cu) — no norm kernel behind the O and W2 GEMMs.  Parity-green, but
-  // measured SLOWER on cfg2 decode (1150 -> 1195 us/step, DESIGN.md "rejected"): B200 places at
+  // measured SLOWER on cfg2 decode (1150 -> 1195 us/step): B200 places at
   // most 15 clusters of 8 such CTAs (16 tiles need a second wave) so the split drops to 6 = 96
   // CTAs streaming the weights instead of 128, and the in-cluster exchange + reduce costs more
   // than the norm launch it removes.  Opt-in: NVLLM_RESID_CLUSTER=1 (read per step).

@@ -1,5 +1,4 @@
-// mamba.cu — Mamba2 block of the Granite-4 hybrid (SURVEY.md §8f rank 4;
-// purego/tensor/mamba2.go:72-351), for a ragged batch of sequences.  The two projections are
+// mamba.cu — Mamba2 block of the Granite-4 hybrid (purego/tensor/mamba2.go:72-351), for a ragged batch of sequences.  The two projections are
 // ordinary GEMMs (forward.cu); this file holds what sits between them:
 //   mamba_conv_rows_kernel  sum of the in_proj split-K slices, causal conv1d over the xBC columns
 //                       (zero-padded at the start of every CALL, like causalConv1d :209-270 — the

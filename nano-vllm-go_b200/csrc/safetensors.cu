@@ -15,7 +15,7 @@
 // Lookup rules follow the reference: a missing name is retried with a "transformer." prefix
 // (:621-629); norm biases are "<key with .weight -> .bias>" (:601); the FFN biases are looked
 // up as "<FFNUpKey>.bias" = "...c_fc.weight.bias", which no checkpoint has, so GPT-2's MLP
-// biases are never loaded (:559-560 — reproduced on purpose, SURVEY.md §8a "quirks"); a
+// biases are never loaded (:559-560 — reproduced on purpose); a
 // missing lm_head falls back to the tied embedding (:255-259).
 #include <fcntl.h>
 #include <string.h>

@@ -1,4 +1,4 @@
-// tp.cu — tensor-parallel plumbing (SURVEY.md §8e, Falcon-7B): one handle per GPU and per
+// tp.cu — tensor-parallel plumbing (Falcon-7B): one handle per GPU and per
 // process (or per thread), joined in an NCCL communicator over NVLink.  The reference has no
 // distributed code at all (Config.TensorParallelSize is validated and never read,
 // nanovllm/config.go:61-63); the split is Megatron's: Q/K/V and W1 by columns, O and W2 by

@@ -1,4 +1,4 @@
-"""Host-side multi-GPU plumbing (SURVEY.md §8e): one process per GPU under torchrun.
+"""Host-side multi-GPU plumbing: one process per GPU under torchrun.
 
 cfg1-3 / cfg5 are data-parallel replicas over disjoint request sets (no data-path collective);
 cfg4 is one tensor-parallel group whose ranks are fed the SAME requests and joined inside the

@@ -2,7 +2,7 @@
 
 Mirrors, method for method, what the Go engine sees:
 
-  ModelRunner interface        /root/reference nanovllm/model_runner.go:9-16
+  ModelRunner interface        nanovllm/model_runner.go:9-16
       Run(seqs, isPrefill) ([]int, error)        -> run(seqs, is_prefill)
       Close() error                              -> close()
   TensorModelRunner extras     nanovllm/tensor_model_runner.go:35-52,100-111

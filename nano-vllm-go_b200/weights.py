@@ -1,12 +1,12 @@
 """Random-init weights in the reference's POST-LOAD layouts (synthetic data).
 
 Layouts are what ``TransformerModel`` holds after
-/root/reference purego/tensor/generic_loader.go:184-265,353-604: every linear
+purego/tensor/generic_loader.go:184-265,353-604: every linear
 is ``[in, out]`` row-major; Llama W1 is ``[gate | up]`` (``:531-536``); Falcon
 KV is ``[H, 2*hd] = [K | V]`` (``:750-765``); MoE expert tensors keep the HF
 layout ``[E, 2I, H]`` / ``[E, H, I]`` (``:578-586``); router is ``[H, E]``.
 
-Distributions follow SURVEY.md §8d: linear / embedding ~ N(0, 0.02^2), output
+Distributions: linear / embedding ~ N(0, 0.02^2), output
 projections ~ N(0, (0.02/sqrt(2L))^2), norm weight 1 + N(0, 0.02^2), biases
 N(0, 0.02^2).  Each tensor has its own seed so tensors can be generated lazily,
 one at a time, identically for the CUDA library and the CPU oracle.
@@ -127,6 +127,6 @@ def random_weights(cfg: C.ModelConfig, seed: int = 1234,
 
 
 def random_prompt(vocab: int, length: int, seed: int) -> np.ndarray:
-    """Token ids uniform in [0, V) (SURVEY §8d: seed 4321 + sequence index)."""
+    """Token ids uniform in [0, V) (seed 4321 + sequence index)."""
     rng = np.random.default_rng(seed)
     return rng.integers(0, vocab, size=length, dtype=np.int32)

@@ -8,7 +8,7 @@
  *
  * PARITY UNPINNED: the reference (hashneo/nano-vllm-go) is Go and there is no
  * Go toolchain in this image, so the reference itself cannot be run here, and
- * none of its own tests executes a forward pass (SURVEY.md §4/§8c).  What IS
+ * none of its own tests executes a forward pass.  What IS
  * pinned: the Falcon QKV de-interleave KAT (purego/tensor/falcon_split_test.go)
  * and the block-manager / sequence tests (restated in
  * nano-vllm-go_b200/engine.py, checked in tests/).  The numerics below are a
@@ -22,7 +22,7 @@
  * per-element accumulation order, so results equal the scalar Go loops).
  *
  * Every function cites the reference file:line it follows
- * (paths relative to /root/reference).
+ * (paths within its project).
  */
 #include <math.h>
 #include <stdint.h>

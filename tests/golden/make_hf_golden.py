@@ -1,6 +1,6 @@
 """Generate golden last-token logits from HuggingFace transformers (CPU, fp32).
 
-The reference's own tests pin no forward-pass numerics (SURVEY.md §4), and the
+The reference's own tests pin no forward-pass numerics, and the
 reference (Go) cannot run in this image.  As an independent cross-check of the
 oracle we load OUR deterministic random-init weights (nano-vllm-go_b200/weights.py,
 reference post-load layouts) into the matching HF architecture by inverting the

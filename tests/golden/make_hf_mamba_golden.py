@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Golden vector for the Mamba2 block (SURVEY.md §8f rank 4): one GraniteMoeHybridMambaLayer of
+"""Golden vector for the Mamba2 block: one GraniteMoeHybridMambaLayer of
 HF transformers (the implementation Granite-4 checkpoints are published for), pure-PyTorch path
 (`torch_forward`, chunked SSD scan), fp32, on seeded weights and a seeded input.
 

@@ -61,7 +61,7 @@ def make_oracle(cfg, seed=1234, round_bf16=False):
 
 
 def rel_err(a, b):
-    """max |a-b| / max |b| — the gate of BASELINE.json's north_star."""
+    """max |a-b| / max |b| — what parity is gated by."""
     a = np.asarray(a, dtype=np.float64)
     b = np.asarray(b, dtype=np.float64)
     return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-30))

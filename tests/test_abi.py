@@ -96,4 +96,4 @@ def test_noalloc_entry_point_source_allocates_nothing():
     assert "cudaGetSymbolAddress" in code
     hdr = open(HEADER).read()
     m = re.search(r"#define\s+NVLLM_NOALLOC_MAX_SCRATCH_FLOATS\s+\(1\s*<<\s*(\d+)\)", hdr)
-    assert m and int(m.group(1)) == 20  # 4 MiB: the limit DESIGN.md and INTEGRATION.md state
+    assert m and int(m.group(1)) == 20  # 4 MiB: the limit that the documents state

@@ -1,4 +1,4 @@
-"""SURVEY.md §8f rank 3 (engine-side fixes): mixed prefill / decode steps with chunked prompts
+"""Engine-side fixes: mixed prefill / decode steps with chunked prompts
 through the unchanged C ABI, outputs by request, KV-pool sizing from free HBM, block-size check.
 The scheduler logic runs on the CPU against a scripted runner; the GPU test drives the library
 and demands the oracle's greedy tokens."""

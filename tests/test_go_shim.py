@@ -145,7 +145,7 @@ def test_defaults_match_new_tensor_model_runner():
     assert R.DEFAULT_SAMPLING == dict(temperature=1.0, top_p=1.0, top_k=0, repetition_penalty=1.2)
 
 
-# ---- go/engine_fixes.go (SURVEY 8f rank 3): same static discipline
+# ---- go/engine_fixes.go: same static discipline
 FIXES = os.path.join(ROOT, "go", "engine_fixes.go")
 FIX_VARS = {  # variable -> struct of package nanovllm
     "seq": "Sequence", "last": "Sequence", "v": "Sequence", "s": "Scheduler", "config": "Config",

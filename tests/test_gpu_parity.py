@@ -2,7 +2,7 @@
 (include/nvllm.h via nano-vllm-go_b200/lib.py + runner.py), against the CPU oracle on the
 same seeded random-init weights and prompts.
 
-Gates (BASELINE.json north_star / SURVEY.md §8d):
+Gates:
   fp32 mode  max|dlogit| / max|logit| <= 1e-4, greedy tokens identical
   bf16 mode  (weights rounded once to bf16, the same values fed to the oracle as fp32,
               fp32 accumulate) <= 2e-2, greedy tokens identical for 32 steps
@@ -113,7 +113,7 @@ STRICT_SEEDS = {"gpt2": 4322, "llama": 4321, "granite": 4321, "falcon": 4391, "g
 
 def _greedy_parity(name, prec, prompt_len, steps, table=None, strict_seed=None):
     """strict_seed given: FREE-RUNNING — the device's own tokens are fed back, every one of them
-    must equal the oracle's (north_star: identical greedy tokens), logits within the gate at every
+    must equal the oracle's (identical greedy tokens), logits within the gate at every
     step.  Otherwise (kernel-variant coverage on prompts whose margins were not screened): the
     oracle's token is fed back, logits within the gate, and a token may differ only where the
     oracle's own top-2 margin is inside the measured numerical error (reported, never > 2)."""
@@ -163,7 +163,7 @@ def test_fp32_logits_and_greedy_tokens(name):
 
 @pytest.mark.parametrize("name", list(TINY))
 def test_bf16_logits_and_greedy_tokens(name):
-    """north_star: <= 2e-2 and identical greedy tokens for the first 32 steps, free-running."""
+    """<= 2e-2 and identical greedy tokens for the first 32 steps, free-running."""
     _greedy_parity(name, C.PREC_BF16, prompt_len=40, steps=32, strict_seed=STRICT_SEEDS[name])
 
 
@@ -297,7 +297,7 @@ def test_engine_batch_with_prefix_cache(name):
 
 def test_fully_cached_prompt_still_yields_logits():
     """A prompt that is an exact multiple of 256 and fully cached (NumCachedTokens == Len) must
-    still compute its last token (SURVEY.md §7 hard part 2)."""
+    still compute its last token."""
     cfg = TINY["llama"]()
     orc = make_oracle(cfg)
     run = _runner(cfg, C.PREC_FP32)
@@ -580,7 +580,7 @@ def test_profile_reports_every_kernel_class():
 
 
 def test_resident_ragged_batch_stops_at_each_sequences_own_table():
-    """in a ragged batch the shorter table is padded with block 0 on the device; the
+    """In a ragged batch the shorter table is padded with block 0 on the device; the
     resident loop must refuse to step a sequence past ITS OWN table (NVLLM_ERR_RANGE) instead of
     appending its K/V into pool block 0, which here belongs to the other sequence."""
     L = nvllm_pkg.sub("lib")
@@ -636,7 +636,7 @@ def test_resident_ragged_batch_stops_at_each_sequences_own_table():
 
 @pytest.mark.parametrize("batch", [1, 64])
 def test_resident_and_speculative_loops_1000_steps(batch):
-    """the device-resident loop (advance_kernel -> forward pass, captured in
+    """The device-resident loop (advance_kernel -> forward pass, captured in
     a CUDA graph, every kernel released by programmatic dependent launch) against stepping
     through nvllm_run with speculation off, token for token over 1000 steps; then the same loop
     through nvllm_run with the speculative next step on."""

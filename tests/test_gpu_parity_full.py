@@ -1,4 +1,4 @@
-"""GPU parity at the sizes BASELINE.json names (run with -m gpu on a B200).
+"""GPU parity at full sizes (run with -m gpu on a B200).
 
   * configs[0] at FULL size — GPT-2 small 124M, 32-token prompt: fp32 mode <= 1e-4 on every
     step and 64 identical greedy tokens; bf16 mode <= 2e-2 and 32 identical greedy tokens.  Both
@@ -243,7 +243,7 @@ def test_decode_fused_residual_through_cluster_shared_memory(hidden, heads, kv, 
     k-splits as one thread-block cluster per output tile, reduce the slices through distributed
     shared memory and apply the residual update + the folded-norm outputs themselves
     (gemm_tcgen05.cu, TC5_EPI_RESID with S > 1) — no norm kernel in the layer.  Opt-in
-    (NVLLM_RESID_CLUSTER=1: measured slower than partials + norm kernel, DESIGN.md).  Checked
+    (NVLLM_RESID_CLUSTER=1: measured slower than partials + norm kernel).  Checked
     against the oracle (bf16 gate) and against the default path, whose logits must agree to bf16
     noise."""
     cfg = C.tiny_llama(vocab_size=2048, hidden=hidden, num_heads=heads, num_kv_heads=kv, head_dim=64,

@@ -1,4 +1,4 @@
-"""SURVEY.md §8f rank 4 — Granite-4 hybrid (Mamba2 + attention blocks): the CUDA path against the
+"""Granite-4 hybrid (Mamba2 + attention blocks): the CUDA path against the
 oracle's restatement of purego/tensor/mamba2.go (itself pinned to an independent numpy
 restatement in tests/test_oracle.py).  Ragged batches, decode steps that carry the SSM state
 through the per-KV-block snapshots, a sequence crossing a 256-token block boundary."""

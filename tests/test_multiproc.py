@@ -1,6 +1,6 @@
 """world_size-2 gloo tests (CPU) of the N > 1 host logic bench.py runs under torchrun: replica
 vs tensor-parallel planning, disjoint / shared request sets, the broadcast of the group's NCCL
-id, max-over-ranks timing and the whole-job aggregate (SURVEY.md §8e)."""
+id, max-over-ranks timing and the whole-job aggregate."""
 import json
 import os
 import socket

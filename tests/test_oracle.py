@@ -188,7 +188,7 @@ def _np_mamba(cfg, wl, x, state):
 
 
 def test_mamba2_layer_matches_independent_numpy_restatement():
-    """the oracle's Mamba2 layer against a vectorised float64 restatement, a
+    """The oracle's Mamba2 layer against a vectorised float64 restatement, a
     prompt and then single-token steps that carry the SSM state (and re-start the convolution,
     the reference's own behaviour: causalConv1d never reads ConvCache)."""
     cfg = C.tiny_hybrid()

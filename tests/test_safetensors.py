@@ -1,4 +1,4 @@
-"""nvllm_load_safetensors (SURVEY.md §8f-1, the half that needs no Go): checkpoints written in
+"""nvllm_load_safetensors (the half that needs no Go): checkpoints written in
 the HuggingFace layouts of the four families the reference maps (generic_loader.go:60-182) load
 straight into the library and give logits BIT-IDENTICAL to the nvllm_set_weight path fed with
 the reference's post-load layouts of the same weights (so every transpose / fused-QKV split /

@@ -1,7 +1,7 @@
-"""Tensor-parallel parity (SURVEY.md §8e, cfg4): one process per GPU, each holding one rank's
+"""Tensor-parallel parity: one process per GPU, each holding one rank's
 handle, joined through NCCL inside the library.  Every rank must reproduce the single-device
 CPU oracle within the precision's gate.  Needs >= 2 GPUs (skipped on a 1-GPU box):
-  gpurun --gpus 2 -- python -m pytest tests/test_tp.py -m gpu -q
+  python -m pytest tests/test_tp.py -m gpu -q
 """
 import os
 import subprocess
