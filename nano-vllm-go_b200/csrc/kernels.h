@@ -269,7 +269,7 @@ constexpr int GEMV_MMA_ROWS = 2;  // from this many rows on; one row: gemv_kerne
 struct GemvMmaArgs {
   const __nv_bfloat16* A;  // [M, lda], rows 16-byte aligned
   const __nv_bfloat16* W;  // [N, K], K a multiple of 8
-  int lda, M, N, K, KC;    // KC: k range of a split-K slice, a multiple of 32
+  int lda, M, N, K, KC;    // KC: k range of a split-K slice, a multiple of 64
   float* out;              // [S][M][ldo] (TC5_EPI_PARTIAL)
   int ldo;
   size_t split_stride;
