@@ -58,13 +58,13 @@ static SplitRoom split_room(const nvllm_handle* h, int T, int n) {
   return r;
 }
 // The fp32 GEMM takes as many slices as there is room for: a step gets the room that a workspace made for it alone has,
-// so that its sums, which fp32 mode is compared by, don't depend on the steps before it.
+// so that its sums, which fp32 mode is compared by, don't depend on the steps before it.  (The GEMV's slices depend on its
+// sizes only: it may use all that there is.)
 static void fit_split_room(nvllm_handle* h) {
-  if (h->adt != DT_F32) return;
   const SplitRoom r = split_room(h, h->lay.T, std::max(h->lay.n, h->lay.n_out));
-  h->ws.ws_a_floats = r.a;
-  h->ws.ws_b_floats = r.b;
-  h->ws.logits_p_floats = r.head;
+  h->ws.fit_a = r.a;
+  h->ws.fit_b = r.b;
+  h->ws.fit_head = r.head;
 }
 
 int ensure_workspace(nvllm_handle* h, int T, int n) {
@@ -696,6 +696,8 @@ int forward_step_auto(nvllm_handle* h) {
     // split-K partial buffers: one half each
     v.ws_a_floats = W0.ws_a_floats / 2;
     v.ws_b_floats = W0.ws_b_floats / 2;
+    v.fit_a = W0.fit_a / 2;
+    v.fit_b = W0.fit_b / 2;
     if (role == 2) {
       v.ws_a = W0.ws_a + v.ws_a_floats;
       v.ws_b = W0.ws_b + v.ws_b_floats;

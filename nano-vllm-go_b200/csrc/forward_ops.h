@@ -106,6 +106,15 @@ struct RouterArgs {  // expert routing fused into the FFN norm of a MoE layer
                      __FILE__, __LINE__);                                                     \
   } while (0)
 
+// floats that the slices of an fp32 GEMM may take at `out`: as many as in a workspace made for this step (see split_room)
+static size_t split_capacity(const nvllm_handle* h, const float* out, size_t cap) {
+  const Workspace& w = h->ws;
+  if (h->adt != DT_F32) return cap;
+  const bool in_a = out >= w.ws_a && out < w.ws_a + w.ws_a_floats;
+  const size_t at = in_a ? (size_t)(out - w.ws_a) : 0, fit = in_a ? w.fit_a : out == w.logits_p ? w.fit_head : w.fit_b;
+  return std::min(cap, fit > at ? fit - at : 0);
+}
+
 // C = A @ W^T into fp32 split-K partials at `out`
 // epi != 0 asks for the FFN activation to be fused into the GEMM epilogue (bf16 hidden state
 // written to epi_out); granted in bf16 mode to steps of 2 .. 8 rows and, on the tcgen05 path, when the GEMM
@@ -199,7 +208,7 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
   GemmArgs g{};
   g.A = A; g.adt = h->adt; g.lda = lda; g.W = W; g.wdt = h->wdt;
   g.M = M; g.N = N; g.K = K; g.out = out; g.ldo = ldo; g.split_stride = res->stride;
-  g.alpha = alpha; g.out_capacity = cap;
+  g.alpha = alpha; g.out_capacity = split_capacity(h, out, cap);
   ProfScope ps(h, NVLLM_K_GEMM_SIMT, io, flops, a_in + 4.0 * M * N);
   LAUNCH(h, launch_gemm_simt(h->stream, g));
   res->S = g.S;

@@ -154,6 +154,7 @@ struct Workspace {
   float *xn_f32 = nullptr, *xn2_f32 = nullptr;  // [T, H] fp32 normed rows (MoE router input; inputs of the convolutions)
   float *ws_a = nullptr, *ws_b = nullptr, *ws_c = nullptr;
   size_t ws_a_floats = 0, ws_b_floats = 0;
+  size_t fit_a = 0, fit_b = 0, fit_head = 0;  // of ws_a, ws_b / ws_c and logits_p: what a workspace of this step alone has
   void* q = nullptr;         // [T, nh hd]
   void* attn_out = nullptr;  // [T, nh hd]
   void* hbuf = nullptr;      // [T, F] or [T k, I]

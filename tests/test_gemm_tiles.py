@@ -76,6 +76,25 @@ def test_fp32_step_does_not_depend_on_the_steps_before_it(lens):
         run.close()
 
 
+def test_fp32_rows_may_use_the_room_of_an_earlier_step():
+    """Eight decoding sequences of a wide feed-forward: 72 slices of the second product, more than a workspace of eight rows
+    has room for, but the prompts' has."""
+    R = nvllm_pkg.sub("runner")
+    cfg = C.tiny_gpt2(hidden=64, num_heads=4, num_kv_heads=4, head_dim=16, ffn_dim=36864)
+    run = R.CudaModelRunner(cfg, W.random_weights(cfg, 5), precision=C.PREC_FP32, num_kv_blocks=8, sampling=None)
+    prompts = [W.random_prompt(cfg.vocab_size, 90, 60 + i) for i in range(8)]
+    tables, zeros = [[i] for i in range(8)], [0.0] * 8
+    try:
+        toks, _ = run.run_flat(prompts, True, [0] * 8, tables, zeros)
+        texts = [np.append(p, t) for p, t in zip(prompts, toks)]
+        _, eight = run.run_flat(texts, False, None, tables, zeros, want_logits=True)
+        for i in range(8):
+            _, one = run.run_flat([texts[i]], False, None, [tables[i]], [0.0], want_logits=True)
+            assert rel_err(eight[i], one[0]) <= 1e-4
+    finally:
+        run.close()
+
+
 @pytest.mark.parametrize("H", [8, 72, 1024, 2048, 2056, 4544, 8192])
 @pytest.mark.parametrize("layer_norm", [False, True])
 def test_norm_of_many_rows(H, layer_norm):
