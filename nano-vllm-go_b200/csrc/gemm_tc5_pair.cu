@@ -15,8 +15,9 @@
 //
 // Measured inside whole steps, TFLOP/s of all products against the one-CTA kernel: Llama-3.2-1B layers, 64 prompts of 256
 // to 512 tokens 1078 -> 1383; Llama-3.2-3B layers, 7936 rows 1207 -> 1352; Falcon-7B layers, 2048 rows 1278 -> 1386;
-// squared-ReLU layers of 2048 x 12288, 18 k rows 1345 -> 1518; routed experts of 1024 x 512, 150 k rows 783 -> 953.  With
-// four epilogue warps instead of eight the same were 1200, 1292, 1331, 1280 and 781: at 1024 to 2048 of k a tile's
+// squared-ReLU layers of 2048 x 12288, 18 k rows 1345 -> 1518; routed experts of 1024 x 512, 150 k rows 783 -> 953, and
+// 975 with their second product (512 of k) on the one-CTA kernel, where it is now.  With
+// four epilogue warps instead of eight the first five were 1200, 1292, 1331, 1280 and 781: at 1024 to 2048 of k a tile's
 // epilogue took longer than its products.  What bounds it now is the clock under the power limit (tensor pipe 92 %
 // busy at 1.3 GHz in the widest product) and, below 2048 of k, the epilogue.
 //
