@@ -208,7 +208,7 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
   GemmArgs g{};
   g.A = A; g.adt = h->adt; g.lda = lda; g.W = W; g.wdt = h->wdt;
   g.M = M; g.N = N; g.K = K; g.out = out; g.ldo = ldo; g.split_stride = res->stride;
-  g.alpha = alpha; g.out_capacity = split_capacity(h, out, cap);
+  g.alpha = alpha; g.out_capacity = split_capacity(h, out, cap); g.wait_flag = h->waits.dev;
   ProfScope ps(h, NVLLM_K_GEMM_SIMT, io, flops, a_in + 4.0 * M * N);
   LAUNCH(h, launch_gemm_simt(h->stream, g));
   res->S = g.S;

@@ -4,9 +4,8 @@
 //    Weights [N,K] are read exactly once with 16-byte streaming loads (L1 no-allocate), one
 //    warp per R output rows, activations staged in shared memory as fp32, fp32 accumulate.
 //    HBM-bound: algorithmic bytes = N*K*sizeof(W).
-//  * gemm_f32_kernel: register-tiled packed-FMA GEMM.  This is the fp32 PARITY-mode
-//    engine (1e-4 gate: TF32/bf16 tensor cores are not accurate enough) and its grouped
-//    (MoE expert) GEMM with row gather.
+//  * gemm_f32_kernel: register-tiled packed-FMA GEMM of the fp32 PARITY mode for few rows and small weights (the others:
+//    gemm_f32_tc5.cu), and its grouped (MoE expert) GEMM with row gather.
 //  * gemm_simt_kernel: 64x64x16 fp32-FMA tiles on bf16 operands that the tcgen05 path cannot address.
 //
 // All compute C[m,n] = alpha * sum_k A[m,k] * W[n,k]  (reference tensor.go:62-88 MatMul with
@@ -358,9 +357,9 @@ gemm_simt_kernel(GemmArgs g, Trace tr) {
 // memory each, for 8 MI packed FMAs, at MI = 8 48 passes beside 32 cycles of the FMA lanes; with 138 registers three
 // CTAs (nine warps) fit an SM, and both are little more than half busy (57 % and 55 % in a product of 300 x 2304 x 768).
 // MI = 2 / 4 keep tiles of 16 / 32 rows for small steps, which are bound by the weights.
-// GPT-2 small, four prompts of 50 to 100 tokens: the step's 48 matrix products 7.24 -> 2.04 ms against tiles of 64 x 64
-// x 16 with scalar FMAs, operands transposed through registers and one k range (60 to 240 CTAs of the chip's 296); 32
-// TFLOP/s in the widest, three CTAs per SM (four at 128 registers each: 2.50 ms).
+// GPT-2 small, four prompts of 50 to 100 tokens (now on gemm_f32_tc5.cu): the step's 48 matrix products 7.24 -> 2.04 ms
+// against tiles of 64 x 64 x 16 with scalar FMAs, operands transposed through registers and one k range (60 to 240 CTAs of
+// the chip's 296); 32 TFLOP/s in the widest, three CTAs per SM (four at 128 registers each: 2.50 ms).
 constexpr int FG_BN = 64, FG_BK = 32, FG_PITCH = 36, FG_STAGES = 3, FG_THREADS = 128;
 
 template <int MI>
@@ -503,6 +502,7 @@ static cudaError_t launch_gemm_f32(cudaStream_t st, GemmArgs& g) {
 
 cudaError_t launch_gemm_simt(cudaStream_t st, GemmArgs& g) {
   if ((g.K % 8) != 0) return cudaErrorInvalidValue;
+  if (gemm_f32_tc5_fits(g)) return launch_gemm_f32_tc5(st, g);
   if (g.adt == DT_F32 && g.wdt == DT_F32) return launch_gemm_f32(st, g);
   g.S = 1;
   dim3 grid(g.tile_expert ? g.max_tiles : ceil_div(g.M, SBM), ceil_div(g.N, SBN));

@@ -1,5 +1,5 @@
-// gemm_tc5.cuh — what the two tcgen05 GEMM kernels share: the one-CTA kernel of gemm_tcgen05.cu and the
-// CTA-pair kernel of gemm_tc5_pair.cu.
+// gemm_tc5.cuh — what the tcgen05 GEMM kernels share: the one-CTA kernel of gemm_tcgen05.cu, the CTA-pair
+// kernel of gemm_tc5_pair.cu and the fp32 kernel of gemm_f32_tc5.cu.
 #pragma once
 #include <cuda.h>
 
@@ -77,6 +77,38 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
     }
   }
   return v[0];
+}
+// ---- bounded waits: a kernel whose wait ran out raises its caller's flag, lets its copies land and returns
+constexpr unsigned long long TC_WAIT_NS = 2000000000ull, TC_DRAIN_NS = 20000000ull;
+// whole warp; false when the wait ran out (here or anywhere in the CTA)
+__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity, volatile uint32_t* dead, int* flag) {
+  for (int i = 0; i < 64; i++)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const unsigned long long t0 = gtime();
+  for (;;) {
+    for (int i = 0; i < 64; i++)
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const bool over = *dead != 0 || gtime() - t0 > TC_WAIT_NS;
+    if (__any_sync(0xffffffffu, over)) {
+      *dead = 1;
+      *reinterpret_cast<volatile int*>(flag) = 1;
+      return false;
+    }
+  }
+}
+// the N threads of the epilogue warps go on together or not at all (they share barriers further on)
+template <int N>
+__device__ __forceinline__ bool warps_agree(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 4, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"((uint32_t)ok), "n"(N)
+      : "memory");
+  return all != 0;
 }
 // rot: CTAs working on the same k range start at different k-blocks (and wrap), so that at any
 // instant they pull DIFFERENT activation tiles out of L2 — otherwise every CTA of a skinny

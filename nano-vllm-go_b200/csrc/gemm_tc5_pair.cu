@@ -41,41 +41,11 @@ constexpr uint32_t PR_A_BYTES = (PR_BT / 2) * TC_BK * 2; // and its half of the 
 constexpr uint32_t PR_STAGE_BYTES = PR_W_BYTES + PR_A_BYTES;
 constexpr int PR_EPI = 8, PR_THREADS = 64 + 32 * PR_EPI; // epilogue warps: two for each 32 lanes of tensor memory
 constexpr size_t PR_SMEM = (size_t)PR_STAGES * PR_STAGE_BYTES + 1024 + 16 * PR_STAGES + 64;
-constexpr unsigned long long PR_WAIT_NS = 2000000000ull, PR_DRAIN_NS = 20000000ull;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
-}
-// whole warp; false when the wait ran out (here or anywhere in the CTA)
-__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity, volatile uint32_t* dead, int* flag) {
-  for (int i = 0; i < 64; i++)
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  const unsigned long long t0 = gtime();
-  for (;;) {
-    for (int i = 0; i < 64; i++)
-      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    const bool over = *dead != 0 || gtime() - t0 > PR_WAIT_NS;
-    if (__any_sync(0xffffffffu, over)) {
-      *dead = 1;
-      *reinterpret_cast<volatile int*>(flag) = 1;
-      return false;
-    }
-  }
-}
-// the epilogue warps go on together or not at all (they share barriers further on)
-__device__ __forceinline__ bool epilogue_agrees(bool ok) {
-  uint32_t all;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 4, 256, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(all)
-      : "r"((uint32_t)ok)
-      : "memory");
-  return all != 0;
 }
 // a load of this CTA's tile that reports to the barrier of the pair's leader (peer bit of the address cleared)
 __device__ __forceinline__ void tma_load_pair(uint32_t dst, const void* map, uint32_t bar, int c0, int c1, uint64_t policy) {
@@ -291,7 +261,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         for (int c = 0; c < 32; c++) xv[c] = n_ok && m0 + c0 + c < Me ? x[(size_t)c * N] : 0.f;
       };
       if (resid) fetch_x(32 * half);
-      if (!epilogue_agrees(wait_limited(bar_tfull + 8 * buf, (lu >> 1) & 1, dead, flag))) break;
+      if (!warps_agree<256>(wait_limited(bar_tfull + 8 * buf, (lu >> 1) & 1, dead, flag))) break;
       tc_fence_after();
       auto load_acc = [&](int c0, uint32_t (&r)[32]) {
         __syncwarp();  // the load is the whole warp's: lanes past the last column have skipped the previous chunk's stores
@@ -423,7 +393,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   __syncwarp();
   if (*dead) {  // a wait ran out: the copies in flight land before the shared memory is given up
     const unsigned long long t0 = gtime();
-    while (gtime() - t0 < PR_DRAIN_NS) __nanosleep(1000);
+    while (gtime() - t0 < TC_DRAIN_NS) __nanosleep(1000);
   }
   tc_fence_before();
   __syncthreads();

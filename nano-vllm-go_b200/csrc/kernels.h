@@ -239,6 +239,7 @@ struct GemmArgs {
   const int* n_tiles;      // device scalar: number of valid tiles
   size_t expert_stride;    // elements
   int max_tiles;
+  int* wait_flag;          // WaitFlag::dev; null: kernels with bounded waits are not used
 };
 // Single-sequence decode (M <= 8) is a chain of ~100 dependent launches of ~3 us: the W2 GEMV
 // builds its own activation from the W1 GEMV's split-K slices instead of reading what an
@@ -262,6 +263,9 @@ struct GemvPre {
 int gemv_splits(int M, int N, int K);
 cudaError_t launch_gemv(cudaStream_t st, GemmArgs& g, const GemvPre* pre = nullptr);  // M <= 8
 cudaError_t launch_gemm_simt(cudaStream_t st, GemmArgs& g);  // any M (fp32 parity mode, MoE)
+// fp32 on the tensor cores (gemm_f32_tc5.cu); launch_gemm_simt takes it where gemm_f32_tc5_fits
+bool gemm_f32_tc5_fits(const GemmArgs& g);
+cudaError_t launch_gemm_f32_tc5(cudaStream_t st, GemmArgs& g);
 
 // ---------------------------------------------------------------- gemv_mma.cu
 // bf16 activations and weights, 2 <= M <= 8 (launch_gemv takes this path by itself; run_gemm calls it with an epilogue)

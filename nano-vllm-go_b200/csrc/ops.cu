@@ -88,7 +88,7 @@ extern "C" int nvllm_op_matmul(int device, int prec, int kernel, int M, int N, i
     GemmArgs g{};
     g.A = dA; g.adt = dt; g.lda = K; g.W = dWt; g.wdt = dt; g.M = M; g.N = N; g.K = K;
     g.out = dOut; g.ldo = ldo; g.split_stride = (size_t)M * ldo; g.alpha = 1.f;
-    g.out_capacity = cap;
+    g.out_capacity = cap; g.wait_flag = s.waits.dev;
     cudaError_t e = (kernel == 1) ? launch_gemv(s.st, g) : launch_gemm_simt(s.st, g);
     S = g.S;
     return e;

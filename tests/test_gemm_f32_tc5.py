@@ -1,0 +1,79 @@
+"""The fp32 product on split operands (gemm_f32_tc5.cu): against float64 at the edges of its tiles and slices, and with
+operands whose split is not finite."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import C, W
+import nvllm_pkg
+
+L = nvllm_pkg.sub("lib")
+pytestmark = pytest.mark.gpu
+
+KERNEL = 49  # its id in the timeline
+
+
+def _run(A, Wm):
+    """The product and whether this kernel made it."""
+    cfg = C.tiny_gpt2()
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 1), num_kv_blocks=1, sampling=None)
+    try:
+        run.trace_begin(1 << 16)
+        out, _ = L.op_matmul(A, Wm, prec=C.PREC_FP32, kernel=2)
+        rec = run.trace_end(1 << 16)
+    finally:
+        run.close()
+    return out, bool((rec[:, 1] == KERNEL).any())
+
+
+def _operands(M, N, K):
+    g = torch.Generator().manual_seed(M * 31 + N * 7 + K)
+    return torch.randn(M, K, generator=g).numpy(), torch.randn(K, N, generator=g).numpy()
+
+
+def _error(out, A, Wm):
+    """Largest error over its bound: in units of 2^-24 times the sum of the magnitudes of an element's terms, two for each of
+    the 24 tensor-core sums of a stage, one per stage for the fp32 sums, one per slice, and 2 for the parts left out."""
+    a, w = torch.from_numpy(A).cuda().double(), torch.from_numpy(Wm).cuda().double()
+    bound = 2.0 ** -24 * (48 + A.shape[1] / 64 + 8 + 2) * (a.abs() @ w.abs())
+    return float(((torch.from_numpy(out).cuda().double() - a @ w).abs() / bound).max())
+
+
+@pytest.mark.parametrize("M,N,K,tc", [
+    (17, 4096, 256, True),      # the fewest rows, the least k
+    (32, 1001, 1096, True),     # a full tile of 32; N and k off the tiles
+    (33, 130, 264, True),       # one row over; two columns in the second weight tile
+    (64, 768, 768, True),
+    (65, 769, 776, True),
+    (129, 2304, 768, True),     # one row in the last token tile
+    (300, 3072, 768, True),
+    (512, 512, 3080, True),
+    (1500, 5003, 328, True),    # several units per CTA
+    (16, 4096, 256, False),
+    (32, 768, 768, False),      # few rows of small weights
+    (300, 768, 248, False),     # little k
+])
+def test_product(M, N, K, tc):
+    A, Wm = _operands(M, N, K)
+    out, ran = _run(A, Wm)
+    assert _error(out, A, Wm) <= 1.0
+    assert ran == tc
+
+
+@pytest.mark.parametrize("M", [40, 200])
+def test_operands_without_finite_parts(M):
+    A, Wm = _operands(M, 300, 520)
+    A[3, 7], A[5, 100], A[5, 101], A[20, 519] = np.inf, np.inf, -np.inf, np.nan
+    Wm[300, 140] = -np.inf
+    A[9, 64] = 3.4e38  # finite, but not when rounded to bf16
+    A[10, 2] = -3.4e38
+    Wm[64], Wm[2] = Wm[64] * 1e-3, Wm[2] * 1e-3
+    out, ran = _run(A, Wm)
+    assert ran
+    with np.errstate(invalid="ignore"):
+        want = A.astype(np.float64) @ Wm.astype(np.float64)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isnan(out), np.isnan(want))
+    assert np.array_equal(out[~finite & ~np.isnan(want)], want[~finite & ~np.isnan(want)].astype(np.float32))
+    bound = 2.0 ** -24 * 520 * (np.abs(np.where(np.isfinite(A), A, 0)).astype(np.float64) @ np.abs(np.where(np.isfinite(Wm), Wm, 0)))
+    assert (np.abs(out[finite] - want[finite]) <= bound[finite]).all()
