@@ -444,38 +444,39 @@ int forward_step(nvllm_handle* h) {
     // ---- attention sub-block
     if ((rc = tp_reduce_pending(h, &p1, &p2, T))) return rc;
     Pending qkv;
+    void* kp = (char*)h->kpool + (size_t)l * kv_layer_bytes;
+    void* vp = (char*)h->vpool + (size_t)l * kv_layer_bytes;
+    const float *cosT = h->use_rope ? h->cosT : nullptr, *sinT = h->use_rope ? h->sinT : nullptr;
+    const Tc5Heads heads{h->nh, h->nkv, h->hd, d_pos, d_slots, cosT, sinT, (bf16*)kp, (bf16*)vp};
+    const Tc5Heads* hp = is_prefill && h->adt == DT_BF16 && h->kvdt == DT_BF16 && (h->hd == 64 || h->hd == 128) ? &heads : nullptr;
     if (xb_parts > 0 && fold_gemm_ok(h, T, h->qkv_cols, H, H)) {
       RowScale rsc{w.ssq, xb_parts};
       if ((rc = run_gemm(h, w.xb, H, lw.wqkv, T, h->qkv_cols, H, 1.f, w.ws_a, w.ws_a_floats,
-                         h->qkv_cols, &qkv, 0, nullptr, 0, nullptr, nullptr, 0, 0.0, &rsc)))
+                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, nullptr, 0, 0.0, &rsc, nullptr, nullptr, hp, w.q)))
         return rc;
     } else {
       if ((rc = run_norm(h, w.x, &p1, &p2, lw.attn_norm_w, lw.attn_norm_b, w.xn,
                          nullptr, nullptr, T)))
         return rc;
       if ((rc = run_gemm(h, w.xn, H, lw.wqkv, T, h->qkv_cols, H, 1.f, w.ws_a, w.ws_a_floats,
-                         h->qkv_cols, &qkv)))
+                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, nullptr, 0, 0.0, nullptr, nullptr, nullptr, hp, w.q)))
         return rc;
     }
     xb_parts = 0;
-    void* kp = (char*)h->kpool + (size_t)l * kv_layer_bytes;
-    void* vp = (char*)h->vpool + (size_t)l * kv_layer_bytes;
     const bool fuse_rope = !is_prefill && attn_decode_fuses_rope(h->adt, h->kvdt, h->hd);
     if (fuse_rope) {
       at.qkv_p = qkv.p; at.qkv_S = qkv.S; at.qkv_stride = qkv.stride; at.qkv_ld = h->qkv_cols;
       at.qkv_bias = lw.bqkv;
-      at.cosT = h->use_rope ? h->cosT : nullptr;
-      at.sinT = h->use_rope ? h->sinT : nullptr;
-    } else {
+      at.cosT = cosT;
+      at.sinT = sinT;
+    } else if (qkv.S > 0) {
       ProfScope ps(h, NVLLM_K_ROPE_KV,
                    (double)T * h->qkv_cols * 4 + (double)T * h->q_cols * asz +
                        2.0 * T * h->kv_cols * kvsz, 0, (double)T * h->qkv_cols * 4 * (qkv.S - 1));
       LAUNCH(h, launch_rope_kv(st, h->adt, h->kvdt, T, h->nh, h->nkv, h->hd, qkv.p, qkv.S,
-                               qkv.stride, lw.bqkv, d_pos, d_slots,
-                               h->use_rope ? h->cosT : nullptr, h->use_rope ? h->sinT : nullptr, w.q,
-                               kp, vp));
-      if (h->pipe_role == 1) NV_CHECK(h, cudaEventRecord(h->pipe_kv[l], st));
+                               qkv.stride, lw.bqkv, d_pos, d_slots, cosT, sinT, w.q, kp, vp));
     }
+    if (h->pipe_role == 1) NV_CHECK(h, cudaEventRecord(h->pipe_kv[l], st));
     at.kpool = kp;
     at.vpool = vp;
     if (is_prefill) {

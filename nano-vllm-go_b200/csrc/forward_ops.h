@@ -119,12 +119,14 @@ static size_t split_capacity(const nvllm_handle* h, const float* out, size_t cap
 // epi != 0 asks for the FFN activation to be fused into the GEMM epilogue (bf16 hidden state
 // written to epi_out); granted in bf16 mode to steps of 2 .. 8 rows and, on the tcgen05 path, when the GEMM
 // needs no split-K: res->S then comes back 0 (no partials to reduce).
+// heads: the projections of an attention layer (bias: epi_bias); where the product takes the kernel for many rows,
+// its epilogue rotates and places them (queries to q_out) and res->S comes back 0.
 static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int M, int N, int K,
                     float alpha, float* out, size_t cap, int ldo, Pending* res, int epi = 0,
                     void* epi_out = nullptr, int epi_ld = 0, const float* epi_bias = nullptr,
                     const void* pf_ptr = nullptr, size_t pf_bytes = 0, double alg_out = 0.0,
                     const RowScale* rs = nullptr, const Resid* rd = nullptr,
-                    const GemvPre* gp = nullptr) {
+                    const GemvPre* gp = nullptr, const Tc5Heads* heads = nullptr, void* q_out = nullptr) {
   res->p = out;
   res->stride = (size_t)M * ldo;
   const double flops = 2.0 * M * N * K;
@@ -188,6 +190,16 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
     if (M <= 128) {  // weight-streaming regime: warm L2 with the next big matrix
       t.pf_ptr = pf_ptr;
       t.pf_bytes = pf_bytes;
+    }
+    if (heads && t.S == 1) {
+      t.heads = heads; t.epi_out = q_out; t.epi_ld = heads->nh * heads->hd; t.epi_bias = epi_bias;
+      if (tc5_pair_fits(t, tc5_box_rows_act(M), 1)) {
+        ProfScope ps(h, NVLLM_K_GEMM_TC5, io, flops, a_in + 2.0 * M * N);
+        LAUNCH(h, launch_gemm_tc5(h->stream, t, nullptr));
+        res->S = 0;
+        return NVLLM_OK;
+      }
+      t.heads = nullptr; t.epi_out = nullptr; t.epi_bias = nullptr;
     }
     const long tiles = (long)ceil_div(N, 128) * ceil_div(M, tc5_box_rows_act(M));
     if (epi && (t.S == 1 || 2 * tiles >= h->sm_count)) {

@@ -40,6 +40,7 @@ constexpr uint32_t PR_W_BYTES = TC_BN * TC_BK * 2;       // of one CTA: its 128 
 constexpr uint32_t PR_A_BYTES = (PR_BT / 2) * TC_BK * 2; // and its half of the token rows
 constexpr uint32_t PR_STAGE_BYTES = PR_W_BYTES + PR_A_BYTES;
 constexpr int PR_EPI = 8, PR_THREADS = 64 + 32 * PR_EPI; // epilogue warps: two for each 32 lanes of tensor memory
+constexpr int HEADS_TOKENS = 16, HEADS_PITCH = TC_BN + 4;
 constexpr size_t PR_SMEM = (size_t)PR_STAGES * PR_STAGE_BYTES + 1024 + 16 * PR_STAGES + 64;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -97,10 +98,14 @@ __device__ __forceinline__ Tc5Unit pair_unit(const Tc5Sched& sc, int u, int M, i
 __global__ void __launch_bounds__(PR_THREADS, 1)
 gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, int M, int N, Tc5Sched sc,
                      float* __restrict__ out, int ldo, float alpha, int w_reused, int epi, bf16* __restrict__ epi_out,
-                     int epi_ld, const float* __restrict__ epi_bias, Tc5Fuse fz, int* flag, Trace tr) {
+                     int epi_ld, const float* __restrict__ epi_bias, Tc5Fuse fz, Tc5Heads hs, int* flag, Trace tr) {
   const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
   unsigned long long t_wait = 0;
-  __shared__ __align__(16) uint8_t epi_stage[PR_EPI][32 * 48];
+  __shared__ __align__(16) union {
+    uint8_t act[PR_EPI][32 * 48];
+    float heads[2][HEADS_TOKENS][HEADS_PITCH];
+  } epi_stage;
+  __shared__ int pos_s[2][PR_BT], slot_s[2][PR_BT];
   __shared__ float rstd_s[2][PR_BT];
   __shared__ float ssq_s[2][2][4][32];  // [half][chunk parity]
   __shared__ uint32_t dead_s;
@@ -247,8 +252,15 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
           }
           w[c] = 1.0f / sqrtf(ssum * fz.rs_inv_h + fz.rs_eps);
         }
-        named_bar(1, 32 * PR_EPI);
+        if (!hs.hd) named_bar(1, 32 * PR_EPI);
         rs = w;
+      }
+      if (hs.hd) {
+        for (int c = et; c < PR_BT && m0 + c < Me; c += 32 * PR_EPI) {
+          pos_s[buf][c] = __ldcg(hs.positions + m0 + c);
+          slot_s[buf][c] = __ldcg(hs.slots + m0 + c);
+        }
+        named_bar(1, 32 * PR_EPI);
       }
       const int n = n0 + q * 32 + lane;
       const bool n_ok = n < N;
@@ -271,7 +283,93 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
           for (int c = 0; c < 32; c++) r[c] = __float_as_uint(__uint_as_float(r[c]) * rs[c0 + c]);
         }
       };
-      if (epi == TC5_EPI_PARTIAL) {
+      if (hs.hd) {
+        // Query, key and value heads, instead of fp32 sums that a kernel of their own reads back: 24.4 k rows of 32 + 16
+        // heads of 64, K = 2048: 229 us and 151-169 for that kernel -> one product of 206 (whole steps: Llama-3.2-1B layers,
+        // 64 prompts 11.58 -> 11.14 ms; 3B layers, 4 k rows 3.93 -> 3.73; 18.7 k rows of 16 + 16 heads 5.17 -> 4.97): bias, rotation of the halves of a head (rope.go), bf16; queries to epi_out, keys and
+        // values to their pages.  A head's halves are in the accumulators of different warps, so 16 tokens at a time go
+        // through shared memory; there a thread takes eight entries of either half of one token's head.
+        float (*stg)[HEADS_PITCH] = epi_stage.heads[half];
+        const int tid = et & 127, tt = tid >> 3, g = tid & 7, hd = hs.hd, hh = hd == 64 ? g >> 2 : 0;
+        const int j = hd == 64 ? (g & 3) * 8 : g * 8;      // entry of the half
+        const int col = hh * 64 + j, swap = hh;            // (odd heads read their second 16 bytes first: other banks)
+        const int head = (n0 + hh * 64) / hd;
+        const bool is_v = head >= hs.nh + hs.nkv, live = head < hs.nh + 2 * hs.nkv;
+        const bool rot = hs.cosT && !is_v && live;
+        float ba[8], bb[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) ba[i] = bb[i] = 0.f;
+        if (epi_bias && live) {
+          load8(epi_bias + n0 + col, ba);
+          load8(epi_bias + n0 + col + hd / 2, bb);
+        }
+        float cs[8], sn[8];
+        auto fetch_rotation = [&](int c) {  // of the coming token
+          if (rot && m0 + c < Me) {
+            const size_t at = (size_t)pos_s[buf][c] * (hd / 2) + j;
+            load8(hs.cosT + at, cs);
+            load8(hs.sinT + at, sn);
+          }
+        };
+        fetch_rotation(32 * half + tt);
+#pragma unroll 1
+        for (int c0 = 32 * half; c0 < PR_BT && m0 + c0 < Me; c0 += 64) {
+          uint32_t r[32];
+          load_acc(c0, r);
+#pragma unroll
+          for (int s = 0; s < 32; s += HEADS_TOKENS) {
+#pragma unroll
+            for (int c = 0; c < HEADS_TOKENS; c++) stg[c][q * 32 + lane] = alpha * __uint_as_float(r[s + c]);
+            named_bar(2 + half, 128);
+            const int c = c0 + s + tt, m = m0 + c;
+            if (live && m < Me) {
+              float a[8], b[8];
+#pragma unroll
+              for (int i = 0; i < 2; i++) {
+                const int o = 4 * (i ^ swap);
+                const float4 va = *reinterpret_cast<const float4*>(&stg[tt][col + o]);
+                const float4 vb = *reinterpret_cast<const float4*>(&stg[tt][col + hd / 2 + o]);
+                const int e = 4 * i;
+                a[e] = va.x; a[e + 1] = va.y; a[e + 2] = va.z; a[e + 3] = va.w;
+                b[e] = vb.x; b[e + 1] = vb.y; b[e + 2] = vb.z; b[e + 3] = vb.w;
+              }
+              if (swap) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                  const float ta = a[i], tb = b[i];
+                  a[i] = a[i + 4]; a[i + 4] = ta;
+                  b[i] = b[i + 4]; b[i + 4] = tb;
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                a[i] += ba[i];
+                b[i] += bb[i];
+              }
+              if (rot) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                  const float ra = a[i] * cs[i] - b[i] * sn[i], rb = b[i] * cs[i] + a[i] * sn[i];
+                  a[i] = ra;
+                  b[i] = rb;
+                }
+              }
+              bf16* dst;
+              if (head < hs.nh) {
+                dst = epi_out + (size_t)m * epi_ld + head * hd + j;
+              } else {
+                const int slot = slot_s[buf][c], kvh = head - hs.nh - (is_v ? hs.nkv : 0);
+                dst = (is_v ? hs.vpool : hs.kpool) + (((size_t)(slot / KV_BLOCK) * hs.nkv + kvh) * KV_BLOCK + slot % KV_BLOCK) * hd + j;
+              }
+              store8(dst, a);
+              store8(dst + hd / 2, b);
+            }
+            const int cn = s == 0 ? c + HEADS_TOKENS : c + 64 - HEADS_TOKENS;
+            if (cn < PR_BT) fetch_rotation(cn);
+            named_bar(2 + half, 128);
+          }
+        }
+      } else if (epi == TC5_EPI_PARTIAL) {
 #pragma unroll 1
         for (int c0 = 32 * half; c0 < PR_BT && m0 + c0 < Me; c0 += 64) {
           uint32_t r[32];
@@ -291,7 +389,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         // interleaved gate / up rows (weights.cu): even lane = gate j, odd lane = up j; the pair splits the 32 tokens.
         // Staged per warp in shared memory ([32 tokens][16 columns], rows 48 B apart) for 16-byte stores.
         const int odd = lane & 1, p = lane >> 1;
-        uint8_t* stg = epi_stage[warp - 2];
+        uint8_t* stg = epi_stage.act[warp - 2];
         const int j0 = (n0 + q * 32) >> 1;
 #pragma unroll 1
         for (int c0 = 32 * half; c0 < PR_BT && m0 + c0 < Me; c0 += 64) {
@@ -464,7 +562,8 @@ int tc5_pair_init(int dev) {
 // Products of 256-row token tiles with one k range are taken over, where rounding the weight tiles up to 256 rows does not
 // cost more rounds of the persistent schedule than the pair gains:
 //  * epilogues that work on the accumulator (activation, residual, the row scales of a folded norm), for which the pair has
-//    twice the warps: up to 1.15 times the rounds.  All products of a step's layers with these on pairs against
+//    twice the warps, and attention projections, which save the launch that would rotate and place them: up to 1.15 times
+//    the rounds.  All products of a step's layers with these on pairs against
 //    not, 384 to 4544 wide, 520 to 20000 rows: activations 1.06 to 1.6 times as fast, residuals 1.0 to 1.08.  (With more
 //    rounds they lose: Falcon-7B layers, 780 rows 627 us against 590, 2040 rows 1252 against 1220.)
 //  * plain fp32 results: up to 1.1 times the rounds; from 768 of k on, a single round from 3072 of k on.  Time of the
@@ -483,7 +582,7 @@ bool tc5_pair_fits(const Tc5Args& a, int bt, int S) {
   const long mt = a.g_experts > 0 ? a.M / PR_BT + a.g_experts : ceil_div(a.M, PR_BT);
   const long one = (mt * ceil_div(a.N, TC_BN) + sms - 1) / sms;
   const long two = (mt * ceil_div(a.N, 2 * TC_BN) + pairs - 1) / pairs;
-  const bool plain = a.epi == TC5_EPI_PARTIAL && !a.rs_ssq;
+  const bool plain = a.epi == TC5_EPI_PARTIAL && !a.rs_ssq && !a.heads;
   if (plain) return two * 10 <= one * 11 && a.K >= (one > 1 ? 768 : 3072);
   return two * 20 <= one * 23;
 }
@@ -493,6 +592,7 @@ cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDes
   cudaGetDevice(&dev);
   const int pairs = g_pair_dev[dev].pairs;
   if (pairs <= 0 || !a.wait_flag) return cudaErrorInvalidValue;
+  if (a.heads && (a.epi != TC5_EPI_PARTIAL || !a.epi_out || a.g_experts > 0 || (a.heads->hd != 64 && a.heads->hd != 128))) return cudaErrorInvalidValue;
   if (a.epi == TC5_EPI_RESID && (!a.res_x || !a.res_xb || !a.res_ssq || a.g_experts > 0)) return cudaErrorInvalidValue;
   Tc5Sched sc{};
   sc.nkb_total = sc.kbps = ceil_div(a.K, TC_BK);
@@ -515,7 +615,8 @@ cudaError_t launch_gemm_tc5_pair(cudaStream_t st, const Tc5Args& a, const TmaDes
                    a.res_ssq_ld, a.res_bias, a.res_m, a.res_g, 0, a.glu_limit};
   return launch_k_cluster(gemm_tc5_pair_kernel, dim3(2 * n), dim3(PR_THREADS), PR_SMEM, st, 2,
                           *reinterpret_cast<const CUtensorMap*>(tw), *reinterpret_cast<const CUtensorMap*>(ta), a.M, a.N, sc,
-                          a.out, a.ldo, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias, fz, a.wait_flag,
+                          a.out, a.ldo, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias, fz,
+                          a.heads ? *a.heads : Tc5Heads{}, a.wait_flag,
                           next_trace(46));
 }
 

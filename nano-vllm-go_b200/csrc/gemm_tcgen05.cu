@@ -1013,7 +1013,9 @@ cudaError_t launch_gemm_tc5(cudaStream_t st, const Tc5Args& a, int* S_out) {
       default: return cudaErrorInvalidValue;
     }
   }
-  if (tc5_pair_fits(a, bt, S)) {
+  const bool pair = tc5_pair_fits(a, bt, S);
+  if (a.heads && !pair) return cudaErrorInvalidValue;
+  if (pair) {
     const TmaDesc* half = cached_map(a.A, a.M, a.K, bt / 2);
     return half ? launch_gemm_tc5_pair(st, a, tw, half) : cudaErrorInvalidValue;
   }

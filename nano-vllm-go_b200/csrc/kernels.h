@@ -310,6 +310,13 @@ struct WaitFlag {
   void raise();  // from the host (tests of the error path)
   bool take();   // after a synchronise: did a wait run out since the last call?
 };
+// Where the plain sums of an attention layer's projections go: the columns are nh query, nkv key and nkv value heads of hd = 64 or 128
+struct Tc5Heads {
+  int nh, nkv, hd;
+  const int *positions, *slots;  // [M] of the rows
+  const float *cosT, *sinT;      // [max_pos, hd / 2], or null: no rotation
+  bf16 *kpool, *vpool;           // the layer's pages
+};
 struct Tc5Args {
   const void* A;  // activations [M, K] bf16, K contiguous
   const void* W;  // weights     [N, K] bf16, K contiguous
@@ -363,6 +370,8 @@ struct Tc5Args {
   const int* g_tile_rows;
   const int* g_n_tiles;  // [1] on the device
   int* wait_flag;        // WaitFlag::dev; null: kernels with bounded waits are not used
+  const Tc5Heads* heads; // TC5_EPI_PARTIAL, the pair kernel only: instead of fp32 sums, heads with epi_bias added, rotated and
+                         // rounded to bf16; queries to epi_out [M, epi_ld], keys and values to their pages
 };
 // TC5_EPI_RELU2: like TC5_EPI_GELU (bf16 activation written, no bias needed) with relu(h)^2
 enum { TC5_EPI_PARTIAL = 0, TC5_EPI_SWIGLU = 1, TC5_EPI_GELU = 2, TC5_EPI_RESID = 3, TC5_EPI_RELU2 = 4 };
