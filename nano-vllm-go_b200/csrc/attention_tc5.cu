@@ -12,24 +12,35 @@
 // transform of every score in the softmax warps (tried: 3.5 to 5.7 ms against 0.97 ms plain, 16 x 4096 tokens,
 // 16 heads of 64) made this kernel slower than those.
 //
-// One CTA = 128 queries of one sequence x one query head; the SM holds two such CTAs, so that
-// one's softmax runs under the other's MMAs.  Per key tile j (BN keys):
-//   TMA warp      K_j / V_j tiles of the paged pool (one (block, kv head) slab is contiguous;
-//                 2-D tensor map over the layer's pool, SWIZZLE_128B) -> shared memory
-//   MMA warp      S = Q K_j^T   (128 x BN, K-major x K-major, accumulator in TMEM)
-//                 O_j = P_j V_j (128 x hd; P from shared memory, V as the MN-major operand —
+// Persistent, two CTAs per SM: an item is 128 queries of one sequence x one query head, dealt out by a counter, heaviest
+// first.  Per key tile (BN keys):
+//   scheduler     the next items' rows, positions and key tiles, up to four ahead
+//   TMA warp      Q of the item, K / V tiles of the paged pool (one (block, kv head) slab is contiguous;
+//                 2-D tensor map over the layer's pool, SWIZZLE_128B) -> shared memory, two stages each
+//   MMA warp      S = Q K^T   (128 x BN, K-major x K-major, accumulator in TMEM), issued as soon as the softmax warps
+//                 have the tile before in registers
+//                 O += P V    (128 x hd; P from tensor memory, V as the MN-major operand —
 //                 the pool keeps V [key][hd], so no transpose anywhere)
 //   softmax warps thread r owns query row r (TMEM lane r): the S row is read into registers
 //                 once (all tcgen05.ld issued, one wait), row max, exp2 / row sum, bf16 P
-//                 written in the swizzled K-major operand layout.  O stays in TMEM across the
+//                 back to tensor memory.  O stays in TMEM across the
 //                 tiles (accumulating MMAs); it is rescaled there only when the running
 //                 maximum has grown by more than a factor 2^8 ("lazy" flash rescaling), and
-//                 read once at the end — nothing but P and the final output leaves the SM
+//                 read once, under the next item's first tile — nothing but the final output leaves the SM
+// Bound by the softmax warps of the SM's two CTAs: row maximum and 128 exp2 a row take 2400 cycles a tile of 128 keys where
+// the special-function units alone would take 1024 of each, and 2600 an item go to its hand-over (prompts of 256 to 512
+// tokens, 2.1 tiles an item).  With one CTA per item, S only after the P V before it and P through shared memory (which
+// costs a proxy fence): 4150 a tile and 4000 an item.  Per launch, 64 such prompts, 32 heads of 64: 255 -> 195 us; 16 heads
+// 73 -> 58; 16 x 256 queries on 3840 cached keys, 24 heads of 128: 409 -> 348 (711 -> 834 TFLOP/s); one prompt of 2048, 71
+// heads of 64: 97 -> 86.
 #include <cuda.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
+#include "gemm_tc5.cuh"
 #include "tc5.cuh"
 #include "tma.cuh"
 
@@ -38,24 +49,28 @@ namespace nvllm {
 namespace {
 
 constexpr int PT_BM = 128;       // queries per CTA (UMMA M)
-constexpr int PT_THREADS = 256;  // warps 0-3 softmax (warpgroup 0), warp 4 TMA, warp 5 MMA, 6-7 idle
+constexpr int PT_THREADS = 256;  // warps 0-3 softmax (warpgroup 0), warp 4 TMA, warp 5 MMA, warp 6 scheduler, 7 idle
+constexpr int PT_ITEMS = 4;      // items known ahead
+
+// a query tile of one head: its first row and query position, rows in use, key tiles (0: no more items)
+struct PtItem {
+  int seq, head, row, pos, rows, n_tiles;
+};
 
 template <int HD>
 struct PtCfg {
   static constexpr int BN = HD == 64 ? 128 : 64;  // keys per tile
-  static constexpr int KST = 2;                    // K stages
+  static constexpr int ST = 2;                     // stages of K and of V
   static constexpr int SUB = HD / 64;              // 64-column (128-byte) sub-tiles of a head row
   static constexpr uint32_t Q_BYTES = PT_BM * HD * 2;
   static constexpr uint32_t KV_BYTES = BN * HD * 2;
-  static constexpr uint32_t P_BYTES = PT_BM * BN * 2;
-  static constexpr uint32_t TILES = Q_BYTES + KST * KV_BYTES + KV_BYTES + P_BYTES;
-  static constexpr uint32_t SMEM = 1024 + TILES + 128;
-  static constexpr uint32_t TMEM_COLS = 256;  // S: BN columns at 0, O: HD columns at BN
+  static constexpr uint32_t TILES = Q_BYTES + 2 * ST * KV_BYTES;
+  static constexpr uint32_t SMEM = TILES + 512;    // barriers, items, tensor-memory address
+  static constexpr uint32_t TMEM_COLS = 256;       // S: BN columns at 0, O: HD columns at BN, P: BN / 2 columns behind
+  static_assert(BN + HD + BN / 2 <= 256, "two CTAs share the tensor memory");
+  static_assert(2 * (SMEM + 1024) <= 233472, "and the shared memory");
 };
 
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -70,53 +85,54 @@ __global__ void __launch_bounds__(PT_THREADS, 2)
 attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, AttnArgs a, Trace tr) {
   using Cf = PtCfg<HD>;
-  constexpr int BN = Cf::BN, SUB = Cf::SUB, KST = Cf::KST;
+  constexpr int BN = Cf::BN, SUB = Cf::SUB, ST = Cf::ST;
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];  // (no static shared memory in front of it)
+  const uint32_t base = smem_u32(smem_raw);
   const uint32_t sQ = base;
   const uint32_t sK = sQ + Cf::Q_BYTES;
-  const uint32_t sV = sK + KST * Cf::KV_BYTES;
-  const uint32_t sP = sV + Cf::KV_BYTES;
-  const uint32_t bars = sP + Cf::P_BYTES;
-  // barriers: q_full, k_full[2], k_empty[2], v_full, v_empty, s_full, p_ready, o_full
-  const uint32_t b_qfull = bars, b_kfull = bars + 8, b_kempty = bars + 24, b_vfull = bars + 40,
-                 b_vempty = bars + 48, b_sfull = bars + 56, b_pready = bars + 64, b_ofull = bars + 72;
-  const uint32_t tmem_slot = bars + 80;
-  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-
+  const uint32_t sV = sK + ST * Cf::KV_BYTES;
+  const uint32_t bars = sV + ST * Cf::KV_BYTES;
+  const uint32_t b_qfull = bars, b_qempty = bars + 8, b_kfull = bars + 16, b_kempty = bars + 32, b_vfull = bars + 48,
+                 b_vempty = bars + 64, b_sfull = bars + 80, b_sread = bars + 88, b_pready = bars + 96, b_ofull = bars + 104,
+                 b_ifull = bars + 112, b_iempty = bars + 112 + 8 * PT_ITEMS;
+  uint8_t* tail = smem_raw + Cf::TILES + 112 + 16 * PT_ITEMS;
+  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(tail);
+  volatile uint32_t* dead = reinterpret_cast<uint32_t*>(tail + 4);
+  PtItem* items = reinterpret_cast<PtItem*>(tail + 16);
+  static_assert(112 + 16 * PT_ITEMS + 16 + PT_ITEMS * sizeof(PtItem) <= 512, "the tail of the shared memory");
+  if (base & 1023) {  // (the swizzle's atoms would not line up; the host's layout rules this out)
+    if (threadIdx.x == 0 && a.wait_flag) *reinterpret_cast<volatile int*>(a.wait_flag) = 1;
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heaviest tiles (latest queries of a sequence see the most keys) first
-  const int tile = a.n_qtiles - 1 - (int)blockIdx.x, head = blockIdx.y;
-  const int seq = a.tile_seq[tile], q0 = a.tile_q0[tile];
-  const int row0 = a.cu_q[seq];
-  const int n_new = a.cu_q[seq + 1] - row0;
-  const int start = a.seq_start[seq];
-  const int kvh = head / (a.nh / a.nkv);
-  const int rows_valid = min(PT_BM, n_new - q0);
-  const int kv_end = start + q0 + rows_valid;  // keys [0, kv_end) are visible to this tile
-  const int n_tiles = (kv_end + BN - 1) / BN;
-  const int* bt = a.block_tables + (size_t)seq * a.max_blocks;
 
   if (warp == 4 && lane == 0) {
     mbar_init(b_qfull, 1);
-    for (int s = 0; s < KST; s++) {
+    mbar_init(b_qempty, 1);
+    for (int s = 0; s < ST; s++) {
       mbar_init(b_kfull + 8 * s, 1);
       mbar_init(b_kempty + 8 * s, 1);
+      mbar_init(b_vfull + 8 * s, 1);
+      mbar_init(b_vempty + 8 * s, 1);
     }
-    mbar_init(b_vfull, 1);
-    mbar_init(b_vempty, 1);
     mbar_init(b_sfull, 1);
-    mbar_init(b_pready, 4);  // one arrival per softmax warp
+    mbar_init(b_sread, 4);   // one arrival per softmax warp
+    mbar_init(b_pready, 4);
     mbar_init(b_ofull, 1);
+    for (int s = 0; s < PT_ITEMS; s++) {
+      mbar_init(b_ifull + 8 * s, 1);
+      mbar_init(b_iempty + 8 * s, 6);  // TMA, MMA and softmax warps
+    }
+    *dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmQ) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmK) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmV) : "memory");
   }
   if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot_ptr)),
                  "r"(Cf::TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -125,38 +141,89 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  const uint32_t tS = tmem_base, tO = tmem_base + BN;
+  const uint32_t tS = tmem_base, tO = tmem_base + BN, tP = tO + HD;
+  auto wait = [&](uint32_t bar, int parity) { return wait_short(bar, (uint32_t)parity & 1, dead, a.wait_flag); };
+  // item `it` once it is known (n_tiles == 0: there are no more); false when the wait ran out
+  auto next_item = [&](int it, PtItem& w) {
+    const int s = it % PT_ITEMS;
+    if (!wait(b_ifull + 8 * s, it / PT_ITEMS)) return false;
+    w = items[s];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(b_iempty + 8 * s);
+    return true;
+  };
 
   if (warp >= 4) {
-    // warpgroup 1 (TMA warp 4, MMA warp 5, two idle warps) hands its registers to the softmax
+    // warpgroup 1 (TMA warp 4, MMA warp 5, scheduler warp 6, an idle warp) hands its registers to the softmax
     // warpgroup, whose threads carry a whole fp32 output row
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 4) {
-      // ---------------------------------------------------------------- TMA producer
-      pdl_wait();  // Q and this step's K / V rows are the previous kernels' output
-      if (elect_one()) {
-        mbar_expect_tx(b_qfull, Cf::Q_BYTES);
-        for (int s = 0; s < SUB; s++)
-          tma_load_2d(sQ + s * (PT_BM * 128), &tmQ, b_qfull, head * HD + 64 * s, row0 + q0);
+    // Q and this step's K / V rows are the previous kernels' output (and the limit of the waits counts from here)
+    pdl_wait();
+    if (warp == 6) {
+      // ---------------------------------------------------------------- scheduler
+      const int n_items = a.n_qtiles * a.nh, grid = (int)gridDim.x;
+      int t = blockIdx.x;
+      for (int it = 0;; it++) {
+        int draw = 0;  // the item after this one
+        if (t < n_items && lane == 0) draw = a.tickets ? grid + atomicAdd(a.tickets, 1) : t + grid;
+        PtItem w{};
+        if (t < n_items) {
+          // heaviest tiles (latest queries of a sequence see the most keys) first, the heads of a tile next to each other
+          const int tile = a.n_qtiles - 1 - t / a.nh;
+          w.head = t % a.nh;
+          w.seq = a.tile_seq[tile];
+          const int q0 = a.tile_q0[tile], first = a.cu_q[w.seq];
+          w.row = first + q0;
+          w.rows = min(PT_BM, a.cu_q[w.seq + 1] - first - q0);
+          w.pos = a.seq_start[w.seq] + q0;
+          w.n_tiles = (w.pos + w.rows + BN - 1) / BN;  // keys [0, pos + rows) are visible to this tile
+        }
+        const int s = it % PT_ITEMS;
+        if (!wait(b_iempty + 8 * s, it / PT_ITEMS + 1)) break;
+        if (elect_one()) {
+          items[s] = w;
+          mbar_arrive(b_ifull + 8 * s);
+        }
+        __syncwarp();
+        if (w.n_tiles == 0) break;
+        draw = __shfl_sync(0xffffffffu, draw, 0);
+        // the counter is zero again for the next launch: n_items draws in all, of each CTA one past the end
+        if (a.tickets && draw - grid == n_items - 1 && lane == 0) *a.tickets = 0;
+        t = draw;
       }
-      __syncwarp();
-      for (int j = 0; j < n_tiles; j++) {
-        const int k0 = j * BN;
-        const int prow = (bt[k0 / KV_BLOCK] * a.nkv + kvh) * KV_BLOCK + (k0 % KV_BLOCK);
-        const int ks = j % KST;
-        if (j >= KST) mbar_wait(b_kempty + 8 * ks, ((j / KST) & 1) ^ 1);
+    } else if (warp == 4) {
+      // ---------------------------------------------------------------- TMA producer
+      int g = 0;  // key tiles so far
+      bool ok = true;
+      for (int it = 0; ok; it++) {
+        PtItem w;
+        if (!next_item(it, w) || w.n_tiles == 0) break;
+        const int* bt = a.block_tables + (size_t)w.seq * a.max_blocks;
+        const int kvh = w.head / (a.nh / a.nkv);
+        if (it > 0 && !wait(b_qempty, it - 1)) break;
         if (elect_one()) {
-          mbar_expect_tx(b_kfull + 8 * ks, Cf::KV_BYTES);
-          for (int s = 0; s < SUB; s++)
-            tma_load_2d(sK + ks * Cf::KV_BYTES + s * (BN * 128), &tmK, b_kfull + 8 * ks, 64 * s, prow);
+          mbar_expect_tx(b_qfull, Cf::Q_BYTES);
+          for (int s = 0; s < SUB; s++) tma_load_2d(sQ + s * (PT_BM * 128), &tmQ, b_qfull, w.head * HD + 64 * s, w.row);
         }
         __syncwarp();
-        if (j >= 1) mbar_wait(b_vempty, (j & 1) ^ 1);
-        if (elect_one()) {
-          mbar_expect_tx(b_vfull, Cf::KV_BYTES);
-          for (int s = 0; s < SUB; s++) tma_load_2d(sV + s * (BN * 128), &tmV, b_vfull, 64 * s, prow);
+        for (int j = 0; j < w.n_tiles; j++, g++) {
+          const int k0 = j * BN, st = g % ST;
+          const int prow = (bt[k0 / KV_BLOCK] * a.nkv + kvh) * KV_BLOCK + (k0 % KV_BLOCK);
+          if (!(ok = wait(b_kempty + 8 * st, g / ST + 1))) break;
+          if (elect_one()) {
+            mbar_expect_tx(b_kfull + 8 * st, Cf::KV_BYTES);
+            for (int s = 0; s < SUB; s++)
+              tma_load_2d(sK + st * Cf::KV_BYTES + s * (BN * 128), &tmK, b_kfull + 8 * st, 64 * s, prow);
+          }
+          __syncwarp();
+          if (!(ok = wait(b_vempty + 8 * st, g / ST + 1))) break;
+          if (elect_one()) {
+            mbar_expect_tx(b_vfull + 8 * st, Cf::KV_BYTES);
+            for (int s = 0; s < SUB; s++)
+              tma_load_2d(sV + st * Cf::KV_BYTES + s * (BN * 128), &tmV, b_vfull + 8 * st, 64 * s, prow);
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
     } else if (warp == 5) {
       // ---------------------------------------------------------------- MMA issuer
@@ -166,45 +233,61 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                                    ((uint32_t)(PT_BM >> 4) << 24);
       constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
                                    ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(PT_BM >> 4) << 24);
-      mbar_wait(b_qfull, 0);
-      for (int j = 0; j < n_tiles; j++) {
-        const int ks = j % KST;
-        mbar_wait(b_kfull + 8 * ks, (j / KST) & 1);
+      auto scores = [&](int g, bool last) {
+        const int st = g % ST;
+        if (!wait(b_kfull + 8 * st, g / ST)) return false;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
           for (int s = 0; s < SUB; s++) {
             const uint64_t qd = make_smem_desc(sQ + s * (PT_BM * 128));
-            const uint64_t kd = make_smem_desc(sK + ks * Cf::KV_BYTES + s * (BN * 128));
+            const uint64_t kd = make_smem_desc(sK + st * Cf::KV_BYTES + s * (BN * 128));
 #pragma unroll
             for (int kk = 0; kk < 4; kk++) tc_mma_bf16(tS, qd + 2 * kk, kd + 2 * kk, idesc_s, (s | kk) != 0);
           }
-          tc_commit(b_kempty + 8 * ks);
+          tc_commit(b_kempty + 8 * st);
           tc_commit(b_sfull);
+          if (last) tc_commit(b_qempty);  // the next item's queries may come
         }
         __syncwarp();
-        mbar_wait(b_pready, j & 1);  // P_j is in shared memory; S_j and O_{j-1} have been read
-        mbar_wait(b_vfull, j & 1);
-        tc_fence_after();
-        if (elect_one()) {
+        return true;
+      };
+      int g = 0;
+      bool ok = true;
+      PtItem w, wn;
+      if (!next_item(0, w)) w.n_tiles = 0;
+      for (int it = 0; ok && w.n_tiles > 0; it++, w = wn) {
+        const int n_tiles = w.n_tiles;
+        // (the previous item's last S has been read: its P V came after)
+        if (!wait(b_qfull, it) || !scores(g, n_tiles == 1)) break;
+        for (int j = 0; j < n_tiles; j++, g++) {
+          // under the softmax of this tile: S of the next one, or what the next item is (its S ahead of this item's last
+          // P V: 216 us instead of 198 in the prompts below)
+          if (j + 1 < n_tiles) ok = wait(b_sread, g) && scores(g + 1, j + 2 == n_tiles);
+          else ok = next_item(it + 1, wn);
+          const int st = g % ST;
+          // P_j is in tensor memory, its O there may be written
+          if (!(ok = ok && wait(b_vfull + 8 * st, g / ST) && wait(b_pready, g))) break;
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BN / 16; kk++) {
-            const uint64_t pd = make_smem_desc(sP + (kk / 4) * (PT_BM * 128)) + 2 * (kk % 4);
-            const uint64_t vd = make_smem_desc_mn(sV + kk * 2048, BN * 128);
-            tc_mma_bf16(tO, pd, vd, idesc_o, (j | kk) != 0);
+            for (int kk = 0; kk < BN / 16; kk++) {
+              const uint64_t vd = make_smem_desc_mn(sV + st * Cf::KV_BYTES + kk * 2048, BN * 128);
+              tc_mma_bf16_ta(tO, tP + 8 * kk, vd, idesc_o, (j | kk) != 0);
+            }
+            tc_commit(b_vempty + 8 * st);
+            tc_commit(b_ofull);
           }
-          tc_commit(b_vempty);
-          tc_commit(b_ofull);
+          __syncwarp();
         }
-        __syncwarp();
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax + output
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    pdl_wait();
     const int q = warp;  // TMEM lane quadrant of this warp
     const int r = q * 32 + lane;
-    const int qpos = start + q0 + r;
     constexpr float LOG2E = 1.4426950408889634f;
     const float sl2 = a.scale * LOG2E;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
@@ -213,37 +296,98 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     // 2^RESCALE_LOG2 in probability — then, and only then, O (TMEM) and l are rescaled; in
     // between, p = exp2(s - m_used) may exceed 1 by at most that factor, harmless in fp32 / bf16.
     constexpr float RESCALE_LOG2 = 8.f;
-    float m_used = -INFINITY, l_run = 0.f;
-    for (int j = 0; j < n_tiles; j++) {
-      const int k0 = j * BN;
-      // the warp's rows see every key of the tile when its last key <= the first row's position
-      const bool need_mask = (k0 + BN - 1) > (start + q0 + q * 32);
-      mbar_wait(b_sfull, j & 1);  // also: every earlier P V MMA has retired (in-order pipe)
-      tc_fence_after();
-      // the whole S row of this tile in registers: all loads issued, one wait
-      uint32_t sr[BN];
+    int g = 0;
+    bool ok = true;
+    // the finished item whose O waits in tensor memory
+    bf16* o_row = nullptr;
+    float o_inv = 0.f;
+    bool o_pending = false;
+    auto output = [&] {
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD; c0 += 32) {
+        uint32_t rr[32];
+        tmem_ld_32x32(tO + lane_off + (uint32_t)c0, rr);
+        if (o_row) {
 #pragma unroll
-      for (int c0 = 0; c0 < BN; c0 += 32) tmem_ld_32x32_nowait(tS + lane_off + (uint32_t)c0, &sr[c0]);
-      tmem_ld_wait();
-      float mx = -INFINITY;
-      if (need_mask) {
+          for (int c = 0; c < 32; c += 8) {
+            float v[8];
 #pragma unroll
-        for (int c = 0; c < BN; c++) {
-          if (k0 + c > qpos) sr[c] = 0xff800000u;  // -inf: p = 0
-          mx = fmaxf(mx, __uint_as_float(sr[c]));
+            for (int i = 0; i < 8; i++) v[i] = __uint_as_float(rr[c + i]) * o_inv;
+            store8(o_row + c0 + c, v);
+          }
         }
-      } else {
-#pragma unroll
-        for (int c = 0; c < BN; c++) mx = fmaxf(mx, __uint_as_float(sr[c]));
       }
-      // rows of the tile that see no key yet (mx = -inf) keep their reference
-      const bool grow = (mx - m_used) * sl2 > RESCALE_LOG2 || (m_used == -INFINITY && mx > -INFINITY);
-      if (__any_sync(0xffffffffu, grow)) {
+      __syncwarp();
+      o_pending = false;
+    };
+    for (int it = 0; ok; it++) {
+      PtItem w;
+      if (!(ok = next_item(it, w)) || w.n_tiles == 0) break;
+      const int n_tiles = w.n_tiles;
+      float m_used = -INFINITY, l_run = 0.f;
+      for (int j = 0; j < n_tiles; j++, g++) {
+        // columns of this tile up to which the warp's first row sees keys (its last row: 31 more)
+        const int lim = w.pos + q * 32 - j * BN;
+        if (!(ok = wait(b_sfull, g))) break;
+        tc_fence_after();
+        // the whole S row of this tile in registers: all loads issued, one wait
+        uint32_t sr[BN];
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 32) tmem_ld_32x32_nowait(tS + lane_off + (uint32_t)c0, &sr[c0]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_sread);
+        float mx = -INFINITY;
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          if (c0 > lim + 31) continue;  // no row of the warp sees these keys: p = 0 below
+          if (c0 + 31 > lim) {
+#pragma unroll
+            for (int c = 0; c < 32; c++)
+              if (c0 + c > lim + lane) sr[c0 + c] = 0xff800000u;  // -inf: p = 0
+          }
+          float m[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) m[c] = __uint_as_float(sr[c0 + c]);
+#pragma unroll
+          for (int c = 4; c < 32; c++) m[c & 3] = fmaxf(m[c & 3], __uint_as_float(sr[c0 + c]));
+          mx = fmaxf(mx, fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])));
+        }
+        // rows of the tile that see no key yet (mx = -inf) keep their reference
+        const bool grow = (mx - m_used) * sl2 > RESCALE_LOG2 || (m_used == -INFINITY && mx > -INFINITY);
         const float m_new = grow ? mx : m_used;
         const float corr = (m_used == -INFINITY) ? 0.f : ex2((m_used - m_new) * sl2);
-        l_run *= corr;
+        const bool rescale = __any_sync(0xffffffffu, grow);
+        if (rescale) l_run *= corr;
         m_used = m_new;
-        if (j > 0) {  // tile 0's P V overwrites O: nothing to rescale yet
+        const float mb = (m_used == -INFINITY) ? 0.f : m_used * sl2;
+        const unsigned long long sl2_2 = pack2(sl2, sl2), mb_2 = pack2(-mb, -mb);
+        float sum = 0.f;
+        uint32_t pk[BN / 2];
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          if (c0 > lim + 31) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) pk[(c0 + c) / 2] = 0;
+            continue;
+          }
+#pragma unroll
+          for (int c = 0; c < 32; c += 2) {
+            float p0, p1;
+            unpack2(fma2(pack2(__uint_as_float(sr[c0 + c]), __uint_as_float(sr[c0 + c + 1])), sl2_2, mb_2), p0, p1);
+            p0 = ex2(p0);
+            p1 = ex2(p1);
+            sum += p0 + p1;
+            __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+            pk[(c0 + c) / 2] = *reinterpret_cast<uint32_t*>(&b2);
+          }
+        }
+        l_run += sum;
+        // the P V before has retired: P may be overwritten, and O rescaled or read
+        if (g > 0 && !(ok = wait(b_ofull, g - 1))) break;
+        tc_fence_after();
+        if (rescale && j > 0) {  // tile 0's P V overwrites O: nothing to rescale yet
 #pragma unroll 1
           for (int c0 = 0; c0 < HD; c0 += 32) {
             uint32_t rr[32];
@@ -254,61 +398,34 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           }
           tmem_st_wait();
         }
+        if (o_pending) output();
+#pragma unroll
+        for (int c = 0; c < BN / 2; c += 32)
+          tmem_st_32x32(tP + lane_off + (uint32_t)c, reinterpret_cast<const uint32_t(&)[32]>(pk[c]));
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_pready);
       }
-      const float mb = (m_used == -INFINITY) ? 0.f : m_used * sl2;
-      float sum = 0.f;
-#pragma unroll
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t pk[16];
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          const float p0 = ex2(fmaf(__uint_as_float(sr[c0 + c]), sl2, -mb));
-          const float p1 = ex2(fmaf(__uint_as_float(sr[c0 + c + 1]), sl2, -mb));
-          sum += p0 + p1;
-          __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
-          pk[c >> 1] = *reinterpret_cast<uint32_t*>(&b2);
-        }
-        const uint32_t prow_addr = sP + (uint32_t)(c0 >> 6) * (PT_BM * 128) + (uint32_t)r * 128;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const uint32_t ch = (uint32_t)(((c0 & 63) >> 3) + i);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow_addr + ((ch ^ (uint32_t)(r & 7)) << 4)),
-                       "r"(pk[4 * i]), "r"(pk[4 * i + 1]), "r"(pk[4 * i + 2]), "r"(pk[4 * i + 3])
-                       : "memory");
-        }
-      }
-      l_run += sum;
-      tc_fence_before();
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(b_pready);
+      if (!ok) break;
+      if (OPT && a.sink && m_used > -INFINITY)  // the sink: a term of the denominator without key or value
+        l_run += ex2((a.sink_w ? a.sink_w[w.head] : 0.f) * LOG2E - m_used * sl2);
+      o_inv = 1.0f / l_run;
+      if (OPT && a.head_gate && r < w.rows) o_inv *= a.head_gate[(size_t)(w.row + r) * a.gate_ld + w.head];
+      o_row = r < w.rows ? (bf16*)a.out + (size_t)(w.row + r) * a.nh * HD + (size_t)w.head * HD : nullptr;
+      o_pending = true;
     }
-    // o_full completes once per tile and is only waited for here.  s_full of the last tile
-    // implied that P V of tile n_tiles - 2 had retired, so the barrier is at least in phase
-    // n_tiles - 1 now and the parity test below can only pass on the last tile's completion.
-    mbar_wait(b_ofull, (n_tiles - 1) & 1);
-    tc_fence_after();
-    if (OPT && a.sink && m_used > -INFINITY)  // the sink: a term of the denominator without key or value
-      l_run += ex2((a.sink_w ? a.sink_w[head] : 0.f) * LOG2E - m_used * sl2);
-    float inv = 1.0f / l_run;
-    if (OPT && a.head_gate && r < rows_valid) inv *= a.head_gate[(size_t)(row0 + q0 + r) * a.gate_ld + head];
-    bf16* op = (bf16*)a.out + (size_t)(row0 + q0 + r) * a.nh * HD + (size_t)head * HD;
-#pragma unroll 1
-    for (int c0 = 0; c0 < HD; c0 += 32) {
-      uint32_t rr[32];
-      tmem_ld_32x32(tO + lane_off + (uint32_t)c0, rr);
-      if (r < rows_valid) {
-#pragma unroll
-        for (int c = 0; c < 32; c += 8) {
-          float v[8];
-#pragma unroll
-          for (int i = 0; i < 8; i++) v[i] = __uint_as_float(rr[c + i]) * inv;
-          store8(op + c0 + c, v);
-        }
-      }
+    if (ok && o_pending && wait(b_ofull, g - 1)) {
+      tc_fence_after();
+      output();
     }
-    tc_fence_before();
   }
+  __syncwarp();
+  if (*dead) {  // a wait ran out: the copies in flight land before the shared memory is given up
+    const unsigned long long t0 = gtime();
+    while (gtime() - t0 < TC_DRAIN_NS) __nanosleep(1000);
+  }
+  tc_fence_before();
   __syncthreads();
   if (warp == 5) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
@@ -339,7 +456,8 @@ static cudaError_t prefill_tc5_launch(cudaStream_t st, const AttnArgs& a) {
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  (void)launch_k(attn_prefill_tc5_kernel<HD, OPT>, dim3(a.n_qtiles, a.nh), dim3(PT_THREADS), Cf::SMEM, st,
+  const int ctas = std::min(a.n_qtiles * a.nh, 2 * std::max(1, a.sm_count));
+  (void)launch_k(attn_prefill_tc5_kernel<HD, OPT>, dim3(ctas), dim3(PT_THREADS), Cf::SMEM, st,
                  *reinterpret_cast<const CUtensorMap*>(tq), *reinterpret_cast<const CUtensorMap*>(tk),
                  *reinterpret_cast<const CUtensorMap*>(tv), a, next_trace(13));
   return cudaGetLastError();

@@ -398,6 +398,8 @@ int forward_step(nvllm_handle* h) {
   at.pool_blocks = h->num_blocks;
   at.total_rows = h->view_T > 0 ? h->view_T : T;
   at.sm_count = h->sm_count;
+  at.tickets = (int*)w.chain_ctr + (h->pipe_role == 2 ? 32 : 16);  // (two chunks of a step may be in flight)
+  at.wait_flag = h->waits.dev;
   if (!is_prefill)
     at.n_splits = attn_decode_splits(h->adt, h->kvdt, n, h->nh, h->nkv, h->hd, L.max_len, h->sm_count);
   const double qo_bytes = 2.0 * T * h->q_cols * asz;

@@ -1287,6 +1287,7 @@ static int mixer_attention(nvllm_handle* h, const ListedLayer& y, int run_idx, P
       t.cu_q = a.cu_q; t.seq_start = a.seq_start; t.seq_len = a.seq_len;
       t.tile_seq = a.tile_seq; t.tile_q0 = a.tile_q0; t.n_qtiles = L.n_qtiles;
       t.pool_blocks = h->num_blocks; t.total_rows = T; t.sm_count = h->sm_count;
+      t.tickets = (int*)w.chain_ctr + 16; t.wait_flag = h->waits.dev;
       t.sink = s.sink; t.sink_w = a.sink_w;
       t.head_gate = s.head_gate ? w.att_gate : nullptr; t.gate_ld = s.heads;
       LAUNCH(h, launch_attn_prefill_tc5(h->stream, t));

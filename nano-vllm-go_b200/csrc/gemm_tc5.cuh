@@ -82,19 +82,25 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
 constexpr unsigned long long TC_WAIT_NS = 2000000000ull, TC_DRAIN_NS = 20000000ull;
 // whole warp; false when the wait ran out (here or anywhere in the CTA)
 __device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity, volatile uint32_t* dead, int* flag) {
+#pragma unroll 1
   for (int i = 0; i < 64; i++)
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const unsigned long long t0 = gtime();
   for (;;) {
+#pragma unroll 1
     for (int i = 0; i < 64; i++)
       if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     const bool over = *dead != 0 || gtime() - t0 > TC_WAIT_NS;
     if (__any_sync(0xffffffffu, over)) {
       *dead = 1;
-      *reinterpret_cast<volatile int*>(flag) = 1;
+      if (flag) *reinterpret_cast<volatile int*>(flag) = 1;
       return false;
     }
   }
+}
+// the same for short paths: a wait that need not wait costs little more than the test
+__device__ __forceinline__ bool wait_short(uint32_t bar, uint32_t parity, volatile uint32_t* dead, int* flag) {
+  return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || wait_limited(bar, parity, dead, flag);
 }
 // the N threads of the epilogue warps go on together or not at all (they share barriers further on)
 template <int N>

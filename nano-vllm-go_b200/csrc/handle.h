@@ -167,7 +167,9 @@ struct Workspace {
   // per-column-tile row sums of squares [parts][T_cap] of it
   void* xb = nullptr;
   float* ssq = nullptr;
-  unsigned* chain_ctr = nullptr;  // [2] counters of the chained W1 -> W2 GEMM launch (zero between launches)
+  // zero between launches: [0, 2) counters of the chained W1 -> W2 GEMM launch, [16] and [32] (second chunk of a step) those
+  // that deal out the items of the prefill attention
+  unsigned* chain_ctr = nullptr;
   float* logits_p = nullptr; // [S][n][ldl]
   float* logits = nullptr;   // [n][ldl]  (tp > 1: [tp][n][Vl], rank-major slices)
   float* tp_buf = nullptr;   // [T, H] fp32 partial sums handed to the all-reduce (tp > 1)

@@ -431,9 +431,8 @@ struct AttnArgs {
   const float* cosT;      // [max_pos, hd/2] or null (no RoPE)
   const float* sinT;
   int newkv_off;          // set by the launcher: smem offset of the new K / V rows
-  // stream-K decode (attention_mma.cu): ticket per (seq, kv head, head chunk), zero between
-  // kernels; total_tiles = host LOWER bound of the key tiles in the step (caps the grid)
-  int* tickets;        // unused (stream-K experiment removed)
+  int* tickets;        // tcgen05 prefill kernel: counter that deals its items out, zero between kernels (null: in turn)
+  int* wait_flag;      // WaitFlag::dev of its waits
   // options of the tcgen05 prefill kernel (all zero / null: plain causal softmax)
   int sink;                // 1: the softmax denominator holds one more term, exp(sink_w[h]) (exp(0) without sink_w)
   const float* sink_w;     // [nh] or null
@@ -442,7 +441,6 @@ struct AttnArgs {
   int pool_blocks;     // blocks in the layer's K / V pool (tensor-map extent)
   int total_rows;      // rows of q / out in this step (tensor-map extent; tcgen05 prefill kernel)
   int sm_count;
-  long long total_tiles;
 };
 constexpr int ATTN_PREFILL_QTILE = 32;  // SIMT (fp32 parity) kernel; the mma kernel uses 64
 // queries per tile of the kernel launch_attn_prefill will pick: the host builds tile_seq /

@@ -155,7 +155,9 @@ static int check_waits(nvllm_handle* h) {
   if (!h->waits.take()) return NVLLM_OK;
   h->resident_ok = h->run_lay_ok = h->spec_pending = false;
   h->fetched_rows = 0;
-  return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a GEMM ran out");
+  // kernels that gave up may have left their counters anywhere
+  if (h->ws.chain_ctr) NV_CHECK(h, cudaMemsetAsync(h->ws.chain_ctr, 0, 256, h->stream));
+  return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a kernel ran out");
 }
 static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, const int32_t* block_tables,
                           const int32_t* cu_blocks) {
