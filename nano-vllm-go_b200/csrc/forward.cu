@@ -374,6 +374,13 @@ int forward_step(nvllm_handle* h) {
   // tests switch it).
   const char* gpre_env = getenv("NVLLM_GEMV_PRE");
   const bool gpre_act = !(gpre_env && atoi(gpre_env) == 0) && T <= 8 && !h->moe;
+  // Steps of one bf16 row: norms in front of the products, residual updates behind them (sequential blocks)
+  const bool one_row = T == 1 && h->adt == DT_BF16 && h->wdt == DT_BF16 && !h->parallel && h->tp == 1 && gemv_row_fits(H);
+  auto row_args = [&](const void* A, const void* W, int N, int K, int epi, const float* bias, float m) {
+    GemvRowArgs r{};
+    r.A = (const bf16*)A; r.W = (const bf16*)W; r.N = N; r.K = K; r.epi = epi; r.bias = bias; r.m = m; r.x = w.x; r.eps = c.norm_eps;
+    return r;
+  };
   int xb_parts = h->fold ? 1 : 0;
   const int h_tiles = ceil_div(H, 128);
   // generic_model.go:359-365: res + rm * x when ResidualMultiplier != 0, else plain add
@@ -451,7 +458,12 @@ int forward_step(nvllm_handle* h) {
     const float *cosT = h->use_rope ? h->cosT : nullptr, *sinT = h->use_rope ? h->sinT : nullptr;
     const Tc5Heads heads{h->nh, h->nkv, h->hd, d_pos, d_slots, cosT, sinT, (bf16*)kp, (bf16*)vp};
     const Tc5Heads* hp = is_prefill && h->adt == DT_BF16 && h->kvdt == DT_BF16 && (h->hd == 64 || h->hd == 128) ? &heads : nullptr;
-    if (xb_parts > 0 && fold_gemm_ok(h, T, h->qkv_cols, H, H)) {
+    if (one_row && !p1.p && !p2.p) {
+      GemvRowArgs r = row_args(nullptr, lw.wqkv, h->qkv_cols, H, TC5_EPI_PARTIAL, nullptr, 0.f);
+      r.norm_w = lw.attn_norm_w; r.norm_b = lw.attn_norm_b; r.out = w.ws_a;
+      if ((rc = run_gemv_row(h, r))) return rc;
+      qkv.p = w.ws_a; qkv.S = 1; qkv.stride = h->qkv_cols;
+    } else if (xb_parts > 0 && fold_gemm_ok(h, T, h->qkv_cols, H, H)) {
       RowScale rsc{w.ssq, xb_parts};
       if ((rc = run_gemm(h, w.xb, H, lw.wqkv, T, h->qkv_cols, H, 1.f, w.ws_a, w.ws_a_floats,
                          h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, nullptr, 0, 0.0, &rsc, nullptr, nullptr, hp, w.q)))
@@ -494,7 +506,10 @@ int forward_step(nvllm_handle* h) {
       LAUNCH(h, launch_attn_decode(st, at));
       if (at.n_splits > 1) h->launches++;
     }
-    if (resid_gemm_ok(h, T, H, h->q_cols, h->q_cols)) {
+    if (one_row && gemv_row_fits(h->q_cols)) {
+      if ((rc = run_gemv_row(h, row_args(w.attn_out, lw.wo, H, h->q_cols, TC5_EPI_RESID, lw.bo, m_res)))) return rc;
+      p1 = Pending();
+    } else if (resid_gemm_ok(h, T, H, h->q_cols, h->q_cols)) {
       Resid rd{m_res, lw.bo, 0, lw.ffn_norm_w};
       if ((rc = run_gemm(h, w.attn_out, h->q_cols, lw.wo, T, H, h->q_cols, 1.f, w.ws_b,
                          w.ws_b_floats, H, &p1, 0, nullptr, 0, nullptr, nullptr, 0, 0.0, nullptr, &rd)))
@@ -509,6 +524,13 @@ int forward_step(nvllm_handle* h) {
     }
     }  // attention / Mamba2 sub-block
     // ---- feed-forward sub-block
+    if (one_row && !h->moe && !p1.p && gemv_row_fits(h->F)) {
+      GemvRowArgs r = row_args(nullptr, lw.w1, h->w1_cols, H, h->swiglu ? TC5_EPI_SWIGLU : TC5_EPI_GELU, lw.b1, 0.f);
+      r.norm_w = lw.ffn_norm_w; r.norm_b = lw.ffn_norm_b; r.act = (bf16*)w.hbuf;
+      if ((rc = run_gemv_row(h, r))) return rc;
+      if ((rc = run_gemv_row(h, row_args(w.hbuf, lw.w2, H, h->F, TC5_EPI_RESID, lw.b2, m_res)))) return rc;
+      continue;
+    }
     float* ffn_out = w.ws_b;
     if (h->parallel) {
       ffn_out = w.ws_c;  // FFN reads the same normed input (generic_model.go:395-418)

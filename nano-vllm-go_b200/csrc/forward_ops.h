@@ -227,6 +227,15 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
   return NVLLM_OK;
 }
 
+// One row's product with its norm in front (norm_w: of x) and its activation or residual update behind (gemv_row.cu)
+static int run_gemv_row(nvllm_handle* h, const GemvRowArgs& a) {
+  const bool act = a.epi == TC5_EPI_SWIGLU || a.epi == TC5_EPI_GELU;
+  ProfScope ps(h, NVLLM_K_GEMV, 2.0 * a.N * a.K, 2.0 * a.N * a.K,
+               (a.norm_w ? 4.0 : 2.0) * a.K + (act ? 2.0 : a.epi == TC5_EPI_RESID ? 8.0 : 4.0) * a.N);
+  LAUNCH(h, launch_gemv_row(h->stream, a));
+  return NVLLM_OK;
+}
+
 // can (M, N, K) with this activation stride take the tcgen05 path (and with it the folded-norm
 // epilogues)?
 static bool fold_gemm_ok(const nvllm_handle* h, int M, int N, int K, int lda) {

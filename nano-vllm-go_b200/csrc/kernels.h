@@ -247,8 +247,7 @@ struct GemmArgs {
 // so nothing is read twice).  In bf16 mode only at one row: from two on the W1 GEMV writes the activation (gemv_mma.cu).
 //  mode 2: A = act(sum_s hp[s] + hbias): SwiGLU over interleaved gate / up columns, or tanh-GELU,
 //          rounded to `adt` exactly like the stand-alone kernel rounds what it stores.
-// (The same trick for the norms — every CTA re-deriving the row statistics from x + the pending
-// slices — was measured on cfg1 and lost: 313 -> 334 us per decode step; removed.)
+// (Norms in front of a product too: one bf16 row, gemv_row.cu.)
 struct GemvPre {
   int mode;  // 0 = none, 2 = activation
   const float* hp;  // [Sh][M][hld] split-K slices of the FFN up projection
@@ -290,6 +289,23 @@ struct GemvMmaPlan {
 };
 GemvMmaPlan gemv_mma_plan(int N, int K, int most);
 cudaError_t launch_gemv_mma(cudaStream_t st, const GemvMmaArgs& a, const GemvMmaPlan& p);
+
+// gemv_row.cu: one bf16 row, its norm in front and what follows behind in the same launch
+struct GemvRowArgs {
+  const __nv_bfloat16* A;         // [K], or norm_w: the row is x, normed
+  const __nv_bfloat16* W;         // [N, K]
+  int N, K;
+  float* x;                       // residual stream: read by the norm [K], updated by TC5_EPI_RESID [N]
+  const float *norm_w, *norm_b;   // norm_b: LayerNorm, otherwise RMSNorm
+  float eps;
+  int epi;                        // TC5_EPI_PARTIAL: out; RESID: x += m (sum + bias); SWIGLU (interleaved rows), GELU: act
+  float* out;
+  __nv_bfloat16* act;
+  const float* bias;
+  float m;
+};
+bool gemv_row_fits(int K);
+cudaError_t launch_gemv_row(cudaStream_t st, const GemvRowArgs& a);
 
 // ---------------------------------------------------------------- gemm_tcgen05.cu
 struct TmaDesc {
