@@ -220,7 +220,9 @@ struct nvllm_handle {
   nvllm_config cfg{};
   int dev = 0, sm_count = 148;
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the last step issued
+  cudaEvent_t ev0_prev = nullptr, ev1_prev = nullptr;  // and around the one before, while that is speculative
+  cudaEvent_t ev_done = nullptr;  // a step's results are in pinned memory
   cudaEvent_t tm0 = nullptr, tm1 = nullptr;  // nvllm_timer_record
   nvllm::WaitFlag waits;                     // of the kernels launched for this handle
   std::string err;
@@ -317,8 +319,6 @@ struct nvllm_handle {
   int32_t* d_stage = nullptr;
   size_t stage_words = 0;
   int32_t* h_out = nullptr;  // pinned [n_cap]
-  float* h_logits = nullptr;  // pinned, grown on demand
-  size_t h_logits_floats = 0;
   nvllm::StepLayout lay;
   nvllm::Workspace ws;
   // sampling
@@ -326,6 +326,10 @@ struct nvllm_handle {
   int top_k = 0;
   // SampleWithHistory filters (sampling.cu): the step's flattened token history
   // [cu_hist (n + 1) | tokens] and the per-row probability scratch, grown on demand
+  float* h_logits = nullptr;  // pinned, on their way to the caller
+  size_t h_logits_bytes = 0;
+  int32_t* h_hist = nullptr;  // pinned, on its way to d_hist
+  size_t h_hist_bytes = 0;
   int32_t* d_hist = nullptr;
   size_t hist_words = 0;
   int hist_n = 0;           // sequences of the uploaded history (0 = none for this step)
@@ -374,7 +378,7 @@ struct nvllm_handle {
   int spec_enabled = 1;
   bool spec_pending = false;
   bool spec_used_graph = false;  // the in-flight speculative step replayed a graph
-  int spec_skip = 0;  // calls that do not speculate (set after a miss)
+  int spec_misses = 0, spec_skip = 0;  // misses in a row, calls that do not speculate because of them
   std::vector<int32_t> spec_len, spec_nb, spec_bt;  // per-sequence lengths / block tables of the last call
   // device-resident decode state as the host knows it: context length (incl. the token the last
   // step appended) and block-table extent of every sequence — nvllm_run_resident refuses to step

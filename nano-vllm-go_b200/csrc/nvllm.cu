@@ -339,11 +339,13 @@ int nvllm_destroy(nvllm_handle* h) {
   }
   if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->h_out) cudaFreeHost(h->h_out);
+  if (h->h_hist) cudaFreeHost(h->h_hist);
   if (h->h_logits) cudaFreeHost(h->h_logits);
   nvllm::free_workspace(h);
   nvllm::tp_destroy(h);
   if (h->ev0) cudaEventDestroy(h->ev0);
-  if (h->ev1) cudaEventDestroy(h->ev1);
+  for (cudaEvent_t e : {h->ev1, h->ev0_prev, h->ev1_prev, h->ev_done})
+    if (e) cudaEventDestroy(e);
   h->waits.destroy();
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;

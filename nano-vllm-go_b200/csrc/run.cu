@@ -68,13 +68,14 @@ static float next_uniform(nvllm_handle* h) {
   return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
+// timed: with the device time between these two events
 static void fill_stats(nvllm_handle* h, nvllm_run_stats* stats, int T, uint64_t h2d, uint64_t d2h,
-                       bool timed) {
+                       cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr) {
   if (!stats) return;
   memset(stats, 0, sizeof *stats);
-  if (timed) {
+  if (ev0) {
     float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, h->ev0, h->ev1) == cudaSuccess) stats->device_ms = ms;
+    if (cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess) stats->device_ms = ms;
   }
   stats->kernel_launches = h->launches;
   stats->new_tokens = T;
@@ -142,12 +143,16 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
 // ---- speculative next step.  ModelRunner.Run is synchronous (the engine needs the tokens to
 // schedule the next step), so between two calls the GPU would idle for the host's turnaround
 // (sync, Go/cgo, staging, launch: ~100 us of a ~1.1 ms cfg2 step).  A decode batch is almost
-// always followed by the same batch one token longer, so nvllm_run ends by issuing exactly that
-// step on the device (what nvllm_run_resident does).  The next call either asks for it — same
+// always followed by the same batch one token longer, so nvllm_run issues exactly that
+// step on the device (what nvllm_run_resident does), behind its own step's results and before it waits for them: the GPU
+// goes from one step to the next without the host (a step of 64 / 128 / 1 sequences used to be followed by 49 / 61 / 35 us
+// of waking, launching and graph start).  The next call either asks for it — same
 // sequences, one token longer, last token = the one just returned, same block tables, greedy —
 // and only has to wait for it, or asks for something else and restages everything as usual.
 // A speculative step that is thrown away has only written K/V at the next position of each
-// sequence, a slot nothing reads before its owner writes it.
+// sequence, a slot nothing reads before its owner writes it; but the call after it waits for it, so misses in a row pause
+// the speculation: 1, 2, 4, ... 16 calls from the second one on.  (A workload of prompts alone threw a decode step
+// away at every second call.)
 static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_graph = nullptr);
 // After a synchronise: did a bounded wait of this handle's kernels run out?  Then neither the results nor the device state
 // that a resident, speculative or repeated step would start from are used.
@@ -216,6 +221,74 @@ static bool speculation_hit(const nvllm_handle* h, int n, int is_prefill, const 
   return true;
 }
 
+// Grows a pinned buffer of the handle (nothing is in flight between two calls: every run ends with a synchronisation).
+static int ensure_pinned(nvllm_handle* h, void** p, size_t* have, size_t bytes) {
+  if (bytes <= *have) return NVLLM_OK;
+  if (*p) cudaFreeHost(*p);
+  *p = nullptr;
+  *have = 0;
+  NV_CHECK(h, cudaMallocHost(p, bytes));
+  *have = bytes;
+  return NVLLM_OK;
+}
+
+// The n rows of logits for the caller, after the step on the stream: enqueue, and finish once the stream is done.  Up to 4
+// MB travel through a pinned buffer of the handle, as one copy that runs beside the host; a copy to the caller's pageable
+// memory is staged by the driver, which waits for the step first.  Larger ones stay with the driver.
+constexpr size_t LOGITS_PINNED = (size_t)4 << 20;
+static int enqueue_logits(nvllm_handle* h, float* out, int n) {
+  const size_t bytes = (size_t)n * h->V * 4;
+  float* dst = out;
+  if (bytes <= LOGITS_PINNED) {
+    if (const int rc = ensure_pinned(h, (void**)&h->h_logits, &h->h_logits_bytes, bytes)) return rc;
+    dst = h->h_logits;
+  }
+  // rows are ldl apart on the device; copy them packed [n, V]
+  if (h->ldl == h->V) NV_CHECK(h, cudaMemcpyAsync(dst, h->ws.logits_final, bytes, cudaMemcpyDeviceToHost, h->stream));
+  else
+    NV_CHECK(h, cudaMemcpy2DAsync(dst, (size_t)h->V * 4, h->ws.logits_final, (size_t)h->ldl * 4, (size_t)h->V * 4, n,
+                                  cudaMemcpyDeviceToHost, h->stream));
+  return NVLLM_OK;
+}
+static void finish_logits(nvllm_handle* h, float* out, int n) {
+  const size_t bytes = (size_t)n * h->V * 4;
+  if (bytes <= LOGITS_PINNED) memcpy(out, h->h_logits, bytes);
+}
+
+// The end of a step whose results are on their way to pinned memory: the next step is issued, then this one is waited for.
+static int finish_step(nvllm_handle* h, int n, const int32_t* cu_seqlens, const int32_t* block_tables, const int32_t* cu_blocks,
+                       const float* temperature, int32_t* out_tokens, float* out_logits, nvllm_run_stats* stats, int T,
+                       uint64_t h2d, uint64_t d2h, bool used_graph) {
+  if (!h->ev_done) {
+    NV_CHECK(h, cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming));
+    NV_CHECK(h, cudaEventCreate(&h->ev0_prev));
+    NV_CHECK(h, cudaEventCreate(&h->ev1_prev));
+  }
+  NV_CHECK(h, cudaEventRecord(h->ev_done, h->stream));
+  h->resident_ok = true;
+  remember_call(h, n, cu_seqlens, block_tables, cu_blocks);
+  // this step's events keep its time, the next one gets the other two
+  auto other_events = [&] {
+    std::swap(h->ev0, h->ev0_prev);
+    std::swap(h->ev1, h->ev1_prev);
+  };
+  other_events();
+  try_speculate(h, n, temperature);
+  const cudaEvent_t ev0 = h->ev0_prev, ev1 = h->ev1_prev;
+  if (!h->spec_pending) other_events();
+  const cudaError_t e = cudaEventSynchronize(h->ev_done);
+  if (e != cudaSuccess) {
+    h->resident_ok = h->run_lay_ok = h->spec_pending = false;
+    return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
+  }
+  if (const int rc = check_waits(h)) return rc;
+  memcpy(out_tokens, h->h_out, (size_t)n * 4);
+  if (out_logits && h->tp == 1) finish_logits(h, out_logits, n);
+  fill_stats(h, stats, T, h2d, d2h, ev0, ev1);
+  if (stats) stats->used_graph = used_graph ? 1 : 0;
+  return NVLLM_OK;
+}
+
 extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* token_ids,
                          const int32_t* cu_seqlens, const int32_t* num_cached,
                          const int32_t* block_tables, const int32_t* cu_blocks,
@@ -237,24 +310,18 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
       NV_CHECK(h, cudaMemcpyAsync(h->h_out, h->ws.out_tokens, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
       uint64_t d2h = (uint64_t)n * 4;
       if (out_logits) {
-        NV_CHECK(h, cudaMemcpy2DAsync(out_logits, (size_t)h->V * 4, h->ws.logits_final,
-                                      (size_t)h->ldl * 4, (size_t)h->V * 4, n, cudaMemcpyDeviceToHost, st));
+        if (const int rc = enqueue_logits(h, out_logits, n)) return rc;
         d2h += (uint64_t)n * h->V * 4;
       }
-      cudaError_t e = cudaStreamSynchronize(st);
-      if (e != cudaSuccess)
-        return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
-      if (const int rc = check_waits(h)) return rc;
-      memcpy(out_tokens, h->h_out, (size_t)n * 4);
       h->run_lay = h->lay;
       h->run_lay_ok = true;
-      fill_stats(h, stats, n, 0, d2h, true);
-      if (stats) stats->used_graph = h->spec_used_graph ? 1 : 0;
-      remember_call(h, n, cu_seqlens, block_tables, cu_blocks);
-      try_speculate(h, n, temperature);
-      return NVLLM_OK;
+      h->spec_misses = 0;
+      return finish_step(h, n, cu_seqlens, block_tables, cu_blocks, temperature, out_tokens, out_logits, stats, n, 0, d2h,
+                         h->spec_used_graph);
     }
-    h->spec_skip = 1;  // missed: the caller is not stepping one batch; back off once
+    // missed: the caller is not stepping one batch
+    h->spec_misses = std::min(h->spec_misses + 1, 6);
+    h->spec_skip = h->spec_misses > 1 ? 1 << (h->spec_misses - 2) : 0;
   }
   h->resident_ok = false;
   h->run_lay_ok = false;
@@ -405,14 +472,11 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
         NV_CHECK(h, cudaMalloc((void**)&h->d_probs, pf * 4));
         h->probs_floats = pf;
       }
-      // offsets relative to the first token, then the tokens themselves (the caller's buffers
-      // are pageable: these copies are staged by the driver before the call returns)
-      std::vector<int32_t> cu(n + 1);
-      for (int i = 0; i <= n; i++) cu[i] = cu_seqlens[i] - cu_seqlens[0];
-      NV_CHECK(h, cudaMemcpyAsync(h->d_hist, cu.data(), (size_t)(n + 1) * 4, cudaMemcpyHostToDevice, st));
-      NV_CHECK(h, cudaMemcpyAsync(h->d_hist + (n + 1), token_ids + cu_seqlens[0], total * 4,
-                                  cudaMemcpyHostToDevice, st));
-      NV_CHECK(h, cudaStreamSynchronize(st));  // `cu` is a stack temporary
+      // offsets relative to the first token, then the tokens themselves, as one copy
+      if ((rc = ensure_pinned(h, (void**)&h->h_hist, &h->h_hist_bytes, words * 4))) return rc;
+      for (int i = 0; i <= n; i++) h->h_hist[i] = cu_seqlens[i] - cu_seqlens[0];
+      memcpy(h->h_hist + n + 1, token_ids + cu_seqlens[0], total * 4);
+      NV_CHECK(h, cudaMemcpyAsync(h->d_hist, h->h_hist, words * 4, cudaMemcpyHostToDevice, st));
       h->hist_n = n;
     }
   }
@@ -429,7 +493,6 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   NV_CHECK(h, cudaMemcpyAsync(h->h_out, h->ws.out_tokens, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
   uint64_t d2h = (uint64_t)n * 4;
   if (out_logits) {
-    // rows are ldl apart on the device; copy them packed [n, V]
     if (h->tp > 1) {  // gathered rank-major vocabulary slices [tp][n][Vl]
       for (int r = 0; r < h->tp; r++) {
         const int c0 = r * h->Vl, cn = std::min(h->Vl, h->V - c0);
@@ -440,26 +503,15 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
                                       cudaMemcpyDeviceToHost, st));
       }
     } else {
-      NV_CHECK(h, cudaMemcpy2DAsync(out_logits, (size_t)h->V * 4, h->ws.logits_final,
-                                    (size_t)h->ldl * 4, (size_t)h->V * 4, n,
-                                    cudaMemcpyDeviceToHost, st));
+      if ((rc = enqueue_logits(h, out_logits, n))) return rc;
     }
     d2h += (uint64_t)n * h->V * 4;
   }
-  cudaError_t e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess)
-    return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: %s", cudaGetErrorString(e));
-  if ((rc = check_waits(h))) return rc;
-  memcpy(out_tokens, h->h_out, (size_t)n * 4);
-  h->resident_ok = true;
   h->run_lay = L;
   h->run_lay_ok = true;
   h->fetched_rows = n_extra;
-  fill_stats(h, stats, T, L.words * 4, d2h, true);
-  if (stats) stats->used_graph = used_graph ? 1 : 0;
-  remember_call(h, n, cu_seqlens, block_tables, cu_blocks);
-  try_speculate(h, n, temperature);
-  return NVLLM_OK;
+  return finish_step(h, n, cu_seqlens, block_tables, cu_blocks, temperature, out_tokens, out_logits, stats, T, L.words * 4, d2h,
+                     used_graph);
 }
 
 extern "C" int nvllm_set_state_slots(nvllm_handle* h, const int32_t* slots, int n) {
@@ -563,7 +615,7 @@ static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_gra
       bool used = false;
       if ((rc = graphed_step(h, 0, advance, &used))) return rc;
       NV_CHECK(h, cudaEventRecord(h->ev1, st));
-      fill_stats(h, stats, n, 0, 0, false);
+      fill_stats(h, stats, n, 0, 0);
       if (stats) stats->used_graph = 1;
       if (used_graph) *used_graph = true;
       return NVLLM_OK;
@@ -572,7 +624,7 @@ static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_gra
   }
   if ((rc = forward_step(h))) return rc;
   NV_CHECK(h, cudaEventRecord(h->ev1, st));
-  fill_stats(h, stats, n, 0, 0, false);
+  fill_stats(h, stats, n, 0, 0);
   return NVLLM_OK;
 }
 
@@ -580,7 +632,7 @@ extern "C" int nvllm_run_resident(nvllm_handle* h, nvllm_run_stats* stats) {
   if (!h) return NVLLM_ERR_INVALID;
   if (h->spec_pending) {  // the step asked for is the one already in flight
     h->spec_pending = false;
-    fill_stats(h, stats, h->lay.n, 0, 0, false);
+    fill_stats(h, stats, h->lay.n, 0, 0);
     if (stats) stats->used_graph = h->spec_used_graph ? 1 : 0;
     return NVLLM_OK;
   }
@@ -606,7 +658,7 @@ extern "C" int nvllm_rerun(nvllm_handle* h, nvllm_run_stats* stats) {
   if (rc) return rc;
   NV_CHECK(h, cudaEventRecord(h->ev1, h->stream));
   h->resident_ok = true;
-  fill_stats(h, stats, h->lay.T, 0, 0, false);
+  fill_stats(h, stats, h->lay.T, 0, 0);
   return NVLLM_OK;
 }
 
