@@ -919,6 +919,20 @@ __global__ void __launch_bounds__(256) delta_out_vec_kernel(DeltaArgs a, Trace t
   const bool on = 4 * lane < vdim;
   const float4 w = on ? *reinterpret_cast<const float4*>(a.onorm_w + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
   pdl_wait();
+  if (a.roll) {  // behind delta_step_kernel: the tail of the q and k channels moves on by the row that it left in qkv
+    float* tail = a.state_pool + (size_t)a.state_slots[t] * a.slot_floats + a.tail_off;
+    for (int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x); c < a.n_q + a.n_k; c += 4 * gridDim.y * blockDim.x) {
+      float4 nv[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (k + 2 < a.taps) nv[k] = __ldcg(reinterpret_cast<const float4*>(tail + (size_t)(k + 1) * a.conv_ch + c));
+      const float4 last = __ldcg(reinterpret_cast<const float4*>(a.qkv + (size_t)t * a.conv_ch + c));
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (k + 2 < a.taps) *reinterpret_cast<float4*>(tail + (size_t)k * a.conv_ch + c) = nv[k];
+      *reinterpret_cast<float4*>(tail + (size_t)(a.taps - 2) * a.conv_ch + c) = last;
+    }
+  }
   OT* out = (OT*)a.out + (size_t)t * a.o_ld;
   const float* gate = a.in_p + (size_t)t * a.in_ld + a.conv_ch + 2 * a.H + 4 * lane;
   const float* o = a.o + (size_t)t * a.H * vdim + 4 * lane;
@@ -982,11 +996,160 @@ __global__ void __launch_bounds__(256) delta_out_kernel(DeltaArgs a, Trace tr) {
   TRACE_EXIT(tr);
 }
 
+static bool delta_out_vec_fits(const DeltaArgs& a) {  // (the gates' columns start behind 2 H entries of the projection)
+  return a.vdim <= 128 && a.vdim % 4 == 0 && (a.conv_ch + 2 * a.H) % 4 == 0 && a.in_ld % 4 == 0 && a.in_stride % 4 == 0 && a.o_ld % 4 == 0;
+}
+
+// ------------------------------------------------------------------ one token per sequence
+// Decode steps, preparation and scan as one launch: a CTA per (sequence, head, 64 value columns) makes its head's q and k
+// and its own v itself and holds its DIM x 64 entries of the state, two columns per lane and DIM / 8 rows per warp, in
+// registers.  State, tail and filter are loaded before the wait for the projection (the kernels that wrote them belong to
+// the step before), so the state streams in under the projection's end; then one round of loads (the projection's
+// slices), two block sums.  Bound by the state's stream, once in and once out.  The tail of the v channels moves on here;
+// that of q and k, which other CTAs still read, in the kernel behind (roll).  32 sequences, 16 heads of 128 x 128, us a layer
+// with the gated norm: 48 -> 20.
+constexpr int DS_VC = 64;
+__device__ __forceinline__ float sum_slices8(const float* __restrict__ p, int S, size_t stride) {
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) v[i] = i < S ? p[(size_t)i * stride] : 0.f;  // all in flight
+  float acc = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    if (i < S) acc += v[i];
+  return acc;
+}
+template <int DIM, int TAPS, bool FAST>
+__global__ void __launch_bounds__(256, 3) delta_step_kernel(DeltaArgs a, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_launch_dependents();
+  constexpr int RW = DIM / 8, NCH = 2 * DIM + DS_VC, NI = (NCH + 255) / 256;
+  __shared__ float qkv[NCH];  // q | k | v
+  __shared__ float part[8][DS_VC];
+  __shared__ float bg[2];
+  const int t = blockIdx.x, h = blockIdx.y, vbase = blockIdx.z * DS_VC;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int hpg = a.H / a.G, kvh = h / hpg;
+  const int pos = a.positions[t];  // (one row per sequence)
+  float* slot = a.state_pool + (size_t)a.state_slots[t] * a.slot_floats;
+  float* tail = slot + a.tail_off;
+  float2* S_g = reinterpret_cast<float2*>(slot + a.state_off + ((size_t)h * DIM + warp * RW) * a.vdim + vbase) + lane;
+  const int ld2 = a.vdim / 2;
+  float2 st[RW];
+#pragma unroll
+  for (int r = 0; r < RW; r++) st[r] = pos > 0 ? __ldcg(S_g + (size_t)r * ld2) : make_float2(0.f, 0.f);
+  int ch[NI];
+  float old[NI][TAPS - 1], cw[NI][TAPS];
+#pragma unroll
+  for (int i = 0; i < NI; i++) {
+    const int j = tid + 256 * i;
+    ch[i] = j < DIM ? kvh * DIM + j : j < 2 * DIM ? a.n_q + kvh * DIM + (j - DIM) : a.n_q + a.n_k + h * a.vdim + vbase + (j - 2 * DIM);
+    if (j >= NCH) continue;
+#pragma unroll
+    for (int k = 0; k < TAPS; k++) cw[i][k] = a.conv_w[(size_t)ch[i] * TAPS + k];
+#pragma unroll
+    for (int k = 0; k + 1 < TAPS; k++) old[i][k] = pos - (TAPS - 1 - k) >= 0 ? __ldcg(tail + (size_t)k * a.conv_ch + ch[i]) : 0.f;
+  }
+  pdl_wait();
+  const float* in = a.in_p + (size_t)t * a.in_ld;
+#pragma unroll
+  for (int i = 0; i < NI; i++) {
+    const int j = tid + 256 * i;
+    if (j >= NCH) continue;
+    const float x = sum_slices8(in + ch[i], a.in_S, a.in_stride);
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k + 1 < TAPS; k++) v = fmaf(old[i][k], cw[i][k], v);
+    v = fmaf(x, cw[i][TAPS - 1], v);
+    qkv[j] = silu_t<FAST>(v);
+    if (j >= 2 * DIM) {
+#pragma unroll
+      for (int k = 0; k + 2 < TAPS; k++) tail[(size_t)k * a.conv_ch + ch[i]] = old[i][k + 1];
+      tail[(size_t)(TAPS - 2) * a.conv_ch + ch[i]] = x;
+    } else if (blockIdx.z == 0 && h % hpg == 0) {
+      a.qkv[(size_t)t * a.conv_ch + ch[i]] = x;  // for the roll
+    }
+  }
+  if (tid >= 254) {
+    const float* p = in + a.conv_ch;
+    if (tid == 254) bg[0] = 1.0f / (1.0f + expf(-sum_slices8(p + h, a.in_S, a.in_stride)));
+    else bg[1] = expf(-expf(a.a_log[h]) * softplus(sum_slices8(p + a.H + h, a.in_S, a.in_stride) + a.dt_bias[h]));
+  }
+  __syncthreads();
+  if (warp < 2) {  // unit lengths of q and k; the query also carries 1 / sqrt(dim)
+    float* v = qkv + warp * DIM;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < DIM / 32; i++) ss += v[lane + 32 * i] * v[lane + 32 * i];
+    float mul = 1.0f / sqrtf(warp_sum(ss) + 1e-6f);
+    if (warp == 0) mul *= 1.0f / sqrtf((float)DIM);
+#pragma unroll
+    for (int i = 0; i < DIM / 32; i++) v[lane + 32 * i] *= mul;
+  }
+  __syncthreads();
+  const float beta = bg[0], g = bg[1];
+  const float *q = qkv + warp * RW, *k = qkv + DIM + warp * RW;
+  auto column_sum = [&](float2 mine) {  // over the warps, every thread its two columns
+    *reinterpret_cast<float2*>(&part[warp][2 * lane]) = mine;
+    __syncthreads();
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const float2 o = *reinterpret_cast<const float2*>(&part[w][2 * lane]);
+      s.x += o.x;
+      s.y += o.y;
+    }
+    return s;
+  };
+  float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < RW; r++) {
+    st[r].x *= g;
+    st[r].y *= g;
+    acc.x = fmaf(st[r].x, k[r], acc.x);
+    acc.y = fmaf(st[r].y, k[r], acc.y);
+  }
+  const float2 sk = column_sum(acc);
+  const float2 v = *reinterpret_cast<const float2*>(&qkv[2 * DIM + 2 * lane]);
+  const float2 u = make_float2(beta * (v.x - sk.x), beta * (v.y - sk.y));
+  acc = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < RW; r++) {
+    st[r].x = fmaf(k[r], u.x, st[r].x);
+    st[r].y = fmaf(k[r], u.y, st[r].y);
+    S_g[(size_t)r * ld2] = st[r];
+    acc.x = fmaf(st[r].x, q[r], acc.x);
+    acc.y = fmaf(st[r].y, q[r], acc.y);
+  }
+  __syncthreads();  // `part` has been read
+  const float2 o = column_sum(acc);
+  if (warp == 0) *reinterpret_cast<float2*>(a.o + (size_t)t * a.H * a.vdim + (size_t)h * a.vdim + vbase + 2 * lane) = o;
+  TRACE_EXIT(tr);
+}
+// sizes that divide into the kernel's tiles, a read-out that the vector form of the gated norm takes (it rolls the tail)
+bool delta_step_fits(const DeltaArgs& a) {
+  return a.T == a.n_seqs && (a.dim == 64 || a.dim == 128) && a.vdim % DS_VC == 0 && a.taps >= 2 && a.taps <= 4 && a.in_S <= 8 &&
+         a.H % a.G == 0 && delta_out_vec_fits(a) && a.n_q % 4 == 0 && a.n_k % 4 == 0 && a.conv_ch % 4 == 0 && a.tail_off % 4 == 0 &&
+         a.state_off % 2 == 0 && a.slot_floats % 4 == 0;
+}
+template <int DIM, int TAPS>
+static cudaError_t delta_step_launch(cudaStream_t st, const DeltaArgs& a) {
+  const dim3 grid(a.T, a.H, a.vdim / DS_VC);
+  return a.fast_act ? launch_k(delta_step_kernel<DIM, TAPS, true>, grid, dim3(256), 0, st, a, next_trace(51))
+                    : launch_k(delta_step_kernel<DIM, TAPS, false>, grid, dim3(256), 0, st, a, next_trace(51));
+}
+cudaError_t launch_delta_step(cudaStream_t st, const DeltaArgs& a) {
+  if (a.T <= 0) return cudaSuccess;
+  if (!delta_step_fits(a)) return cudaErrorInvalidValue;
+  if (a.dim == 64) return a.taps == 4 ? delta_step_launch<64, 4>(st, a) : a.taps == 3 ? delta_step_launch<64, 3>(st, a) : delta_step_launch<64, 2>(st, a);
+  return a.taps == 4 ? delta_step_launch<128, 4>(st, a) : a.taps == 3 ? delta_step_launch<128, 3>(st, a) : delta_step_launch<128, 2>(st, a);
+}
+
 cudaError_t launch_delta_out(cudaStream_t st, int odt, const DeltaArgs& a) {
   if (a.T <= 0) return cudaSuccess;
   const dim3 grid(a.T, a.T >= 1024 ? 1 : ceil_div(a.H, 8));  // few rows (decode): a row's heads spread over several CTAs
-  // (the gates' columns start behind 2 H entries of the projection)
-  if (a.vdim <= 128 && a.vdim % 4 == 0 && (a.conv_ch + 2 * a.H) % 4 == 0 && a.in_ld % 4 == 0 && a.in_stride % 4 == 0 && a.o_ld % 4 == 0)
+  if (a.roll && !delta_out_vec_fits(a)) return cudaErrorInvalidValue;
+  if (delta_out_vec_fits(a))
     return odt == DT_F32 ? launch_k(delta_out_vec_kernel<float>, grid, dim3(256), 0, st, a, next_trace(36))
                          : launch_k(delta_out_vec_kernel<bf16>, grid, dim3(256), 0, st, a, next_trace(36));
   if (odt == DT_F32) (void)launch_k(delta_out_kernel<float, 8>, grid, dim3(256), 0, st, a, next_trace(36));

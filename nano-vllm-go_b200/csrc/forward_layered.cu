@@ -731,7 +731,8 @@ static int mixer_delta(nvllm_handle* h, const ListedLayer& y, Pending* out) {
   a.qkv = w.dl_qkv; a.bg = w.dl_bg; a.o = w.dl_o;
   a.out = w.attn_out; a.o_ld = y.ov_p;
   const double hv = (double)s.heads * s.vdim;
-  {
+  a.roll = delta_step_fits(a) ? 1 : 0;
+  if (!a.roll) {
     ProfScope ps(h, NVLLM_K_RECUR, (double)T * (y.conv_ch + 2 * s.heads) * 8, 0,
                  (double)T * y.n_in * 4 * (pin.S - 1) + (double)T * y.conv_ch * 4 * (s.conv - 1));
     LAUNCH(h, launch_delta_prep(h->stream, a));
@@ -740,7 +741,8 @@ static int mixer_delta(nvllm_handle* h, const ListedLayer& y, Pending* out) {
     // algorithmic: every sequence's state once in and once out, the token inputs once, the read-outs once
     const double state = (double)L.n * s.heads * s.dim * s.vdim * 4 * 2;
     ProfScope ps(h, NVLLM_K_RECUR, state + (double)T * (y.conv_ch + 2 * s.heads + hv) * 4, 6.0 * T * hv * s.dim);
-    LAUNCH(h, launch_delta_scan(h->stream, a));
+    if (a.roll) LAUNCH(h, launch_delta_step(h->stream, a));
+    else LAUNCH(h, launch_delta_scan(h->stream, a));
   }
   {
     ProfScope ps(h, NVLLM_K_RECUR, (double)T * hv * (4 + 4 + asz), 0, (double)T * hv * 4 * (pin.S - 1));

@@ -636,7 +636,11 @@ struct DeltaArgs {
   float* bg;             // [T, 2 H]     write strength | decay
   float* o;              // [T, H vdim]  read-outs
   void* out; int o_ld;   // [T, o_ld] act dtype: input of the output projection
+  int roll;              // launch_delta_out behind launch_delta_step: it also moves the tail of the q and k channels on
 };
+// one token per sequence: launch_delta_prep and launch_delta_scan in one
+bool delta_step_fits(const DeltaArgs& a);
+cudaError_t launch_delta_step(cudaStream_t st, const DeltaArgs& a);
 cudaError_t launch_delta_prep(cudaStream_t st, const DeltaArgs& a);
 cudaError_t launch_delta_scan(cudaStream_t st, const DeltaArgs& a);
 cudaError_t launch_delta_out(cudaStream_t st, int odt, const DeltaArgs& a);
