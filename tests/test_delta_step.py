@@ -17,7 +17,7 @@ KERNEL = 51  # its id in the timeline
     (2, 2, 64, 64, 2, True),     # one block of columns, one older row in the tail
     (4, 1, 128, 64, 3, True),
     (3, 1, 128, 64, 3, False),   # gates off the 16-byte boundaries
-    (1, 1, 64, 128, 4, True),
+    (2, 1, 64, 128, 4, True),
     (2, 1, 64, 96, 4, False),    # columns that don't fill its blocks
     (2, 1, 64, 64, 1, False),    # no tail
 ])
