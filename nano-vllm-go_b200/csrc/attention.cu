@@ -8,13 +8,18 @@
 // head h / (n_heads / n_kv_heads) (attention.go:337-339).
 //
 //  * attn_prefill_kernel: flash-style (online softmax, no S x S score tensor).
-//    CTA = 32 queries of one sequence x one head; 4 threads per query each owning
-//    hd/4 dims; K/V tiles of 64 keys staged in shared memory as fp32.
+//    CTA = 32 queries of one sequence x one head; four groups of 128 threads share the keys of a
+//    tile (16 each) and merge at the end; in a group 4 threads per query each own
+//    hd/4 dims; K/V tiles of 64 keys staged in shared memory as fp32.  Bound by the latency of its
+//    shared-memory reads and sums: a prompt's step has one or two such CTAs per SM, and with one group a
+//    scheduler has one warp to issue from.  Four prompts of 50 to 100 tokens, 12 heads of 64: 20 -> 14 us.
 //  * attn_decode_kernel: one new token per sequence.  CTA = (sequence, group of
 //    GC query heads sharing a kv head, KV split).  HBM-bound: each K/V row is
 //    read once with 16-byte loads by hd/8 lanes; online softmax in registers;
 //    split partials merged by attn_combine_kernel.
 #include <stdlib.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -22,12 +27,15 @@
 namespace nvllm {
 
 constexpr int PF_KT = 64;  // keys per shared-memory tile (divides KV_BLOCK)
+constexpr int PF_GROUPS = 4, PF_THREADS = 128 * PF_GROUPS;
+constexpr size_t pf_smem(int hd) {  // K and V tiles; then the groups' results: m, l and a row each
+  return sizeof(float) * std::max((size_t)2 * PF_KT * hd, (size_t)(PF_GROUPS - 1) * ATTN_PREFILL_QTILE * (hd + 4));
+}
 
 template <typename QT, typename KT, int HD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(PF_THREADS)
 attn_prefill_kernel(AttnArgs a) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ float smem[];
   float* Ks = smem;               // [PF_KT][HD]
   float* Vs = smem + PF_KT * HD;  // [PF_KT][HD]
@@ -40,16 +48,18 @@ attn_prefill_kernel(AttnArgs a) {
   const int n_new = a.cu_q[seq + 1] - a.cu_q[seq];
   const int start = a.seq_start[seq];
   const int kvh = head / (a.nh / a.nkv);
-  const int qi = threadIdx.x >> 2, sub = threadIdx.x & 3;
+  const int grp = threadIdx.x >> 7, qi = (threadIdx.x & 127) >> 2, sub = threadIdx.x & 3;
   const int qidx = q0 + qi;  // index among the new tokens of this sequence
   const bool qvalid = qidx < n_new;
   const int qpos = start + qidx;
   const int row = a.cu_q[seq] + qidx;
   const int* bt = a.block_tables + (size_t)seq * a.max_blocks;
 
+  const int blk0 = bt[0];
   float q[DPT], acc[DPT];
 #pragma unroll
   for (int i = 0; i < DPT; i++) acc[i] = 0.f;
+  pdl_wait();  // (what is read above came with the step)
   if (qvalid) {
     const QT* qp = (const QT*)a.q + (size_t)row * a.nh * HD + head * HD;
 #pragma unroll
@@ -67,7 +77,7 @@ attn_prefill_kernel(AttnArgs a) {
 
   for (int k0 = 0; k0 < kv_end; k0 += PF_KT) {
     const int nk = min(PF_KT, kv_end - k0);
-    const int blk = bt[k0 / KV_BLOCK];
+    const int blk = k0 == 0 ? blk0 : bt[k0 / KV_BLOCK];
     const size_t base = (((size_t)blk * a.nkv + kvh) * KV_BLOCK + (k0 % KV_BLOCK)) * HD;
     __syncthreads();
     for (int i = threadIdx.x * 8; i < nk * HD; i += blockDim.x * 8) {
@@ -82,8 +92,8 @@ attn_prefill_kernel(AttnArgs a) {
     // shuffles below name all 32 lanes), so every lane runs to the warp's largest jmax and
     // masks its own tail.
     const int jmax = qvalid ? max(0, min(nk, qpos - k0 + 1)) : 0;
-    const int jlim = __reduce_max_sync(0xffffffffu, jmax);
-    for (int j0 = 0; j0 < jlim; j0 += 8) {
+    const int jlim = min(__reduce_max_sync(0xffffffffu, jmax), (grp + 1) * (PF_KT / PF_GROUPS));
+    for (int j0 = grp * (PF_KT / PF_GROUPS); j0 < jlim; j0 += 8) {
       float s[8];
       float cmax = -INFINITY;
 #pragma unroll
@@ -132,7 +142,45 @@ attn_prefill_kernel(AttnArgs a) {
       m = m_new;
     }
   }
-  if (qvalid) {
+  // the groups' results meet in the first one
+  __syncthreads();
+  float* mine = smem + ((size_t)(grp - 1) * ATTN_PREFILL_QTILE + qi) * (HD + 4);
+  if (grp > 0) {
+    if (sub == 0) {
+      mine[HD] = m;
+      mine[HD + 1] = l;
+    }
+#pragma unroll
+    for (int v = 0; v < NV; v++)
+      *reinterpret_cast<float4*>(mine + v * 16 + sub * 4) = make_float4(acc[v * 4], acc[v * 4 + 1], acc[v * 4 + 2], acc[v * 4 + 3]);
+  }
+  __syncthreads();
+  if (grp == 0 && qvalid) {
+    // (key 0 is the first group's: its m is finite)
+    const float* other[PF_GROUPS - 1];
+    float top = m;
+#pragma unroll
+    for (int g = 0; g < PF_GROUPS - 1; g++) {
+      other[g] = smem + ((size_t)g * ATTN_PREFILL_QTILE + qi) * (HD + 4);
+      top = fmaxf(top, other[g][HD]);
+    }
+    const float c0 = expf(m - top);
+    l *= c0;
+#pragma unroll
+    for (int i = 0; i < DPT; i++) acc[i] *= c0;
+#pragma unroll
+    for (int g = 0; g < PF_GROUPS - 1; g++) {
+      const float c = expf(other[g][HD] - top);  // a group that saw no key: exp(-inf) = 0
+      l = fmaf(other[g][HD + 1], c, l);
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const float4 o = *reinterpret_cast<const float4*>(other[g] + v * 16 + sub * 4);
+        acc[v * 4] = fmaf(o.x, c, acc[v * 4]);
+        acc[v * 4 + 1] = fmaf(o.y, c, acc[v * 4 + 1]);
+        acc[v * 4 + 2] = fmaf(o.z, c, acc[v * 4 + 2]);
+        acc[v * 4 + 3] = fmaf(o.w, c, acc[v * 4 + 3]);
+      }
+    }
     const float inv = 1.0f / l;
     QT* op = (QT*)a.out + (size_t)row * a.nh * HD + head * HD;
 #pragma unroll
@@ -145,13 +193,13 @@ attn_prefill_kernel(AttnArgs a) {
 template <typename QT, typename KT>
 static cudaError_t prefill_dispatch(cudaStream_t st, const AttnArgs& a) {
   dim3 grid(a.n_qtiles, a.nh);
-  size_t smem = (size_t)2 * PF_KT * a.hd * sizeof(float);
+  const size_t smem = pf_smem(a.hd);
 #define PF(HD)                                                                               \
   {                                                                                          \
     if (smem > 48 * 1024)                                                                    \
       cudaFuncSetAttribute(attn_prefill_kernel<QT, KT, HD>,                                  \
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-    (void)launch_k(attn_prefill_kernel<QT, KT, HD>, dim3(grid), dim3(128), smem, st, a);                             \
+    (void)launch_k(attn_prefill_kernel<QT, KT, HD>, dim3(grid), dim3(PF_THREADS), smem, st, a);                      \
   }
   switch (a.hd) {
     case 16: PF(16); break;
