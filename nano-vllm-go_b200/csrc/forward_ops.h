@@ -263,7 +263,17 @@ static int launch_norm_routed(nvllm_handle* h, NormArgs a) {
     n.router = nullptr;
     n.y_f32 = h->ws.xn_f32;
     LAUNCH(h, launch_norm(h->stream, n));
-    LAUNCH(h, launch_moe_route_rows(h->stream, a, h->ws.xn_f32));
+    // logits [experts, rows] into the experts' results, whose last reader is the norm above
+    GemmArgs g{};
+    g.A = a.router; g.W = h->ws.xn_f32; g.adt = g.wdt = DT_F32; g.lda = a.H; g.M = a.E; g.N = a.n_rows; g.K = a.H;
+    g.out = h->ws.moe_Y; g.ldo = (a.n_rows + 3) / 4 * 4; g.split_stride = (size_t)a.E * g.ldo; g.alpha = 1.f;
+    g.out_capacity = (size_t)a.n_rows * h->topk * h->H; g.wait_flag = h->waits.dev; g.w_late = 1;
+    if (g.split_stride <= g.out_capacity && moe_route_product_fits(a, g)) {
+      LAUNCH(h, launch_gemm_f32_tc5(h->stream, g));
+      LAUNCH(h, launch_moe_select_rows(h->stream, a, g));
+    } else {
+      LAUNCH(h, launch_moe_route_rows(h->stream, a, h->ws.xn_f32));
+    }
     return NVLLM_OK;
   }
   LAUNCH(h, launch_norm(h->stream, a));

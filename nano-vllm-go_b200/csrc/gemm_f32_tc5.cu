@@ -56,19 +56,15 @@ struct F32Tc5Args {
   float alpha;
   int* flag;
   int wide;  // rows of `out` start on 16-byte boundaries
+  int late;  // W comes from the kernel in front
 };
 
 struct F8 {  // eight consecutive values, as the packed operations take them
   unsigned long long v[4];
 };
 // 32 bytes on their own boundary, no line kept in L1
-__device__ __forceinline__ F8 ld_weights(const float* p) {
-  F8 r;
-  asm("ld.global.nc.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.v[0]), "=l"(r.v[1]), "=l"(r.v[2]), "=l"(r.v[3]) : "l"(p));
-  return r;
-}
 // (volatile: not before the wait for the kernel that wrote them)
-__device__ __forceinline__ F8 ld_rows(const float* p) {
+__device__ __forceinline__ F8 ld_piece(const float* p) {
   F8 r;
   asm volatile("ld.global.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
                : "=l"(r.v[0]), "=l"(r.v[1]), "=l"(r.v[2]), "=l"(r.v[3]) : "l"(p));
@@ -167,14 +163,14 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
       const float* p = g.W + (size_t)n * g.K + k + 8 * q;
       const bool in = k + 8 * q < k1;
 #pragma unroll
-      for (int i = 0; i < NW; i++) w[i] = in && n + 64 * i < g.N ? ld_weights(p + (size_t)(64 * i) * g.K) : F8{};
+      for (int i = 0; i < NW; i++) w[i] = in && n + 64 * i < g.N ? ld_piece(p + (size_t)(64 * i) * g.K) : F8{};
     };
     auto fetch_a = [&](int m0, int k, int k1) {
       const int m = m0 + r0;
       const float* p = g.A + (size_t)m * g.lda + k + 8 * q;
       const bool in = k + 8 * q < k1 && (BT >= 64 || r0 < BT);
 #pragma unroll
-      for (int i = 0; i < NA; i++) a[i] = in && m + 64 * i < g.M ? ld_rows(p + (size_t)(64 * i) * g.lda) : F8{};
+      for (int i = 0; i < NA; i++) a[i] = in && m + 64 * i < g.M ? ld_piece(p + (size_t)(64 * i) * g.lda) : F8{};
     };
     const uint32_t at0 = (uint32_t)(r0 * 128) + (((q ^ r0) & 7) << 4);  // 64 rows on: 8192 bytes on, the same swizzle
     auto put = [&](const F8& v, uint32_t at, uint32_t part, __nv_bfloat162& t) {
@@ -187,8 +183,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
     };
     int u = blockIdx.x, n0, m0, split, k, k1, lu = 0, i = 0;
     unit(u, n0, m0, split, k, k1);
-    fetch_w(n0, k, k1);  // weights don't change: before the kernel in front is done
+    if (!g.late) fetch_w(n0, k, k1);  // weights don't change: before the kernel in front is done
     pdl_wait();
+    if (g.late) fetch_w(n0, k, k1);
     fetch_a(m0, k, k1);
     for (;; i++) {
       const int lun = lu;
@@ -352,10 +349,12 @@ static cudaError_t launch_f32_tc5(cudaStream_t st, const F32Tc5Args& a, int ctas
 //     32   11.2 / 12.2   14.0 / 12.6  19.1 / 16.7  40.4 / 32.7     300   35.7 / 23.7  54.7 / 24.7   120 / 63     294 / 109
 //     64   13.2 / 12.4   15.9 / 13.3  22.0 / 18.5  60.9 / 35.5    2048   75.4 / 30.0   179 / 52     275 / 83    1548 / 366
 // K below 256 leaves nothing to split: 300 x 64 x 64 9.4 / 10.3.
-bool gemm_f32_tc5_fits(const GemmArgs& g) {
-  return g.adt == DT_F32 && g.wdt == DT_F32 && g.wait_flag && !g.tile_expert && !g.a_rows && g.K >= 256 &&
-         (g.M > 32 || (g.M > 16 && (size_t)g.N * g.K >= (size_t)1 << 20)) && (g.K % 8) == 0 && (g.lda % 8) == 0 &&
+bool gemm_f32_tc5_takes(const GemmArgs& g) {
+  return g.adt == DT_F32 && g.wdt == DT_F32 && g.wait_flag && !g.tile_expert && !g.a_rows && (g.K % 8) == 0 && (g.lda % 8) == 0 &&
          (((uintptr_t)g.A | (uintptr_t)g.W) & 31) == 0;  // 32-byte loads
+}
+bool gemm_f32_tc5_fits(const GemmArgs& g) {
+  return gemm_f32_tc5_takes(g) && g.K >= 256 && (g.M > 32 || (g.M > 16 && (size_t)g.N * g.K >= (size_t)1 << 20));
 }
 
 // Token tile and slices (up to the eight that a consumer sums with one batch of loads, as many as the buffer has room
@@ -364,7 +363,7 @@ bool gemm_f32_tc5_fits(const GemmArgs& g) {
 cudaError_t launch_gemm_f32_tc5(cudaStream_t st, GemmArgs& g) {
   F32Tc5Args a{};
   a.A = (const float*)g.A; a.W = (const float*)g.W; a.lda = g.lda; a.M = g.M; a.N = g.N; a.K = g.K;
-  a.out = g.out; a.ldo = g.ldo; a.split_stride = g.split_stride; a.alpha = g.alpha; a.flag = g.wait_flag;
+  a.out = g.out; a.ldo = g.ldo; a.split_stride = g.split_stride; a.alpha = g.alpha; a.flag = g.wait_flag; a.late = g.w_late;
   a.wide = (((uintptr_t)g.out | (uintptr_t)(g.ldo * 4) | (uintptr_t)(g.split_stride * 4)) & 15) == 0;
   a.n_tiles = ceil_div(g.N, TC_BN);
   int dev = 0, sms = 0;

@@ -132,6 +132,9 @@ cudaError_t launch_norm(cudaStream_t st, const NormArgs& a);
 // arguments of the routed norm; rows: those fp32 rows.
 bool moe_route_rows_fits(int n_rows, int H, int E);
 cudaError_t launch_moe_route_rows(cudaStream_t st, const NormArgs& a, const float* rows);
+struct GemmArgs;
+bool moe_route_product_fits(const NormArgs& a, const GemmArgs& g);
+cudaError_t launch_moe_select_rows(cudaStream_t st, const NormArgs& a, const GemmArgs& g);  // g: the logits' product, launched
 
 // SwiGLU: out[t,j] = silu(h[t,j]) * h[t,F+j]   (transformer.go:50-66, mamba2.go:360-367)
 // GELU:   out[t,j] = gelu_tanh(h[t,j] + b1[j]) (transformer.go:67-78, tensor.go:181-190)
@@ -240,6 +243,7 @@ struct GemmArgs {
   size_t expert_stride;    // elements
   int max_tiles;
   int* wait_flag;          // WaitFlag::dev; null: kernels with bounded waits are not used
+  int w_late;              // W is the previous kernel's output (gemm_f32_tc5.cu)
 };
 // Single-sequence decode (M <= 8) is a chain of ~100 dependent launches of ~3 us: the W2 GEMV
 // builds its own activation from the W1 GEMV's split-K slices instead of reading what an
@@ -262,7 +266,8 @@ struct GemvPre {
 int gemv_splits(int M, int N, int K);
 cudaError_t launch_gemv(cudaStream_t st, GemmArgs& g, const GemvPre* pre = nullptr);  // M <= 8
 cudaError_t launch_gemm_simt(cudaStream_t st, GemmArgs& g);  // any M (fp32 parity mode, MoE)
-// fp32 on the tensor cores (gemm_f32_tc5.cu); launch_gemm_simt takes it where gemm_f32_tc5_fits
+// fp32 on the tensor cores (gemm_f32_tc5.cu); launch_gemm_simt takes it where gemm_f32_tc5_fits; takes: operands it can address
+bool gemm_f32_tc5_takes(const GemmArgs& g);
 bool gemm_f32_tc5_fits(const GemmArgs& g);
 cudaError_t launch_gemm_f32_tc5(cudaStream_t st, GemmArgs& g);
 

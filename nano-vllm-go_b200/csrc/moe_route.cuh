@@ -88,7 +88,7 @@ __device__ __forceinline__ void moe_select_row(float* probs, float* chs, float* 
       const unsigned key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
       const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
       bi = (int)__reduce_min_sync(0xffffffffu, (key == kmax && bi != 0x7fffffff) ? (unsigned)bi : 0x7fffffffu);
-      bv = probs[bi];  // the weight comes from the score itself
+      bv = probs[min(bi, E - 1)];  // the weight comes from the score itself
     } else {
       // warp arg-max in two redux operations instead of five shuffle rounds: probabilities are
       // >= 0, so their bit patterns order like the values (+1 keeps a genuine 0.0 above the -1 of
@@ -98,6 +98,7 @@ __device__ __forceinline__ void moe_select_row(float* probs, float* chs, float* 
       bi = (int)__reduce_min_sync(0xffffffffu, key == kmax ? (unsigned)bi : 0x7fffffffu);
       bv = kmax ? __uint_as_float(kmax - 1u) : -1.f;
     }
+    if (bi >= E) bi = s;  // no candidate left (scores that are not numbers)
     if (lane == s) {
       sel_p = bv;
       sel_i = bi;
@@ -117,6 +118,41 @@ __device__ __forceinline__ void moe_select_row(float* probs, float* chs, float* 
   if (identity_w) {
     id_w = warp_sum(id_w);
     if (lane == 0) *identity_w = id_w;
+  }
+}
+
+// The same for up to 32 experts chosen by their own scores, without groups or identity experts: a lane per expert, all in
+// registers (z: the lane's logit).
+__device__ __forceinline__ void moe_select_lanes(float z, int E, int k, size_t t, int* __restrict__ topk_idx, float* __restrict__ topk_w,
+                                                 const RouteOpts& ro) {
+  const int lane = threadIdx.x & 31;
+  float p;
+  if (ro.sigmoid) {
+    p = 1.0f / (1.0f + expf(-z));
+  } else {
+    const float mx = warp_max(lane < E ? z : -INFINITY);
+    const float e = lane < E ? expf(z - mx) : 0.f;
+    p = e / warp_sum(e);
+  }
+  unsigned key = lane < E && p >= 0.f ? __float_as_uint(p) + 1u : 0u;  // (scores that are not numbers: no candidates)
+  float sel_p = 0.f, ksum = 0.f;
+  int sel_i = 0;
+  for (int s = 0; s < k; s++) {
+    const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+    const int bi = kmax ? __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1 : s;
+    const float bv = kmax ? __uint_as_float(kmax - 1u) : -1.f;
+    if (lane == s) {
+      sel_p = bv;
+      sel_i = bi;
+    }
+    ksum += bv;
+    if (lane == bi) key = 0u;
+  }
+  if (ro.sigmoid && !ro.raw) ksum += 1e-20f;
+  if (lane < k) {
+    topk_idx[t * k + lane] = sel_i;
+    const float wgt = ro.raw ? sel_p * ro.scale : sel_p / ksum;
+    topk_w[t * k + lane] = ro.square ? wgt * wgt : wgt;
   }
 }
 
