@@ -6,9 +6,9 @@
 // the scheduler's block tables, the cached prefix of a sequence (NumCachedTokens) attended but
 // not recomputed.
 //
-// Options (AttnArgs, compiled in by the OPT template flag): a sink in the softmax's denominator (score 0 or
-// learned per head) and the output of a head times a gate per (token, head) — both outside the per-score
-// loop.  Capped scores and distance penalties stay with the mma.sync kernels of attention_window.cu: a
+// Options (AttnArgs, compiled in by OPT): a sink in the softmax's denominator (score 0 or
+// learned per head) and the output of a head times a gate per (token, head), both outside the per-score
+// loop (OPT 1); besides, a window of keys (OPT 2), whose key tiles start at the first query's first key.  Capped scores and distance penalties stay with the mma.sync kernels of attention_window.cu: a
 // transform of every score in the softmax warps (tried: 3.5 to 5.7 ms against 0.97 ms plain, 16 x 4096 tokens,
 // 16 heads of 64) made this kernel slower than those.
 //
@@ -33,6 +33,9 @@
 // costs a proxy fence): 4150 a tile and 4000 an item.  Per launch, 64 such prompts, 32 heads of 64: 255 -> 195 us; 16 heads
 // 73 -> 58; 16 x 256 queries on 3840 cached keys, 24 heads of 128: 409 -> 348 (711 -> 834 TFLOP/s); one prompt of 2048, 71
 // heads of 64: 97 -> 86.
+// Windows, per launch against the mma.sync kernel of attention_window.cu, 32 heads of 64 / 128, us: 8 x 2000 tokens, window 32
+// 170 -> 76 / 307 -> 102, 128 232 -> 76 / 413 -> 112, 1024 618 -> 219 / 1051 -> 257; 16 x 600, window 512 229 -> 85 / 375 -> 99;
+// one prompt of 40 tokens 10.4 -> 7.8 / 12.7 -> 7.6; faster at every size tried, so every layer that fits takes this kernel.
 #include <cuda.h>
 #include <stdlib.h>
 
@@ -54,7 +57,7 @@ constexpr int PT_ITEMS = 4;      // items known ahead
 
 // a query tile of one head: its first row and query position, rows in use, key tiles (0: no more items)
 struct PtItem {
-  int seq, head, row, pos, rows, n_tiles;
+  int seq, head, row, pos, rows, n_tiles, first;  // first: key tile
 };
 
 template <int HD>
@@ -79,8 +82,8 @@ __device__ __forceinline__ float ex2(float x) {
 
 }  // namespace
 
-// OPT: the options of AttnArgs (sink, gate per head) are compiled in
-template <int HD, bool OPT>
+// OPT: which options of AttnArgs are compiled in (1: sink, gate per head; 2: the window too)
+template <int HD, int OPT>
 __global__ void __launch_bounds__(PT_THREADS, 2)
 attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, AttnArgs a, Trace tr) {
@@ -176,7 +179,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           w.row = first + q0;
           w.rows = min(PT_BM, a.cu_q[w.seq + 1] - first - q0);
           w.pos = a.seq_start[w.seq] + q0;
-          w.n_tiles = (w.pos + w.rows + BN - 1) / BN;  // keys [0, pos + rows) are visible to this tile
+          w.first = OPT > 1 ? max(0, w.pos - a.window + 1) / BN : 0;
+          w.n_tiles = (w.pos + w.rows + BN - 1) / BN - w.first;  // keys up to pos + rows are visible to this tile
         }
         const int s = it % PT_ITEMS;
         if (!wait(b_iempty + 8 * s, it / PT_ITEMS + 1)) break;
@@ -207,7 +211,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         __syncwarp();
         for (int j = 0; j < w.n_tiles; j++, g++) {
-          const int k0 = j * BN, st = g % ST;
+          const int k0 = (w.first + j) * BN, st = g % ST;
           const int prow = (bt[k0 / KV_BLOCK] * a.nkv + kvh) * KV_BLOCK + (k0 % KV_BLOCK);
           if (!(ok = wait(b_kempty + 8 * st, g / ST + 1))) break;
           if (elect_one()) {
@@ -327,7 +331,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       float m_used = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_tiles; j++, g++) {
         // columns of this tile up to which the warp's first row sees keys (its last row: 31 more)
-        const int lim = w.pos + q * 32 - j * BN;
+        const int lim = w.pos + q * 32 - (w.first + j) * BN;
+        const int low = lim - a.window + 1;  // and from which on (OPT 2)
         if (!(ok = wait(b_sfull, g))) break;
         tc_fence_after();
         // the whole S row of this tile in registers: all loads issued, one wait
@@ -341,7 +346,12 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         float mx = -INFINITY;
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (c0 > lim + 31) continue;  // no row of the warp sees these keys: p = 0 below
+          if (c0 > lim + 31 || (OPT > 1 && c0 + 31 < low)) continue;  // no row of the warp sees these keys: p = 0 below
+          if (OPT > 1 && c0 < low + 31) {
+#pragma unroll
+            for (int c = 0; c < 32; c++)
+              if (c0 + c < low + lane) sr[c0 + c] = 0xff800000u;
+          }
           if (c0 + 31 > lim) {
 #pragma unroll
             for (int c = 0; c < 32; c++)
@@ -367,7 +377,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         uint32_t pk[BN / 2];
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (c0 > lim + 31) {
+          if (c0 > lim + 31 || (OPT > 1 && c0 + 31 < low)) {
 #pragma unroll
             for (int c = 0; c < 32; c += 2) pk[(c0 + c) / 2] = 0;
             continue;
@@ -441,7 +451,7 @@ bool attn_prefill_tc5_enabled() {
   return on;
 }
 
-template <int HD, bool OPT>
+template <int HD, int OPT>
 static cudaError_t prefill_tc5_launch(cudaStream_t st, const AttnArgs& a) {
   using Cf = PtCfg<HD>;
   const int pool_rows = a.pool_blocks * a.nkv * KV_BLOCK;
@@ -467,9 +477,9 @@ static cudaError_t prefill_tc5_launch(cudaStream_t st, const AttnArgs& a) {
 cudaError_t launch_attn_prefill_tc5(cudaStream_t st, const AttnArgs& a) {
   if (a.n_qtiles <= 0) return cudaSuccess;
   if (a.pool_blocks <= 0 || a.total_rows <= 0) return cudaErrorInvalidValue;
-  if (a.sink || a.head_gate)
-    return a.hd == 64 ? prefill_tc5_launch<64, true>(st, a) : prefill_tc5_launch<128, true>(st, a);
-  return a.hd == 64 ? prefill_tc5_launch<64, false>(st, a) : prefill_tc5_launch<128, false>(st, a);
+  if (a.window > 0) return a.hd == 64 ? prefill_tc5_launch<64, 2>(st, a) : prefill_tc5_launch<128, 2>(st, a);
+  if (a.sink || a.head_gate) return a.hd == 64 ? prefill_tc5_launch<64, 1>(st, a) : prefill_tc5_launch<128, 1>(st, a);
+  return a.hd == 64 ? prefill_tc5_launch<64, 0>(st, a) : prefill_tc5_launch<128, 0>(st, a);
 }
 
 }  // namespace nvllm

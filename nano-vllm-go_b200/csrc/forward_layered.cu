@@ -665,6 +665,28 @@ static int run_postnorm(nvllm_handle* h, Pending* p, const float* w, int T, bool
   return NVLLM_OK;
 }
 
+static bool attention_on_tc5(const nvllm_handle* h, const nvllm_layer_spec& s) {
+  return h->adt == DT_BF16 && h->kvdt == DT_BF16 && s.dim == s.vdim && (s.dim == 64 || s.dim == 128) &&
+         s.softcap == 0.f && s.dist_slope == 0.f && !s.diff_maps && attn_prefill_tc5_enabled();
+}
+// a prompt step's attention on the tcgen05 kernel, from the arguments of the other kernels
+static int attention_tc5(nvllm_handle* h, const nvllm_layer_spec& s, const WinAttnArgs& a, const float* head_gate) {
+  const StepLayout& L = h->lay;
+  AttnArgs t{};
+  t.q = a.q; t.out = a.out; t.qdt = h->adt; t.kvdt = h->kvdt;
+  t.kpool = a.kpool; t.vpool = a.vpool;
+  t.n_seqs = L.n; t.nh = s.heads; t.nkv = s.kv_heads; t.hd = s.dim; t.scale = s.scale;
+  t.block_tables = a.block_tables; t.max_blocks = a.max_blocks;
+  t.cu_q = a.cu_q; t.seq_start = a.seq_start; t.seq_len = a.seq_len;
+  t.tile_seq = a.tile_seq; t.tile_q0 = a.tile_q0; t.n_qtiles = L.n_qtiles;
+  t.pool_blocks = h->num_blocks; t.total_rows = L.T; t.sm_count = h->sm_count;
+  t.tickets = (int*)h->ws.chain_ctr + 16; t.wait_flag = h->waits.dev;
+  t.window = s.window; t.sink = s.sink; t.sink_w = a.sink_w;
+  t.head_gate = head_gate; t.gate_ld = s.heads;
+  LAUNCH(h, launch_attn_prefill_tc5(h->stream, t));
+  return NVLLM_OK;
+}
+
 static int mixer_window_attention(nvllm_handle* h, const ListedLayer& y, Pending* out) {
   const StepLayout& L = h->lay;
   Workspace& w = h->ws;
@@ -704,7 +726,11 @@ static int mixer_window_attention(nvllm_handle* h, const ListedLayer& y, Pending
     const double pairs = std::min(L.attn_pairs, (double)T * win);
     ProfScope ps(h, L.prefill ? NVLLM_K_ATTN_PREFILL : NVLLM_K_ATTN_DECODE, keys * s.kv_heads * (s.dim + s.vdim) * kvsz,
                  2.0 * s.heads * (s.dim + s.vdim) * pairs, (double)T * (s.heads * s.dim + y.ov_p) * asz);
-    LAUNCH(h, launch_winattn(h->stream, h->adt, h->kvdt, a));
+    if (L.prefill && h->attn_qtile == 128 && attention_on_tc5(h, s)) {
+      if ((rc = attention_tc5(h, s, a, nullptr))) return rc;
+    } else {
+      LAUNCH(h, launch_winattn(h->stream, h->adt, h->kvdt, a));
+    }
   }
   return run_gemm(h, w.attn_out, y.ov_p, y.w_o, T, H, y.ov_p, 1.f, w.ws_b, w.ws_b_floats, H, out);
 }
@@ -1210,10 +1236,6 @@ static int ffn_moe_gated(nvllm_handle* h, const ListedLayer& y, float* topk_w, P
 // Prefill steps of an attention layer whose keys and values have one size, 64 or 128, in bf16, and whose scores are
 // neither capped nor biased by the distance nor windowed nor two maps (a sink and head gates are fine) run on the tcgen05 kernel
 // (attention_tc5.cu, 128 queries per tile); everything else on the window kernels (attention_window.cu)
-static bool attention_on_tc5(const nvllm_handle* h, const nvllm_layer_spec& s) {
-  return h->adt == DT_BF16 && h->kvdt == DT_BF16 && s.dim == s.vdim && (s.dim == 64 || s.dim == 128) &&
-         s.softcap == 0.f && s.dist_slope == 0.f && s.window == 0 && !s.diff_maps && attn_prefill_tc5_enabled();
-}
 
 // Grouped-query attention over the cached prefix (or a window of it) with the options of the spec
 static int mixer_attention(nvllm_handle* h, const ListedLayer& y, int run_idx, Pending* out) {
@@ -1281,18 +1303,7 @@ static int mixer_attention(nvllm_handle* h, const ListedLayer& y, int run_idx, P
                  keys * s.kv_heads * (maps * s.dim + s.vdim) * kvsz, 2.0 * s.heads * maps * (s.dim + s.vdim) * pairs_seen,
                  (double)T * (y.n_q + y.ov_p) * asz);
     if (L.prefill && h->attn_qtile == 128 && attention_on_tc5(h, s)) {
-      AttnArgs t{};
-      t.q = w.q; t.out = w.attn_out; t.qdt = h->adt; t.kvdt = h->kvdt;
-      t.kpool = a.kpool; t.vpool = a.vpool;
-      t.n_seqs = L.n; t.nh = s.heads; t.nkv = s.kv_heads; t.hd = s.dim; t.scale = s.scale;
-      t.block_tables = a.block_tables; t.max_blocks = a.max_blocks;
-      t.cu_q = a.cu_q; t.seq_start = a.seq_start; t.seq_len = a.seq_len;
-      t.tile_seq = a.tile_seq; t.tile_q0 = a.tile_q0; t.n_qtiles = L.n_qtiles;
-      t.pool_blocks = h->num_blocks; t.total_rows = T; t.sm_count = h->sm_count;
-      t.tickets = (int*)w.chain_ctr + 16; t.wait_flag = h->waits.dev;
-      t.sink = s.sink; t.sink_w = a.sink_w;
-      t.head_gate = s.head_gate ? w.att_gate : nullptr; t.gate_ld = s.heads;
-      LAUNCH(h, launch_attn_prefill_tc5(h->stream, t));
+      if ((rc = attention_tc5(h, s, a, s.head_gate ? w.att_gate : nullptr))) return rc;
     } else {
       LAUNCH(h, launch_winattn(h->stream, h->adt, h->kvdt, a));
     }
@@ -2182,7 +2193,7 @@ extern "C" int nvllm_create_layered(const nvllm_layered_config* c, const nvllm_l
         y.n_v = own ? s.kv_heads * s.vdim : 0;
         y.n_in = y.n_q + y.n_k + y.n_v;
         // every prefill tile list of the step is built for one query-tile size: the smallest any layer wants
-        const int qt = winattn_qtile(h->adt, h->kvdt, s.dim, s.vdim);
+        const int qt = attention_on_tc5(h, s) ? 128 : winattn_qtile(h->adt, h->kvdt, s.dim, s.vdim);
         win_qtile = win_qtile ? std::min(win_qtile, qt) : qt;
       }
       AL(y.post1_w, (size_t)W * 4);

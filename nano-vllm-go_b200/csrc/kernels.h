@@ -455,6 +455,7 @@ struct AttnArgs {
   int* tickets;        // tcgen05 prefill kernel: counter that deals its items out, zero between kernels (null: in turn)
   int* wait_flag;      // WaitFlag::dev of its waits
   // options of the tcgen05 prefill kernel (all zero / null: plain causal softmax)
+  int window;              // > 0: a query sees its last `window` keys, itself included
   int sink;                // 1: the softmax denominator holds one more term, exp(sink_w[h]) (exp(0) without sink_w)
   const float* sink_w;     // [nh] or null
   const float* head_gate;  // [rows, gate_ld] or null: the output of (row, head) times head_gate[row * gate_ld + head]
