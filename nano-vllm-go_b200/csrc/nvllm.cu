@@ -294,7 +294,6 @@ int nvllm_set_layer_types(nvllm_handle* h, const int32_t* types, int n_layers) {
       h->weight_bytes += sizes[i];
     }
   }
-  h->spec_enabled = 0;  // a discarded speculative step would leave its SSM state in the block
   return NVLLM_OK;
 }
 
@@ -390,7 +389,7 @@ int nvllm_set_graphs(nvllm_handle* h, int enabled) {
 
 int nvllm_set_speculation(nvllm_handle* h, int enabled) {
   if (!h) return NVLLM_ERR_INVALID;
-  h->spec_enabled = (enabled && h->n_mamba == 0) ? 1 : 0;  // see nvllm_set_layer_types
+  h->spec_enabled = enabled ? 1 : 0;  // (models with recurrent state never speculate: run.cu)
   return NVLLM_OK;
 }
 

@@ -150,7 +150,7 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
 // sequences, one token longer, last token = the one just returned, same block tables, greedy —
 // and only has to wait for it, or asks for something else and restages everything as usual.
 // A speculative step that is thrown away has only written K/V at the next position of each
-// sequence, a slot nothing reads before its owner writes it; but the call after it waits for it, so misses in a row pause
+// sequence, a slot nothing reads before its owner writes it (models with recurrent state never speculate); but the call after it waits for it, so misses in a row pause
 // the speculation: 1, 2, 4, ... 16 calls from the second one on.  (A workload of prompts alone threw a decode step
 // away at every second call.)
 static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_graph = nullptr);
@@ -179,6 +179,8 @@ static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, con
 static void try_speculate(nvllm_handle* h, int n, const float* temperature) {
   h->spec_pending = false;
   if (!h->spec_enabled || !graph_usable(h, n)) return;
+  // a step that is thrown away would leave recurrent state, which steps update in place, one token ahead
+  if (h->state_slot_floats || h->n_mamba) return;
   if (h->spec_skip > 0) {
     h->spec_skip--;
     return;

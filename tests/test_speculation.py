@@ -5,6 +5,7 @@ import pytest
 
 from helpers import C, W
 import nvllm_pkg
+import test_zozonex as zozonex
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,31 @@ def test_prompts_pause_it_and_decoding_brings_it_back():
         assert (la is None) == (lb is None)
         if la is not None:
             np.testing.assert_array_equal(la, lb)  # same kernels, same order
+
+
+def test_recurrent_state_is_not_stepped_ahead():
+    """Calls that a step issued ahead would not match (another token, another batch), on a model whose steps update state in
+    place: the same with speculation asked for as without."""
+    cfg, w = zozonex.random_weights(zozonex.mixed_model(), 7)
+    prompts = [W.random_prompt(cfg.vocab_size, 9 + 4 * i, 40 + i).tolist() for i in range(3)]
+
+    def drive(spec):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, w.items(), precision=C.PREC_FP32, num_kv_blocks=3, sampling=None, num_state_slots=3)
+        try:
+            run.set_speculation(spec)
+            seqs = [list(p) for p in prompts]
+            outs = [run.run_flat(seqs, True, [0] * 3, [[0], [1], [2]], [0.0] * 3, want_logits=True, state_slots=[2, 0, 1])]
+            for k in range(8):
+                for i, (s, t) in enumerate(zip(seqs, outs[-1][0])):
+                    s.append(5 if (k, i) == (2, 1) else int(t))
+                if k == 5:  # the first sequence alone, before all three
+                    outs.append(run.run_flat(seqs[:1], False, None, [[0]], [0.0], want_logits=True, state_slots=[2]))
+                    seqs[0].append(int(outs[-1][0][0]))
+                outs.append(run.run_flat(seqs, False, None, [[0], [1], [2]], [0.0] * 3, want_logits=True, state_slots=[2, 0, 1]))
+            return outs
+        finally:
+            run.close()
+
+    for (a, la), (b, lb) in zip(drive(False), drive(True)):
+        np.testing.assert_array_equal(a, b)
+        np.testing.assert_array_equal(la, lb)
