@@ -181,6 +181,7 @@ static void try_speculate(nvllm_handle* h, int n, const float* temperature) {
   if (!h->spec_enabled || !graph_usable(h, n)) return;
   // a step that is thrown away would leave recurrent state, which steps update in place, one token ahead
   if (h->state_slot_floats || h->n_mamba) return;
+  if (h->fetched_rows > 0) return;  // its logits would land on rows that the caller is still to fetch
   if (h->spec_skip > 0) {
     h->spec_skip--;
     return;
@@ -307,7 +308,8 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   const nvllm_config& c = h->cfg;
   if (h->spec_pending) {
     h->spec_pending = false;
-    if (speculation_hit(h, n, is_prefill, token_ids, cu_seqlens, block_tables, cu_blocks, temperature)) {
+    // (a step issued ahead has none of the further logits rows that this call may have to bring)
+    if (h->want_rows.empty() && speculation_hit(h, n, is_prefill, token_ids, cu_seqlens, block_tables, cu_blocks, temperature)) {
       // the requested step is already running (or done): collect it
       cudaStream_t st = h->stream;
       NV_CHECK(h, cudaMemcpyAsync(h->h_out, h->ws.out_tokens, (size_t)n * 4, cudaMemcpyDeviceToHost, st));

@@ -70,3 +70,32 @@ def test_recurrent_state_is_not_stepped_ahead():
     for (a, la), (b, lb) in zip(drive(False), drive(True)):
         np.testing.assert_array_equal(a, b)
         np.testing.assert_array_equal(la, lb)
+
+
+def test_requested_logits_rows():
+    """Further rows asked for (nvllm_request_logits) in calls that a step issued ahead would answer or overwrite."""
+    cfg = C.tiny_llama(hidden=1032)  # the head's products of few rows are split along k: another step's slices are elsewhere
+    prompts = [W.random_prompt(cfg.vocab_size, 18 + 7 * i, 300 + i).tolist() for i in range(3)]
+    weights = list(W.random_weights(cfg, 5))
+
+    def drive(spec):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, weights, precision=C.PREC_FP32, num_kv_blocks=3, sampling=None)
+        try:
+            run.set_speculation(spec)
+            seqs, rows, outs, hits = [list(p) for p in prompts], [3, 20, 40, 7], [], 0
+            for k in range(9):
+                want = rows if k == 0 else [2, 0] if k in (4, 7) else []
+                run.request_logits(want)
+                out, logits = run.run_flat(seqs, k == 0, [0] * 3, [[0], [1], [2]], [0.0] * 3, want_logits=True)
+                hits += run.last_stats.h2d_bytes == 0
+                outs += [out, logits] + ([run.fetch_logits(len(want))] if want else [])
+                for s, t in zip(seqs, out):
+                    s.append(int(t))
+            return outs, hits
+        finally:
+            run.close()
+
+    (want, none), (got, hits) = drive(False), drive(True)
+    assert none == 0 and hits >= 3
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
