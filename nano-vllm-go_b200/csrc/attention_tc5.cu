@@ -477,7 +477,12 @@ static cudaError_t prefill_tc5_launch(cudaStream_t st, const AttnArgs& a) {
 cudaError_t launch_attn_prefill_tc5(cudaStream_t st, const AttnArgs& a) {
   if (a.n_qtiles <= 0) return cudaSuccess;
   if (a.pool_blocks <= 0 || a.total_rows <= 0) return cudaErrorInvalidValue;
-  if (a.window > 0) return a.hd == 64 ? prefill_tc5_launch<64, 2>(st, a) : prefill_tc5_launch<128, 2>(st, a);
+  if (a.window > 0) {
+    AttnArgs b = a;
+    // (a window past the longest sequence limits nothing, and the masks' differences of positions stay within 32 bits)
+    b.window = (int)std::min((long long)a.window, (long long)a.max_blocks * KV_BLOCK);
+    return a.hd == 64 ? prefill_tc5_launch<64, 2>(st, b) : prefill_tc5_launch<128, 2>(st, b);
+  }
   if (a.sink || a.head_gate) return a.hd == 64 ? prefill_tc5_launch<64, 1>(st, a) : prefill_tc5_launch<128, 1>(st, a);
   return a.hd == 64 ? prefill_tc5_launch<64, 0>(st, a) : prefill_tc5_launch<128, 0>(st, a);
 }
