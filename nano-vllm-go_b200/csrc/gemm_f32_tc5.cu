@@ -12,8 +12,9 @@
 // warps sum the stages (tensor memory, double-buffered) and write the tile.  Persistent: units (weight tile, token tile,
 // k slice) go round the CTAs.
 //
-// An operand with a part that is not finite (infinity, NaN, or a value that bf16 rounds to infinity) would turn into NaN
-// in the split where fp32 arithmetic has an infinity: units that met one are computed again with FMAs.
+// An operand with a part that is not finite (infinity, NaN, or a value that bf16 rounds to infinity) turns into NaN in the
+// split, and products out of range into infinities of both signs, where fp32 arithmetic may have an infinity: results that
+// are not finite are computed again with FMAs, by a warp each, until the sum is NaN.
 //
 // Bound by the MMAs' reads of shared memory (24 MMAs a stage, 60 cycles each at BT = 64, 79 at 128) with the splitters
 // close behind: with eight of their warps instead of sixteen a stage took 1.57 / 1.85 us instead of 1.19 / 1.55.
@@ -84,13 +85,11 @@ __device__ __forceinline__ uint32_t round_bf16x2(unsigned long long v) {
 __device__ __forceinline__ unsigned long long widen_bf16x2(uint32_t h) {
   return pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u));
 }
-// the three parts of two values; t turns into NaN where a part is not finite
-__device__ __forceinline__ void split2(unsigned long long x, uint32_t& hi, uint32_t& mid, uint32_t& lo, __nv_bfloat162& t) {
+__device__ __forceinline__ void split2(unsigned long long x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = round_bf16x2(x);
   const unsigned long long r = sub2(x, widen_bf16x2(hi));
   mid = round_bf16x2(r);
   lo = round_bf16x2(sub2(r, widen_bf16x2(mid)));
-  t = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo), __float2bfloat162_rn(0.f), t);
 }
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t (&v)[4]) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
@@ -102,6 +101,24 @@ __device__ __forceinline__ void tmem_ld_32x8_nowait(uint32_t taddr, uint32_t (&r
                : "memory");
 }
 
+// the whole warp: sum of a[k] w[k], k0 <= k < k1 (multiples of 8), in fp32; ends early once it is NaN.  Rare: kept out of the
+// kernel's registers.
+__device__ __noinline__ float warp_dot(const float* a, const float* w, int k0, int k1, int lane) {
+  float v = 0.f;
+  for (int k = k0 + 4 * lane; __any_sync(0xffffffffu, k < k1) && !__any_sync(0xffffffffu, v != v);) {
+#pragma unroll
+    for (int i = 0; i < 4; i++, k += 128) {
+      if (k >= k1) continue;
+      const float4 x = __ldcg(reinterpret_cast<const float4*>(a + k)), y = __ldcg(reinterpret_cast<const float4*>(w + k));
+      v = fmaf(x.x, y.x, v);
+      v = fmaf(x.y, y.y, v);
+      v = fmaf(x.z, y.z, v);
+      v = fmaf(x.w, y.w, v);
+    }
+  }
+  return warp_sum(v);
+}
+
 template <int BT>
 __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args g, Trace tr) {
   using Z = FtSizes<BT>;
@@ -109,7 +126,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) unsigned long long bar_s[2 * Z::STAGES + 4];
   __shared__ uint32_t tmem_s, dead_s;
-  __shared__ volatile uint32_t odd_s[8];  // units with an operand that is not finite (a splitter is at most six units ahead)
   const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_full = smem_u32(bar_s), bar_empty = bar_full + 8 * Z::STAGES;
   const uint32_t bar_dfull = bar_empty + 8 * Z::STAGES, bar_dempty = bar_dfull + 16;
@@ -129,7 +145,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (lane < 8) odd_s[lane] = 0;
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "r"((uint32_t)(2 * Z::ACC))
                  : "memory");
@@ -173,40 +188,36 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
       for (int i = 0; i < NA; i++) a[i] = in && m + 64 * i < g.M ? ld_piece(p + (size_t)(64 * i) * g.lda) : F8{};
     };
     const uint32_t at0 = (uint32_t)(r0 * 128) + (((q ^ r0) & 7) << 4);  // 64 rows on: 8192 bytes on, the same swizzle
-    auto put = [&](const F8& v, uint32_t at, uint32_t part, __nv_bfloat162& t) {
+    auto put = [&](const F8& v, uint32_t at, uint32_t part) {
       uint32_t h[4], m[4], l[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) split2(v.v[e], h[e], m[e], l[e], t);
+      for (int e = 0; e < 4; e++) split2(v.v[e], h[e], m[e], l[e]);
       st_shared_v4(at, h);
       st_shared_v4(at + part, m);
       st_shared_v4(at + 2 * part, l);
     };
-    int u = blockIdx.x, n0, m0, split, k, k1, lu = 0, i = 0;
+    int u = blockIdx.x, n0, m0, split, k, k1, i = 0;
     unit(u, n0, m0, split, k, k1);
     if (!g.late) fetch_w(n0, k, k1);  // weights don't change: before the kernel in front is done
     pdl_wait();
     if (g.late) fetch_w(n0, k, k1);
     fetch_a(m0, k, k1);
     for (;; i++) {
-      const int lun = lu;
       k += TC_BK;  // the next stage
       if (k >= k1) {
         u += gridDim.x;
-        lu++;
         if (u < units) unit(u, n0, m0, split, k, k1);
       }
       const int s = i % Z::STAGES;
       if (!wait_limited(bar_empty + 8 * s, ((i / Z::STAGES) & 1) ^ 1, dead, g.flag)) break;
       const uint32_t base = tiles + s * Z::STAGE + at0;
-      __nv_bfloat162 t = __float2bfloat162_rn(0.f);
 #pragma unroll
-      for (int j = 0; j < NW; j++) put(w[j], base + 8192 * j, Z::W_PART, t);
+      for (int j = 0; j < NW; j++) put(w[j], base + 8192 * j, Z::W_PART);
       if (u < units) fetch_w(n0, k, k1);
 #pragma unroll
       for (int j = 0; j < NA; j++)
-        if (BT >= 64 || r0 < BT) put(a[j], base + 3 * Z::W_PART + 8192 * j, Z::A_PART, t);
+        if (BT >= 64 || r0 < BT) put(a[j], base + 3 * Z::W_PART + 8192 * j, Z::A_PART);
       if (u < units) fetch_a(m0, k, k1);
-      if (__hisnan(t.x) || __hisnan(t.y)) odd_s[lun & 7] = 1;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_full + 8 * s);
@@ -253,9 +264,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
     constexpr int NC = Z::NC;
     const int qr = warp & 3, c0 = (warp >> 2) * NC;
     pdl_wait();
-    int i = 0, lu = 0;
+    int i = 0;
     bool ok = true;
-    for (int u = blockIdx.x; ok && u < units; u += gridDim.x, lu++) {
+    for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
       int n0, m0, split, k0, k1;
       unit(u, n0, m0, split, k0, k1);
       float sum[NC];
@@ -278,25 +289,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
         }
         tc_fence_before();
         __syncwarp();
-        // the splitters' notes of this unit are read before its last accumulator is handed back
-        if (k + TC_BK < k1 && lane == 0) mbar_arrive(bar_dempty + 8 * b);
+        if (lane == 0) mbar_arrive(bar_dempty + 8 * b);
       }
       if (!warps_agree<32 * FT_SUM>(ok)) break;
       const int n = n0 + qr * 32 + lane;
-      const bool odd = odd_s[lu & 7] != 0;
-      named_bar(1, 32 * FT_SUM);  // all have read it
-      if (threadIdx.x == 0) odd_s[lu & 7] = 0;
-      if (lane == 0) mbar_arrive(bar_dempty + 8 * ((i - 1) & 1));
       float* out = g.out + (size_t)split * g.split_stride + (size_t)(m0 + c0) * g.ldo;
-      if (odd) {
-        if (n < g.N)
-          for (int c = 0; c < NC && m0 + c0 + c < g.M; c++) {
-            float v = 0.f;
-            for (int k = k0; k < k1; k++) v = fmaf(g.A[(size_t)(m0 + c0 + c) * g.lda + k], g.W[(size_t)n * g.K + k], v);
-            out[(size_t)c * g.ldo + n] = g.alpha * v;
-          }
-        continue;
-      }
       // through shared memory, a row of 128 columns per store: short code (what a launch runs once, it also fetches once)
       float* stage = reinterpret_cast<float*>(smem_raw + (tiles - smem_u32(smem_raw)) + Z::STAGES * Z::STAGE) + (warp >> 2) * (Z::CHUNK * TC_BN);
 #pragma unroll
@@ -304,6 +301,20 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc5_kernel(F32Tc5Args 
         named_bar(2 + (warp >> 2), 128);  // the chunk before is out
 #pragma unroll
         for (int c = 0; c < Z::CHUNK; c++) stage[c * TC_BN + qr * 32 + lane] = g.alpha * sum[cc + c];
+        uint32_t odd = 0;  // of the chunk's tokens, those whose result is not finite
+#pragma unroll
+        for (int c = 0; c < Z::CHUNK; c++) odd |= (uint32_t)(fabsf(sum[cc + c]) < INFINITY ? 0 : 1) << c;
+        // (rows past M or N count for nothing: their zeros turn into NaN where the other operand has one)
+        const int valid = n < g.N ? min(Z::CHUNK, g.M - m0 - c0 - cc) : 0;
+        if (valid < Z::CHUNK) odd &= valid > 0 ? (1u << valid) - 1 : 0u;
+        for (unsigned lanes; (lanes = __ballot_sync(0xffffffffu, odd != 0)) != 0;) {
+          const int who = __ffs(lanes) - 1, c = __ffs(__shfl_sync(0xffffffffu, odd, who)) - 1;
+          const float v = g.alpha * warp_dot(g.A + (size_t)(m0 + c0 + cc + c) * g.lda, g.W + (size_t)__shfl_sync(0xffffffffu, n, who) * g.K, k0, k1, lane);
+          if (lane == who) {
+            stage[c * TC_BN + qr * 32 + lane] = v;
+            odd &= odd - 1;
+          }
+        }
         named_bar(2 + (warp >> 2), 128);
         const int nn = n0 + 4 * lane, rows = min(Z::CHUNK, g.M - m0 - c0 - cc);
 #pragma unroll 2

@@ -77,3 +77,33 @@ def test_operands_without_finite_parts(M):
     assert np.array_equal(out[~finite & ~np.isnan(want)], want[~finite & ~np.isnan(want)].astype(np.float32))
     bound = 2.0 ** -24 * 520 * (np.abs(np.where(np.isfinite(A), A, 0)).astype(np.float64) @ np.abs(np.where(np.isfinite(Wm), Wm, 0)))
     assert (np.abs(out[finite] - want[finite]) <= bound[finite]).all()
+
+
+@pytest.mark.parametrize("M", [40, 200])
+def test_products_out_of_range(M):
+    """Finite operands whose products are not: the parts' products overflow to both infinities, the result has one."""
+    A, Wm = _operands(M, 300, 520)
+    A[7] = np.abs(A[7]) * 1e30 + 1e29
+    Wm[:, 33] = -np.abs(Wm[:, 33]) * 1e25 - 1e24
+    out, ran = _run(A, Wm)
+    assert ran
+    want = A.astype(np.float64) @ Wm.astype(np.float64)
+    assert np.isfinite(out).sum() == out.size - 1 and out[7, 33] == -np.inf and want[7, 33] < -1e53
+    bound = 2.0 ** -24 * 520 * (np.abs(A).astype(np.float64) @ np.abs(Wm))
+    finite = np.isfinite(out)
+    assert (np.abs(out - want)[finite] <= bound[finite]).all()
+
+
+@pytest.mark.parametrize("rows,cols", [(slice(None), slice(0)), (slice(0), slice(None)), (slice(130, 131), slice(5, 6))])
+def test_rows_of_nan(rows, cols):
+    """All of A, all of W, a row and a column; token and weight tiles with ends past the matrices, several units per CTA."""
+    A, Wm = _operands(300, 9001, 1096)
+    A[rows, 1095], Wm[0, cols] = np.nan, np.nan
+    out, ran = _run(A, Wm)
+    assert ran
+    nan = np.zeros(out.shape, bool)
+    nan[rows], nan[:, cols] = True, True
+    assert np.array_equal(np.isnan(out), nan)
+    if not nan.all():
+        a, w = np.where(np.isnan(A), 0, A), np.where(np.isnan(Wm), 0, Wm)
+        assert np.abs(out - a.astype(np.float64) @ w)[~nan].max() <= 1e-4  # (of some 30)
