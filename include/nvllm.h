@@ -556,7 +556,8 @@ int nvllm_set_graphs(nvllm_handle* h, int enabled);
  * the GPU does not idle during the host's turnaround.  The next nvllm_run that asks for exactly
  * that step (same lengths + 1, last token = the one returned, same block tables) only waits
  * for it and copies nothing to the device; any other call restages everything as usual.
- * Misses in a row pause it for 1, 2, 4, ... 16 calls. */
+ * Misses in a row pause it for 1, 2, 4, ... 16 calls (steps issued by prefill and by decode calls are counted
+ * apart).  Models with recurrent state, whose steps update it in place, never speculate. */
 int nvllm_set_speculation(nvllm_handle* h, int enabled);
 
 /* GetVocabSize / GetModelConfig (purego/generic_runner.go:184-196). */

@@ -378,7 +378,10 @@ struct nvllm_handle {
   int spec_enabled = 1;
   bool spec_pending = false;
   bool spec_used_graph = false;  // the in-flight speculative step replayed a graph
-  int spec_misses = 0, spec_skip = 0;  // misses in a row, calls that do not speculate because of them
+  struct SpecPause {
+    int misses = 0, skip = 0;  // misses in a row, calls that do not speculate because of them
+  } spec_pause[2];             // of steps issued by decode and by prefill calls (run.cu)
+  int spec_kind = 0;           // which of them issued the last one
   std::vector<int32_t> spec_len, spec_nb, spec_bt;  // per-sequence lengths / block tables of the last call
   // device-resident decode state as the host knows it: context length (incl. the token the last
   // step appended) and block-table extent of every sequence — nvllm_run_resident refuses to step

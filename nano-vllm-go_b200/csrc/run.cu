@@ -150,9 +150,14 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
 // sequences, one token longer, last token = the one just returned, same block tables, greedy —
 // and only has to wait for it, or asks for something else and restages everything as usual.
 // A speculative step that is thrown away has only written K/V at the next position of each
-// sequence, a slot nothing reads before its owner writes it (models with recurrent state never speculate); but the call after it waits for it, so misses in a row pause
-// the speculation: 1, 2, 4, ... 16 calls from the second one on.  (A workload of prompts alone threw a decode step
-// away at every second call.)
+// sequence, a slot nothing reads before its owner writes it (models with recurrent state never speculate); but the call
+// after it waits for it, so misses in a row pause the speculation: 1, 2, 4, ... 16 calls.  Steps issued by prefill calls
+// and by decode calls count apart.  Those of prefill calls miss where prompts arrive while others decode (the next call
+// is the merged batch) or come alone, and pause from the first miss on; those of decode calls miss once per arrival or
+// end of a sequence and hit in between, and pause from the second miss in a row on.  Per 64 decode steps of 32 sequences
+// through four Llama-1B layers, ms: a prompt every step / 3 / 8 steps 57.7 / 30.0 / 21.9 when any miss kept just its own
+// call from issuing, 46.2 / 34.1 / 22.7 with one count for both from the second miss on, 47.2 / 29.5 / 21.1 so; a
+// sequence that ends every second step (48 steps) 24.7, 18.1, 17.6.
 static int resident_step(nvllm_handle* h, nvllm_run_stats* stats, bool* used_graph = nullptr);
 // After a synchronise: did a bounded wait of this handle's kernels run out?  Then neither the results nor the device state
 // that a resident, speculative or repeated step would start from are used.
@@ -182,8 +187,10 @@ static void try_speculate(nvllm_handle* h, int n, const float* temperature) {
   // a step that is thrown away would leave recurrent state, which steps update in place, one token ahead
   if (h->state_slot_floats || h->n_mamba) return;
   if (h->fetched_rows > 0) return;  // its logits would land on rows that the caller is still to fetch
-  if (h->spec_skip > 0) {
-    h->spec_skip--;
+  h->spec_kind = h->lay.prefill ? 1 : 0;
+  nvllm_handle::SpecPause& pause = h->spec_pause[h->spec_kind];
+  if (pause.skip > 0) {
+    pause.skip--;
     return;
   }
   for (int i = 0; i < n; i++) {
@@ -320,13 +327,15 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
       }
       h->run_lay = h->lay;
       h->run_lay_ok = true;
-      h->spec_misses = 0;
+      h->spec_pause[h->spec_kind].misses = 0;
       return finish_step(h, n, cu_seqlens, block_tables, cu_blocks, temperature, out_tokens, out_logits, stats, n, 0, d2h,
                          h->spec_used_graph);
     }
     // missed: the caller is not stepping one batch
-    h->spec_misses = std::min(h->spec_misses + 1, 6);
-    h->spec_skip = h->spec_misses > 1 ? 1 << (h->spec_misses - 2) : 0;
+    nvllm_handle::SpecPause& pause = h->spec_pause[h->spec_kind];
+    pause.misses = std::min(pause.misses + 1, 6);
+    const int pauses = pause.misses - (h->spec_kind == 0 ? 1 : 0);
+    pause.skip = pauses > 0 ? 1 << std::min(pauses - 1, 4) : 0;
   }
   h->resident_ok = false;
   h->run_lay_ok = false;
@@ -637,6 +646,7 @@ extern "C" int nvllm_run_resident(nvllm_handle* h, nvllm_run_stats* stats) {
   if (!h) return NVLLM_ERR_INVALID;
   if (h->spec_pending) {  // the step asked for is the one already in flight
     h->spec_pending = false;
+    h->spec_pause[h->spec_kind].misses = 0;
     fill_stats(h, stats, h->lay.n, 0, 0);
     if (stats) stats->used_graph = h->spec_used_graph ? 1 : 0;
     return NVLLM_OK;

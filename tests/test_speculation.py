@@ -44,6 +44,40 @@ def test_prompts_pause_it_and_decoding_brings_it_back():
             np.testing.assert_array_equal(la, lb)  # same kernels, same order
 
 
+def test_arrivals_discard_one_step_each():
+    """Prompts that arrive while others decode: each costs the step that was issued for the batch without it, and the steps
+    issued behind the prompts themselves, which the merged batch never asks for, die out."""
+    cfg = C.tiny_llama()
+    prompts = [W.random_prompt(cfg.vocab_size, 18 + 7 * i, 300 + i).tolist() for i in range(20)]
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 5), precision=C.PREC_FP32, num_kv_blocks=20, sampling=None)
+
+    def call(which, prefill, hit=None):
+        nonlocal issued
+        seqs = [prompts[i] for i in which]
+        out, _ = run.run_flat(seqs, prefill, [0] * len(seqs), [[i] for i in which], [0.0] * len(seqs))
+        if hit is not None:
+            assert (run.last_stats.h2d_bytes == 0) == hit, (which, hit)
+        issued = run.sync()[1] != run.last_stats.device_ms  # the time of the last step issued is not that of the one asked for
+        for s, t in zip(seqs, out):
+            s.append(int(t))
+
+    issued, live = False, [0, 1, 2]
+    try:
+        call(live, True)
+        for _ in range(3):
+            call(live, False, hit=True)
+        for arrival in range(3, 20):
+            call([arrival], True, hit=False)
+            if arrival - 3 not in (0, 2, 5, 10):  # pauses of 1, 2, 4 and 8 prompts
+                assert not issued, arrival
+            live = live[1:] + [arrival]
+            call(live, False, hit=False)
+            for _ in range(3):  # the merged batch goes on without the host at once
+                call(live, False, hit=True)
+    finally:
+        run.close()
+
+
 def test_recurrent_state_is_not_stepped_ahead():
     """Calls that a step issued ahead would not match (another token, another batch), on a model whose steps update state in
     place: the same with speculation asked for as without."""
