@@ -8,11 +8,11 @@
 // head h / (n_heads / n_kv_heads) (attention.go:337-339).
 //
 //  * attn_prefill_kernel: flash-style (online softmax, no S x S score tensor).
-//    CTA = 32 queries of one sequence x one head; four groups of 128 threads share the keys of a
-//    tile (16 each) and merge at the end; in a group 4 threads per query each own
+//    CTA = 32 queries of one sequence x one head; 4 threads per query each own
 //    hd/4 dims; K/V tiles of 64 keys staged in shared memory as fp32.  Bound by the latency of its
-//    shared-memory reads and sums: a prompt's step has one or two such CTAs per SM, and with one group a
-//    scheduler has one warp to issue from.  Four prompts of 50 to 100 tokens, 12 heads of 64: 20 -> 14 us.
+//    shared-memory reads and sums.  In small steps, with one or two CTAs per SM, a scheduler has one warp to
+//    issue from: there four groups of 128 threads share the keys of a tile (16 each) and merge at the end
+//    (prefill_groups has the rule and both sides' times).
 //  * attn_decode_kernel: one new token per sequence.  CTA = (sequence, group of
 //    GC query heads sharing a kv head, KV split).  HBM-bound: each K/V row is
 //    read once with 16-byte loads by hd/8 lanes; online softmax in registers;
@@ -27,13 +27,56 @@
 namespace nvllm {
 
 constexpr int PF_KT = 64;  // keys per shared-memory tile (divides KV_BLOCK)
-constexpr int PF_GROUPS = 4, PF_THREADS = 128 * PF_GROUPS;
-constexpr size_t pf_smem(int hd) {  // K and V tiles; then the groups' results: m, l and a row each
-  return sizeof(float) * std::max((size_t)2 * PF_KT * hd, (size_t)(PF_GROUPS - 1) * ATTN_PREFILL_QTILE * (hd + 4));
+constexpr size_t pf_smem(int hd, int groups) {  // K and V tiles; then the groups' results: m, l and a row each
+  return sizeof(float) * std::max((size_t)2 * PF_KT * hd, (size_t)(groups - 1) * ATTN_PREFILL_QTILE * (hd + 4));
 }
 
-template <typename QT, typename KT, int HD>
-__global__ void __launch_bounds__(PF_THREADS)
+// the groups' results of a query (maximum, sum, row; 4 threads each) meet in the first one
+template <int HD, int GROUPS>
+__device__ __forceinline__ void merge_groups(float* smem, int grp, int qi, int sub, float m, float& l, float (&acc)[HD / 4]) {
+  constexpr int NV = HD / 16;
+  __syncthreads();
+  if (grp > 0) {
+    float* mine = smem + ((size_t)(grp - 1) * ATTN_PREFILL_QTILE + qi) * (HD + 4);
+    if (sub == 0) {
+      mine[HD] = m;
+      mine[HD + 1] = l;
+    }
+#pragma unroll
+    for (int v = 0; v < NV; v++)
+      *reinterpret_cast<float4*>(mine + v * 16 + sub * 4) = make_float4(acc[v * 4], acc[v * 4 + 1], acc[v * 4 + 2], acc[v * 4 + 3]);
+  }
+  __syncthreads();
+  if (grp > 0) return;
+  // (key 0 is the first group's: a valid query's m is finite)
+  const float* other[GROUPS - 1];
+  float top = m;
+#pragma unroll
+  for (int g = 0; g < GROUPS - 1; g++) {
+    other[g] = smem + ((size_t)g * ATTN_PREFILL_QTILE + qi) * (HD + 4);
+    top = fmaxf(top, other[g][HD]);
+  }
+  const float c0 = expf(m - top);
+  l *= c0;
+#pragma unroll
+  for (int i = 0; i < HD / 4; i++) acc[i] *= c0;
+#pragma unroll
+  for (int g = 0; g < GROUPS - 1; g++) {
+    const float c = expf(other[g][HD] - top);  // a group that saw no key: exp(-inf) = 0
+    l = fmaf(other[g][HD + 1], c, l);
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      const float4 o = *reinterpret_cast<const float4*>(other[g] + v * 16 + sub * 4);
+      acc[v * 4] = fmaf(o.x, c, acc[v * 4]);
+      acc[v * 4 + 1] = fmaf(o.y, c, acc[v * 4 + 1]);
+      acc[v * 4 + 2] = fmaf(o.z, c, acc[v * 4 + 2]);
+      acc[v * 4 + 3] = fmaf(o.w, c, acc[v * 4 + 3]);
+    }
+  }
+}
+
+template <typename QT, typename KT, int HD, int GROUPS>
+__global__ void __launch_bounds__(128 * GROUPS)
 attn_prefill_kernel(AttnArgs a) {
   pdl_launch_dependents();
   extern __shared__ float smem[];
@@ -92,8 +135,8 @@ attn_prefill_kernel(AttnArgs a) {
     // shuffles below name all 32 lanes), so every lane runs to the warp's largest jmax and
     // masks its own tail.
     const int jmax = qvalid ? max(0, min(nk, qpos - k0 + 1)) : 0;
-    const int jlim = min(__reduce_max_sync(0xffffffffu, jmax), (grp + 1) * (PF_KT / PF_GROUPS));
-    for (int j0 = grp * (PF_KT / PF_GROUPS); j0 < jlim; j0 += 8) {
+    const int jlim = min(__reduce_max_sync(0xffffffffu, jmax), (grp + 1) * (PF_KT / GROUPS));
+    for (int j0 = grp * (PF_KT / GROUPS); j0 < jlim; j0 += 8) {
       float s[8];
       float cmax = -INFINITY;
 #pragma unroll
@@ -142,45 +185,8 @@ attn_prefill_kernel(AttnArgs a) {
       m = m_new;
     }
   }
-  // the groups' results meet in the first one
-  __syncthreads();
-  float* mine = smem + ((size_t)(grp - 1) * ATTN_PREFILL_QTILE + qi) * (HD + 4);
-  if (grp > 0) {
-    if (sub == 0) {
-      mine[HD] = m;
-      mine[HD + 1] = l;
-    }
-#pragma unroll
-    for (int v = 0; v < NV; v++)
-      *reinterpret_cast<float4*>(mine + v * 16 + sub * 4) = make_float4(acc[v * 4], acc[v * 4 + 1], acc[v * 4 + 2], acc[v * 4 + 3]);
-  }
-  __syncthreads();
+  if constexpr (GROUPS > 1) merge_groups<HD, GROUPS>(smem, grp, qi, sub, m, l, acc);
   if (grp == 0 && qvalid) {
-    // (key 0 is the first group's: its m is finite)
-    const float* other[PF_GROUPS - 1];
-    float top = m;
-#pragma unroll
-    for (int g = 0; g < PF_GROUPS - 1; g++) {
-      other[g] = smem + ((size_t)g * ATTN_PREFILL_QTILE + qi) * (HD + 4);
-      top = fmaxf(top, other[g][HD]);
-    }
-    const float c0 = expf(m - top);
-    l *= c0;
-#pragma unroll
-    for (int i = 0; i < DPT; i++) acc[i] *= c0;
-#pragma unroll
-    for (int g = 0; g < PF_GROUPS - 1; g++) {
-      const float c = expf(other[g][HD] - top);  // a group that saw no key: exp(-inf) = 0
-      l = fmaf(other[g][HD + 1], c, l);
-#pragma unroll
-      for (int v = 0; v < NV; v++) {
-        const float4 o = *reinterpret_cast<const float4*>(other[g] + v * 16 + sub * 4);
-        acc[v * 4] = fmaf(o.x, c, acc[v * 4]);
-        acc[v * 4 + 1] = fmaf(o.y, c, acc[v * 4 + 1]);
-        acc[v * 4 + 2] = fmaf(o.z, c, acc[v * 4 + 2]);
-        acc[v * 4 + 3] = fmaf(o.w, c, acc[v * 4 + 3]);
-      }
-    }
     const float inv = 1.0f / l;
     QT* op = (QT*)a.out + (size_t)row * a.nh * HD + head * HD;
 #pragma unroll
@@ -190,26 +196,48 @@ attn_prefill_kernel(AttnArgs a) {
   }
 }
 
+// How many groups share a tile's keys.  With four, an SM holds one CTA (two of heads up to 32) and a CTA is through a tile in
+// 0.6 of the time; with one it holds six, and a full chip gets through more tiles.  So four while the time is that of the
+// longest CTA: x = all CTAs' tiles over SMs x the longest one's up to 1.0 where that is one tile, and to 2.8 (4 for heads up
+// to 32) from six on; and one up to 32 keys, of which two groups would have none.  Time with four over time with one, whole
+// fp32 steps of four layers of 768, x in front; heads: 12 of 64, 32 of 64, 12 of 32, 16 of 128:
+//    9 tokens         0.06 1.10   0.17 1.14   0.06 1.07   0.08 1.01      2 x 300    0.96 0.91   2.56 0.97   0.96 0.81   1.28 0.89
+//   48                0.17 0.95   0.45 0.99   0.17 0.94   0.22 0.92      6 x 300    2.87 1.01   7.67 1.16   2.87 0.97   3.83 1.03
+//    4 x 40           0.62 0.90   1.64 1.05   0.62 0.97   0.82 0.96      1000       1.36 0.70   3.63 1.04   1.36 0.61   1.81 0.95
+//   16 x 40           2.47 1.10   6.57 1.22   2.47 1.02   3.29 1.09      3 x 1000   4.08 1.04   10.9 1.17   4.08 0.90   5.44 1.02
+//    8 x 80           1.24 1.03   3.31 1.18   1.24 0.94   1.66 1.07      2000       2.60 0.85   6.92 1.08   2.60 0.81   3.46 0.94
+//    2 x 130          0.43 0.83   1.14 0.91   0.43 0.88   0.57 0.89      2 x 2000   5.19 1.04   13.8 1.16   5.19 0.95   6.92 1.02
+static int prefill_groups(const AttnArgs& a) {
+  if (a.max_len <= PF_KT / 2) return 1;
+  const double longest = ceil_div(a.max_len, PF_KT);
+  const double tiles = a.nh * (a.pairs / (ATTN_PREFILL_QTILE * PF_KT) + 0.75 * a.n_qtiles);  // (a CTA's last tile is half full)
+  const double most = std::min(0.6 + 0.4 * longest, a.hd <= 32 ? 4.0 : 2.8);
+  return tiles <= most * longest * std::max(1, a.sm_count) ? 4 : 1;
+}
+
+template <typename QT, typename KT, int HD, int GROUPS>
+static cudaError_t prefill_launch(cudaStream_t st, const AttnArgs& a) {
+  constexpr size_t smem = pf_smem(HD, GROUPS);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<QT, KT, HD, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  (void)launch_k(attn_prefill_kernel<QT, KT, HD, GROUPS>, dim3(a.n_qtiles, a.nh), dim3(128 * GROUPS), smem, st, a);
+  return cudaGetLastError();
+}
+template <typename QT, typename KT, int HD>
+static cudaError_t prefill_hd(cudaStream_t st, const AttnArgs& a) {
+  return prefill_groups(a) == 4 ? prefill_launch<QT, KT, HD, 4>(st, a) : prefill_launch<QT, KT, HD, 1>(st, a);
+}
 template <typename QT, typename KT>
 static cudaError_t prefill_dispatch(cudaStream_t st, const AttnArgs& a) {
-  dim3 grid(a.n_qtiles, a.nh);
-  const size_t smem = pf_smem(a.hd);
-#define PF(HD)                                                                               \
-  {                                                                                          \
-    if (smem > 48 * 1024)                                                                    \
-      cudaFuncSetAttribute(attn_prefill_kernel<QT, KT, HD>,                                  \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-    (void)launch_k(attn_prefill_kernel<QT, KT, HD>, dim3(grid), dim3(PF_THREADS), smem, st, a);                      \
-  }
   switch (a.hd) {
-    case 16: PF(16); break;
-    case 32: PF(32); break;
-    case 64: PF(64); break;
-    case 128: PF(128); break;
+    case 16: return prefill_hd<QT, KT, 16>(st, a);
+    case 32: return prefill_hd<QT, KT, 32>(st, a);
+    case 64: return prefill_hd<QT, KT, 64>(st, a);
+    case 128: return prefill_hd<QT, KT, 128>(st, a);
     default: return cudaErrorInvalidValue;
   }
-#undef PF
-  return cudaGetLastError();
 }
 
 int attn_prefill_qtile(int qdt, int kvdt, int hd) {

@@ -405,6 +405,7 @@ int forward_step(nvllm_handle* h) {
   at.pool_blocks = h->num_blocks;
   at.total_rows = h->view_T > 0 ? h->view_T : T;
   at.sm_count = h->sm_count;
+  at.pairs = L.attn_pairs; at.max_len = L.max_len;
   at.tickets = (int*)w.chain_ctr + (h->pipe_role == 2 ? 32 : 16);  // (two chunks of a step may be in flight)
   at.wait_flag = h->waits.dev;
   if (!is_prefill)

@@ -463,6 +463,8 @@ struct AttnArgs {
   int pool_blocks;     // blocks in the layer's K / V pool (tensor-map extent)
   int total_rows;      // rows of q / out in this step (tensor-map extent; tcgen05 prefill kernel)
   int sm_count;
+  double pairs;        // (query, key) pairs of a prefill step, and
+  int max_len;         // its longest sequence (how attention.cu shares out a tile's keys)
 };
 constexpr int ATTN_PREFILL_QTILE = 32;  // SIMT (fp32 parity) kernel; the mma kernel uses 64
 // queries per tile of the kernel launch_attn_prefill will pick: the host builds tile_seq /
