@@ -14,7 +14,8 @@
 //
 // Persistent, two CTAs per SM: an item is 128 queries of one sequence x one query head, dealt out by a counter, heaviest
 // first.  Per key tile (BN keys):
-//   scheduler     the next items' rows, positions and key tiles, up to four ahead
+//   scheduler     the next items' rows, positions and key tiles, up to four ahead (every warp finds the CTA's first item
+//                 itself, before the wait for the kernel in front)
 //   TMA warp      Q of the item, K / V tiles of the paged pool (one (block, kv head) slab is contiguous;
 //                 2-D tensor map over the layer's pool, SWIZZLE_128B) -> shared memory, two stages each
 //   MMA warp      S = Q K^T   (128 x BN, K-major x K-major, accumulator in TMEM), issued as soon as the softmax warps
@@ -110,6 +111,21 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_items = a.n_qtiles * a.nh, grid = (int)gridDim.x;
+  auto item_at = [&](int t) {
+    // heaviest tiles (latest queries of a sequence see the most keys) first, the heads of a tile next to each other
+    PtItem w;
+    const int tile = a.n_qtiles - 1 - t / a.nh;
+    w.head = t % a.nh;
+    w.seq = a.tile_seq[tile];
+    const int q0 = a.tile_q0[tile], first = a.cu_q[w.seq];
+    w.row = first + q0;
+    w.rows = min(PT_BM, a.cu_q[w.seq + 1] - first - q0);
+    w.pos = a.seq_start[w.seq] + q0;
+    w.first = OPT > 1 ? max(0, w.pos - a.window + 1) / BN : 0;
+    w.n_tiles = (w.pos + w.rows + BN - 1) / BN - w.first;  // keys up to pos + rows are visible to this tile
+    return w;
+  };
 
   if (warp == 4 && lane == 0) {
     mbar_init(b_qfull, 1);
@@ -146,10 +162,14 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const uint32_t tmem_base = *tmem_slot_ptr;
   const uint32_t tS = tmem_base, tO = tmem_base + BN, tP = tO + HD;
   auto wait = [&](uint32_t bar, int parity) { return wait_short(bar, (uint32_t)parity & 1, dead, a.wait_flag); };
-  // item `it` once it is known (n_tiles == 0: there are no more); false when the wait ran out
+  // the CTA's item `it` > 0 once it is known (n_tiles == 0: there are no more); false when the wait ran out
   auto next_item = [&](int it, PtItem& w) {
-    const int s = it % PT_ITEMS;
-    if (!wait(b_ifull + 8 * s, it / PT_ITEMS)) return false;
+    if (n_items <= grid) {
+      w.n_tiles = 0;
+      return true;
+    }
+    const int s = (it - 1) % PT_ITEMS;
+    if (!wait(b_ifull + 8 * s, (it - 1) / PT_ITEMS)) return false;
     w = items[s];
     __syncwarp();
     if (lane == 0) mbar_arrive(b_iempty + 8 * s);
@@ -160,57 +180,69 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     // warpgroup 1 (TMA warp 4, MMA warp 5, scheduler warp 6, an idle warp) hands its registers to the softmax
     // warpgroup, whose threads carry a whole fp32 output row
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    // Q and this step's K / V rows are the previous kernels' output (and the limit of the waits counts from here)
-    pdl_wait();
+    PtItem w = item_at(blockIdx.x);  // (what it reads came with the step: no kernel writes it)
+    // Q and this step's K / V rows are the previous kernels' output (and the limit of the waits counts from the wait for them)
     if (warp == 6) {
       // ---------------------------------------------------------------- scheduler
-      const int n_items = a.n_qtiles * a.nh, grid = (int)gridDim.x;
-      int t = blockIdx.x;
-      for (int it = 0;; it++) {
-        int draw = 0;  // the item after this one
-        if (t < n_items && lane == 0) draw = a.tickets ? grid + atomicAdd(a.tickets, 1) : t + grid;
-        PtItem w{};
-        if (t < n_items) {
-          // heaviest tiles (latest queries of a sequence see the most keys) first, the heads of a tile next to each other
-          const int tile = a.n_qtiles - 1 - t / a.nh;
-          w.head = t % a.nh;
-          w.seq = a.tile_seq[tile];
-          const int q0 = a.tile_q0[tile], first = a.cu_q[w.seq];
-          w.row = first + q0;
-          w.rows = min(PT_BM, a.cu_q[w.seq + 1] - first - q0);
-          w.pos = a.seq_start[w.seq] + q0;
-          w.first = OPT > 1 ? max(0, w.pos - a.window + 1) / BN : 0;
-          w.n_tiles = (w.pos + w.rows + BN - 1) / BN - w.first;  // keys up to pos + rows are visible to this tile
+      pdl_wait();
+      if (n_items > grid) {
+        auto draw = [&](int t) { return lane != 0 ? 0 : a.tickets ? grid + atomicAdd(a.tickets, 1) : t + grid; };
+        auto drawn = [&](int d) {
+          d = __shfl_sync(0xffffffffu, d, 0);
+          // the counter is zero again for the next launch: n_items draws in all, of each CTA one past the end
+          if (a.tickets && d - grid == n_items - 1 && lane == 0) *a.tickets = 0;
+          return d;
+        };
+        int t = drawn(draw(blockIdx.x));
+        for (int it = 0;; it++) {
+          const bool more = t < n_items;
+          const int d = more ? draw(t) : 0;  // the item after this one
+          w.n_tiles = 0;
+          if (more) w = item_at(t);
+          const int s = it % PT_ITEMS;
+          if (!wait(b_iempty + 8 * s, it / PT_ITEMS + 1)) break;
+          if (elect_one()) {
+            items[s] = w;
+            mbar_arrive(b_ifull + 8 * s);
+          }
+          __syncwarp();
+          if (!more) break;
+          t = drawn(d);
         }
-        const int s = it % PT_ITEMS;
-        if (!wait(b_iempty + 8 * s, it / PT_ITEMS + 1)) break;
-        if (elect_one()) {
-          items[s] = w;
-          mbar_arrive(b_ifull + 8 * s);
-        }
-        __syncwarp();
-        if (w.n_tiles == 0) break;
-        draw = __shfl_sync(0xffffffffu, draw, 0);
-        // the counter is zero again for the next launch: n_items draws in all, of each CTA one past the end
-        if (a.tickets && draw - grid == n_items - 1 && lane == 0) *a.tickets = 0;
-        t = draw;
       }
     } else if (warp == 4) {
       // ---------------------------------------------------------------- TMA producer
-      int g = 0;  // key tiles so far
+      int g = 1;  // key tiles so far
       bool ok = true;
-      for (int it = 0; ok; it++) {
-        PtItem w;
-        if (!next_item(it, w) || w.n_tiles == 0) break;
-        const int* bt = a.block_tables + (size_t)w.seq * a.max_blocks;
-        const int kvh = w.head / (a.nh / a.nkv);
-        if (it > 0 && !wait(b_qempty, it - 1)) break;
-        if (elect_one()) {
+      {  // the first item's queries and first key tile: short code behind the wait, which a launch fetches while it counts
+        const int k0 = w.first * BN;
+        const int prow = (a.block_tables[(size_t)w.seq * a.max_blocks + k0 / KV_BLOCK] * a.nkv + w.head / (a.nh / a.nkv)) * KV_BLOCK + k0 % KV_BLOCK;
+        const bool one = elect_one();
+        if (one) {
           mbar_expect_tx(b_qfull, Cf::Q_BYTES);
+          mbar_expect_tx(b_kfull, Cf::KV_BYTES);
+          mbar_expect_tx(b_vfull, Cf::KV_BYTES);
+        }
+        pdl_wait();
+        if (one) {
           for (int s = 0; s < SUB; s++) tma_load_2d(sQ + s * (PT_BM * 128), &tmQ, b_qfull, w.head * HD + 64 * s, w.row);
+          for (int s = 0; s < SUB; s++) tma_load_2d(sK + s * (BN * 128), &tmK, b_kfull, 64 * s, prow);
+          for (int s = 0; s < SUB; s++) tma_load_2d(sV + s * (BN * 128), &tmV, b_vfull, 64 * s, prow);
         }
         __syncwarp();
-        for (int j = 0; j < w.n_tiles; j++, g++) {
+      }
+      for (int it = 0; ok && w.n_tiles > 0; it++) {
+        const int* bt = a.block_tables + (size_t)w.seq * a.max_blocks;
+        const int kvh = w.head / (a.nh / a.nkv);
+        if (it > 0) {
+          if (!wait(b_qempty, it - 1)) break;
+          if (elect_one()) {
+            mbar_expect_tx(b_qfull, Cf::Q_BYTES);
+            for (int s = 0; s < SUB; s++) tma_load_2d(sQ + s * (PT_BM * 128), &tmQ, b_qfull, w.head * HD + 64 * s, w.row);
+          }
+          __syncwarp();
+        }
+        for (int j = it == 0 ? 1 : 0; j < w.n_tiles; j++, g++) {
           const int k0 = (w.first + j) * BN, st = g % ST;
           const int prow = (bt[k0 / KV_BLOCK] * a.nkv + kvh) * KV_BLOCK + (k0 % KV_BLOCK);
           if (!(ok = wait(b_kempty + 8 * st, g / ST + 1))) break;
@@ -228,6 +260,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           }
           __syncwarp();
         }
+        ok = ok && next_item(it + 1, w);
       }
     } else if (warp == 5) {
       // ---------------------------------------------------------------- MMA issuer
@@ -258,8 +291,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       };
       int g = 0;
       bool ok = true;
-      PtItem w, wn;
-      if (!next_item(0, w)) w.n_tiles = 0;
+      PtItem wn;
+      pdl_wait();
       for (int it = 0; ok && w.n_tiles > 0; it++, w = wn) {
         const int n_tiles = w.n_tiles;
         // (the previous item's last S has been read: its P V came after)
@@ -289,6 +322,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   } else {
     // ------------------------------------------------------------------ softmax + output
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    PtItem w = item_at(blockIdx.x);
     pdl_wait();
     const int q = warp;  // TMEM lane quadrant of this warp
     const int r = q * 32 + lane;
@@ -324,9 +358,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       __syncwarp();
       o_pending = false;
     };
-    for (int it = 0; ok; it++) {
-      PtItem w;
-      if (!(ok = next_item(it, w)) || w.n_tiles == 0) break;
+    for (int it = 0; ok && w.n_tiles > 0; it++) {
       const int n_tiles = w.n_tiles;
       float m_used = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_tiles; j++, g++) {
@@ -424,6 +456,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       if (OPT && a.head_gate && r < w.rows) o_inv *= a.head_gate[(size_t)(w.row + r) * a.gate_ld + w.head];
       o_row = r < w.rows ? (bf16*)a.out + (size_t)(w.row + r) * a.nh * HD + (size_t)w.head * HD : nullptr;
       o_pending = true;
+      ok = next_item(it + 1, w);
     }
     if (ok && o_pending && wait(b_ofull, g - 1)) {
       tc_fence_after();
