@@ -123,11 +123,18 @@ __global__ void __launch_bounds__(256) moe_select_rows_kernel(NormArgs a, const 
 static size_t moe_select_rows_smem(int E) { return (size_t)(MSR_TT * (E + 1) + 16 * E) * sizeof(float); }
 
 // Routing of many rows as a product on the tensor cores (gemm_f32_tc5.cu: fp32 in, fp32 sums; the experts are its token
-// side, the rows its weight side) and the selection: from 1024 rows on, as moe_route_rows_kernel, which reads the router
-// once per eight rows from L2 and keeps what this refuses (identity experts, which need the row itself).  18.7 k rows of
-// 1024, 32 experts: 106 -> 37 us (27 and 10).
+// side, the rows its weight side) and the selection, against moe_route_rows_kernel, which reads the router once per eight
+// rows from L2.  18.7 k rows of 1024, 32 experts: 106 -> 37 us (27 and 10).  The product's launch has a floor of some 15 us
+// and the selection of more than 32 experts another ten, so the other kernel keeps steps of fewer rows, and what this
+// refuses (identity experts, which need the row itself; 256 experts, whose selection is past 48 KB).  All norms of a layer,
+// us, rows kernel / product:
+//   8 experts, rows of 1024: 1024 rows 32.6 / 35.3, 2560 43.9 / 45.1, 4096 62.2 / 57.2    2048: 1024 rows 46.9 / 43.3, 2560 68.7 / 67.2
+//   32 experts, 512: 2560 rows 41.9 / 42.6, 4096 57.3 / 51.0    1024: 1024 rows 39.7 / 42.1, 4096 82.8 / 74.5
+//   40 experts, 512: 1024 rows 31.4 / 45.3    1024: 4096 rows 85.4 / 89.3, 8192 152.6 / 134.0    2048: 1600 rows 70.8 / 78.5
+//   64 experts, 1024: 2560 rows 67.4 / 71.2, 4096 97.4 / 90.0    128: 1024 rows 60.4 / 65.6, 2560 95.2 / 79.6
 bool moe_route_product_fits(const NormArgs& a, const GemmArgs& g) {
-  return a.n_rows >= 1024 && a.route.identity == 0 && a.E <= MOE_MAX_E && moe_select_rows_smem(a.E) <= 48 * 1024 && gemm_f32_tc5_takes(g);
+  const bool worth = a.E <= 32 ? a.n_rows >= 4096 || a.H >= 2048 : (double)a.n_rows * a.E * a.H >= 2.05e8;
+  return a.n_rows >= 1024 && worth && a.route.identity == 0 && a.E <= MOE_MAX_E && moe_select_rows_smem(a.E) <= 48 * 1024 && gemm_f32_tc5_takes(g);
 }
 cudaError_t launch_moe_select_rows(cudaStream_t st, const NormArgs& a, const GemmArgs& g) {
   (void)launch_k(moe_select_rows_kernel, dim3((a.n_rows + MSR_TT - 1) / MSR_TT), dim3(256), moe_select_rows_smem(a.E), st, a,
