@@ -374,11 +374,14 @@ int forward_step(nvllm_handle* h) {
   // tests switch it).
   const char* gpre_env = getenv("NVLLM_GEMV_PRE");
   const bool gpre_act = !(gpre_env && atoi(gpre_env) == 0) && T <= 8 && !h->moe;
-  // Steps of one bf16 row: norms in front of the products, residual updates behind them (sequential blocks)
-  const bool one_row = T == 1 && h->adt == DT_BF16 && h->wdt == DT_BF16 && !h->parallel && h->tp == 1 && gemv_row_fits(H);
+  // Steps of one bf16 row: norms in front of the products, residual updates behind them (sequential blocks); the attention's
+  // output product and the feed-forward together or not at all (gemv_row.cu)
+  const bool one_row = T == 1 && h->adt == DT_BF16 && h->wdt == DT_BF16 && !h->parallel && h->tp == 1 && gemv_row_fits(H, true);
+  const bool row_ffn = one_row && !h->moe && gemv_row_fits(h->q_cols, false) && gemv_row_fits(h->F, false);
   auto row_args = [&](const void* A, const void* W, int N, int K, int epi, const float* bias, float m) {
     GemvRowArgs r{};
     r.A = (const bf16*)A; r.W = (const bf16*)W; r.N = N; r.K = K; r.epi = epi; r.bias = bias; r.m = m; r.x = w.x; r.eps = c.norm_eps;
+    r.sm_count = h->sm_count;
     return r;
   };
   int xb_parts = h->fold ? 1 : 0;
@@ -507,7 +510,7 @@ int forward_step(nvllm_handle* h) {
       LAUNCH(h, launch_attn_decode(st, at));
       if (at.n_splits > 1) h->launches++;
     }
-    if (one_row && gemv_row_fits(h->q_cols)) {
+    if (row_ffn) {
       if ((rc = run_gemv_row(h, row_args(w.attn_out, lw.wo, H, h->q_cols, TC5_EPI_RESID, lw.bo, m_res)))) return rc;
       p1 = Pending();
     } else if (resid_gemm_ok(h, T, H, h->q_cols, h->q_cols)) {
@@ -525,7 +528,7 @@ int forward_step(nvllm_handle* h) {
     }
     }  // attention / Mamba2 sub-block
     // ---- feed-forward sub-block
-    if (one_row && !h->moe && !p1.p && gemv_row_fits(h->F)) {
+    if (row_ffn && !p1.p) {
       GemvRowArgs r = row_args(nullptr, lw.w1, h->w1_cols, H, h->swiglu ? TC5_EPI_SWIGLU : TC5_EPI_GELU, lw.b1, 0.f);
       r.norm_w = lw.ffn_norm_w; r.norm_b = lw.ffn_norm_b; r.act = (bf16*)w.hbuf;
       if ((rc = run_gemv_row(h, r))) return rc;

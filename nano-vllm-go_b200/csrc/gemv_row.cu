@@ -6,8 +6,16 @@
 // instead of seven.  A warp group (WPR warps) owns the whole sum of R output rows; its lanes take 16 bytes of a
 // weight row at a time, all of a row's loads in flight, the first tile's before the wait for the kernel in front
 // (weights don't change).  Sums: 8 NL FMAs a lane, then the lanes and warps in pairs.
-// Bound by the chain: release of the launch, one L2 round trip for the row, the sums.  GPT-2 small, one sequence, us per
-// token: 342 -> 255; Llama-1B layers 245 -> 225.
+// Bound by the chain: release of the launch, one L2 round trip for the row, the sums.
+//
+// Which layers take it (forward.cu), us a token, with their norms and products as launches of their own / here (vocabulary of
+// 4096; width, feed-forward, layers):
+//   768, 3072, 12 (GPT-2 small)  289 / 213     2048, 8192, 4   201 / 187     4096, 8192, 2    189 / 179 (all heads with keys of
+//   1600, 6400, 8                341 / 287     3072, 8192, 4   286 / 264                       their own: 205 / 194)
+// Rows wider than 4096 are better off without the norm in front, which every CTA repeats: 5120, 6144, 2 199 / 217; 8192,
+// 4096, 2 269 / 277; 8192, 8192, 2 344 / 352; 5120, 384, 4 with 8 heads 122 / 144.  And the attention's output product pays only
+// where the feed-forward follows here too: behind it alone a norm is launched all the same, and the residual update that this
+// norm would have done costs the product its split sums (2048, 8192, 4: 201 / 209; 4096, 14336, 2: 251 / 253).
 #include <algorithm>
 
 #include "common.cuh"
@@ -172,17 +180,18 @@ __global__ void __launch_bounds__(GR_THREADS) gemv_row_kernel(GemvRowArgs a, Tra
   TRACE_EXIT(tr);
 }
 
-bool gemv_row_fits(int K) { return K >= 8 && K <= 8192 && (K % 8) == 0; }
+bool gemv_row_fits(int K, bool norm) { return K >= 8 && K <= (norm ? 4096 : 8192) && (K % 8) == 0; }
 
 template <int R, int WPR, int NL, bool NORM>
 static cudaError_t gemv_row_launch(cudaStream_t st, const GemvRowArgs& a) {
-  const int ctas = std::min(ceil_div(a.N, GR_WARPS / WPR * R), 148 * 4);
+  const int ctas = std::min(ceil_div(a.N, GR_WARPS / WPR * R), 4 * std::max(1, a.sm_count));
   return launch_k(gemv_row_kernel<R, WPR, NL, NORM>, dim3(ctas), dim3(GR_THREADS), NORM ? (size_t)a.K * 2 : 0, st, a, next_trace(50));
 }
 // as few warps to a row as take it in four pieces a lane
 template <int R, bool NORM>
 static cudaError_t gemv_row_pick(cudaStream_t st, const GemvRowArgs& a) {
-  if (a.K > 4096) return gemv_row_launch<R, 8, 4, NORM>(st, a);
+  if constexpr (!NORM)
+    if (a.K > 4096) return gemv_row_launch<R, 8, 4, NORM>(st, a);
   if (a.K > 2048) return gemv_row_launch<R, 4, 4, NORM>(st, a);
   if (a.K > 1024) return gemv_row_launch<R, 2, 4, NORM>(st, a);
   if (a.K > 768) return gemv_row_launch<R, 1, 4, NORM>(st, a);
@@ -191,7 +200,7 @@ static cudaError_t gemv_row_pick(cudaStream_t st, const GemvRowArgs& a) {
 }
 
 cudaError_t launch_gemv_row(cudaStream_t st, const GemvRowArgs& a) {
-  if (!gemv_row_fits(a.K) || (a.epi == TC5_EPI_SWIGLU && (a.N & 1)) || a.N < 1) return cudaErrorInvalidValue;
+  if (!gemv_row_fits(a.K, a.norm_w != nullptr) || (a.epi == TC5_EPI_SWIGLU && (a.N & 1)) || a.N < 1) return cudaErrorInvalidValue;
   if (a.epi == TC5_EPI_SWIGLU) return a.norm_w ? gemv_row_pick<2, true>(st, a) : gemv_row_pick<2, false>(st, a);
   return a.norm_w ? gemv_row_pick<1, true>(st, a) : gemv_row_pick<1, false>(st, a);
 }

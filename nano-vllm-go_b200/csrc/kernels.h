@@ -308,8 +308,9 @@ struct GemvRowArgs {
   __nv_bfloat16* act;
   const float* bias;
   float m;
+  int sm_count;
 };
-bool gemv_row_fits(int K);
+bool gemv_row_fits(int K, bool norm);
 cudaError_t launch_gemv_row(cudaStream_t st, const GemvRowArgs& a);
 
 // ---------------------------------------------------------------- gemm_tcgen05.cu
