@@ -1,5 +1,5 @@
 """Decode steps of the delta rule (delta_step_kernel): tokens one at a time against the same texts as prompts, whose
-convolution and scan are other kernels, in the fp32 mode."""
+convolution and scan are other kernels, and against the float64 restatement, in the fp32 mode."""
 import numpy as np
 import pytest
 
@@ -22,7 +22,8 @@ KERNEL = 51  # its id in the timeline
     (2, 1, 64, 64, 1, False),    # no tail
 ])
 def test_tokens_one_at_a_time_match_prompts(heads, kv_heads, dim, vdim, conv, taken):
-    cfg, w = zozonex.random_weights(zozonex.model([zozonex.layer(zozonex.delta(heads, kv_heads, dim, vdim, conv), 96)] * 2, width=128), 5)
+    model = zozonex.model([zozonex.layer(zozonex.delta(heads, kv_heads, dim, vdim, conv), 96)] * 2, width=128)
+    cfg, w = zozonex.random_weights(model, 5)
     n, steps = 3, 7
     texts = [W.random_prompt(cfg.vocab_size, 1 + i * i + steps, 60 + i) for i in range(n)]  # starts of 1, 2 and 5 tokens
     run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, w.items(), precision=C.PREC_FP32, num_kv_blocks=n, sampling=None, num_state_slots=n)
@@ -43,6 +44,10 @@ def test_tokens_one_at_a_time_match_prompts(heads, kv_heads, dim, vdim, conv, ta
         got.append(step([1] * n, True))  # one-token prompts: whatever the slots hold counts as nothing
         got.append(step([2] * n, False))
         assert (KERNEL in run.trace_end(1 << 18)[:, 1]) == taken
+        for i in range(n):
+            exact = zozonex.ref.forward(model, w, texts[i])
+            for k in range(steps + 1):
+                assert rel_err(got[k][i], exact[len(texts[i]) - steps + k - 1]) <= 1e-4, (k, i)  # what the fp32 mode is held to
         for k in range(steps + 1):
             for i in range(n):
                 want = step([len(texts[i]) - steps + k], True, [i])[0]

@@ -1,9 +1,9 @@
 """The projections of an attention layer placed by the product's own epilogue (gemm_tc5_pair.cu): a batch of prompts that takes
-it against the same prompts one at a time, whose heads are rotated and placed by a kernel of their own."""
+it against the same prompts one at a time, whose heads are rotated and placed by a kernel of their own, and against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import C, W
+from helpers import C, W, make_oracle, rel_err
 import nvllm_pkg
 
 pytestmark = pytest.mark.gpu
@@ -39,6 +39,8 @@ def test_batch_matches_prompts_one_at_a_time(family):
         rec = run.trace_end(1 << 18)
         return logits, ROPE_KERNEL in rec[:, 1], PAIR_KERNEL in rec[:, 1]
 
+    oracle = make_oracle(cfg, 7, round_bf16=True)
+    exact = {i: oracle.greedy(prompts[i], 1)[1][0] for i in (0, 1, 24, n - 1)}
     try:
         alone = []
         for i in range(n):
@@ -52,5 +54,7 @@ def test_batch_matches_prompts_one_at_a_time(family):
                 # the same bf16 roundings, sums in another order: an element may round the other way (2^-8 of it)
                 rms = np.sqrt(np.mean((batch[i] - alone[i]) ** 2) / np.mean(alone[i] ** 2))
                 assert rms <= 1e-2, f"sequence {i}: {rms}"
+            for i, want in exact.items():
+                assert rel_err(batch[i], want) <= 2e-2  # what the bf16 mode is held to
     finally:
         run.close()
