@@ -298,8 +298,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         // (the previous item's last S has been read: its P V came after)
         if (!wait(b_qfull, it) || !scores(g, n_tiles == 1)) break;
         for (int j = 0; j < n_tiles; j++, g++) {
-          // under the softmax of this tile: S of the next one, or what the next item is (its S ahead of this item's last
-          // P V: 216 us instead of 198 in the prompts below)
+          // under the softmax of this tile: S of the next one, or what the next item is (with its S ahead of this item's
+          // last P V the 64 prompts above took 216 us, and 198 in this order)
           if (j + 1 < n_tiles) ok = wait(b_sread, g) && scores(g + 1, j + 2 == n_tiles);
           else ok = next_item(it + 1, wn);
           const int st = g % ST;

@@ -665,6 +665,10 @@ static int run_postnorm(nvllm_handle* h, Pending* p, const float* w, int T, bool
   return NVLLM_OK;
 }
 
+// Prefill steps of an attention layer whose keys and values have one size, 64 or 128, in bf16, and whose scores are
+// neither capped nor biased by the distance nor two maps (windows, a sink and head gates are fine) run on the tcgen05 kernel
+// (attention_tc5.cu, 128 queries per tile), if every layer of the model does; everything else on the window kernels
+// (attention_window.cu)
 static bool attention_on_tc5(const nvllm_handle* h, const nvllm_layer_spec& s) {
   return h->adt == DT_BF16 && h->kvdt == DT_BF16 && s.dim == s.vdim && (s.dim == 64 || s.dim == 128) &&
          s.softcap == 0.f && s.dist_slope == 0.f && !s.diff_maps && attn_prefill_tc5_enabled();
@@ -1232,10 +1236,6 @@ static int ffn_moe_gated(nvllm_handle* h, const ListedLayer& y, float* topk_w, P
   if ((rc = run_moe_ffn(h, T, w.xn, s.experts, s.top, y.ff_p, 0.f, y.moe_in, y.moe_out, topk_w, p1))) return rc;
   return s.shared_ff > 0 ? ffn_glu(h, y, y.sff_p, 0.f, p2) : NVLLM_OK;
 }
-
-// Prefill steps of an attention layer whose keys and values have one size, 64 or 128, in bf16, and whose scores are
-// neither capped nor biased by the distance nor windowed nor two maps (a sink and head gates are fine) run on the tcgen05 kernel
-// (attention_tc5.cu, 128 queries per tile); everything else on the window kernels (attention_window.cu)
 
 // Grouped-query attention over the cached prefix (or a window of it) with the options of the spec
 static int mixer_attention(nvllm_handle* h, const ListedLayer& y, int run_idx, Pending* out) {

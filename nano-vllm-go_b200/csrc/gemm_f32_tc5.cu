@@ -1,7 +1,8 @@
 // gemm_f32_tc5.cu — fp32 GEMM on the tensor cores: every fp32 operand as the exact sum of three bf16 parts.
 //
 // x = hi + mid + lo with hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits = 3 x 8, each part rounded to
-// nearest, so mid <= 2^-9 |x| and lo <= 2^-18 |x|).  Of the nine products of parts the six above 2^-27 of the whole are
+// nearest, so mid <= 2^-9 |x| and lo <= 2^-18 |x|).  Exact down to some 2^-110: below, lo falls under bf16's smallest
+// subnormal, and an operand is off by up to 2^-134.  Of the nine products of parts the six above 2^-27 of the whole are
 // summed; what is left out is below the rounding of one fp32 product.  The tensor core's fp32 sums drop bits where an
 // FMA rounds, so no sum stays in it for long: each stage of 64 k starts from zero in tensor memory, in two
 // accumulators by size (hi hi; the other five), and is added to fp32 registers, which round to nearest.
@@ -18,7 +19,7 @@
 //
 // Bound by the MMAs' reads of shared memory (24 MMAs a stage, 60 cycles each at BT = 64, 79 at 128) with the splitters
 // close behind: with eight of their warps instead of sixteen a stage took 1.57 / 1.85 us instead of 1.19 / 1.55.
-// GPT-2 small, four prompts of 50 to 100 tokens: the whole step 2.66 -> 1.65 ms against the SIMT tiles; 2048 x 8192 x
+// GPT-2 small, four prompts of 50 to 100 tokens: the whole step 2.69 -> 1.70 ms against the SIMT tiles; 2048 x 8192 x
 // 2048 44 -> 188 TFLOP/s.  Relative error (2-norm) against float64, SIMT / this kernel: 300 x 2304 x 768 3.5e-7 / 9.7e-8,
 // 300 x 768 x 3072 7.0e-7 / 1.5e-7, 9 to 300 rows and 64 to 8192 of k 1.1e-7..1.1e-6 / 7e-8..2.2e-7.
 #include <cuda.h>

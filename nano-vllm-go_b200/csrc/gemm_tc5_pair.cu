@@ -284,11 +284,12 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         }
       };
       if (hs.hd) {
-        // Query, key and value heads, instead of fp32 sums that a kernel of their own reads back: 24.4 k rows of 32 + 16
-        // heads of 64, K = 2048: 229 us and 151-169 for that kernel -> one product of 206 (whole steps: Llama-3.2-1B layers,
-        // 64 prompts 11.58 -> 11.14 ms; 3B layers, 4 k rows 3.93 -> 3.73; 18.7 k rows of 16 + 16 heads 5.17 -> 4.97): bias, rotation of the halves of a head (rope.go), bf16; queries to epi_out, keys and
-        // values to their pages.  A head's halves are in the accumulators of different warps, so 16 tokens at a time go
-        // through shared memory; there a thread takes eight entries of either half of one token's head.
+        // Query, key and value heads, instead of fp32 sums that a kernel of their own reads back: bias, rotation of the
+        // halves of a head (rope.go), bf16; queries to epi_out, keys and values to their pages.  A head's halves are in the
+        // accumulators of different warps, so 16 tokens at a time go through shared memory; there a thread takes eight
+        // entries of either half of one token's head.  24.4 k rows of 32 + 16 heads of 64, K = 2048: 229 us and 151-169 for
+        // the other kernel -> one product of 206; whole steps: Llama-3.2-1B layers, 64 prompts 11.58 -> 11.14 ms; 3B layers,
+        // 4 k rows 3.93 -> 3.73; 18.7 k rows of 16 + 16 heads 5.17 -> 4.97.
         float (*stg)[HEADS_PITCH] = epi_stage.heads[half];
         const int tid = et & 127, tt = tid >> 3, g = tid & 7, hd = hs.hd, hh = hd == 64 ? g >> 2 : 0;
         const int j = hd == 64 ? (g & 3) * 8 : g * 8;      // entry of the half

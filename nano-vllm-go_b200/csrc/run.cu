@@ -231,7 +231,8 @@ static bool speculation_hit(const nvllm_handle* h, int n, int is_prefill, const 
   return true;
 }
 
-// Grows a pinned buffer of the handle (nothing is in flight between two calls: every run ends with a synchronisation).
+// Grows a pinned buffer of the handle.  Between two calls only a step issued ahead can be in flight, and that one uses none of
+// these buffers: the copies of the call before are done once it has returned.
 static int ensure_pinned(nvllm_handle* h, void** p, size_t* have, size_t bytes) {
   if (bytes <= *have) return NVLLM_OK;
   if (*p) cudaFreeHost(*p);
