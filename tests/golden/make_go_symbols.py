@@ -2,7 +2,7 @@
 """Extracts the Go declarations the cgo shim (go/cuda_model_runner.go) binds against from the
 reference tree and writes them to tests/golden/go_symbols.json.
 
-    python tests/golden/make_go_symbols.py [/root/reference]
+    python tests/golden/make_go_symbols.py SOURCE
 
 No Go toolchain is needed: struct fields, exported package-level identifiers (types, consts,
 vars, funcs) and method sets are read with a small line parser.  tests/test_go_shim.py checks
@@ -84,7 +84,7 @@ def extract(root):
 
 
 if __name__ == "__main__":
-    root = sys.argv[1] if len(sys.argv) > 1 else "/root/reference"
+    root = sys.argv[1]
     out = os.path.join(os.path.dirname(os.path.abspath(__file__)), "go_symbols.json")
     json.dump(extract(root), open(out, "w"), indent=1, sort_keys=True)
     print("wrote", out)

@@ -4,7 +4,7 @@ Every selector the shim uses on a reference type — model.X, mc.X, engineCfg.X,
 a.X inside the attention type switch, s.X, t.X, tensor.X — must exist in the reference's Go
 declarations (tests/golden/go_symbols.json, extracted by tests/golden/make_go_symbols.py), every
 C.X must be declared by include/nvllm.h, and the shim's method set must cover the reference's
-ModelRunner interface plus the TensorModelRunner extras.  When /root/reference is present the
+ModelRunner interface plus the TensorModelRunner extras.  When NANO_VLLM_GO_SOURCE names a checkout of it the
 committed JSON is also checked against a fresh extraction.
 """
 import importlib.util
@@ -18,7 +18,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = os.path.join(ROOT, "go", "cuda_model_runner.go")
 SYMS = os.path.join(ROOT, "tests", "golden", "go_symbols.json")
 HDR = os.path.join(ROOT, "include", "nvllm.h")
-REF = "/root/reference"
+REF = os.environ.get("NANO_VLLM_GO_SOURCE", "")  # a checkout of the reference
 
 # variable -> (package, struct) as declared in the shim
 VAR_TYPES = {

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""profiles/ncu_traffic.json from the committed `ncu --set full` summaries (profiles/r2_full_*.md):
+"""profiles/ncu_traffic.json from the committed `ncu --set full` summaries (profiles/full_*.md):
 per workload and kernel class, the measured DRAM bytes per launch (dram__bytes_read.sum +
 dram__bytes_write.sum), averaged over the launches of that class in the captured window, next to
 the launch count and the mean duration under ncu.  bench.py reports the entry of its dominant
@@ -15,12 +15,12 @@ import sys
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 P = os.path.join(ROOT, "profiles")
 # summary file -> (workload name as bench.py's cfg.name, phase)
-FILES = {"r2_full_cfg2_prefill.md": ("llama-3.2-1b", "prefill", "batch 64 x 512-token prompts"),
-         "r2_full_cfg2_decode.md": ("llama-3.2-1b", "decode", "batch 64, context ~514"),
-         "r2_full_cfg1_decode.md": ("gpt2", "decode", "1 sequence, context ~34"),
-         "r2_full_cfg3_decode.md": ("granite-moe-1b", "decode", "batch 128, context ~130"),
-         "r2_full_cfg5_prefill.md": ("llama-3.2-3b", "prefill", "4 x 4096-token prompts, 2 layers"),
-         "r2_full_cfg4_falcon.md": ("falcon-7b", "mixed", "1 x 512-token prompt + decode steps, 2 layers")}
+FILES = {"full_cfg2_prefill.md": ("llama-3.2-1b", "prefill", "batch 64 x 512-token prompts"),
+         "full_cfg2_decode.md": ("llama-3.2-1b", "decode", "batch 64, context ~514"),
+         "full_cfg1_decode.md": ("gpt2", "decode", "1 sequence, context ~34"),
+         "full_cfg3_decode.md": ("granite-moe-1b", "decode", "batch 128, context ~130"),
+         "full_cfg5_prefill.md": ("llama-3.2-3b", "prefill", "4 x 4096-token prompts, 2 layers"),
+         "full_cfg4_falcon.md": ("falcon-7b", "mixed", "1 x 512-token prompt + decode steps, 2 layers")}
 CLASS = [("gemm_tc5_kernel", "gemm_tc5"), ("gemv_kernel", "gemv"), ("norm_kernel", "norm"),
          ("attn_prefill", "attn_prefill"), ("attn_decode", "attn_decode"), ("attn_combine", "attn_decode"),
          ("rope_kv", "rope_kv"), ("embed", "embed"), ("act_kernel", "act"), ("sample", "sample"),
