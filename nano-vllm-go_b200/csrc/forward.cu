@@ -462,7 +462,7 @@ int forward_step(nvllm_handle* h) {
     const float *cosT = h->use_rope ? h->cosT : nullptr, *sinT = h->use_rope ? h->sinT : nullptr;
     const Tc5Heads heads{h->nh, h->nkv, h->hd, d_pos, d_slots, cosT, sinT, (bf16*)kp, (bf16*)vp};
     const Tc5Heads* hp = is_prefill && h->adt == DT_BF16 && h->kvdt == DT_BF16 && (h->hd == 64 || h->hd == 128) ? &heads : nullptr;
-    if (one_row && !p1.p && !p2.p) {
+    if (one_row && (row_ffn || H <= 2048) && !p1.p && !p2.p) {
       GemvRowArgs r = row_args(nullptr, lw.wqkv, h->qkv_cols, H, TC5_EPI_PARTIAL, nullptr, 0.f);
       r.norm_w = lw.attn_norm_w; r.norm_b = lw.attn_norm_b; r.out = w.ws_a;
       if ((rc = run_gemv_row(h, r))) return rc;
