@@ -232,9 +232,11 @@ static bool speculation_hit(const nvllm_handle* h, int n, int is_prefill, const 
 }
 
 // Grows a pinned buffer of the handle.  Between two calls only a step issued ahead can be in flight, and that one uses none of
-// these buffers: the copies of the call before are done once it has returned.
+// these buffers: the copies of the call before are done once it has returned.  A quarter more than asked for: histories grow
+// by a token a sequence and step (256 sequences of 4000 tokens, locked anew in every call: 7.5 ms a step instead of 2.6).
 static int ensure_pinned(nvllm_handle* h, void** p, size_t* have, size_t bytes) {
   if (bytes <= *have) return NVLLM_OK;
+  bytes += bytes / 4;
   if (*p) cudaFreeHost(*p);
   *p = nullptr;
   *have = 0;
