@@ -127,6 +127,7 @@ attn_decode_t_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     // resolves.  Fused mode patches that row in shared memory, so nothing here depends on the
     // previous kernel at all.
     bool waited = fused;
+    const uint64_t once = l2_once();
     for (int f = 0; f < F; f++) {
       const int stage = f % STAGES;
       const int hh = f % KPC, j = f / KPC;  // heads interleaved tile by tile
@@ -143,8 +144,8 @@ attn_decode_t_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         mbar_expect_tx(full, 2 * TILE_BYTES);
 #pragma unroll
         for (int p = 0; p < PANELS; p++) {
-          tma_load_2d(sK + stage * TILE_BYTES + p * (BN * 128), &tmK, full, p * 64, row);
-          tma_load_2d(sV + stage * TILE_BYTES + p * (BN * 128), &tmV, full, p * 64, row);
+          tma_load_2d_hint(sK + stage * TILE_BYTES + p * (BN * 128), &tmK, full, p * 64, row, once);
+          tma_load_2d_hint(sV + stage * TILE_BYTES + p * (BN * 128), &tmV, full, p * 64, row, once);
         }
       }
       __syncwarp();

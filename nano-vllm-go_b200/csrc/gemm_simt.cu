@@ -40,10 +40,7 @@ int gemv_splits(int M, int N, int K) { return gemv_plan(M, N, K).S; }
 template <typename WT> struct Raw8;
 template <> struct Raw8<bf16> {
   uint4 v;
-  __device__ __forceinline__ void ld(const bf16* p) {
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  }
+  __device__ __forceinline__ void ld(const bf16* p) { v = ld_once16(p); }
   __device__ __forceinline__ void cvt(float (&o)[8]) const {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
@@ -55,16 +52,14 @@ template <> struct Raw8<bf16> {
   }
 };
 template <> struct Raw8<float> {
-  float4 a, b;
+  uint4 a, b;
   __device__ __forceinline__ void ld(const float* p) {
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w) : "l"(p));
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p + 4));
+    a = ld_once16(p);
+    b = ld_once16(p + 4);
   }
   __device__ __forceinline__ void cvt(float (&o)[8]) const {
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-    o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+    o[0] = __uint_as_float(a.x); o[1] = __uint_as_float(a.y); o[2] = __uint_as_float(a.z); o[3] = __uint_as_float(a.w);
+    o[4] = __uint_as_float(b.x); o[5] = __uint_as_float(b.y); o[6] = __uint_as_float(b.z); o[7] = __uint_as_float(b.w);
   }
 };
 

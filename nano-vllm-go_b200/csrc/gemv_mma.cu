@@ -63,7 +63,7 @@ gemv_mma_kernel(GemvMmaArgs a, Trace tr) {
     const bool in = k < ke;
 #pragma unroll
     for (int r = lr; r < 16 * MT; r += 4)
-      cp_async16(st + gm_at(r, lc), a.W + (size_t)min(n0 + r, a.N - 1) * a.K + (in ? k : 0), in);
+      cp_async16_once(st + gm_at(r, lc), a.W + (size_t)min(n0 + r, a.N - 1) * a.K + (in ? k : 0), in);
   };
   auto fetch_a = [&](int i) {
     const uint32_t st = base + (uint32_t)(i % NS) * STAGE + W_BYTES;

@@ -27,11 +27,6 @@ namespace nvllm {
 
 constexpr int GR_THREADS = 256, GR_WARPS = GR_THREADS / 32;
 
-__device__ __forceinline__ uint4 ld_weights16(const bf16* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
 __device__ __forceinline__ void widen8(const uint4& v, float (&o)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
@@ -65,7 +60,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemv_row_kernel(GemvRowArgs a, Tra
 #pragma unroll
       for (int i = 0; i < NL; i++) {
         const int k = k0 + i * kstep;
-        w[r][i] = k < a.K && n < a.N ? ld_weights16(a.W + (size_t)n * a.K + k) : make_uint4(0u, 0u, 0u, 0u);
+        w[r][i] = k < a.K && n < a.N ? ld_once16(a.W + (size_t)n * a.K + k) : make_uint4(0u, 0u, 0u, 0u);
       }
     }
   };
