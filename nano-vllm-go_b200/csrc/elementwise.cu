@@ -440,23 +440,51 @@ __global__ void __launch_bounds__(512) norm_kernel(NormArgs a, Trace tr) {
     trace_rec(tr, t_entry, t_wait, ((t_loads - t_wait) << 32) | (t_red - t_wait));
 }
 
-// The same for many rows whose addends need no summing over slices (prompts): a row stays in registers, four entries per
-// thread and vector, V vectors; all loads of a row, the expert rows of a combine included, are in flight at
-// once.  Bound by memory.  norm_kernel keeps eight entries per thread, sums up to eight slices, stages the row in shared
-// memory and needs 128 registers for all its options, too many for enough loads in flight.  Per launch inside whole
-// steps: 6446 rows of 2048 with one addend 55 -> 31 us (5.9 TB/s); 18 k rows of 2048, norm on the addend 148 -> 86 us;
-// 2048 rows of 4544, LayerNorm and two addends 54 -> 24 us; 18.7 k rows of 1024 through combines of eight expert rows and
-// routing 161 -> 140 us.  From 512 rows on (every SM has more than three); fewer keep norm_kernel, whose CTAs start
-// their weights' loads before the dependency resolves.
-constexpr int NR_MAX_V = 4, NR_THREADS = 512;
-template <typename YT, int V, int COMB>
-__global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Trace tr) {
+// The same with a row in registers, four entries per thread and vector, V vectors, and all loads of a row in flight at once,
+// the expert rows of a combine (COMB) and up to SL slices of an addend included.  norm_kernel keeps eight entries per
+// thread (a warp's 16-byte loads then touch every sector twice), stages the row in shared memory and needs 128 registers
+// for all its options.
+// Prompts (SL = 1; their addends need no summing over slices): bound by memory.  Per launch inside whole steps: 6446 rows of
+// 2048 with one addend 55 -> 31 us (5.9 TB/s); 18 k rows of 2048, norm on the addend 148 -> 86 us; 2048 rows of 4544,
+// LayerNorm and two addends 54 -> 24 us; 18.7 k rows of 1024 through combines of eight expert rows and routing 161 -> 140
+// us.  From 512 rows on (every SM has more than three).
+// Steps of fewer rows (SL = 8): bound by one L2 round trip, two block sums at most and the way in and out of the launch;
+// weights and biases are loaded before the dependency resolves.  64 rows of 2048 with eight slices, from the release to the last
+// exit: 4.9 -> 2.7 us; 16 decode steps of 64 sequences through four Llama-1B layers 4668 -> 4330 us, of 128 through routed
+// experts (every second norm) 5694 -> 5505.
+constexpr int NR_MAX_V = 4, NR_THREADS = 512, NR_STEP_THREADS = 640;
+template <typename YT, int V, int COMB, int SL>
+__global__ void __launch_bounds__(SL > 1 ? NR_STEP_THREADS : NR_THREADS, SL > 1 ? 1 : 2) norm_rows_kernel(NormArgs a, Trace tr) {
   const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
   pdl_launch_dependents();
   __shared__ float red[32];
-  const int H = a.H, r = blockIdx.x;
+  const int H = a.H;
+  constexpr bool STEP = SL > 1, AHEAD = STEP && V <= 2;
+  auto get = [](const float* p, float (&o)[4]) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
+  };
+  float wa[AHEAD ? V : 1][4], ba[AHEAD ? V : 1][4], b1a[AHEAD ? V : 1][4], b2a[AHEAD ? V : 1][4];
+  if constexpr (AHEAD) {
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const int i = ((int)threadIdx.x + k * (int)blockDim.x) * 4;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        wa[k][j] = 1.f;
+        ba[k][j] = b1a[k][j] = b2a[k][j] = 0.f;
+      }
+      if (i >= H) continue;
+      if (a.w) get(a.w + i, wa[k]);
+      if (a.b) get(a.b + i, ba[k]);
+      if (a.p1 && a.bias1) get(a.bias1 + i, b1a[k]);
+      if (a.p2 && a.bias2) get(a.bias2 + i, b2a[k]);
+    }
+  }
   pdl_wait();
   const unsigned long long t_wait = trace_on(tr) ? gtime() : 0ull;
+  const int orow = blockIdx.x;
+  const int r = STEP && a.row_idx ? a.row_idx[orow] - a.row_bias : orow;
   float* xr = a.x + (size_t)r * H;
   float v[V][4], acc[V][4];
   int prow[COMB ? COMB : 1];
@@ -468,10 +496,6 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
       cw[q] = q < a.comb_k ? a.comb_w[(size_t)r * a.comb_k + q] : 0.f;
     }
   }
-  auto get = [](const float* p, float (&o)[4]) {
-    const float4 f = *reinterpret_cast<const float4*>(p);
-    o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
-  };
 #pragma unroll
   for (int k = 0; k < V; k++) {
     const int i = ((int)threadIdx.x + k * (int)blockDim.x) * 4;
@@ -479,6 +503,13 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
     for (int j = 0; j < 4; j++) v[k][j] = acc[k][j] = 0.f;
     if (i >= H) continue;
     get(xr + i, v[k]);
+    float p2[4] = {0.f, 0.f, 0.f, 0.f}, b[4];
+    float s2[SL][4];
+    if (a.p2 && !a.post) {
+#pragma unroll
+      for (int q = 0; q < SL; q++)
+        if (q == 0 || q < a.S2) get(a.p2 + (size_t)q * a.stride2 + (size_t)r * H + i, s2[q]);
+    }
     if constexpr (COMB > 0) {
       float pv[COMB][4];
 #pragma unroll
@@ -491,20 +522,35 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
           for (int j = 0; j < 4; j++) acc[k][j] += cw[q] * pv[q][j];
         }
     } else if (a.p1) {
-      get(a.p1 + (size_t)r * H + i, acc[k]);
+      float s1[SL][4];
+#pragma unroll
+      for (int q = 0; q < SL; q++)
+        if (q == 0 || q < a.S1) get(a.p1 + (size_t)q * a.stride1 + (size_t)r * H + i, s1[q]);
+#pragma unroll
+      for (int q = 0; q < SL; q++)
+        if (q == 0 || q < a.S1) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[k][j] += s1[q][j];
+        }
     }
     if (a.post) continue;
-    float p2[4] = {0.f, 0.f, 0.f, 0.f}, b[4];
-    if (a.p2) get(a.p2 + (size_t)r * H + i, p2);
-    if (a.p1 && a.bias1) {
-      get(a.bias1 + i, b);
+    if (a.p2) {
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[k][j] += b[j];
+      for (int q = 0; q < SL; q++)
+        if (q == 0 || q < a.S2) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) p2[j] += s2[q][j];
+        }
+    }
+    if (a.p1 && a.bias1) {
+      if constexpr (!AHEAD) get(a.bias1 + i, b);
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[k][j] += AHEAD ? b1a[AHEAD ? k : 0][j] : b[j];
     }
     if (a.p2 && a.bias2) {
-      get(a.bias2 + i, b);
+      if constexpr (!AHEAD) get(a.bias2 + i, b);
 #pragma unroll
-      for (int j = 0; j < 4; j++) p2[j] += b[j];
+      for (int j = 0; j < 4; j++) p2[j] += AHEAD ? b2a[AHEAD ? k : 0][j] : b[j];
     }
     if (a.p1)
 #pragma unroll
@@ -544,8 +590,16 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
       const int i = ((int)threadIdx.x + k * (int)blockDim.x) * 4;
       if (i >= H) continue;
       float w[4] = {1.f, 1.f, 1.f, 1.f}, b[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
-      if (a.w) get(a.w + i, w);
-      if (a.b) get(a.b + i, b);
+      if constexpr (AHEAD) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          w[j] = wa[k][j];
+          b[j] = ba[k][j];
+        }
+      } else {
+        if (a.w) get(a.w + i, w);
+        if (a.b) get(a.b + i, b);
+      }
       if (a.post) {
 #pragma unroll
         for (int j = 0; j < 4; j++) o[j] = fmaf(acc[k][j] * inv, w[j], v[k][j]);
@@ -557,27 +611,36 @@ __global__ void __launch_bounds__(NR_THREADS, 2) norm_rows_kernel(NormArgs a, Tr
 #pragma unroll
         for (int j = 0; j < 4; j++) o[j] = v[k][j] * inv * w[j];
       }
-      if (a.y) store4((YT*)a.y + (size_t)r * H + i, o);
-      if (a.y_f32 && !a.post) store4(a.y_f32 + (size_t)r * H + i, o);
+      if (a.y) store4((YT*)a.y + (size_t)orow * H + i, o);
+      if (a.y_f32 && !a.post) store4(a.y_f32 + (size_t)orow * H + i, o);
     }
   }
   if (threadIdx.x == 0 && trace_on(tr))  // what the row took in: 1 an addend (2: expert rows), 4 a second one, 8 normed on it
     trace_rec(tr, t_entry, t_wait, (a.p1 ? 1ull : 0ull) | (COMB ? 2ull : 0ull) | (a.p2 ? 4ull : 0ull) | (a.post ? 8ull : 0ull));
 }
-// many rows, no option of norm_kernel that these kernels lack, at most one slice (or eight expert rows) per addend
-static bool norm_rows_fit(const NormArgs& a) {
-  return a.n_rows >= 512 && a.H % 8 == 0 && a.H <= NR_MAX_V * NR_THREADS * 4 && !a.row_idx && !a.router && !a.gate_w && !a.plain &&
-         a.groups <= 1 && !a.xadd && !a.xadd_table && !a.row_m2 && !a.conv_taps && !a.p1_bf16 &&
-         (!a.p1 || (a.comb_rows ? a.comb_k <= 8 : a.S1 == 1)) && (!a.p2 || a.S2 == 1) &&
+// no option of norm_kernel that these kernels lack; at most eight expert rows
+static bool norm_rows_plain(const NormArgs& a) {
+  return a.H % 8 == 0 && !a.router && !a.gate_w && !a.plain && a.groups <= 1 && !a.xadd && !a.xadd_table && !a.row_m2 &&
+         !a.conv_taps && !a.p1_bf16 && (!a.p1 || !a.comb_rows || a.comb_k <= 8) &&
          (!a.post || (a.p1 && a.w && !a.comb_rows && !a.p2));
 }
-template <typename YT>
+// many rows, at most one slice per addend
+static bool norm_rows_fit(const NormArgs& a) {
+  return norm_rows_plain(a) && a.n_rows >= 512 && a.H <= NR_MAX_V * NR_THREADS * 4 && !a.row_idx &&
+         (!a.p1 || a.comb_rows || a.S1 == 1) && (!a.p2 || a.S2 == 1);
+}
+// few rows, at most eight slices (what the products of a step are split into)
+static bool norm_step_fit(const NormArgs& a) {
+  return norm_rows_plain(a) && a.n_rows < 512 && a.H <= NR_MAX_V * NR_STEP_THREADS * 4 && (!a.p1 || a.comb_rows || a.S1 <= 8) &&
+         (!a.p2 || a.S2 <= 8);
+}
+template <typename YT, int SL>
 static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
-  const int V = ceil_div(a.H, NR_THREADS * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
+  const int V = ceil_div(a.H, (SL > 1 ? NR_STEP_THREADS : NR_THREADS) * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
   const bool comb = a.p1 && a.comb_rows;
-#define NR(V_)                                                                                                       \
-  (comb ? launch_k(norm_rows_kernel<YT, V_, 8>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47))             \
-        : launch_k(norm_rows_kernel<YT, V_, 0>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47)))
+#define NR(V_)                                                                                                           \
+  (comb ? launch_k(norm_rows_kernel<YT, V_, 8, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47))             \
+        : launch_k(norm_rows_kernel<YT, V_, 0, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47)))
   return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
 #undef NR
 }
@@ -585,7 +648,8 @@ static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
 cudaError_t launch_norm(cudaStream_t st, const NormArgs& a) {
   if (a.n_rows <= 0) return cudaSuccess;
   if (a.groups > 64 || (a.groups > 1 && a.H % a.groups) || (a.plain && !a.y)) return cudaErrorInvalidValue;
-  if (norm_rows_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float>(st, a) : launch_norm_rows<bf16>(st, a);
+  if (norm_rows_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float, 1>(st, a) : launch_norm_rows<bf16, 1>(st, a);
+  if (norm_step_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float, 8>(st, a) : launch_norm_rows<bf16, 8>(st, a);
   int threads = min(512, max(64, ((a.H / 8 + 31) / 32) * 32));
   // fused router, decode-sized batches (latency-bound: fewer row CTAs than two waves): 16 warps
   // so that each takes two experts of a 32-expert layer in one pass; prefill keeps the

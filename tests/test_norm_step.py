@@ -1,0 +1,58 @@
+"""Norms of steps of few rows (elementwise.cu norm_rows_kernel, slices of a product summed on the way): a decode step against
+the same tokens as the ends of whole prompts, whose norms are other kernels or part of the products."""
+import numpy as np
+import pytest
+
+from helpers import C, W
+import nvllm_pkg
+
+pytestmark = pytest.mark.gpu
+
+ROWS, GENERAL = 47, 2  # kernel ids in the timeline
+
+
+def gpt2(hidden):
+    return C.tiny_gpt2(hidden=hidden, num_layers=2, num_heads=2, num_kv_heads=2, head_dim=64, ffn_dim=1096)
+
+
+def llama(hidden):
+    return C.tiny_llama(hidden=hidden, num_layers=2, num_heads=4, num_kv_heads=2, head_dim=64, ffn_dim=1096)
+
+
+def falcon(hidden):
+    return C.tiny_falcon(hidden=hidden, num_layers=2, num_heads=3, head_dim=64, ffn_dim=1096)
+
+
+@pytest.mark.parametrize("cfg", [
+    gpt2(64), llama(72),                       # half a warp; a thread more
+    gpt2(2056), llama(2560), falcon(2048),     # one vector, the last one: five slices and more
+    llama(2568), falcon(4544), gpt2(5120),     # two
+    falcon(5128), llama(7688),                 # three; four
+    gpt2(10240), llama(10248),                 # the widest; wider
+], ids=lambda c: f"{c.name}-{c.hidden}")
+def test_step_matches_the_prompts(cfg):
+    n = 12
+    texts = [W.random_prompt(cfg.vocab_size, 61 + 3 * i, 160 + i) for i in range(n)]
+    weights = list(W.random_weights(cfg, 17, round_bf16=True))
+    tables, zeros = [[i] for i in range(n)], [0.0] * n
+
+    def ends(precision, step):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, weights, precision=precision, num_kv_blocks=n, sampling=None)
+        try:
+            run.set_graphs(False)
+            run.set_speculation(False)
+            if not step:
+                return run.run_flat(texts, True, [0] * n, tables, zeros, want_logits=True)[1]
+            run.run_flat([t[:-1] for t in texts], True, [0] * n, tables, zeros)
+            run.trace_begin(1 << 18)
+            out = run.run_flat(texts, False, None, tables, zeros, want_logits=True)[1]
+            ran = set(run.trace_end(1 << 18)[:, 1].tolist())
+            assert (ROWS in ran, GENERAL in ran) == (cfg.hidden <= 10240, cfg.hidden > 10240)
+            return out
+        finally:
+            run.close()
+
+    want, prompts, step = ends(C.PREC_FP32, False), ends(C.PREC_BF16, False), ends(C.PREC_BF16, True)
+    # the same bf16 roundings, sums in another order: as far from float32 as the prompts are (the error's norm over n rows is
+    # known to a tenth or so)
+    assert np.linalg.norm(step - want) <= 1.25 * np.linalg.norm(prompts - want)
