@@ -639,8 +639,8 @@ static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
   const int V = ceil_div(a.H, (SL > 1 ? NR_STEP_THREADS : NR_THREADS) * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
   const bool comb = a.p1 && a.comb_rows;
 #define NR(V_)                                                                                                           \
-  (comb ? launch_k(norm_rows_kernel<YT, V_, 8, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47))             \
-        : launch_k(norm_rows_kernel<YT, V_, 0, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(47)))
+  (comb ? launch_k(norm_rows_kernel<YT, V_, 8, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(SL > 1 ? 53 : 47)) \
+        : launch_k(norm_rows_kernel<YT, V_, 0, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(SL > 1 ? 53 : 47)))
   return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
 #undef NR
 }

@@ -470,14 +470,14 @@ int forward_step(nvllm_handle* h) {
     } else if (xb_parts > 0 && fold_gemm_ok(h, T, h->qkv_cols, H, H)) {
       RowScale rsc{w.ssq, xb_parts};
       if ((rc = run_gemm(h, w.xb, H, lw.wqkv, T, h->qkv_cols, H, 1.f, w.ws_a, w.ws_a_floats,
-                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, nullptr, 0, 0.0, &rsc, nullptr, nullptr, hp, w.q)))
+                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, 0.0, &rsc, nullptr, nullptr, hp, w.q)))
         return rc;
     } else {
       if ((rc = run_norm(h, w.x, &p1, &p2, lw.attn_norm_w, lw.attn_norm_b, w.xn,
                          nullptr, nullptr, T)))
         return rc;
       if ((rc = run_gemm(h, w.xn, H, lw.wqkv, T, h->qkv_cols, H, 1.f, w.ws_a, w.ws_a_floats,
-                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, nullptr, 0, 0.0, nullptr, nullptr, nullptr, hp, w.q)))
+                         h->qkv_cols, &qkv, 0, nullptr, 0, lw.bqkv, 0.0, nullptr, nullptr, nullptr, hp, w.q)))
         return rc;
     }
     xb_parts = 0;
@@ -516,7 +516,7 @@ int forward_step(nvllm_handle* h) {
     } else if (resid_gemm_ok(h, T, H, h->q_cols, h->q_cols)) {
       Resid rd{m_res, lw.bo, 0, lw.ffn_norm_w};
       if ((rc = run_gemm(h, w.attn_out, h->q_cols, lw.wo, T, H, h->q_cols, 1.f, w.ws_b,
-                         w.ws_b_floats, H, &p1, 0, nullptr, 0, nullptr, nullptr, 0, 0.0, nullptr, &rd)))
+                         w.ws_b_floats, H, &p1, 0, nullptr, 0, nullptr, 0.0, nullptr, &rd)))
         return rc;
       xb_parts = h_tiles;
     } else {
@@ -567,7 +567,7 @@ int forward_step(nvllm_handle* h) {
         Tc5Args t1{};
         t1.A = w.xn; t1.W = lw.w1; t1.M = T; t1.N = h->w1_cols; t1.K = H; t1.S = 1; t1.alpha = 1.f;
         t1.epi = h->swiglu ? TC5_EPI_SWIGLU : TC5_EPI_GELU; t1.epi_out = w.hbuf; t1.epi_ld = h->F;
-        t1.epi_bias = lw.b1;
+        t1.epi_bias = lw.b1; t1.wait_flag = h->waits.dev;
         Tc5Args t2{};
         t2.A = w.hbuf; t2.W = lw.w2; t2.M = T; t2.N = H; t2.K = h->F; t2.alpha = 1.f;
         t2.out = ffn_out; t2.ldo = H; t2.split_stride = (size_t)T * H; t2.out_capacity = w.ws_b_floats;
@@ -589,7 +589,7 @@ int forward_step(nvllm_handle* h) {
       RowScale rsc{xb_parts > 0 ? w.ssq : nullptr, xb_parts};
       if ((rc = run_gemm(h, xb_parts > 0 ? w.xb : w.xn, H, lw.w1, T, h->w1_cols, H, 1.f, w.ws_a,
                          w.ws_a_floats, h->w1_cols, &h1, h->swiglu ? TC5_EPI_SWIGLU : TC5_EPI_GELU,
-                         w.hbuf, h->F, lw.b1, nullptr, 0, 0.0, &rsc)))
+                         w.hbuf, h->F, lw.b1, 0.0, &rsc)))
         return rc;
       xb_parts = 0;
       if (h1.S > 0 && gpre_act) {
@@ -597,7 +597,7 @@ int forward_step(nvllm_handle* h) {
         ga.mode = 2; ga.hp = h1.p; ga.Sh = h1.S; ga.hstride = h1.stride; ga.hld = h->w1_cols;
         ga.hbias = lw.b1; ga.swiglu = h->swiglu ? 1 : 0;
         if ((rc = run_gemm(h, w.hbuf, h->F, lw.w2, T, H, h->F, 1.f, ffn_out, w.ws_b_floats, H, &pf, 0,
-                           nullptr, 0, nullptr, nullptr, 0, 0.0, nullptr, nullptr, &ga)))
+                           nullptr, 0, nullptr, 0.0, nullptr, nullptr, &ga)))
           return rc;
         pf.bias = lw.b2;
         pf.m = h->parallel ? (par_scaled ? c.residual_multiplier : 1.f) : m_res;
@@ -613,7 +613,7 @@ int forward_step(nvllm_handle* h) {
         // the next reader of x is layer l + 1's attention norm (the final norm reads fp32 x)
         Resid rd{m_res, lw.b2, 1, l + 1 < h->L ? h->layers[l + 1].attn_norm_w : nullptr};
         if ((rc = run_gemm(h, w.hbuf, h->F, lw.w2, T, H, h->F, 1.f, ffn_out, w.ws_b_floats, H, &pf, 0,
-                           nullptr, 0, nullptr, nullptr, 0, 0.0, nullptr, &rd)))
+                           nullptr, 0, nullptr, 0.0, nullptr, &rd)))
           return rc;
         xb_parts = h_tiles;
       } else {
@@ -655,7 +655,7 @@ int forward_step(nvllm_handle* h) {
     vsplit = Vl;
   } else {
     if ((rc = run_gemm(h, w.xn_last, H, h->lm_head, n_out, h->V, H, alpha, w.logits_p,
-                       w.logits_p_floats, h->ldl, &lg, 0, nullptr, 0, nullptr, nullptr, 0,
+                       w.logits_p_floats, h->ldl, &lg, 0, nullptr, 0, nullptr,
                        (double)n_out * h->V * 4)))
       return rc;
     logits = lg.p;

@@ -795,7 +795,7 @@ static int ffn_dense_unary(nvllm_handle* h, const ListedLayer& y, Pending* out) 
   if (h1.S > 0 && T <= 8 && !(gpre_env && atoi(gpre_env) == 0)) {
     GemvPre ga{};
     ga.mode = 2; ga.hp = h1.p; ga.Sh = h1.S; ga.hstride = h1.stride; ga.hld = ff; ga.swiglu = 2;
-    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, out, 0, nullptr, 0, nullptr, nullptr, 0,
+    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, out, 0, nullptr, 0, nullptr,
                     0.0, nullptr, nullptr, &ga);
   }
   if (h1.S > 0) {
@@ -1175,7 +1175,7 @@ static int ffn_moe_relu2(nvllm_handle* h, const ListedLayer& y, float* topk_w, P
   if (h1.S > 0 && T <= 8 && !(gpre_env && atoi(gpre_env) == 0)) {
     GemvPre ga{};
     ga.mode = 2; ga.hp = h1.p; ga.Sh = h1.S; ga.hstride = h1.stride; ga.hld = ff; ga.swiglu = 2;
-    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, p2, 0, nullptr, 0, nullptr, nullptr, 0,
+    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, p2, 0, nullptr, 0, nullptr,
                     0.0, nullptr, nullptr, &ga);
   }
   if (h1.S > 0) {
@@ -1216,7 +1216,7 @@ static int ffn_glu(nvllm_handle* h, const ListedLayer& y, int ff, float limit, P
   if (h1.S > 0 && T <= 8 && !(gpre_env && atoi(gpre_env) == 0)) {
     GemvPre ga{};
     ga.mode = 2; ga.hp = h1.p; ga.Sh = h1.S; ga.hstride = h1.stride; ga.hld = 2 * ff; ga.swiglu = 1; ga.glu_limit = limit;
-    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, out, 0, nullptr, 0, nullptr, nullptr, 0,
+    return run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_b, w.ws_b_floats, H, out, 0, nullptr, 0, nullptr,
                     0.0, nullptr, nullptr, &ga);
   }
   if (h1.S > 0) {
@@ -1608,7 +1608,7 @@ int forward_step_layered(nvllm_handle* h) {
         ga.mode = 2; ga.hp = h1.p; ga.Sh = h1.S; ga.hstride = h1.stride; ga.hld = 2 * ff;
         ga.swiglu = 1; ga.glu_limit = s.limit;
         if ((rc = run_gemm(h, w.hbuf, ff, y.w2, T, H, ff, 1.f, w.ws_c, w.ws_b_floats, H, &pm, 0, nullptr, 0,
-                           nullptr, nullptr, 0, 0.0, nullptr, nullptr, &ga)))
+                           nullptr, 0.0, nullptr, nullptr, &ga)))
           return rc;
       } else {
         if (h1.S > 0) {
@@ -1636,7 +1636,7 @@ int forward_step_layered(nvllm_handle* h) {
   Pending lg;
   if ((rc = run_gemm(h, w.xn_last, H, h->lm_head, n_out, h->V, H, h->logit_scale != 0.f ? h->logit_scale : 1.f, w.logits_p,
                      w.logits_p_floats, h->ldl, &lg, 0,
-                     nullptr, 0, nullptr, nullptr, 0, (double)n_out * h->V * 4)))
+                     nullptr, 0, nullptr, (double)n_out * h->V * 4)))
     return rc;
   {
     ProfScope ps(h, NVLLM_K_MISC, (double)n_out * h->ldl * 8, 0, (double)n_out * h->ldl * 4 * (lg.S - 1));

@@ -124,7 +124,7 @@ static size_t split_capacity(const nvllm_handle* h, const float* out, size_t cap
 static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int M, int N, int K,
                     float alpha, float* out, size_t cap, int ldo, Pending* res, int epi = 0,
                     void* epi_out = nullptr, int epi_ld = 0, const float* epi_bias = nullptr,
-                    const void* pf_ptr = nullptr, size_t pf_bytes = 0, double alg_out = 0.0,
+                    double alg_out = 0.0,
                     const RowScale* rs = nullptr, const Resid* rd = nullptr,
                     const GemvPre* gp = nullptr, const Tc5Heads* heads = nullptr, void* q_out = nullptr) {
   res->p = out;
@@ -186,10 +186,6 @@ static int run_gemm(nvllm_handle* h, const void* A, int lda, const void* W, int 
       LAUNCH(h, launch_gemm_tc5(h->stream, t, nullptr));
       *res = Pending();
       return NVLLM_OK;
-    }
-    if (M <= 128) {  // weight-streaming regime: warm L2 with the next big matrix
-      t.pf_ptr = pf_ptr;
-      t.pf_bytes = pf_bytes;
     }
     if (heads && t.S == 1) {
       t.heads = heads; t.epi_out = q_out; t.epi_ld = heads->nh * heads->hd; t.epi_bias = epi_bias;

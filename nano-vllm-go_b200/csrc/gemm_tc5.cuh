@@ -13,6 +13,8 @@ namespace nvllm {
 constexpr int TC_BN = 128;  // weight rows per CTA (UMMA M)
 constexpr int TC_BK = 64;   // k elements per stage = one 128-byte swizzle row of bf16
 constexpr int TC_THREADS = 192;
+// k-blocks that a stage of the one-CTA kernel's ring holds (one wait each for producer and MMAs)
+__host__ __device__ constexpr int tc5_stage_blocks(int BT) { return BT <= 128 ? 2 : 1; }
 
 // The work of a launch: units (token tile, weight tile, k split) dealt out round-robin.
 struct Tc5Sched {

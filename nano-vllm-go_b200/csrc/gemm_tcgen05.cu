@@ -52,6 +52,7 @@ struct Tc5Chain {
   float alpha;
   unsigned* ctr;
   int n_waiters;  // CTAs owning at least one unit of problem 2
+  int* flag;      // WaitFlag::dev of the wait (null: none)
 };
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
@@ -81,8 +82,7 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmA2,
                 int M, int N_a, Tc5Sched sc, float* __restrict__ out_a, int ldo_a, size_t split_stride_a,
                 float alpha_a, int w_reused, int epi_a, bf16* __restrict__ epi_out, int epi_ld,
-                const float* __restrict__ epi_bias, int prefetch, const uint8_t* __restrict__ pf_ptr,
-                unsigned long long pf_bytes, Tc5Fuse fz, Tc5Chain ch, Trace tr) {
+                const float* __restrict__ epi_bias, int prefetch, Tc5Fuse fz, Tc5Chain ch, Trace tr) {
   const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
   unsigned long long t_wait = 0;
   __shared__ unsigned long long tr_mma, tr_epi0, tr_epi1, tr_x[6], tr_c[4];
@@ -91,7 +91,8 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   __shared__ float ssq_s[2][4][32];     // RESID: per-warp row sums of squares of a 32-token chunk
   constexpr uint32_t W_BYTES = TC_BN * TC_BK * 2;
   constexpr uint32_t A_BYTES = BT * TC_BK * 2;
-  constexpr uint32_t STAGE_BYTES = W_BYTES + A_BYTES;
+  constexpr int KB = tc5_stage_blocks(BT);
+  constexpr uint32_t STAGE_BYTES = KB * (W_BYTES + A_BYTES);  // [weight blocks][activation blocks]
   extern __shared__ uint8_t smem_raw[];
   const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;  // SWIZZLE_128B needs 1024 B
   const uint32_t bars = tiles + STAGES * STAGE_BYTES;
@@ -144,11 +145,10 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   // each warp right before its phase-B arrival; phase B = "my slices are in the owners' buffers"
   if (fz.cl > 1) cluster_arrive_relaxed();
 
-  // The producer and MMA warps run their loops with ALL 32 lanes (warp-uniform control flow)
-  // and elect one lane only around the issue instructions: TMA and tcgen05 instructions take
-  // uniform-register operands, and inside a divergent `if (lane == 0)` region the compiler
-  // wraps every one of them in an elect/branch loop plus R2UR moves (~120 cycles per MMA
-  // measured on B200 — enough to make a skinny GEMM issue-bound instead of HBM-bound).
+  // Producer and MMA warp: one elected thread runs all of a loop.  With an election around each stage's instructions the
+  // compiler brings every descriptor to the uniform registers anew and the issue takes 335 cycles per 64 k of 64 tokens;
+  // so it takes 237, and 194 with two blocks of k per wait (32 / 64 / 128 tokens 173 / 194 / 257: the rate of the MMAs).
+  // 16 decode steps, 64 sequences through four Llama-1B layers: 4350 -> 4130 us.
   if (warp == 0) {
     // weights read once per step must not displace activations in L2; weights re-read by
     // other token tiles (prefill) stay
@@ -158,26 +158,31 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     else
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_a));
-    // (1) weight tiles of the first STAGES k-blocks, before the dependency resolves (dense
+    // (1) weight tiles of the first STAGES stages, before the dependency resolves (dense
     // mode only: a grouped GEMM learns which expert a tile multiplies from the previous kernel)
+    auto load_weights = [&](int s, const CUtensorMap* map, const Tc5Unit& t, int kb) {  // of a stage, and what it expects
+      const uint32_t full = bars + 8 * s, dst = tiles + s * STAGE_BYTES;
+      const int nb = min(KB, t.nkb - kb);
+      mbar_expect_tx(full, nb * (W_BYTES + A_BYTES));
+#pragma unroll
+      for (int j = 0; j < KB; j++)
+        if (j < nb) tma_load_2d_hint(dst + j * W_BYTES, map, full, tc5_kb(t.kb0, kb + j, t.rot, t.nkb) * TC_BK, t.wrow, pol_w);
+    };
     int pre = 0;
-    {
+    if ((prefetch & 1) && !grouped) {
       int u = blockIdx.x, kb = 0;
-      while ((prefetch & 1) && !grouped && pre < STAGES && u < sc.units) {
+      const bool leader = elect_one();
+      while (pre < STAGES && u < sc.units) {
         const Tc5Unit t = tc5_unit(sc, u, BT, M);
-        const uint32_t full = bars + 8 * pre;
-        if (elect_one()) {
-          mbar_expect_tx(full, (prefetch & 2) ? W_BYTES : STAGE_BYTES);
-          tma_load_2d_hint(tiles + pre * STAGE_BYTES, &tmW, full,
-                           tc5_kb(t.kb0, kb, t.rot, t.nkb) * TC_BK, t.wrow, pol_w);
-        }
-        __syncwarp();
+        if (leader) load_weights(pre, &tmW, t, kb);
         pre++;
-        if (++kb == t.nkb) {
+        kb += KB;
+        if (kb >= t.nkb) {
           kb = 0;
           u += grid;
         }
       }
+      __syncwarp();
     }
     // (1a') grouped mode cannot know its experts before the sort kernel has run, but a decode
     // batch routes a handful of rows to EVERY expert: one token tile per expert, in expert
@@ -198,79 +203,57 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
       }
     }
-    // (1b) L2 prefetch of the weights a LATER kernel streams (immutable, so legal before the
-    // wait): this kernel's own stream leaves HBM idle while it waits for its dependency and
-    // during its epilogue; the next big GEMM then reads L2 instead of HBM.
-    if (pf_bytes) {
-      const unsigned long long per = ((pf_bytes + gridDim.x - 1) / gridDim.x + 127) & ~127ull;
-      const unsigned long long lo = per * blockIdx.x;
-      const unsigned long long hi = lo + per < pf_bytes ? lo + per : pf_bytes;
-      constexpr unsigned long long PIECE = 16384;
-      for (unsigned long long o = lo + (unsigned long long)lane * PIECE; o < hi; o += 32 * PIECE) {
-        const uint32_t sz = (uint32_t)((hi - o < PIECE ? hi - o : PIECE) & ~15ull);
-        if (sz)
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pf_ptr + o), "r"(sz)
-                       : "memory");
-      }
-    }
     pdl_wait();
     if (trace_on(tr)) t_wait = gtime();
     // (2) their activation tiles, then (3) the steady state
-    int i = 0;
-    int ahead_lo = 0, ahead_hi = pre;  // k-block range [lo, hi) whose weight tile is already in flight
-    for (int p = 0; p < 2; p++) {
-      const Tc5Sched& scp = p ? ch.sc : sc;
-      const CUtensorMap* mW = p ? &tmW2 : &tmW;
-      const CUtensorMap* mA = p ? &tmA2 : &tmA;
-      const int units = p ? ch.sc.units : (grouped ? *sc.g_ntiles * sc.n_tiles : sc.units);
-      if (p == 1 && (int)blockIdx.x < units) {
-        // chained GEMM: weight tiles of the first k-blocks now, activations after problem 1 is done
-        const Tc5Unit t = tc5_unit(scp, blockIdx.x, BT, M);
-        const int na = min(STAGES, t.nkb);
-        for (int kb = 0; kb < na; kb++) {
-          const int ii = i + kb, s = ii % STAGES;
-          mbar_wait(bars + 8 * (STAGES + s), ((ii / STAGES) & 1) ^ 1);
-          if (elect_one()) {
-            mbar_expect_tx(bars + 8 * s, STAGE_BYTES);
-            tma_load_2d_hint(tiles + s * STAGE_BYTES, mW, bars + 8 * s,
-                             tc5_kb(t.kb0, kb, t.rot, t.nkb) * TC_BK, t.wrow, pol_w);
+    if (elect_one()) {
+      int i = 0;
+      int ahead_lo = 0, ahead_hi = pre;  // stages [lo, hi) whose weight tiles are already in flight
+      for (int p = 0; p < 2; p++) {
+        const Tc5Sched& scp = p ? ch.sc : sc;
+        const CUtensorMap* mW = p ? &tmW2 : &tmW;
+        const CUtensorMap* mA = p ? &tmA2 : &tmA;
+        const int units = p ? ch.sc.units : (grouped ? *sc.g_ntiles * sc.n_tiles : sc.units);
+        if (p == 1 && (int)blockIdx.x < units) {
+          // chained GEMM: weight tiles of the first stages now, activations after problem 1 is done
+          const Tc5Unit t = tc5_unit(scp, blockIdx.x, BT, M);
+          ahead_lo = ahead_hi = i;
+          for (int kb = 0; kb < t.nkb && ahead_hi < i + STAGES; kb += KB, ahead_hi++) {
+            const int s = ahead_hi % STAGES;
+            mbar_wait(bars + 8 * (STAGES + s), ((ahead_hi / STAGES) & 1) ^ 1);
+            load_weights(s, mW, t, kb);
           }
-          __syncwarp();
-        }
-        ahead_lo = i;
-        ahead_hi = i + na;
-        if (elect_one()) {
-          while (ld_acquire_u32(ch.ctr) < (unsigned)sc.units) {
-          }
+          const unsigned long long t0 = gtime();
+          while (ld_acquire_u32(ch.ctr) < (unsigned)sc.units)
+            if (gtime() - t0 > TC_WAIT_NS) {  // (the result is of no use then: the host reads the flag)
+              if (ch.flag) *reinterpret_cast<volatile int*>(ch.flag) = 1;
+              break;
+            }
           if (atomicAdd(ch.ctr + 1, 1u) == (unsigned)ch.n_waiters - 1) {  // everyone is past the wait
             ch.ctr[0] = 0;
             ch.ctr[1] = 0;
           }
+          // the activations were written through the generic proxy by other CTAs; TMA reads them
+          asm volatile("fence.proxy.async;" ::: "memory");
         }
-        __syncwarp();
-        // the activations were written through the generic proxy by other CTAs; TMA reads them
-        asm volatile("fence.proxy.async;" ::: "memory");
-      }
-      for (int u = blockIdx.x; u < units; u += grid) {
-        const Tc5Unit t = tc5_unit(scp, u, BT, M);
-        for (int kb = 0; kb < t.nkb; kb++, i++) {
-          const int s = i % STAGES;
-          const uint32_t full = bars + 8 * s;
-          const uint32_t dst = tiles + s * STAGE_BYTES;
-          const int k = tc5_kb(t.kb0, kb, t.rot, t.nkb) * TC_BK;
-          const bool w_ahead = i >= ahead_lo && i < ahead_hi;
-          if (!w_ahead) mbar_wait(bars + 8 * (STAGES + s), ((i / STAGES) & 1) ^ 1);
-          if (elect_one()) {
-            if (!w_ahead) {
-              mbar_expect_tx(full, (prefetch & 2) ? W_BYTES : STAGE_BYTES);
-              tma_load_2d_hint(dst, mW, full, k, t.wrow, pol_w);
+        for (int u = blockIdx.x; u < units; u += grid) {
+          const Tc5Unit t = tc5_unit(scp, u, BT, M);
+          for (int kb = 0; kb < t.nkb; kb += KB, i++) {
+            const int s = i % STAGES;
+            if (i < ahead_lo || i >= ahead_hi) {
+              mbar_wait(bars + 8 * (STAGES + s), ((i / STAGES) & 1) ^ 1);
+              load_weights(s, mW, t, kb);
             }
-            if (!(prefetch & 2)) tma_load_2d_hint(dst + W_BYTES, mA, full, k, t.m0, pol_a);
+            const uint32_t dst = tiles + s * STAGE_BYTES + KB * W_BYTES;
+#pragma unroll
+            for (int j = 0; j < KB; j++)
+              if (kb + j < t.nkb)
+                tma_load_2d_hint(dst + j * A_BYTES, mA, bars + 8 * s, tc5_kb(t.kb0, kb + j, t.rot, t.nkb) * TC_BK, t.m0, pol_a);
           }
-          __syncwarp();
         }
       }
     }
+    __syncwarp();
     if (fz.cl > 1) {
       cluster_wait_acquire();
       cluster_arrive_release();
@@ -282,41 +265,39 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BT >> 3) << 17) |
                                ((uint32_t)(TC_BN >> 4) << 24);
     if (grouped) pdl_wait();  // the tile list is the previous kernel's output
-    int i = 0, lu = 0;
-    for (int p = 0; p < 2; p++) {
-    const Tc5Sched& scp = p ? ch.sc : sc;
-    const int units = p ? ch.sc.units : (grouped ? *sc.g_ntiles * sc.n_tiles : sc.units);
-    for (int u = blockIdx.x; u < units; u += grid, lu++) {
-      const int nkb = tc5_unit(scp, u, BT, M).nkb;
-      const int buf = lu & 1;
-      mbar_wait(bar_tempty + 8 * buf, ((lu >> 1) & 1) ^ 1);  // epilogue drained this buffer
-      tc_fence_after();
-      const uint32_t tacc = tmem_base + (uint32_t)(buf * BT);
-      for (int kb = 0; kb < nkb; kb++, i++) {
-        const int s = i % STAGES;
-        mbar_wait(bars + 8 * s, (i / STAGES) & 1);
-        tc_fence_after();
-        if (tr.buf && lane == 0) {
-          if (i == 0) tr_x[0] = gtime();
-          tr_x[1] = gtime();
-        }
-        const uint32_t wt = tiles + s * STAGE_BYTES;
-        const uint64_t wdesc = make_smem_desc(wt);
-        const uint64_t adesc = make_smem_desc(wt + W_BYTES);
-        if (elect_one()) {
+    if (elect_one()) {
+      const uint32_t desc_hi = (uint32_t)(make_smem_desc(tiles) >> 32), desc_lo = (uint32_t)make_smem_desc(tiles);
+      int i = 0, lu = 0;
+      for (int p = 0; p < 2; p++) {
+        const Tc5Sched& scp = p ? ch.sc : sc;
+        const int units = p ? ch.sc.units : (grouped ? *sc.g_ntiles * sc.n_tiles : sc.units);
+        for (int u = blockIdx.x; u < units; u += grid, lu++) {
+          const int nkb = tc5_unit(scp, u, BT, M).nkb;
+          const int buf = lu & 1;
+          mbar_wait(bar_tempty + 8 * buf, ((lu >> 1) & 1) ^ 1);  // epilogue drained this buffer
+          tc_fence_after();
+          const uint32_t tacc = tmem_base + (uint32_t)(buf * BT);
+          for (int kb = 0; kb < nkb; kb += KB, i++) {
+            const int s = i % STAGES;
+            mbar_wait(bars + 8 * s, (i / STAGES) & 1);
+            tc_fence_after();
+            if (tr.buf) {
+              if (i == 0) tr_x[0] = gtime();
+              tr_x[1] = gtime();
+            }
+            const uint32_t w_lo = desc_lo + ((s * STAGE_BYTES) >> 4), a_lo = w_lo + ((KB * W_BYTES) >> 4);
 #pragma unroll
-          for (int kk = 0; kk < TC_BK / 16; kk++) {
-            // advancing 16 bf16 = 32 bytes inside the swizzle row: +2 in the >>4 address field
-            tc_mma_bf16(tacc, wdesc + 2 * kk, adesc + 2 * kk, idesc, (kb | kk) != 0);
+            for (int j = 0; j < KB; j++)
+              if (kb + j < nkb)
+                tc_mma_bf16_k64(tacc, w_lo + ((j * W_BYTES) >> 4), a_lo + ((j * A_BYTES) >> 4), desc_hi, idesc, (kb | j) != 0);
+            tc_commit(bars + 8 * (STAGES + s));  // frees the stage when these MMAs retire
           }
-          tc_commit(bars + 8 * (STAGES + s));  // frees the stage when these MMAs retire
-          if (kb == nkb - 1) tc_commit(bar_tfull + 8 * buf);
+          tc_commit(bar_tfull + 8 * buf);
+          if (tr.buf) tr_mma = gtime();
         }
-        __syncwarp();
       }
-      if (tr.buf && lane == 0) tr_mma = gtime();
     }
-    }
+    __syncwarp();
     if (fz.cl > 1) {
       cluster_wait_acquire();
       cluster_arrive_release();
@@ -751,9 +732,9 @@ int tc5_splits(int M, int N, int K, int sm_count) {
 }
 
 // ring depths of the cluster variant (the receive buffer takes 36 / 20 KB of the ring's room)
-constexpr int CL_STAGES_32 = 9, CL_STAGES_64 = 7;
+constexpr int CL_STAGES_32 = 4, CL_STAGES_64 = 3;
 constexpr size_t tc5_smem_bytes(int BT, int STAGES, bool CL) {
-  return (size_t)STAGES * (TC_BN + BT) * TC_BK * 2 + 1024 + 16 * STAGES + 64 +
+  return (size_t)STAGES * tc5_stage_blocks(BT) * (TC_BN + BT) * TC_BK * 2 + 1024 + 16 * STAGES + 64 +
          (CL ? (size_t)(BT + 8) * TC_BN * 4 + 128 : 0);
 }
 // how many clusters of S CTAs of the fused-residual GEMM can be resident at once on this device
@@ -821,8 +802,7 @@ bool carveout_known(const void* fn) {
   return false;
 }
 
-// bit 0: weight prefetch before the dependency wait (default on); bit 1: timing experiment
-// only — skip the activation loads (results are garbage)
+// bit 0: weight prefetch before the dependency wait (default on)
 static int prefetch_flags() {
   static int v = -1;
   if (v < 0) {
@@ -919,7 +899,7 @@ static cudaError_t launch_bt(cudaStream_t st, const Tc5Args& a, const TmaDesc* t
                             *reinterpret_cast<const CUtensorMap*>(tw),
                             *reinterpret_cast<const CUtensorMap*>(ta), a.M, a.N, sc, a.out, a.ldo,
                             a.split_stride, a.alpha, 0, a.epi, (bf16*)a.epi_out, a.epi_ld, a.epi_bias,
-                            prefetch_flags(), (const uint8_t*)nullptr, 0ull, fz, Tc5Chain{}, next_trace(1));
+                            prefetch_flags(), fz, Tc5Chain{}, next_trace(1));
   }
   const bool w_reused = a.g_experts > 0 ? a.M > 2 * BT * a.g_experts : m_tiles > 1;
   Tc5Chain ch{};
@@ -939,6 +919,7 @@ static cudaError_t launch_bt(cudaStream_t st, const Tc5Args& a, const TmaDesc* t
     ch.split_stride = a2->split_stride;
     ch.alpha = a2->alpha;
     ch.ctr = chain_ctr;
+    ch.flag = a.wait_flag;
     grid_l = min(max(sc.units, ch.sc.units), max(1, sm_counts[dev]));
     ch.n_waiters = min(grid_l, ch.sc.units);
   }
@@ -948,9 +929,7 @@ static cudaError_t launch_bt(cudaStream_t st, const Tc5Args& a, const TmaDesc* t
                   *reinterpret_cast<const CUtensorMap*>(a2 ? tw2 : tw),
                   *reinterpret_cast<const CUtensorMap*>(a2 ? ta2 : ta), a.M, a.N, sc, a.out, a.ldo,
                   a.split_stride, a.alpha, w_reused ? 1 : 0, a.epi, (bf16*)a.epi_out, a.epi_ld,
-                  a.epi_bias, prefetch_flags(),
-                  (const uint8_t*)((prefetch_flags() & 4) ? nullptr : a.pf_ptr),
-                  (unsigned long long)((prefetch_flags() & 4) ? 0 : a.pf_bytes), fz, ch, next_trace(1));
+                  a.epi_bias, prefetch_flags(), fz, ch, next_trace(1));
 }
 
 // a1: GEMM with a fused activation epilogue (S = 1) writing the bf16 matrix that is a2's A;
@@ -974,9 +953,9 @@ cudaError_t launch_gemm_tc5_chain(cudaStream_t st, const Tc5Args& a1, const Tc5A
   if (S2_out) *S2_out = S2;
   if (a2.out_capacity && (size_t)S2 * a2.split_stride > a2.out_capacity) return cudaErrorInvalidValue;
   switch (bt) {
-    case 32: return launch_bt<32, 10>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
-    case 64: return launch_bt<64, 8>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
-    default: return launch_bt<128, 6>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
+    case 32: return launch_bt<32, 5>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
+    case 64: return launch_bt<64, 4>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
+    default: return launch_bt<128, 3>(st, a1, tw, ta, 1, &a2, tw2, ta2, S2, ctr);
   }
 }
 
@@ -1018,9 +997,9 @@ cudaError_t launch_gemm_tc5(cudaStream_t st, const Tc5Args& a, int* S_out) {
     return half ? launch_gemm_tc5_pair(st, a, tw, half) : cudaErrorInvalidValue;
   }
   switch (bt) {
-    case 32: return launch_bt<32, 10>(st, a, tw, ta, S);
-    case 64: return launch_bt<64, 8>(st, a, tw, ta, S);
-    case 128: return launch_bt<128, 6>(st, a, tw, ta, S);
+    case 32: return launch_bt<32, 5>(st, a, tw, ta, S);
+    case 64: return launch_bt<64, 4>(st, a, tw, ta, S);
+    case 128: return launch_bt<128, 3>(st, a, tw, ta, S);
     default: return launch_bt<256, 4>(st, a, tw, ta, S);
   }
 }

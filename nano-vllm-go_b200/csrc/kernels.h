@@ -378,9 +378,6 @@ struct Tc5Args {
   float res_m;
   const float* res_g;    // [N] weight of the norm that consumes x next: res_xb = bf16(x * g)
   int max_ctas;  // > 0: cap of the persistent grid (leave SMs to a concurrent collective)
-  // weights of a later GEMM to pull into L2 while this one waits / drains (decode only)
-  const void* pf_ptr;
-  size_t pf_bytes;
   // grouped (mixture-of-experts) GEMM, g_experts > 0: A is the expert-sorted activation matrix
   // [M, K]; W stacks g_experts matrices of [N, K]; the token tiles (g_tile rows each, device
   // lists written by moe_sort_kernel) say which rows meet which expert.  S must be 1.

@@ -28,6 +28,24 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t tmem_d, uint64_t adesc, uin
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the four of 64 k (one 128-byte swizzle row of bf16): the operands' descriptors by their low words, the high word is common
+// to both (advancing 16 bf16 = 32 bytes inside the row: +2 in the >>4 address field)
+__device__ __forceinline__ void tc_mma_bf16_k64(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, t;\n\t.reg .b64 a, b;\n\t.reg .b32 x, y;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t"
+      "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 a, {x, %3};\n\tmov.b64 b, {y, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
+      "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 a, {x, %3};\n\tmov.b64 b, {y, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
+      "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 a, {x, %3};\n\tmov.b64 b, {y, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t}"
+      ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // the same with A in tensor memory: lane = row, two consecutive k of bf16 per column
 __device__ __forceinline__ void tc_mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

@@ -8,7 +8,7 @@ import nvllm_pkg
 
 pytestmark = pytest.mark.gpu
 
-ROWS, GENERAL = 47, 2  # kernel ids in the timeline
+ROWS, GENERAL = 53, 2  # kernel ids in the timeline
 
 
 def gpt2(hidden):
