@@ -645,11 +645,187 @@ static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
 #undef NR
 }
 
+// The step form with the row's routing behind it (mixture-of-experts layers, up to 1024 rows): 16 warps, each the logits of
+// experts w, w + 16, ... from the normed row in shared memory.  The first RT_AHEAD 16-byte pieces of a lane's router rows
+// are loaded before the dependency resolves (32 experts of 1024: all of them), neighbouring lanes neighbouring pieces, and up to
+// 32 experts are chosen with a lane each.  128 rows of 1024 with eight slices and 32 experts, from the release to the last exit:
+// 10 -> 5.9 us; with the sort of moe.cu, 16 decode steps of 128 sequences through four layers of 32 experts 5410 -> 5100 us.
+constexpr int RT_THREADS = 512, RT_AHEAD = 16, RT_MAX_V = 4;
+template <typename YT, int V, int COMB>
+__global__ void __launch_bounds__(RT_THREADS, 1) norm_route_kernel(NormArgs a, Trace tr) {
+  const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float row[];
+  __shared__ float red[32], probs[MOE_MAX_E], chs[MOE_MAX_E], gsc[MOE_MAX_E];
+  const int H = a.H, r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = RT_THREADS / 32;
+  auto get = [](const float* p, float (&o)[4]) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
+  };
+  // piece m of this warp's router rows: expert warp + NW (m / nch), entries 128 (m % nch) + 4 lane
+  const int nch = (H + 127) / 128, pieces = (a.E > warp ? (a.E - warp + NW - 1) / NW : 0) * nch;
+  auto piece = [&](int j, int c, float (&o)[4]) {
+    const int i = 128 * c + 4 * lane;
+    o[0] = o[1] = o[2] = o[3] = 0.f;
+    if (i < H) get(a.router + (size_t)(warp + NW * j) * H + i, o);
+  };
+  float ahead[RT_AHEAD][4];
+  {
+    int j = 0, c = 0;
+#pragma unroll
+    for (int m = 0; m < RT_AHEAD; m++) {
+      if (m < pieces) piece(j, c, ahead[m]);
+      if (++c == nch) c = 0, j++;
+    }
+  }
+  pdl_wait();
+  const unsigned long long t_wait = trace_on(tr) ? gtime() : 0ull;
+  float* xr = a.x + (size_t)r * H;
+  int prow[COMB ? COMB : 1];
+  float cw[COMB ? COMB : 1];
+  if constexpr (COMB > 0) {
+#pragma unroll
+    for (int q = 0; q < COMB; q++) {
+      prow[q] = q < a.comb_k ? a.comb_rows[(size_t)r * a.comb_k + q] : -1;
+      cw[q] = q < a.comb_k ? a.comb_w[(size_t)r * a.comb_k + q] : 0.f;
+    }
+  }
+  const bool ln = a.b != nullptr || a.centered != 0;
+  float v[V][4], part = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = ((int)threadIdx.x + k * RT_THREADS) * 4;
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[k][j] = 0.f;
+    if (i >= H) continue;
+    get(xr + i, v[k]);
+    if (a.p1) {
+      float s1[8][4], acc[4] = {0.f, 0.f, 0.f, 0.f}, b[4];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if (COMB ? prow[COMB ? q : 0] >= 0 : q < a.S1)
+          get(a.p1 + (COMB ? (size_t)prow[COMB ? q : 0] * H : (size_t)q * a.stride1 + (size_t)r * H) + i, s1[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (COMB ? prow[COMB ? q : 0] >= 0 : q < a.S1) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[j] += COMB ? cw[COMB ? q : 0] * s1[q][j] : s1[q][j];
+        }
+      if (a.bias1) {
+        get(a.bias1 + i, b);
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[j] += b[j];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[k][j] = v[k][j] + a.m1 * acc[j];
+      store4(xr + i, v[k]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) part += ln ? v[k][j] : v[k][j] * v[k][j];
+  }
+  const float tot = block_sum(part, red);
+  float mean = 0.f, inv;
+  if (ln) {
+    mean = tot / (float)H;
+    float lv = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      if (((int)threadIdx.x + k * RT_THREADS) * 4 < H) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float d = v[k][j] - mean;
+          lv += d * d;
+        }
+      }
+    inv = 1.0f / sqrtf(block_sum(lv, red) / (float)H + a.eps);
+  } else {
+    inv = 1.0f / sqrtf(tot / (float)H + a.eps);
+  }
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = ((int)threadIdx.x + k * RT_THREADS) * 4;
+    if (i >= H) continue;
+    float w[4] = {1.f, 1.f, 1.f, 1.f}, b[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
+    if (a.w) get(a.w + i, w);
+    if (a.b) get(a.b + i, b);
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = ln ? (v[k][j] - mean) * inv * w[j] + b[j] : v[k][j] * inv * w[j];
+    if (a.y) store4((YT*)a.y + (size_t)r * H + i, o);
+    if (a.y_f32) store4(a.y_f32 + (size_t)r * H + i, o);
+    store4(row + i, o);
+  }
+  __syncthreads();
+  {
+    int j = 0, c = 0;
+    float acc = 0.f;
+    auto take = [&](const float (&p)[4]) {
+      const int i = 128 * c + 4 * lane;
+      if (i < H) {
+        float y[4];
+        get(row + i, y);
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc = fmaf(y[e], p[e], acc);
+      }
+      if (++c == nch) {
+        acc = warp_sum(acc);
+        const int e = warp + NW * j;
+        if (lane == 0) probs[e] = a.route.bias ? acc + a.route.bias[e] : acc;
+        acc = 0.f;
+        c = 0;
+        j++;
+      }
+    };
+#pragma unroll
+    for (int m = 0; m < RT_AHEAD; m++)
+      if (m < pieces) take(ahead[m]);
+    for (int m = RT_AHEAD; m < pieces; m += 8) {
+      float p[8][4];
+      int jj = j, cc = c;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if (m + q < pieces) piece(jj, cc, p[q]);
+        if (++cc == nch) cc = 0, jj++;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (m + q < pieces) take(p[q]);
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    if (a.E <= 32 && !a.route.correction && !(a.route.groups > 1 && a.route.keep < a.route.groups))
+      moe_select_lanes(lane < a.E ? probs[lane] : 0.f, a.E, a.topk, (size_t)r, a.topk_idx, a.topk_w, a.route);
+    else
+      moe_select_row(probs, chs, gsc, a.E, a.topk, (size_t)r, a.topk_idx, a.topk_w, a.route);
+  }
+  if (threadIdx.x == 0 && trace_on(tr)) trace_rec(tr, t_entry, t_wait, 0ull);
+}
+// (identity experts need the row itself again; more rows fill the SMs without 16 warps to a row)
+static bool norm_route_fit(const NormArgs& a) {
+  return a.router && a.route.identity == 0 && a.n_rows <= 1024 && a.E <= MOE_MAX_E && a.topk <= 32 && a.H % 8 == 0 &&
+         a.H <= RT_MAX_V * RT_THREADS * 4 && !a.p2 && !a.row_idx && !a.gate_w && !a.plain && !a.post && a.groups <= 1 && !a.xadd &&
+         !a.xadd_table && !a.row_m2 && !a.conv_taps && !a.p1_bf16 && (!a.p1 || (a.comb_rows ? a.comb_k <= 8 : a.S1 <= 8));
+}
+template <typename YT>
+static cudaError_t launch_norm_route(cudaStream_t st, const NormArgs& a) {
+  const int V = ceil_div(a.H, RT_THREADS * 4);
+  const size_t smem = (size_t)a.H * sizeof(float);
+  const bool comb = a.p1 && a.comb_rows;
+#define NR(V_)                                                                                                        \
+  (comb ? launch_k(norm_route_kernel<YT, V_, 8>, dim3(a.n_rows), dim3(RT_THREADS), smem, st, a, next_trace(54))       \
+        : launch_k(norm_route_kernel<YT, V_, 0>, dim3(a.n_rows), dim3(RT_THREADS), smem, st, a, next_trace(54)))
+  return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
+#undef NR
+}
+
 cudaError_t launch_norm(cudaStream_t st, const NormArgs& a) {
   if (a.n_rows <= 0) return cudaSuccess;
   if (a.groups > 64 || (a.groups > 1 && a.H % a.groups) || (a.plain && !a.y)) return cudaErrorInvalidValue;
   if (norm_rows_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float, 1>(st, a) : launch_norm_rows<bf16, 1>(st, a);
   if (norm_step_fit(a)) return a.ydt == DT_F32 ? launch_norm_rows<float, 8>(st, a) : launch_norm_rows<bf16, 8>(st, a);
+  if (norm_route_fit(a)) return a.ydt == DT_F32 ? launch_norm_route<float>(st, a) : launch_norm_route<bf16>(st, a);
   int threads = min(512, max(64, ((a.H / 8 + 31) / 32) * 32));
   // fused router, decode-sized batches (latency-bound: fewer row CTAs than two waves): 16 warps
   // so that each takes two experts of a 32-expert layer in one pass; prefill keeps the

@@ -350,6 +350,10 @@ cudaError_t launch_moe_gather(cudaStream_t st, int rows, int H, const void* x, c
 // (row of pair p = offset of its expert + number of earlier pairs routed to that expert —
 // deterministic, so all CTAs agree), CTA 0 publishes the lists the grouped GEMMs and the
 // combine read, and each CTA copies its share of the sorted activation rows.
+//
+// Bound by round trips: the choices are read once, each thread's up to four stay in registers.  A warp counts its 32 pairs
+// per expert (match), one warp per expert scans those counts over all warps, one warp the experts: four block barriers.
+// 128 rows, 8 of 32 experts, from the end of the routing to the last exit: 8.0 -> 6.4 us.
 constexpr int MOE_SG_MAX_P = 4096, MOE_SG_MAX_E = 64;
 __global__ void __launch_bounds__(1024)
 moe_sort_gather_kernel(const int* __restrict__ topk_idx, int n_pairs, int k, int E, MoeSortBufs b,
@@ -357,17 +361,55 @@ moe_sort_gather_kernel(const int* __restrict__ topk_idx, int n_pairs, int k, int
                        uint4* __restrict__ xs, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
+  constexpr int CH = MOE_SG_MAX_P / 1024, VW = 32 * CH;  // pairs of a thread; groups of 32 pairs
+  __shared__ unsigned short s_w[MOE_SG_MAX_E][VW];       // pairs of a group per expert, then those of the groups before
   __shared__ int s_cnt[MOE_SG_MAX_E];
   __shared__ int s_off[MOE_SG_MAX_E + 1];
-  __shared__ int s_base[MOE_SG_MAX_E];
-  __shared__ int s_wcnt[32][MOE_SG_MAX_E];
-  __shared__ int s_inv[MOE_SG_MAX_P];
+  __shared__ unsigned short s_inv[MOE_SG_MAX_P];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < MOE_SG_MAX_E) s_cnt[tid] = s_base[tid] = 0;
+  const int chunks = (n_pairs + 1023) / 1024;
+  for (int i = tid; i < MOE_SG_MAX_E * VW / 2; i += 1024) reinterpret_cast<unsigned*>(&s_w[0][0])[i] = 0u;
   pdl_wait();
+  int e[CH], rank[CH];
+#pragma unroll
+  for (int c = 0; c < CH; c++) {
+    const int p = c * 1024 + tid;
+    e[c] = c < chunks && p < n_pairs ? topk_idx[p] : -1;
+  }
   __syncthreads();
-  for (int p = tid; p < n_pairs; p += 1024)
-    if (topk_idx[p] < E) atomicAdd(&s_cnt[topk_idx[p]], 1);  // (others are identity experts: no row)
+#pragma unroll
+  for (int c = 0; c < CH; c++) {
+    if (c >= chunks) break;
+    if (e[c] >= E) {  // identity experts: no row
+      e[c] = -1;
+      if (blockIdx.x == 0) b.pair_row[c * 1024 + tid] = -1;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, e[c]);
+    rank[c] = __popc(same & ((1u << lane) - 1));
+    if (e[c] >= 0 && rank[c] == 0) s_w[e[c]][c * 32 + warp] = (unsigned short)__popc(same);
+  }
+  __syncthreads();
+  for (int x_ = warp; x_ < E; x_ += 32) {  // a lane takes the CH groups that follow one another
+    int n[CH], sum = 0;
+#pragma unroll
+    for (int c = 0; c < CH; c++) {
+      n[c] = s_w[x_][lane * CH + c];
+      sum += n[c];
+    }
+    int run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += up;
+    }
+    if (lane == 31) s_cnt[x_] = run;
+    run -= sum;
+#pragma unroll
+    for (int c = 0; c < CH; c++) {
+      s_w[x_][lane * CH + c] = (unsigned short)run;
+      run += n[c];
+    }
+  }
   __syncthreads();
   if (warp == 0) {
     // expert offsets and the tile list by warp scans (E <= 64: lane holds experts lane and
@@ -421,46 +463,28 @@ moe_sort_gather_kernel(const int* __restrict__ topk_idx, int n_pairs, int k, int
       }
     }
   }
-  for (int c0 = 0; c0 < n_pairs; c0 += 1024) {
-    for (int i = tid; i < 32 * MOE_SG_MAX_E; i += 1024) (&s_wcnt[0][0])[i] = 0;
-    __syncthreads();
-    const int p = c0 + tid;
-    int e = p < n_pairs ? topk_idx[p] : -1;
-    if (e >= E) {
-      e = -1;
-      if (blockIdx.x == 0) b.pair_row[p] = -1;
-    }
-    const unsigned same = __match_any_sync(0xffffffffu, e);
-    const int rank = __popc(same & ((1u << lane) - 1));
-    if (e >= 0 && rank == 0) s_wcnt[warp][e] = __popc(same);
-    __syncthreads();
-    if (tid < E) {  // exclusive prefix over the warps, continuing from the earlier chunks
-      int run = s_base[tid];
-      for (int w = 0; w < 32; w++) {
-        const int n = s_wcnt[w][tid];
-        s_wcnt[w][tid] = run;
-        run += n;
-      }
-      s_base[tid] = run;
-    }
-    __syncthreads();
-    if (e >= 0) {
-      const int row = s_off[e] + s_wcnt[warp][e] + rank;
-      s_inv[row] = p;
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < CH; c++) {
+    if (c >= chunks) break;
+    if (e[c] >= 0) {
+      const int p = c * 1024 + tid, row = s_off[e[c]] + s_w[e[c]][c * 32 + warp] + rank[c];
+      s_inv[row] = (unsigned short)(p / k);
       if (blockIdx.x == 0) {
         b.sorted_pair[row] = p;
         b.pair_row[p] = row;
         b.a_rows[row] = p / k;
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
   const int n_rows = s_off[E];
   const int rpc = (n_rows + gridDim.x - 1) / gridDim.x;
   const int r0 = blockIdx.x * rpc;
+#pragma unroll 2
   for (int idx = tid; idx < rpc * vpr; idx += 1024) {
     const int r = r0 + idx / vpr, j = idx % vpr;
-    if (r < n_rows) xs[(size_t)r * vpr + j] = x[(size_t)(s_inv[r] / k) * vpr + j];
+    if (r < n_rows) xs[(size_t)r * vpr + j] = x[(size_t)s_inv[r] * vpr + j];
   }
   TRACE_EXIT(tr);
 }
