@@ -180,6 +180,8 @@ cudaError_t launch_sample(cudaStream_t st, const float* logits, int ldl, int V, 
                           unsigned long long* amax = nullptr, int* ticket = nullptr, int vsplit = 0);
 
 // advance device-resident decode state by one token (nvllm_run_resident)
+// a step's tokens, and its logits where out_logits is given, to pinned memory
+cudaError_t launch_copy_out(cudaStream_t st, int n, const int* tokens, int* out_tokens, const float* logits, int ldl, int V, float* out_logits);
 cudaError_t launch_advance(cudaStream_t st, int n, const int* sampled, int* tokens, int* positions,
                            int* slots, int* seq_len, const int* block_tables, int max_blocks,
                            int max_pos);

@@ -245,22 +245,24 @@ static int ensure_pinned(nvllm_handle* h, void** p, size_t* have, size_t bytes) 
   return NVLLM_OK;
 }
 
-// The n rows of logits for the caller, after the step on the stream: enqueue, and finish once the stream is done.  Up to 256
-// KB travel through a pinned buffer of the handle, as a copy that runs beside the host; the driver stages a copy to the
-// caller's pageable memory itself, and waits for the step first (a sampled step of 8 x 4096: 345 -> 335 us).  Larger ones
-// gain nothing from it, and locking their pages costs a new handle's first call (2 MB: 1.4 ms).
+// The tokens and, if asked for, the n rows of logits for the caller, after the step on the stream: enqueue, and finish once the
+// stream is done.  Up to 256 KB of logits travel through a pinned buffer of the handle with the tokens, by a kernel; the
+// driver stages a copy to the caller's pageable memory itself, and waits for the step first (a sampled step of 8 x 4096:
+// 345 -> 335 us).  Larger ones gain nothing from it, and locking their pages costs a new handle's first call (2 MB: 1.4 ms).
 constexpr size_t LOGITS_PINNED = (size_t)256 << 10;
-static int enqueue_logits(nvllm_handle* h, float* out, int n) {
+static int enqueue_results(nvllm_handle* h, float* out, int n) {
   const size_t bytes = (size_t)n * h->V * 4;
-  float* dst = out;
-  if (bytes <= LOGITS_PINNED) {
+  float* pinned = nullptr;
+  if (out && bytes <= LOGITS_PINNED) {
     if (const int rc = ensure_pinned(h, (void**)&h->h_logits, &h->h_logits_bytes, bytes)) return rc;
-    dst = h->h_logits;
+    pinned = h->h_logits;
   }
+  NV_CHECK(h, launch_copy_out(h->stream, n, h->ws.out_tokens, h->h_out, h->ws.logits_final, h->ldl, h->V, pinned));
+  if (!out || pinned) return NVLLM_OK;
   // rows are ldl apart on the device; copy them packed [n, V]
-  if (h->ldl == h->V) NV_CHECK(h, cudaMemcpyAsync(dst, h->ws.logits_final, bytes, cudaMemcpyDeviceToHost, h->stream));
+  if (h->ldl == h->V) NV_CHECK(h, cudaMemcpyAsync(out, h->ws.logits_final, bytes, cudaMemcpyDeviceToHost, h->stream));
   else
-    NV_CHECK(h, cudaMemcpy2DAsync(dst, (size_t)h->V * 4, h->ws.logits_final, (size_t)h->ldl * 4, (size_t)h->V * 4, n,
+    NV_CHECK(h, cudaMemcpy2DAsync(out, (size_t)h->V * 4, h->ws.logits_final, (size_t)h->ldl * 4, (size_t)h->V * 4, n,
                                   cudaMemcpyDeviceToHost, h->stream));
   return NVLLM_OK;
 }
@@ -321,13 +323,9 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
     // (a step issued ahead has none of the further logits rows that this call may have to bring)
     if (h->want_rows.empty() && speculation_hit(h, n, is_prefill, token_ids, cu_seqlens, block_tables, cu_blocks, temperature)) {
       // the requested step is already running (or done): collect it
-      cudaStream_t st = h->stream;
-      NV_CHECK(h, cudaMemcpyAsync(h->h_out, h->ws.out_tokens, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
       uint64_t d2h = (uint64_t)n * 4;
-      if (out_logits) {
-        if (const int rc = enqueue_logits(h, out_logits, n)) return rc;
-        d2h += (uint64_t)n * h->V * 4;
-      }
+      if (const int rc = enqueue_results(h, out_logits, n)) return rc;
+      if (out_logits) d2h += (uint64_t)n * h->V * 4;
       h->run_lay = h->lay;
       h->run_lay_ok = true;
       h->spec_pause[h->spec_kind].misses = 0;
@@ -507,8 +505,8 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
     return rc;
   }
   NV_CHECK(h, cudaEventRecord(h->ev1, st));
-  NV_CHECK(h, cudaMemcpyAsync(h->h_out, h->ws.out_tokens, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
   uint64_t d2h = (uint64_t)n * 4;
+  if ((rc = enqueue_results(h, h->tp > 1 ? nullptr : out_logits, n))) return rc;
   if (out_logits) {
     if (h->tp > 1) {  // gathered rank-major vocabulary slices [tp][n][Vl]
       for (int r = 0; r < h->tp; r++) {
@@ -519,8 +517,6 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
                                       (size_t)h->Vl * 4, (size_t)cn * 4, n,
                                       cudaMemcpyDeviceToHost, st));
       }
-    } else {
-      if ((rc = enqueue_logits(h, out_logits, n))) return rc;
     }
     d2h += (uint64_t)n * h->V * 4;
   }
