@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(512) norm_kernel(NormArgs a, Trace tr) {
 #pragma unroll
       for (int j = 0; j < 8; j++) v[j] = fmaf(p[j], m, v[j]);
     }
-    if (upd) store8(xr + i, v);
+    if (upd && !a.row_idx) store8(xr + i, v);  // (gathered rows may repeat: the last norm, whose input nothing reads again)
     store8(row + i, v);
     if (ln) {
 #pragma unroll
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(SL > 1 ? NR_STEP_THREADS : NR_THREADS, SL > 1 
     if (a.p2)
 #pragma unroll
       for (int j = 0; j < 4; j++) v[k][j] = v[k][j] + a.m2 * p2[j];
-    if (a.p1 || a.p2) store4(xr + i, v[k]);
+    if ((a.p1 || a.p2) && !(STEP && a.row_idx)) store4(xr + i, v[k]);  // (gathered rows may repeat, see norm_kernel)
   }
   if (a.y || a.y_f32 || a.post) {
     const bool ln = a.b != nullptr || a.centered != 0;
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(SL > 1 ? NR_STEP_THREADS : NR_THREADS, SL > 1 
 static bool norm_rows_plain(const NormArgs& a) {
   return a.H % 8 == 0 && !a.router && !a.gate_w && !a.plain && a.groups <= 1 && !a.xadd && !a.xadd_table && !a.row_m2 &&
          !a.conv_taps && !a.p1_bf16 && (!a.p1 || !a.comb_rows || a.comb_k <= 8) &&
-         (!a.post || (a.p1 && a.w && !a.comb_rows && !a.p2));
+         (!a.post || (a.p1 && a.w && !a.comb_rows && !a.p2 && !a.row_idx));
 }
 // many rows, at most one slice per addend
 static bool norm_rows_fit(const NormArgs& a) {

@@ -56,3 +56,22 @@ def test_step_matches_the_prompts(cfg):
     # the same bf16 roundings, sums in another order: as far from float32 as the prompts are (the error's norm over n rows is
     # known to a tenth or so)
     assert np.linalg.norm(step - want) <= 1.25 * np.linalg.norm(prompts - want)
+
+
+@pytest.mark.parametrize("cfg", [C.tiny_llama(hidden=24), falcon(64), C.tiny_granite(hidden=264)], ids=lambda c: c.name)
+def test_rows_asked_for_twice(cfg):
+    """The logits of rows that are a sequence's last one as well: the last norm meets them twice, and takes their pending results
+    in each time from the same residual row."""
+    n = 24
+    texts = [W.random_prompt(cfg.vocab_size, 3 + i % 5, 60 + i) for i in range(n)]
+    last = (np.cumsum([len(t) for t in texts]) - 1).tolist()
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 3), precision=C.PREC_FP32, num_kv_blocks=n, sampling=None)
+    try:
+        for _ in range(40):
+            run.request_logits(last + last)
+            _, once = run.run_flat(texts, True, [0] * n, [[i] for i in range(n)], [0.0] * n, want_logits=True)
+            again = run.fetch_logits(2 * n)
+            np.testing.assert_array_equal(again[:n], once)
+            np.testing.assert_array_equal(again[n:], once)
+    finally:
+        run.close()
