@@ -557,7 +557,8 @@ int nvllm_set_graphs(nvllm_handle* h, int enabled);
  * that step (same lengths + 1, last token = the one returned, same block tables) only waits
  * for it and copies nothing to the device; any other call restages everything as usual.
  * Misses in a row pause it for 1, 2, 4, ... 16 calls (steps issued by prefill and by decode calls are counted
- * apart).  Models with recurrent state, whose steps update it in place, never speculate. */
+ * apart).  Recurrent state, which steps update in place, is copied aside first (up to 128 MB a step; more, or
+ * Mamba2 state in KV blocks: no step is issued) and put back by the next call that does not ask for the step. */
 int nvllm_set_speculation(nvllm_handle* h, int enabled);
 
 /* GetVocabSize / GetModelConfig (purego/generic_runner.go:184-196). */

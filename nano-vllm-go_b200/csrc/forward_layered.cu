@@ -77,7 +77,10 @@ void layered_free(nvllm_handle* h) {
   F(h->pos_freq);
   h->pos_freq = nullptr;
   F(h->state_pool);
-  h->state_pool = nullptr;
+  F(h->state_copy);
+  h->state_pool = h->state_copy = nullptr;
+  h->state_copy_bytes = 0;
+  h->state_copy_n = 0;
   for (auto& r : h->ropes) {
     F(r.inv_freq); F(r.cosT); F(r.sinT);
   }
@@ -1885,7 +1888,6 @@ extern "C" int nvllm_create_layered(const nvllm_layered_config* c, const nvllm_l
     }
   }
   h->num_state_slots = c->num_state_slots > 0 ? c->num_state_slots : g.max_num_seqs;
-  h->spec_enabled = 0;  // the speculative next step is keyed on the uniform models' shapes
   if (const char* env = getenv("NVLLM_SKIP")) h->skip_mask = (unsigned)strtoul(env, nullptr, 0);
   auto fail = [&](cudaError_t ce, const char* what) {
     int code = (ce == cudaErrorMemoryAllocation) ? NVLLM_ERR_NOMEM : NVLLM_ERR_CUDA;

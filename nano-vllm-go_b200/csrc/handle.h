@@ -382,6 +382,11 @@ struct nvllm_handle {
     int misses = 0, skip = 0;  // misses in a row, calls that do not speculate because of them
   } spec_pause[2];             // of steps issued by decode and by prefill calls (run.cu)
   int spec_kind = 0;           // which of them issued the last one
+  // models with recurrent state: what it was before the step issued ahead, and the sequences whose state that is (0: none)
+  float* state_copy = nullptr;  // [n][state_slot_floats], then the n slots
+  size_t state_copy_bytes = 0;
+  int state_copy_n = 0;
+  std::vector<int32_t> spec_slots;
   std::vector<int32_t> spec_len, spec_nb, spec_bt;  // per-sequence lengths / block tables of the last call
   // device-resident decode state as the host knows it: context length (incl. the token the last
   // step appended) and block-table extent of every sequence — nvllm_run_resident refuses to step

@@ -180,6 +180,9 @@ cudaError_t launch_sample(cudaStream_t st, const float* logits, int ldl, int V, 
                           unsigned long long* amax = nullptr, int* ticket = nullptr, int vsplit = 0);
 
 // advance device-resident decode state by one token (nvllm_run_resident)
+// the recurrent state of a step's n sequences aside, or back to where it was
+cudaError_t launch_state_copy(cudaStream_t st, int n, const int* slots, float* pool, size_t slot_floats, float* copy, int* copy_slots,
+                              bool restore);
 // a step's tokens, and its logits where out_logits is given, to pinned memory
 cudaError_t launch_copy_out(cudaStream_t st, int n, const int* tokens, int* out_tokens, const float* logits, int ldl, int V, float* out_logits);
 cudaError_t launch_advance(cudaStream_t st, int n, const int* sampled, int* tokens, int* positions,

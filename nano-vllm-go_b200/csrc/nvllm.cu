@@ -389,7 +389,7 @@ int nvllm_set_graphs(nvllm_handle* h, int enabled) {
 
 int nvllm_set_speculation(nvllm_handle* h, int enabled) {
   if (!h) return NVLLM_ERR_INVALID;
-  h->spec_enabled = enabled ? 1 : 0;  // (models with recurrent state never speculate: run.cu)
+  h->spec_enabled = enabled ? 1 : 0;
   return NVLLM_OK;
 }
 

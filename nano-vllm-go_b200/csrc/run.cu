@@ -150,8 +150,8 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
 // sequences, one token longer, last token = the one just returned, same block tables, greedy —
 // and only has to wait for it, or asks for something else and restages everything as usual.
 // A speculative step that is thrown away has only written K/V at the next position of each
-// sequence, a slot nothing reads before its owner writes it (models with recurrent state never speculate); but the call
-// after it waits for it, so misses in a row pause the speculation: 1, 2, 4, ... 16 calls.  Steps issued by prefill calls
+// sequence, a slot nothing reads before its owner writes it, and recurrent state, which the next call puts back from a copy
+// made ahead of the step (save_state); but the call after it waits for it, so misses in a row pause the speculation: 1, 2, 4, ... 16 calls.  Steps issued by prefill calls
 // and by decode calls count apart.  Those of prefill calls miss where prompts arrive while others decode (the next call
 // is the merged batch) or come alone, and pause from the first miss on; those of decode calls miss once per arrival or
 // end of a sequence and hit in between, and pause from the second miss in a row on.  Per 64 decode steps of 32 sequences
@@ -169,6 +169,41 @@ static int check_waits(nvllm_handle* h) {
   if (h->ws.chain_ctr) NV_CHECK(h, cudaMemsetAsync(h->ws.chain_ctr, 0, 256, h->stream));
   return set_err(h, NVLLM_ERR_CUDA, "forward pass failed: a wait inside a kernel ran out");
 }
+// Recurrent state is updated in place: it is copied aside before a step is issued ahead, and back if that step is not the one
+// asked for.  The copy costs its stream twice per step where the host's turn costs some 80 us, so steps of more state than
+// STATE_COPY are left to the host.  Decode steps of a delta-rule layer (16 heads of 128 x 128; 1.1 MB a sequence) and a window
+// attention layer, us without / with: 4 sequences 160 / 113, 32 201 / 145, 64 260 / 193, 120 360 / 273.  Mamba-2 state that lives in KV blocks is not copied: those models wait for the host.
+constexpr size_t STATE_COPY = (size_t)128 << 20;
+static bool save_state(nvllm_handle* h, int n) {
+  const size_t floats = (size_t)n * h->state_slot_floats, bytes = (floats + n) * 4;
+  if (bytes > STATE_COPY) return false;
+  if (bytes > h->state_copy_bytes) {
+    if (h->state_copy) cudaFree(h->state_copy);
+    h->state_copy = nullptr;
+    h->state_copy_bytes = 0;
+    const size_t room = std::min(STATE_COPY, bytes + bytes / 4);
+    if (cudaMalloc((void**)&h->state_copy, room) != cudaSuccess) {
+      (void)cudaGetLastError();
+      h->state_copy = nullptr;
+      return false;
+    }
+    h->state_copy_bytes = room;
+  }
+  if (launch_state_copy(h->stream, n, h->lay.d + h->lay.state_slots, h->state_pool, h->state_slot_floats, h->state_copy,
+                        reinterpret_cast<int*>(h->state_copy + floats), false) != cudaSuccess)
+    return false;
+  h->state_copy_n = n;
+  return true;
+}
+// a step issued ahead is not taken: the state it changed is put back before anything else runs on the stream
+static int restore_state(nvllm_handle* h) {
+  const int n = h->state_copy_n;
+  if (n == 0) return NVLLM_OK;
+  h->state_copy_n = 0;
+  NV_CHECK(h, launch_state_copy(h->stream, n, nullptr, h->state_pool, h->state_slot_floats, h->state_copy,
+                                reinterpret_cast<int*>(h->state_copy + (size_t)n * h->state_slot_floats), true));
+  return NVLLM_OK;
+}
 static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, const int32_t* block_tables,
                           const int32_t* cu_blocks) {
   h->spec_len.resize(n);
@@ -184,8 +219,7 @@ static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, con
 static void try_speculate(nvllm_handle* h, int n, const float* temperature) {
   h->spec_pending = false;
   if (!h->spec_enabled || !graph_usable(h, n)) return;
-  // a step that is thrown away would leave recurrent state, which steps update in place, one token ahead
-  if (h->state_slot_floats || h->n_mamba) return;
+  if (h->n_mamba) return;
   if (h->fetched_rows > 0) return;  // its logits would land on rows that the caller is still to fetch
   h->spec_kind = h->lay.prefill ? 1 : 0;
   nvllm_handle::SpecPause& pause = h->spec_pause[h->spec_kind];
@@ -198,7 +232,8 @@ static void try_speculate(nvllm_handle* h, int n, const float* temperature) {
     if (h->spec_len[i] >= h->spec_nb[i] * KV_BLOCK) return;  // next position needs a new block
     if (h->use_rope && h->spec_len[i] + 1 > h->cfg.max_seq_len) return;
   }
-  // a failed speculative step must leave no trace: layout, per-sequence extents and the
+  if (h->state_slot_floats && !save_state(h, n)) return;
+  // a failed speculative step must leave no trace (its state goes back with the next call): layout, per-sequence extents and the
   // caller-visible error string are restored
   const int saved = h->launches;
   const StepLayout lay0 = h->lay;
@@ -219,6 +254,7 @@ static bool speculation_hit(const nvllm_handle* h, int n, int is_prefill, const 
                             const int32_t* cu_seqlens, const int32_t* block_tables,
                             const int32_t* cu_blocks, const float* temperature) {
   if (is_prefill || n != (int)h->spec_len.size() || h->filters_active()) return false;
+  if (h->state_slot_floats && h->next_state_slots != h->spec_slots) return false;
   size_t o = 0;
   for (int i = 0; i < n; i++) {
     const int len = cu_seqlens[i + 1] - cu_seqlens[i], nb = cu_blocks[i + 1] - cu_blocks[i];
@@ -323,6 +359,8 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
     // (a step issued ahead has none of the further logits rows that this call may have to bring)
     if (h->want_rows.empty() && speculation_hit(h, n, is_prefill, token_ids, cu_seqlens, block_tables, cu_blocks, temperature)) {
       // the requested step is already running (or done): collect it
+      h->state_copy_n = 0;
+      h->next_state_slots.clear();
       uint64_t d2h = (uint64_t)n * 4;
       if (const int rc = enqueue_results(h, out_logits, n)) return rc;
       if (out_logits) d2h += (uint64_t)n * h->V * 4;
@@ -338,6 +376,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
     const int pauses = pause.misses - (h->spec_kind == 0 ? 1 : 0);
     pause.skip = pauses > 0 ? 1 << std::min(pauses - 1, 4) : 0;
   }
+  if (const int rc = restore_state(h)) return rc;
   h->resident_ok = false;
   h->run_lay_ok = false;
 
@@ -356,6 +395,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
       for (int j = 0; j < i; j++)
         if (sslots[j] == sslots[i]) return set_err(h, NVLLM_ERR_INVALID, "sequences %d and %d share state slot %d", j, i, sslots[i]);
     }
+    h->spec_slots = sslots;
   }
   long long sum_len = 0;
   double pairs = 0;
@@ -645,11 +685,13 @@ extern "C" int nvllm_run_resident(nvllm_handle* h, nvllm_run_stats* stats) {
   if (!h) return NVLLM_ERR_INVALID;
   if (h->spec_pending) {  // the step asked for is the one already in flight
     h->spec_pending = false;
+    h->state_copy_n = 0;
     h->spec_pause[h->spec_kind].misses = 0;
     fill_stats(h, stats, h->lay.n, 0, 0);
     if (stats) stats->used_graph = h->spec_used_graph ? 1 : 0;
     return NVLLM_OK;
   }
+  if (const int rc = restore_state(h)) return rc;
   return resident_step(h, stats);
 }
 
@@ -662,6 +704,7 @@ extern "C" int nvllm_rerun(nvllm_handle* h, nvllm_run_stats* stats) {
     return set_err(h, NVLLM_ERR_STATE,
                    "nvllm_rerun replays prefill steps only (a decode step's staged state is "
                    "advanced in place by nvllm_run_resident)");
+  if (const int rc = restore_state(h)) return rc;
   h->lay = h->run_lay;
   h->spec_pending = false;
   h->res_len = h->spec_len;  // the device state is the replayed step's again

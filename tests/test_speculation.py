@@ -1,5 +1,7 @@
 """The speculative next step of nvllm_run: calls that never ask for it pause it, a decode loop gets it back, and results (tokens,
 logits, device time of the step that was asked for) are those of a runner without it."""
+import importlib
+
 import numpy as np
 import pytest
 
@@ -102,6 +104,57 @@ def test_recurrent_state_is_not_stepped_ahead():
             run.close()
 
     for (a, la), (b, lb) in zip(drive(False), drive(True)):
+        np.testing.assert_array_equal(a, b)
+        np.testing.assert_array_equal(la, lb)
+
+
+@pytest.mark.parametrize("family", ["zozonex", "lazovik", "sutuvik", "sozurax", "defilorn"])
+def test_recurrent_state_goes_back(family):
+    """Steps issued ahead on models whose steps update state in place: taken where they match; where the next call has another
+    token, batch, order or slots, or is a prompt or a repetition, the state they changed is put back."""
+    m = importlib.import_module("test_" + family)
+    cfg, w = m.random_weights(m.mixed_model(), 7)
+    prompts = [W.random_prompt(cfg.vocab_size, 9 + 4 * i, 40 + i).tolist() for i in range(4)]
+
+    def drive(spec):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, w.items(), precision=C.PREC_FP32, num_kv_blocks=4, sampling=None, num_state_slots=5)
+        try:
+            run.set_speculation(spec)
+            seqs, slots, outs, hits = [list(p) for p in prompts], [2, 0, 1, 4], [], 0
+
+            def call(which, prompt=False):
+                nonlocal hits
+                out, logits = run.run_flat([seqs[i] for i in which], prompt, [0] * len(which), [[i] for i in which], [0.0] * len(which),
+                                           want_logits=True, state_slots=[slots[i] for i in which])
+                hits += run.last_stats.h2d_bytes == 0
+                outs.append((out, logits))
+                for i, t in zip(which, out):
+                    seqs[i].append(int(t))
+
+            call([0, 1, 2], prompt=True)
+            for k in range(24):
+                if k in (3, 15):
+                    seqs[1][-1] = 5  # another token than the one that came out
+                if k == 6:
+                    call([0])        # one of them alone
+                if k == 9:
+                    call([2, 0, 1])  # another order
+                if k == 12:          # a new sequence joins; one ends and its slot is the next one's
+                    call([3], prompt=True)
+                if k == 18:
+                    seqs[3], slots[3] = list(prompts[3]), 3
+                    call([3], prompt=True)
+                if k == 21:
+                    run.sync()
+                call([0, 1, 2])
+            call([3])
+            return outs, hits
+        finally:
+            run.close()
+
+    (want, none), (got, hits) = drive(False), drive(True)
+    assert none == 0 and hits >= 10
+    for (a, la), (b, lb) in zip(want, got):
         np.testing.assert_array_equal(a, b)
         np.testing.assert_array_equal(la, lb)
 
