@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(256) mamba_conv_rows_kernel(MambaArgs a, Trace
 // dt / c are made once per token and head.
 // Bound by instruction issue, half of it those operations; a 16-byte read of shared memory brings eight different pieces
 // to eight lanes (four lanes per row where the state has only 16 entries).  6446 rows in 16 sequences, 64 heads of
-// 64 x 128: 683 us; 730 us with four lanes and three operations per entry, 7405 us with a thread per row, scalar
+// 64 x 128: 582 us (659 with the CTAs in the order of the sequences: 1024 of them in 592 places); before that, 730 us with
+// four lanes and three operations per entry, 7405 us with a thread per row, scalar
 // operations and the decay computed in every thread.  Half the rows per lane doubles the threads of a head when few
 // (sequence, head) pairs are to be shared out.
 constexpr int MS_TC = 16;
@@ -244,12 +245,30 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
   constexpr int N = 4 * L * NJ;
   extern __shared__ __align__(16) float sm[];
   __shared__ float4 tok_s[2 * MS_TC * MS_MAX_HPC];  // [half][token][head]: c, dt / c, what multiplies the state before it
-  const int s = blockIdx.x, h0 = blockIdx.y * hpc;
+  __shared__ int seq_s;
   const int tid = threadIdx.x, nt = blockDim.x, tph = L * a.hd / R;
-  const int hl = tid / tph, ht = tid % tph, q = ht % L, d0 = ht / L * R, h = h0 + hl;
+  const int hl = tid / tph, ht = tid % tph, q = ht % L, d0 = ht / L * R;
   const int uw = hpc * a.hd, row = 2 * N + uw + 2 * hpc;  // floats of a staged token: B | C | u | (step, decay)
   const int rowp = (row + 3) & ~3;
   pdl_wait();
+  // the CTAs of the longest sequence first, then the next one's: what starts last, in SMs that others have left, is short
+  int s = blockIdx.x, part = blockIdx.y;
+  if (a.n_seqs > 1 && a.n_seqs <= 512) {
+    const int at = blockIdx.x + gridDim.x * blockIdx.y;
+    part = at % gridDim.y;
+    for (int i = tid; i < a.n_seqs; i += nt) {
+      const int mine = a.cu_q[i + 1] - a.cu_q[i];
+      int rank = 0;
+      for (int j = 0; j < a.n_seqs; j++) {
+        const int n = a.cu_q[j + 1] - a.cu_q[j];
+        rank += n > mine || (n == mine && j < i);
+      }
+      if (rank == at / (int)gridDim.y) seq_s = i;
+    }
+    __syncthreads();
+    s = seq_s;
+  }
+  const int h0 = part * hpc, h = h0 + hl;
   const int r0 = a.cu_q[s], r1 = a.cu_q[s + 1];
   if (r0 >= r1) return;
   const int start = a.positions[r0];  // position of the first new token
@@ -324,7 +343,11 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
     if (t0 + MS_TC < r1) fetch(t0 + MS_TC, buf ^ 1);
     __syncthreads();
     if (c_end != 1.f) scale(c_end);
-    for (int t = 0; t < n; t++) {
+    float* yp = a.y + (size_t)t0 * a.E + (size_t)h * a.hd + d0 + q;
+    // snapshots: the state after the last token written into a block
+    const int pos0 = start + (t0 - r0);
+    int snap = min(KV_BLOCK - 1 - pos0 % KV_BLOCK, r1 - 1 - t0);
+    for (int t = 0; t < n; t++, yp += a.E) {
       const float* x = sm + (buf * MS_TC + t) * rowp;
       const float4 tk = tok_s[(buf * MS_TC + t) * MS_MAX_HPC + hl];
       const float* u = x + 2 * N + hl * a.hd + d0;
@@ -335,7 +358,6 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
       for (int r = 0; r < R; r++) {
         const float v = tk.y * u[r];
         du[r] = pack2(v, v);
-        acc[r] = 0ull;
       }
 #pragma unroll
       for (int j = 0; j < NJ; j++) {
@@ -345,7 +367,7 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
         for (int r = 0; r < R; r++) {
           st[r][2 * j] = fma2(du[r], B.x, st[r][2 * j]);  // mamba2.go:325-331
           st[r][2 * j + 1] = fma2(du[r], B.y, st[r][2 * j + 1]);
-          acc[r] = fma2(Cc.x, st[r][2 * j], acc[r]);      // :335-340
+          acc[r] = j == 0 ? mul2(Cc.x, st[r][0]) : fma2(Cc.x, st[r][2 * j], acc[r]);  // :335-340
           acc[r] = fma2(Cc.y, st[r][2 * j + 1], acc[r]);
         }
       }
@@ -369,11 +391,10 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
       float out = y[0];
 #pragma unroll
       for (int o = R; o < L; o <<= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
-      if (q < R) a.y[(size_t)(t0 + t) * a.E + (size_t)h * a.hd + d0 + q] = tk.x * out + Dh * u[q];
-      const int pos = start + (t0 + t - r0);
-      if ((pos + 1) % KV_BLOCK == 0 || t0 + t == r1 - 1) {
-        // snapshot: the state after the last token written into this block
-        float* dst = a.ssm_pool + (size_t)bt[pos / KV_BLOCK] * per_block + mine;
+      if (q < R) *yp = tk.x * out + Dh * u[q];
+      if (t == snap) {
+        snap = min(snap + KV_BLOCK, r1 - 1 - t0);
+        float* dst = a.ssm_pool + (size_t)bt[(pos0 + t) / KV_BLOCK] * per_block + mine;
         const unsigned long long cc = pack2(tk.x, tk.x);
 #pragma unroll
         for (int r = 0; r < R; r++)
