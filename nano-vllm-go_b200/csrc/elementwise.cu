@@ -74,11 +74,95 @@ __global__ void embed_kernel(const int* __restrict__ tokens, const int* __restri
   TRACE_EXIT(tr);
 }
 
+// The same for prompts: a warp per row, four neighbouring entries per lane (whole sectors in every access), eight pieces of the
+// row in flight, no block barriers.  Bound by memory.  24 k rows of 2048, bf16 copy and sums of squares: 174 -> 95 us; 18.7 k of
+// 1024 50 -> 23.
+constexpr int EMBED_WARPS = 8, EMBED_MIN_ROWS = 512;
+template <typename WT>
+__global__ void __launch_bounds__(32 * EMBED_WARPS) embed_rows_kernel(const int* __restrict__ tokens, const int* __restrict__ positions, int T,
+                                                                      const WT* __restrict__ wte, const WT* __restrict__ wpe, int max_pos,
+                                                                      float mult, float* __restrict__ x, int H, bf16* __restrict__ xb,
+                                                                      float* __restrict__ ssq, const float* __restrict__ g,
+                                                                      const double* __restrict__ pos_freq, WT* __restrict__ y, Trace tr) {
+  TRACE_ENTRY(tr);
+  pdl_wait();  // step prologue, as above
+  pdl_launch_dependents();
+  constexpr int U = 8;
+  const int lane = threadIdx.x & 31, t = blockIdx.x * EMBED_WARPS + (threadIdx.x >> 5);
+  if (t < T) {
+    const int tok = tokens[t], pos = positions[t];
+    const WT* er = wte + (size_t)tok * H;
+    const WT* pr = wpe != nullptr && pos < max_pos ? wpe + (size_t)pos * H : nullptr;
+    auto get = [](const WT* p, float (&o)[4]) {
+      if constexpr (sizeof(WT) == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
+      } else {
+        const uint2 u = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+      }
+    };
+    float lsq = 0.f;
+    for (int i0 = 4 * lane; i0 < H; i0 += 128 * U) {
+      float v[U][4];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (i0 + 128 * u < H) get(er + i0 + 128 * u, v[u]);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + 128 * u;
+        if (i >= H) break;
+        if (pr) {
+          float p[4];
+          get(pr + i, p);
+#pragma unroll
+          for (int j = 0; j < 4; j++) v[u][j] += p[j];
+        }
+        if (mult != 0.f) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) v[u][j] *= mult;
+        }
+        if (pos_freq) {
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            double sn, cs;
+            sincos((double)pos * pos_freq[(i + j) >> 1], &sn, &cs);
+            v[u][j] += (float)sn;
+            v[u][j + 1] += (float)cs;
+          }
+        }
+        store4(x + (size_t)t * H + i, v[u]);
+        if (y) store4(y + (size_t)t * H + i, v[u]);
+        if (xb) {
+          const float4 gv = *reinterpret_cast<const float4*>(g + i);
+          const float o[4] = {v[u][0] * gv.x, v[u][1] * gv.y, v[u][2] * gv.z, v[u][3] * gv.w};
+#pragma unroll
+          for (int j = 0; j < 4; j++) lsq += v[u][j] * v[u][j];
+          store4(xb + (size_t)t * H + i, o);
+        }
+      }
+    }
+    if (xb) {
+      lsq = warp_sum(lsq);
+      if (lane == 0) ssq[t] = lsq;
+    }
+  }
+  TRACE_EXIT(tr);
+}
+
 cudaError_t launch_embed(cudaStream_t st, int wdt, const int* tokens, const int* positions,
                          const void* wte, const void* wpe, int max_pos, float mult, float* x, int T,
                          int H, void* xb, float* ssq, const float* g, const double* pos_freq, void* y) {
   if (T <= 0) return cudaSuccess;
   if ((xb == nullptr) != (ssq == nullptr) || (xb && !g)) return cudaErrorInvalidValue;
+  if (T >= EMBED_MIN_ROWS && H % 8 == 0) {  // (fewer rows: a block each is the shorter way)
+    const dim3 grid(ceil_div(T, EMBED_WARPS)), block(32 * EMBED_WARPS);
+    return wdt == DT_F32 ? launch_k(embed_rows_kernel<float>, grid, block, 0, st, tokens, positions, T, (const float*)wte, (const float*)wpe,
+                                    max_pos, mult, x, H, (bf16*)xb, ssq, g, pos_freq, (float*)y, next_trace(5))
+                         : launch_k(embed_rows_kernel<bf16>, grid, block, 0, st, tokens, positions, T, (const bf16*)wte, (const bf16*)wpe,
+                                    max_pos, mult, x, H, (bf16*)xb, ssq, g, pos_freq, (bf16*)y, next_trace(5));
+  }
   int threads = min(256, max(32, ((H / 8 + 31) / 32) * 32));
   if (wdt == DT_F32)
     (void)launch_k(embed_kernel<float>, dim3(T), dim3(threads), 0, st, tokens, positions, (const float*)wte,
