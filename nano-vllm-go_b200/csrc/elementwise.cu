@@ -1309,6 +1309,7 @@ __global__ void sample_kernel(const float* __restrict__ logits, int ldl, int V,
                               int vsplit, Trace tr) {
   TRACE_ENTRY(tr);
   pdl_launch_dependents();
+  const float temp = temperature ? temperature[blockIdx.x] : 0.f;  // step state: stable before the wait
   pdl_wait();
   __shared__ float red[32];
   __shared__ ArgMax amred[32];
@@ -1322,7 +1323,6 @@ __global__ void sample_kernel(const float* __restrict__ logits, int ldl, int V,
     return;
   }
   const float* l = logits + (size_t)s * ldl;
-  const float temp = temperature ? temperature[s] : 0.f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (!(temp > 0.f)) {
     const int chunks = gridDim.y;
@@ -1332,17 +1332,26 @@ __global__ void sample_kernel(const float* __restrict__ logits, int ldl, int V,
     // the forward pass has ldl % 8 == 0 and `per` % 4 == 0 (16-byte aligned slices); the
     // single-operator entry point may pass any row stride
     const bool vec = ((reinterpret_cast<uintptr_t>(l + lo)) & 15) == 0;
-    for (int i = lo + threadIdx.x * 4; i < hi; i += blockDim.x * 4) {
-      if (vec && i + 3 < hi) {
-        const float4 v = *reinterpret_cast<const float4*>(l + i);
-        if (v.x > am.v) { am.v = v.x; am.i = i; }
-        if (v.y > am.v) { am.v = v.y; am.i = i + 1; }
-        if (v.z > am.v) { am.v = v.z; am.i = i + 2; }
-        if (v.w > am.v) { am.v = v.w; am.i = i + 3; }
-      } else {
-        for (int j = i; j < min(hi, i + 4); j++) {
-          const float v = l[j];
-          if (v > am.v) { am.v = v; am.i = j; }
+    constexpr int U = 4;  // pieces of a thread in flight
+    const int step = (int)blockDim.x * 4;
+    for (int i0 = lo + (int)threadIdx.x * 4; i0 < hi; i0 += U * step) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (vec && i0 + u * step + 3 < hi) v[u] = *reinterpret_cast<const float4*>(l + i0 + u * step);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * step;
+        if (vec && i + 3 < hi) {
+          if (v[u].x > am.v) { am.v = v[u].x; am.i = i; }
+          if (v[u].y > am.v) { am.v = v[u].y; am.i = i + 1; }
+          if (v[u].z > am.v) { am.v = v[u].z; am.i = i + 2; }
+          if (v[u].w > am.v) { am.v = v[u].w; am.i = i + 3; }
+        } else {
+          for (int j = i; j < min(hi, i + 4); j++) {
+            const float w_ = l[j];
+            if (w_ > am.v) { am.v = w_; am.i = j; }
+          }
         }
       }
     }
@@ -1426,8 +1435,8 @@ cudaError_t launch_sample(cudaStream_t st, const float* logits, int ldl, int V, 
                           const float* temperature, const float* uniforms, int* out_tokens,
                           unsigned long long* amax, int* ticket, int vsplit) {
   if (n <= 0) return cudaSuccess;
-  // ~8K logits per CTA keeps >= 2 waves of CTAs in flight for a large vocabulary
-  const int chunks = (amax && ticket && vsplit == 0) ? max(1, min(64, V / 8192)) : 1;
+  // a CTA of a large vocabulary: 4096 logits, all its loads in flight (8192 one after another: 16 steps of GPT-2 alone 3800 us, 3763 so)
+  const int chunks = (amax && ticket && vsplit == 0 && V >= 8192) ? min(64, V / 4096) : 1;
   (void)launch_k(sample_kernel, dim3(n, chunks), dim3(chunks > 1 ? 256 : 1024), 0, st, logits, ldl,
                  V, temperature, uniforms, out_tokens, amax, ticket, vsplit, next_trace(7));
   return cudaGetLastError();
