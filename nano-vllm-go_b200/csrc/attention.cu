@@ -252,6 +252,15 @@ int attn_decode_splits(int qdt, int kvdt, int n_seqs, int nh, int nkv, int hd, i
     const int G = nh / nkv;
     ctas = n_seqs * nkv * ((G + 15) / 16);
     max_splits = (max_len + attn_decode_mma_tile(hd) - 1) / attn_decode_mma_tile(hd);
+    // Where a context is left whole: its second half would cost less than the launch that joins the parts.  The more CTAs
+    // there are, the more of their memory time one hides under another's, and the longer that holds.  Resident steps, us
+    // split / whole (12 GPT-2 layers, heads by themselves; four Llama-1B layers, groups of four; two of Falcon, one group):
+    //   GPT-2    1 x 250 226 / 213, 350 230 / 220, 500 225 / 228    4 x 250 256 / 242, 420 251 / 258    8 x 450 302 / 270, 900 319 / 306
+    //   Llama    1 x 250 196 / 190, 500 190 / 192    8 x 500 189 / 182, 1500 206 / 202, 2500 219 / 226    16 x 700 221 / 205, 2500 256 / 254
+    //            24 x 1500 250 / 228    32 x 1000 240 / 219
+    //   Falcon   8 x 250 197 / 195, 700 200 / 202    16 x 700 210 / 217
+    const int whole = G > 8 ? 256 : ctas >= 56 ? max(352, 20 * ctas) : 352;
+    if (max_len <= whole) return 1;
   } else {
     const int G = nh / nkv;
     int gc = 1;
