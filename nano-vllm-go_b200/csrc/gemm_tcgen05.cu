@@ -713,7 +713,9 @@ int tc5_splits(int M, int N, int K, int sm_count) {
   // The consumer of the partials sums up to 8 slices with one batch of loads (sum_partials8); a
   // 9th slice costs it a second L2 round trip, more than the GEMM gains from the finer split
   // (cfg2 decode, W2 GEMM K = 8192: S = 9 -> 1105 us/step, capped at 8 -> 1079; 6 -> 1099 /
-  // 1219 with the fused residual; 4 -> 1371).
+  // 1219 with the fused residual; 4 -> 1371).  What a slice costs, in blocks of k: 0.1 / 0.35 / 0.7 / 1.2 / 2 give 128
+  // sequences through routed experts 5096 / 5099 / 4964 / 4969 / 5105 us for 16 steps, 64 through Llama-1B layers 4028 / 4037 /
+  // 4026 / 4067 / 4061.
   constexpr int smax = 8;
   for (int s = 1; s <= smax && s <= nkb; s++) {
     const int kbps = ceil_div(nkb, s);
@@ -722,7 +724,7 @@ int tc5_splits(int M, int N, int K, int sm_count) {
     if (s_eff != s) continue;
     const long units = tiles * s;
     const long rounds = (units + sm_count - 1) / sm_count;
-    const double cost = (double)rounds * (kbps + 1.5) + 0.35 * s;
+    const double cost = (double)rounds * (kbps + 1.5) + 0.7 * s;
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
       best = s;
