@@ -1477,7 +1477,7 @@ cudaError_t launch_advance(cudaStream_t st, int n, const int* sampled, int* toke
 
 // ------------------------------------------------------------- recurrent state
 // The state of a step's sequences aside (restore = 0) and back: copy [n][slot_floats], behind it the n slots.  Bound by
-// memory, once in and once out; the copy leaves L2 first.  32 slots of 1.1 MB: 13 us.
+// memory, once in and once out; the copy leaves L2 first.  32 slots of 1.1 MB: 16 us.
 __global__ void __launch_bounds__(256) state_copy_kernel(int n, const int* __restrict__ slots, float* __restrict__ pool, size_t slot_floats,
                                                          float* __restrict__ copy, int* __restrict__ copy_slots, int restore, Trace tr) {
   TRACE_ENTRY(tr);
