@@ -510,9 +510,11 @@ static cudaError_t decode_t_launch(cudaStream_t st, const AttnArgs& a, int G) {
 }
 
 // kv heads per CTA can be forced with NVLLM_ATTN_T_KPC (1, 2, 4) for experiments.
-cudaError_t launch_attn_decode_t(cudaStream_t st, const AttnArgs& a) {
-  if (a.n_seqs <= 0) return cudaSuccess;
-  const int G = a.nh / a.nkv;
+// The order of a row's sums follows it: a replayed graph is kept for one choice only (run.cu), so that a step's results
+// do not depend on the lengths that the handle saw before.
+int attn_decode_heads(int n_seqs, int nh, int nkv, int max_len, int n_splits, int sm_count) {
+  if (nkv <= 0 || nh % nkv) return 1;
+  const int G = nh / nkv;
   // read per launch (not cached): the parity tests switch it between runners
   const char* kpc_s = getenv("NVLLM_ATTN_T_KPC");
   const int kpc_env = kpc_s ? atoi(kpc_s) : 0;
@@ -522,16 +524,22 @@ cudaError_t launch_attn_decode_t(cudaStream_t st, const AttnArgs& a) {
   // one stage per head measured slower — cfg3 1810 vs 1775 us/step, cfg2 1231 vs 1088 — and is
   // only reachable through the knob.)
   int kpc = 1;
-  if (a.n_splits == 1) {
-    const int sm = a.sm_count > 0 ? a.sm_count : 148;
-    while (kpc < 2 && a.nkv % (kpc * 2) == 0 &&
-           (long)a.n_seqs * (a.nkv / (kpc * 2)) * 10 >= (long)sm * 16)
+  if (n_splits == 1) {
+    const int sm = sm_count > 0 ? sm_count : 148;
+    while (kpc < 2 && nkv % (kpc * 2) == 0 &&
+           (long)n_seqs * (nkv / (kpc * 2)) * 10 >= (long)sm * 16)
       kpc *= 2;
     // heads by themselves (G = 1) and short contexts: two of them to a CTA merge over two warps each instead of four
     // (GPT-2 alone, us a step: 30 tokens 220 -> 210, 150 209 -> 201, 300 216 -> 213; eight sequences of 450 268 -> 271)
-    if (kpc == 1 && G == 1 && a.nkv % 2 == 0 && a.max_len <= 256) kpc = 2;
-    if ((kpc_env == 1 || kpc_env == 2 || kpc_env == 4) && a.nkv % kpc_env == 0) kpc = kpc_env;
+    if (kpc == 1 && G == 1 && nkv % 2 == 0 && max_len <= 256) kpc = 2;
+    if ((kpc_env == 1 || kpc_env == 2 || kpc_env == 4) && nkv % kpc_env == 0) kpc = kpc_env;
   }
+  return kpc;
+}
+
+cudaError_t launch_attn_decode_t(cudaStream_t st, const AttnArgs& a) {
+  if (a.n_seqs <= 0) return cudaSuccess;
+  const int G = a.nh / a.nkv, kpc = attn_decode_heads(a.n_seqs, a.nh, a.nkv, a.max_len, a.n_splits, a.sm_count);
   if (a.hd == 64) {
     // 4 heads: one 16 KB stage per head (3 CTAs / SM, 12 head streams per SM in flight)
     if (kpc == 4) return decode_t_launch<64, 64, 4, 4>(st, a, G);

@@ -490,6 +490,7 @@ bool attn_prefill_tc5_enabled();
 cudaError_t launch_attn_prefill_tc5(cudaStream_t st, const AttnArgs& a);
 // attention_dec.cu: decode kernel for query-head groups of <= 8 (needs AttnArgs::pool_blocks)
 bool attn_decode_t_supported(const AttnArgs& a);
+int attn_decode_heads(int n_seqs, int nh, int nkv, int max_len, int n_splits, int sm_count);  // K / V heads of a CTA
 cudaError_t launch_attn_decode_t(cudaStream_t st, const AttnArgs& a);
 
 // ---------------------------------------------------------------- attention_latent.cu

@@ -87,7 +87,7 @@ static void fill_stats(nvllm_handle* h, nvllm_run_stats* stats, int T, uint64_t 
 // pointer or a constant of the launch shape (the step state itself lives in device memory), so
 // the ~100 launches are captured once — programmatic dependent-launch edges included — and
 // replayed with one cudaGraphLaunch until the shape changes (staging buffer, batch,
-// block-table width, KV split count).  slot 0 = nvllm_run_resident (`pre` launches the advance
+// block-table width, KV split count, K / V heads of an attention CTA).  slot 0 = nvllm_run_resident (`pre` launches the advance
 // kernel), slot 1 = nvllm_run's decode step (`pre` does nothing; the H2D copy stays outside).
 static bool graph_usable(const nvllm_handle* h, int n) {
   return h->graphs_enabled && !h->profile && !trace_active() && h->tp == 1 && h->skip_mask == 0 &&
@@ -109,6 +109,7 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
         sig.n_splits += latent_attn_splits(L.n, y.s.heads, L.max_len, y.s.window, h->sm_count);
   } else {
     sig.n_splits = attn_decode_splits(h->adt, h->kvdt, L.n, h->nh, h->nkv, h->hd, L.max_len, h->sm_count);
+    if (attn_mma_supported(h->adt, h->kvdt, h->hd)) sig.heads = attn_decode_heads(L.n, h->nh, h->nkv, L.max_len, sig.n_splits, h->sm_count);
   }
   if (!h->step_graph[slot] || !(sig == h->graph_sig[slot])) {
     if (h->step_graph[slot]) cudaGraphExecDestroy(h->step_graph[slot]);

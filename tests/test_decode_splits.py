@@ -57,3 +57,43 @@ def test_step_matches_the_prompts(make, n, longest, split):
     # the same bf16 roundings, sums in another order: as far from float32 as the prompts are; one row's error is known to
     # a third or so, that of n rows to the square root of n better
     assert np.linalg.norm(step - want) <= (1.2 + 0.4 / np.sqrt(n)) * np.linalg.norm(prompts - want)
+
+
+def test_replayed_steps_choose_by_their_own_lengths():
+    """Block tables with room to spare, so that nothing else of a step's shape changes where its kernels do: replayed steps give
+    what launched ones give, bit for bit, whatever lengths the handle saw before."""
+    cfg = gpt2()
+    weights = list(W.random_weights(cfg, 17, round_bf16=True))
+    texts = [W.random_prompt(cfg.vocab_size, n, 160 + i).tolist() for i, n in enumerate((250, 341, 30))]
+
+    def drive(graphs):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, weights, precision=C.PREC_BF16, num_kv_blocks=6, sampling=None)
+        try:
+            run.set_graphs(graphs)
+            run.set_speculation(False)
+            outs, used = [], 0
+
+            def steps(i, n):
+                nonlocal used
+                for k in range(n):
+                    seq = texts[i] + [7 + j for j in range(k)]
+                    outs.append(run.run_flat([seq], False, None, [[2 * i, 2 * i + 1]], [0.0], want_logits=True)[1])
+                    used += run.last_stats.used_graph
+
+            run.run_flat([t[:-1] for t in texts], True, [0] * 3, [[0, 1], [2, 3], [4, 5]], [0.0] * 3)
+            steps(0, 12)  # across 256 tokens
+            steps(2, 2)   # a short context after long ones
+            steps(1, 14)  # a long one after short ones, across 352
+            run.run_flat([texts[0]], False, None, [[0, 1]], [0.0])
+            for _ in range(12):  # the same on the device's own tokens
+                run.run_resident()
+                used += run.last_stats.used_graph
+                outs.append(run.sync(1)[0])
+            return outs, used
+        finally:
+            run.close()
+
+    (want, none), (got, all_) = drive(False), drive(True)
+    assert none == 0 and all_ == len(got)
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
