@@ -438,7 +438,7 @@ int forward_step(nvllm_handle* h) {
       ma.conv_w = lw.m_conv_w; ma.conv_b = lw.m_conv_b; ma.dt_bias = lw.m_dt_bias; ma.a_log = lw.m_a_log;
       ma.d_skip = lw.m_d; ma.norm_w = lw.m_norm;
       ma.xbc = w.m_xbc; ma.dt = w.m_dt; ma.y = w.m_y;
-      ma.cu_q = d + L.cu_q; ma.positions = d_pos; ma.block_tables = d + L.block_tables;
+      ma.cu_q = d + L.cu_q; ma.order = L.by_length ? d + L.seq_order : nullptr; ma.positions = d_pos; ma.block_tables = d + L.block_tables;
       ma.max_blocks = L.max_blocks;
       ma.ssm_pool = h->ssm_pool; ma.n_mamba = h->n_mamba; ma.layer = h->mamba_idx[l];
       {

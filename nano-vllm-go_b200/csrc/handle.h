@@ -144,7 +144,8 @@ struct StepLayout {
   size_t words = 0;  // 4-byte words in use
   // offsets (in words) of each array
   size_t tokens, positions, slots, cu_q, seq_start, seq_len, last_row, block_tables, tile_seq,
-      tile_q0, temperature, uniforms, state_slots;
+      tile_q0, temperature, uniforms, state_slots, seq_order;
+  bool by_length = false;  // seq_order holds the sequences by their new tokens, the most first
 };
 
 struct Workspace {

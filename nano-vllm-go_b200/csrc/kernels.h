@@ -764,6 +764,7 @@ struct MambaArgs {
   float2* dt;          // [T, nh]    {softplus(dt + bias), exp(-exp(A_log) of it)}
   float* y;            // [T, E]     scan output
   const int* cu_q;         // [n_seqs + 1] rows of each sequence
+  const int* order;        // [n_seqs] sequences by their rows, the most first; null: all alike
   const int* positions;    // [T]
   const int* block_tables; // [n_seqs, max_blocks]
   int max_blocks;

@@ -233,7 +233,9 @@ __global__ void __launch_bounds__(256) mamba_conv_rows_kernel(MambaArgs a, Trace
 // to eight lanes (four lanes per row where the state has only 16 entries).  6446 rows in 16 sequences, 64 heads of
 // 64 x 128: 582 us (659 with the CTAs in the order of the sequences: 1024 of them in 592 places); before that, 730 us with
 // four lanes and three operations per entry, 7405 us with a thread per row, scalar
-// operations and the decay computed in every thread.  Half the rows per lane doubles the threads of a head when few
+// operations and the decay computed in every thread.  The order comes from the host, which knows the lengths, and only where
+// they differ: counted in every CTA it made a decode step of 128 / 256 / 512 sequences (one such layer and one of attention)
+// 305 / 746 / 3120 us long, 280 / 483 / 816 so.  Half the rows per lane doubles the threads of a head when few
 // (sequence, head) pairs are to be shared out.
 constexpr int MS_TC = 16;
 constexpr float MS_RESCALE = 1e-18f;
@@ -245,7 +247,6 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
   constexpr int N = 4 * L * NJ;
   extern __shared__ __align__(16) float sm[];
   __shared__ float4 tok_s[2 * MS_TC * MS_MAX_HPC];  // [half][token][head]: c, dt / c, what multiplies the state before it
-  __shared__ int seq_s;
   const int tid = threadIdx.x, nt = blockDim.x, tph = L * a.hd / R;
   const int hl = tid / tph, ht = tid % tph, q = ht % L, d0 = ht / L * R;
   const int uw = hpc * a.hd, row = 2 * N + uw + 2 * hpc;  // floats of a staged token: B | C | u | (step, decay)
@@ -253,20 +254,10 @@ __global__ void __launch_bounds__(512) mamba_scan_tile_kernel(MambaArgs a, int h
   pdl_wait();
   // the CTAs of the longest sequence first, then the next one's: what starts last, in SMs that others have left, is short
   int s = blockIdx.x, part = blockIdx.y;
-  if (a.n_seqs > 1 && a.n_seqs <= 512) {
+  if (a.order) {
     const int at = blockIdx.x + gridDim.x * blockIdx.y;
     part = at % gridDim.y;
-    for (int i = tid; i < a.n_seqs; i += nt) {
-      const int mine = a.cu_q[i + 1] - a.cu_q[i];
-      int rank = 0;
-      for (int j = 0; j < a.n_seqs; j++) {
-        const int n = a.cu_q[j + 1] - a.cu_q[j];
-        rank += n > mine || (n == mine && j < i);
-      }
-      if (rank == at / (int)gridDim.y) seq_s = i;
-    }
-    __syncthreads();
-    s = seq_s;
+    s = a.order[at / gridDim.y];
   }
   const int h0 = part * hpc, h = h0 + hl;
   const int r0 = a.cu_q[s], r1 = a.cu_q[s + 1];

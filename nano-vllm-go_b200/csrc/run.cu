@@ -31,7 +31,7 @@ static int ensure_stage(nvllm_handle* h, size_t words) {
 }
 
 // offsets of a step's arrays inside its staging buffer (every array 16-byte aligned)
-static void plan_layout(StepLayout& L, int T, int n, int max_blocks, int n_qtiles, int n_extra = 0) {
+static void plan_layout(StepLayout& L, int T, int n, int max_blocks, int n_qtiles, int n_extra = 0, bool by_length = false) {
   L.T = T;
   L.n = n;
   L.n_out = n + n_extra;
@@ -56,6 +56,8 @@ static void plan_layout(StepLayout& L, int T, int n, int max_blocks, int n_qtile
   L.temperature = take(n);
   L.uniforms = take(n);
   L.state_slots = take(n);
+  L.by_length = by_length;
+  L.seq_order = take(by_length ? n : 0);
   L.words = o;
 }
 
@@ -382,7 +384,8 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   h->run_lay_ok = false;
 
   // ---- pass 1: sizes and validation
-  int T = 0, max_blocks = 0, n_qtiles = 0, max_len = 0;
+  int T = 0, max_blocks = 0, n_qtiles = 0, max_len = 0, first_new = 0;
+  bool by_length = false;  // Mamba2 scans of prompts of unequal length take the sequences by it (mamba.cu)
   const int qtile = h->layered ? h->attn_qtile : attn_prefill_qtile(h->adt, h->kvdt, h->hd);
   // recurrent mixers: every sequence of the step names its state slot (nvllm_set_state_slots)
   std::vector<int32_t> sslots;
@@ -425,6 +428,8 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
                        "ones; disable prefix caching / chunked prefill for them", i, len - start, start);
     }
     const int n_new = len - start;
+    if (i == 0) first_new = n_new;
+    by_length = by_length || (h->n_mamba && n_new != first_new);
     T += n_new;
     n_qtiles += (n_new + qtile - 1) / qtile;
     max_blocks = std::max(max_blocks, nb);
@@ -441,7 +446,7 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
   for (int r : want)
     if (r < 0 || r >= T) return set_err(h, NVLLM_ERR_RANGE, "requested logits row %d outside the step's %d rows", r, T);
   StepLayout& L = h->lay;
-  plan_layout(L, T, n, max_blocks, is_prefill ? n_qtiles : 0, n_extra);
+  plan_layout(L, T, n, max_blocks, is_prefill ? n_qtiles : 0, n_extra, by_length);
   L.prefill = is_prefill != 0;
   L.max_len = max_len;
   L.sum_len = sum_len;
@@ -499,6 +504,11 @@ extern "C" int nvllm_run(nvllm_handle* h, int n, int is_prefill, const int32_t* 
     s_uni[i] = (t > 0.f) ? (uniforms ? uniforms[i] : next_uniform(h)) : 0.f;
   }
   s[L.cu_q + n] = row;
+  if (by_length) {
+    int32_t *order = s + L.seq_order, *rows = s + L.cu_q;
+    for (int i = 0; i < n; i++) order[i] = i;
+    std::stable_sort(order, order + n, [rows](int a, int b) { return rows[a + 1] - rows[a] > rows[b + 1] - rows[b]; });
+  }
   for (int i = 0; i < n_extra; i++) s[L.last_row + n + i] = want[i];
 
   cudaStream_t st = h->stream;

@@ -162,3 +162,52 @@ def test_hybrid_decays_of_every_strength(N, hd, n):
         assert max(rel_err(row, want[1][1]) for row in logits) <= 1e-4
     finally:
         run.close()
+
+
+CONV, SCAN = 20, 21  # ids in the timeline
+
+
+def test_hybrid_decode_scan_grows_with_the_batch_only():
+    """A decode step's scan is bound by the state that it reads and writes: four times the sequences, four times the time."""
+    cfg = C.tiny_hybrid(vocab_size=256, num_layers=1, hybrid_layers=(True,), mamba_num_heads=64, mamba_head_dim=64,
+                        mamba_state_size=128, mamba_n_groups=1, mamba_conv_kernel=4)
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 7), precision=C.PREC_BF16, num_kv_blocks=512, sampling=None)
+    times = {}
+    try:
+        for n in (128, 512):
+            seqs, tables = [[i % 256, 3] for i in range(n)], [[i] for i in range(n)]
+            for _ in range(3):
+                run.trace_begin(1 << 17)
+                run.run_flat(seqs, False, None, tables, [0.0] * n)
+                rec = run.trace_end(1 << 17)
+                took = int(rec[rec[:, 1] == SCAN, 6].max()) - int(rec[rec[:, 1] == CONV, 6].max())
+                times[n] = min(times.get(n, took), took)
+    finally:
+        run.close()
+    assert times[512] <= 6 * times[128], times  # (four, and half as much again for what a small batch hides)
+
+
+@pytest.mark.parametrize("lengths", [
+    (9, 9, 9), (3, 40, 3), tuple(1 + i % 2 for i in range(7)),                         # all alike; one of them longer; ties
+    tuple(5 + 37 * i % 61 for i in range(64)), tuple(1 + 7 * i % 19 for i in range(520)),  # in no order; more than 512 of them
+], ids=lambda v: str(len(v)))
+def test_hybrid_prompts_of_any_lengths_are_what_each_is_alone(lengths):
+    """The scan takes the sequences of a step by length (mamba.cu): each ends as it does alone, now and in a step that is repeated."""
+    cfg = C.tiny_hybrid(vocab_size=256, num_layers=2, hybrid_layers=(True, True), mamba_num_heads=4, mamba_head_dim=16,
+                        mamba_state_size=32, mamba_n_groups=1, mamba_conv_kernel=4)
+    n = len(lengths)
+    seqs = [W.random_prompt(cfg.vocab_size, k, 50 + i).tolist() for i, k in enumerate(lengths)]
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 7), precision=C.PREC_FP32, num_kv_blocks=n + 1, sampling=None)
+    try:
+        out, logits = run.run_flat(seqs, True, [0] * n, [[i] for i in range(n)], [0.0] * n, want_logits=True)
+        after = run.run_flat([s + [int(t)] for s, t in zip(seqs, out)], False, None, [[i] for i in range(n)], [0.0] * n, want_logits=True)
+        for i in sorted({0, 1, n // 2, n - 1, int(np.argmax(lengths)), int(np.argmin(lengths))}):
+            one, alone = run.run_flat([seqs[i]], True, [0], [[n]], [0.0], want_logits=True)
+            assert rel_err(logits[i], alone[0]) <= TOL[C.PREC_FP32] and int(one[0]) == int(out[i])
+            _, alone = run.run_flat([seqs[i] + [int(out[i])]], False, None, [[n]], [0.0], want_logits=True)
+            assert rel_err(after[1][i], alone[0]) <= TOL[C.PREC_FP32]
+        run.run_flat(seqs, True, [0] * n, [[i] for i in range(n)], [0.0] * n)
+        run.rerun()
+        np.testing.assert_array_equal(run.sync(n)[0], out)
+    finally:
+        run.close()
