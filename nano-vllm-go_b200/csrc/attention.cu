@@ -246,7 +246,7 @@ int attn_prefill_qtile(int qdt, int kvdt, int hd) {
 }
 
 int attn_decode_splits(int qdt, int kvdt, int n_seqs, int nh, int nkv, int hd, int max_len,
-                       int sm_count) {
+                       long long sum_len, int sm_count) {
   int ctas, max_splits;
   if (attn_mma_supported(qdt, kvdt, hd)) {
     const int G = nh / nkv;
@@ -259,8 +259,20 @@ int attn_decode_splits(int qdt, int kvdt, int n_seqs, int nh, int nkv, int hd, i
     //   Llama    1 x 250 196 / 190, 500 190 / 192    8 x 500 189 / 182, 1500 206 / 202, 2500 219 / 226    16 x 700 221 / 205, 2500 256 / 254
     //            24 x 1500 250 / 228    32 x 1000 240 / 219
     //   Falcon   8 x 250 197 / 195, 700 200 / 202    16 x 700 210 / 217
-    const int whole = G > 8 ? 256 : ctas >= 56 ? max(352, 20 * ctas) : 352;
-    if (max_len <= whole) return 1;
+    // The others' work has to be there for that: the longest context may exceed what they keep the chip busy with (mean * ctas
+    // / 300 tokens of one CTA's time; twice that at head size 128, with twice the bytes) by the cost of the launch and of the
+    // parts' own starts (800 tokens, and 6 per CTA).  One context of the first length, the others as long / half / a quarter /
+    // a twentieth, us split / whole:
+    //   Llama-1B  16 x 2000  245 / 242  233 / 233  225 / 229  220 / 226     32 x 4000  348 / 330  293 / 294  268 / 279  248 / 266
+    //             36 x 4000  384 / 366  318 / 320  289 / 299  265 / 285
+    //   head size 128 (two Llama-3B layers)
+    //              7 x 500   149 / 138  148 / 136  147 / 137  145 / 136     14 x 1500  175 / 159  164 / 156  161 / 155  158 / 154
+    //             16 x 2000  186 / 171  172 / 165  166 / 163  162 / 162     28 x 4000  298 / 281  226 / 236  201 / 215  184 / 198
+    // (Not met by it: 160 to 230 CTAs of head size 128, some SMs with twice the CTAs of the others: 20 x 3000 229 / 239 stays
+    // whole, and so does 28 x 4000 with halves.)
+    const int whole = G > 8 ? 256 : 352;
+    const double rest = (double)sum_len / n_seqs * ctas * hd / (300 * 64);
+    if (max_len <= whole || (G <= 8 && ctas >= 56 && max_len <= min(20.0 * ctas, 800 + 6.0 * ctas + rest))) return 1;
   } else {
     const int G = nh / nkv;
     int gc = 1;

@@ -412,7 +412,7 @@ int forward_step(nvllm_handle* h) {
   at.tickets = (int*)w.chain_ctr + (h->pipe_role == 2 ? 32 : 16);  // (two chunks of a step may be in flight)
   at.wait_flag = h->waits.dev;
   if (!is_prefill)
-    at.n_splits = attn_decode_splits(h->adt, h->kvdt, n, h->nh, h->nkv, h->hd, L.max_len, h->sm_count);
+    at.n_splits = attn_decode_splits(h->adt, h->kvdt, n, h->nh, h->nkv, h->hd, L.max_len, L.sum_len, h->sm_count);
   const double qo_bytes = 2.0 * T * h->q_cols * asz;
   const double attn_flops = 4.0 * h->nh * h->hd * L.attn_pairs;
   // algorithmic: every K/V row of the contexts once (+ the new rows appended by a fused decode

@@ -473,9 +473,9 @@ constexpr int ATTN_PREFILL_QTILE = 32;  // SIMT (fp32 parity) kernel; the mma ke
 // queries per tile of the kernel launch_attn_prefill will pick: the host builds tile_seq /
 // tile_q0 with it
 int attn_prefill_qtile(int qdt, int kvdt, int hd);
-// KV splits for a decode step of n_seqs sequences whose longest context is max_len
+// KV splits for a decode step of n_seqs sequences whose longest context is max_len, all together sum_len
 int attn_decode_splits(int qdt, int kvdt, int n_seqs, int nh, int nkv, int hd, int max_len,
-                       int sm_count);
+                       long long sum_len, int sm_count);
 cudaError_t launch_attn_prefill(cudaStream_t st, const AttnArgs& a);
 cudaError_t launch_attn_decode(cudaStream_t st, const AttnArgs& a);
 bool attn_decode_fuses_rope(int qdt, int kvdt, int hd);

@@ -110,7 +110,7 @@ static int graphed_step(nvllm_handle* h, int slot, Pre pre, bool* used) {
       if (y.s.mixer == NVLLM_MIXER_LATENT_ATTENTION)
         sig.n_splits += latent_attn_splits(L.n, y.s.heads, L.max_len, y.s.window, h->sm_count);
   } else {
-    sig.n_splits = attn_decode_splits(h->adt, h->kvdt, L.n, h->nh, h->nkv, h->hd, L.max_len, h->sm_count);
+    sig.n_splits = attn_decode_splits(h->adt, h->kvdt, L.n, h->nh, h->nkv, h->hd, L.max_len, L.sum_len, h->sm_count);
     if (attn_mma_supported(h->adt, h->kvdt, h->hd)) sig.heads = attn_decode_heads(L.n, h->nh, h->nkv, L.max_len, sig.n_splits, h->sm_count);
   }
   if (!h->step_graph[slot] || !(sig == h->graph_sig[slot])) {

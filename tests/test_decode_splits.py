@@ -32,8 +32,18 @@ def falcon():
     (falcon, 2, 256, False), (falcon, 2, 257, True),                          # one group of nine heads
 ], ids=lambda v: v if not callable(v) else "m")
 def test_step_matches_the_prompts(make, n, longest, split):
-    cfg = make()
-    texts = [W.random_prompt(cfg.vocab_size, longest - (7 * i) % 31, 160 + i) for i in range(n)]
+    check_step(make(), [longest - (7 * i) % 31 for i in range(n)], split)
+
+
+@pytest.mark.parametrize("rest,split", [(60, True), (1699, False)])
+def test_one_long_context_among_short_ones(rest, split):
+    """128 CTAs leave contexts whole where all are long, not where one is: the others' memory time does not hide it then."""
+    check_step(llama(8), [1700] + [rest - (7 * i) % 31 for i in range(15)], split)
+
+
+def check_step(cfg, lengths, split):
+    n, longest = len(lengths), lengths[0]
+    texts = [W.random_prompt(cfg.vocab_size, k, 160 + i) for i, k in enumerate(lengths)]
     weights = list(W.random_weights(cfg, 17, round_bf16=True))
     blocks = -(-longest // 256)
     tables, zeros = [list(range(blocks * i, blocks * i + blocks)) for i in range(n)], [0.0] * n
