@@ -537,15 +537,17 @@ __global__ void __launch_bounds__(512) norm_kernel(NormArgs a, Trace tr) {
 // Steps of fewer rows (SL = 8): bound by one L2 round trip, two block sums at most and the way in and out of the launch;
 // weights and biases are loaded before the dependency resolves.  64 rows of 2048 with eight slices, from the release to the last
 // exit: 4.9 -> 2.7 us; 16 decode steps of 64 sequences through four Llama-1B layers 4668 -> 4330 us, of 128 through routed
-// experts (every second norm) 5694 -> 5505.
-constexpr int NR_MAX_V = 4, NR_THREADS = 512, NR_STEP_THREADS = 640;
+// experts (every second norm) 5694 -> 5505.  Threads and vectors are such that no form spills (two vectors with the weights
+// ahead did; a step of 64 sequences through two Llama-3B layers 147.8 us so, 144.5 without).
+constexpr int NR_MAX_V = 4, NR_THREADS = 512, NR_STEP_MAX_V = 5;
+constexpr int nr_step_threads(int V, bool comb) { return V <= (comb ? 1 : 2) ? 640 : 512; }
 template <typename YT, int V, int COMB, int SL>
-__global__ void __launch_bounds__(SL > 1 ? NR_STEP_THREADS : NR_THREADS, SL > 1 ? 1 : 2) norm_rows_kernel(NormArgs a, Trace tr) {
+__global__ void __launch_bounds__(SL > 1 ? nr_step_threads(V, COMB > 0) : NR_THREADS, SL > 1 ? 1 : 2) norm_rows_kernel(NormArgs a, Trace tr) {
   const unsigned long long t_entry = trace_on(tr) ? gtime() : 0ull;
   pdl_launch_dependents();
   __shared__ float red[32];
   const int H = a.H;
-  constexpr bool STEP = SL > 1, AHEAD = STEP && V <= 2;
+  constexpr bool STEP = SL > 1, AHEAD = STEP && V == 1;  // (two vectors leave no registers for the weights)
   auto get = [](const float* p, float (&o)[4]) {
     const float4 f = *reinterpret_cast<const float4*>(p);
     o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
@@ -715,18 +717,29 @@ static bool norm_rows_fit(const NormArgs& a) {
   return norm_rows_plain(a) && a.n_rows >= 512 && a.H <= NR_MAX_V * NR_THREADS * 4 && !a.row_idx &&
          (!a.p1 || a.comb_rows || a.S1 == 1) && (!a.p2 || a.S2 == 1);
 }
+struct NrShape {
+  int V, threads;
+};
+static NrShape nr_shape(int H, bool step, bool comb) {
+  NrShape s{1, 0};
+  while (H > s.V * 4 * (step ? nr_step_threads(s.V, comb) : NR_THREADS)) s.V++;
+  s.threads = ceil_div(ceil_div(H, 4 * s.V), 32) * 32;
+  return s;
+}
 // few rows, at most eight slices (what the products of a step are split into)
 static bool norm_step_fit(const NormArgs& a) {
-  return norm_rows_plain(a) && a.n_rows < 512 && a.H <= NR_MAX_V * NR_STEP_THREADS * 4 && (!a.p1 || a.comb_rows || a.S1 <= 8) &&
-         (!a.p2 || a.S2 <= 8);
+  return norm_rows_plain(a) && a.n_rows < 512 && a.H <= NR_STEP_MAX_V * nr_step_threads(NR_STEP_MAX_V, false) * 4 &&
+         (!a.p1 || a.comb_rows || a.S1 <= 8) && (!a.p2 || a.S2 <= 8);
 }
 template <typename YT, int SL>
 static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
-  const int V = ceil_div(a.H, (SL > 1 ? NR_STEP_THREADS : NR_THREADS) * 4), threads = ceil_div(ceil_div(a.H, 4 * V), 32) * 32;
   const bool comb = a.p1 && a.comb_rows;
+  const auto [V, threads] = nr_shape(a.H, SL > 1, comb);
 #define NR(V_)                                                                                                           \
   (comb ? launch_k(norm_rows_kernel<YT, V_, 8, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(SL > 1 ? 53 : 47)) \
         : launch_k(norm_rows_kernel<YT, V_, 0, SL>, dim3(a.n_rows), dim3(threads), 0, st, a, next_trace(SL > 1 ? 53 : 47)))
+  if constexpr (SL > 1)
+    if (V == 5) return NR(5);
   return V == 1 ? NR(1) : V == 2 ? NR(2) : V == 3 ? NR(3) : NR(4);
 #undef NR
 }

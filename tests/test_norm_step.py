@@ -28,6 +28,7 @@ def falcon(hidden):
     gpt2(2056), llama(2560), falcon(2048),     # one vector, the last one: five slices and more
     llama(2568), falcon(4544), gpt2(5120),     # two
     falcon(5128), llama(7688),                 # three; four
+    llama(6144), falcon(6152), gpt2(8192), llama(8200),  # the last of three, of four; five
     gpt2(10240), llama(10248),                 # the widest; wider
 ], ids=lambda c: f"{c.name}-{c.hidden}")
 def test_step_matches_the_prompts(cfg):
