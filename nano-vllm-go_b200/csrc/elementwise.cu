@@ -726,10 +726,30 @@ static NrShape nr_shape(int H, bool step, bool comb) {
   s.threads = ceil_div(ceil_div(H, 4 * s.V), 32) * 32;
   return s;
 }
-// few rows, at most eight slices (what the products of a step are split into)
+// Few rows, at most eight slices (what the products of a step are split into).  Up to which row: norm_kernel has two CTAs of
+// up to 2048 entries on an SM where these take all of its registers, and is ahead from the fourth wave of them on, with
+// expert rows from the second; rows of four vectors and more are too long a chain for a second wave.  Whole steps of few
+// layers, norm_kernel / these:
+//   rows            1            16           64           128          192          256          384          448          511
+//   width  768  199 / 198    437 / 363    490 / 425    613 / 548    789 / 734    891 / 828   1143 / 1107  1219 / 1200  1311 / 1298
+//         2048  188 / 187    200 / 188    218 / 195    261 / 250    376 / 367    404 / 397    563 / 560    585 / 591    612 / 622
+//         3072  144 / 144    134 / 132    150 / 145    179 / 176    247 / 244    268 / 265    389 / 391    414 / 416    432 / 434
+//         4544  259 / 259    208 / 202    234 / 228    277 / 272    377 / 367    410 / 403    574 / 565    605 / 591    628 / 615
+//         5120  278 / 270    274 / 255    292 / 270    335 / 317    432 / 411    468 / 449    612 / 590    658 / 634    706 / 678
+//         6144  332 / 330    295 / 286    313 / 302    360 / 352    458 / 452    497 / 493    655 / 650    707 / 704    747 / 750
+//         8192  373 / 378    346 / 343    363 / 360    419 / 418    521 / 527    566 / 575    668 / 663    689 / 687    749 / 748
+//        10240  327 / 329    326 / 319    354 / 344    427 / 420    611 / 612    684 / 689    929 / 950    988 /1012   1020 / 1043
+//   experts 1024  182 / 172  197 / 189    222 / 213    250 / 244    314 / 309    342 / 337    430 / 429    454 / 455    485 / 485
+//           2048  171 / 162  190 / 181    204 / 195    240 / 233    308 / 308    350 / 351    439 / 444    478 / 486    512 / 520
 static bool norm_step_fit(const NormArgs& a) {
-  return norm_rows_plain(a) && a.n_rows < 512 && a.H <= NR_STEP_MAX_V * nr_step_threads(NR_STEP_MAX_V, false) * 4 &&
-         (!a.p1 || a.comb_rows || a.S1 <= 8) && (!a.p2 || a.S2 <= 8);
+  if (!norm_rows_plain(a) || a.n_rows >= 512 || a.H > NR_STEP_MAX_V * nr_step_threads(NR_STEP_MAX_V, false) * 4 ||
+      (a.p1 && !a.comb_rows && a.S1 > 8) || (a.p2 && a.S2 > 8))
+    return false;
+  const bool comb = a.p1 && a.comb_rows;
+  const NrShape s = nr_shape(a.H, true, comb);
+  if (s.V >= 4) return a.n_rows <= 148;
+  const bool alone = s.threads * (comb ? 80 : 96) > 32768;  // on its SM, by its registers
+  return !alone || a.H > 2048 || a.n_rows <= (comb ? 148 : 3 * 148);
 }
 template <typename YT, int SL>
 static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
@@ -749,6 +769,8 @@ static cudaError_t launch_norm_rows(cudaStream_t st, const NormArgs& a) {
 // are loaded before the dependency resolves (32 experts of 1024: all of them), neighbouring lanes neighbouring pieces, and up to
 // 32 experts are chosen with a lane each.  128 rows of 1024 with eight slices and 32 experts, from the release to the last exit:
 // 10 -> 5.9 us; with the sort of moe.cu, 16 decode steps of 128 sequences through four layers of 32 experts 5410 -> 5100 us.
+// One step of 64 / 192 / 384 / 512 sequences, norm_kernel / this: 222 / 209, 336 / 308, 464 / 420, 524 / 477; prompts of 1008
+// rows in all 703 / 638.
 constexpr int RT_THREADS = 512, RT_AHEAD = 16, RT_MAX_V = 4;
 template <typename YT, int V, int COMB>
 __global__ void __launch_bounds__(RT_THREADS, 1) norm_route_kernel(NormArgs a, Trace tr) {

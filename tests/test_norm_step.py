@@ -32,8 +32,21 @@ def falcon(hidden):
     gpt2(10240), llama(10248),                 # the widest; wider
 ], ids=lambda c: f"{c.name}-{c.hidden}")
 def test_step_matches_the_prompts(cfg):
-    n = 12
-    texts = [W.random_prompt(cfg.vocab_size, 61 + 3 * i, 160 + i) for i in range(n)]
+    check_step(cfg, [61 + 3 * i for i in range(12)], cfg.hidden <= 10240)
+
+
+@pytest.mark.parametrize("cfg,n,rows", [
+    (llama(2048), 444, True), (llama(2048), 445, False),    # three waves, one CTA to an SM
+    (llama(2056), 511, True),                               # norm_kernel has no more of them there
+    (gpt2(8192), 148, True), (gpt2(8192), 149, False),      # four vectors: one wave
+], ids=lambda v: v.hidden if hasattr(v, "hidden") else str(v))
+def test_wide_batches(cfg, n, rows):
+    check_step(cfg, [2 + i % 3 for i in range(n)], rows)
+
+
+def check_step(cfg, lengths, rows):
+    n = len(lengths)
+    texts = [W.random_prompt(cfg.vocab_size, k, 160 + i) for i, k in enumerate(lengths)]
     weights = list(W.random_weights(cfg, 17, round_bf16=True))
     tables, zeros = [[i] for i in range(n)], [0.0] * n
 
@@ -48,7 +61,7 @@ def test_step_matches_the_prompts(cfg):
             run.trace_begin(1 << 18)
             out = run.run_flat(texts, False, None, tables, zeros, want_logits=True)[1]
             ran = set(run.trace_end(1 << 18)[:, 1].tolist())
-            assert (ROWS in ran, GENERAL in ran) == (cfg.hidden <= 10240, cfg.hidden > 10240)
+            assert (ROWS in ran, GENERAL in ran) == (rows, not rows)
             return out
         finally:
             run.close()
