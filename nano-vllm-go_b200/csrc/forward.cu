@@ -28,7 +28,7 @@ void free_workspace(nvllm_handle* h) {
                   w.sort.counts, w.sort.offsets, w.sort.cursor, w.sort.sorted_pair, w.sort.pair_row,
                   w.sort.a_rows, w.sort.tile_expert, w.sort.tile_row0, w.sort.tile_rows,
                   w.sort.n_tiles, w.sort.part, w.moe_Y, w.moe_y, w.moe_xs, w.lr_qkw, w.lr_v, w.lr_o, w.att_gate, w.sh_gate, w.mx_in,
-                  w.m2_xbc, w.m2_dtx, w.m2_decay, w.v_first, w.side_g, w.att_split, w.att_split_cnt, w.ml_gates, w.ml_nq};
+                  w.m2_xbc, w.m2_dtx, w.m2_decay, w.v_first, w.side_g, w.att_split, w.att_split_cnt, w.ml_gates, w.ml_nq, w.state_copy};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& r : h->ropes) {
@@ -233,6 +233,13 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
     WS(w.moe_y, Tc * H * 4);
   }
 #undef WS
+  // last, so that it takes room from nothing else; a handle without it does not issue steps ahead
+  if (h->state_slot_floats && h->n_mamba == 0) {
+    const size_t one = (h->state_slot_floats + 1) * 4;
+    const int seqs = (int)std::min<size_t>(std::min(nc, h->num_state_slots), STATE_COPY / one);
+    if (seqs > 0 && A((void**)&w.state_copy, seqs * one) == cudaSuccess) w.state_copy_seqs = seqs;
+    else (void)cudaGetLastError();
+  }
   return NVLLM_OK;
 }
 

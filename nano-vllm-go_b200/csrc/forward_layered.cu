@@ -77,9 +77,7 @@ void layered_free(nvllm_handle* h) {
   F(h->pos_freq);
   h->pos_freq = nullptr;
   F(h->state_pool);
-  F(h->state_copy);
-  h->state_pool = h->state_copy = nullptr;
-  h->state_copy_bytes = 0;
+  h->state_pool = nullptr;
   h->state_copy_n = 0;
   for (auto& r : h->ropes) {
     F(r.inv_freq); F(r.cosT); F(r.sinT);

@@ -148,6 +148,8 @@ struct StepLayout {
   bool by_length = false;  // seq_order holds the sequences by their new tokens, the most first
 };
 
+constexpr size_t STATE_COPY = (size_t)128 << 20;  // recurrent state of a step that is copied aside at most (run.cu save_state)
+
 struct Workspace {
   int T_cap = 0, n_cap = 0;
   float* x = nullptr;        // [T, H] fp32 residual stream
@@ -176,6 +178,10 @@ struct Workspace {
   float* tp_buf = nullptr;   // [T, H] fp32 partial sums handed to the all-reduce (tp > 1)
   const float* logits_final = nullptr;  // where the last step's summed logits live
   int n_cap_out = 0;
+  // models with recurrent state: that of a step's sequences before the step issued ahead, [n][state_slot_floats], then the n
+  // slots; for up to state_copy_seqs of them (run.cu save_state)
+  float* state_copy = nullptr;
+  int state_copy_seqs = 0;
   size_t logits_p_floats = 0;
   float* attn_ws = nullptr;
   size_t attn_ws_floats = 0;
@@ -383,10 +389,7 @@ struct nvllm_handle {
     int misses = 0, skip = 0;  // misses in a row, calls that do not speculate because of them
   } spec_pause[2];             // of steps issued by decode and by prefill calls (run.cu)
   int spec_kind = 0;           // which of them issued the last one
-  // models with recurrent state: what it was before the step issued ahead, and the sequences whose state that is (0: none)
-  float* state_copy = nullptr;  // [n][state_slot_floats], then the n slots
-  size_t state_copy_bytes = 0;
-  int state_copy_n = 0;
+  int state_copy_n = 0;        // sequences whose recurrent state before the step issued ahead is in ws.state_copy (0: none)
   std::vector<int32_t> spec_slots;
   std::vector<int32_t> spec_len, spec_nb, spec_bt;  // per-sequence lengths / block tables of the last call
   // device-resident decode state as the host knows it: context length (incl. the token the last

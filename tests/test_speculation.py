@@ -159,6 +159,51 @@ def test_recurrent_state_goes_back(family):
         np.testing.assert_array_equal(la, lb)
 
 
+@pytest.mark.parametrize("n,ahead", [(31, True), (32, False)])
+def test_room_for_the_state(n, ahead):
+    """4 MB of state a sequence: up to 128 MB are copied aside, a step of more waits for the host.  The room is made with the
+    workspace, not between decode steps, and is part of what memory_info says."""
+    torch = pytest.importorskip("torch")
+    z = zozonex
+    cfg, w = z.random_weights(z.model([z.layer(z.delta(heads=64, kv_heads=8, dim=128, vdim=128, conv=2), 48),
+                                       z.layer(z.attn(heads=2, kv_heads=1, dim=16, vdim=16, window=40))]), 7)
+    prompts = [W.random_prompt(cfg.vocab_size, 3 + i % 3, 40 + i).tolist() for i in range(n)]
+
+    def drive(spec):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, w.items(), precision=C.PREC_FP32, num_kv_blocks=n, sampling=None, num_state_slots=n)
+        try:
+            run.set_speculation(spec)
+            seqs, outs, hits, start = [list(p) for p in prompts], [], 0, torch.cuda.mem_get_info()[0]
+
+            def call(which, prompt, temperature):
+                nonlocal hits
+                out, logits = run.run_flat([seqs[i] for i in which], prompt, [0] * len(which), [[i] for i in which],
+                                           [temperature] * len(which), [0.5] * len(which), want_logits=True, state_slots=list(which))
+                hits += run.last_stats.h2d_bytes == 0
+                outs.extend((out, logits))
+                for i, t in zip(which, out):
+                    seqs[i].append(int(t))
+
+            call(range(n), True, 1.0)  # (nothing is issued behind a step with draws)
+            free, room = torch.cuda.mem_get_info()[0], run.memory_info()["workspace"]
+            for _ in range(4):
+                call(range(2), False, 0.0)
+            two = hits
+            for _ in range(6):
+                call(range(n), False, 0.0)
+            end = torch.cuda.mem_get_info()[0]
+            assert free - end < 16 << 20 and run.memory_info()["workspace"] == room  # (graphs)
+            return outs, two, hits - two, start - end - room
+        finally:
+            run.close()
+
+    (want, *none, beside), (got, two, hits, beside_ahead) = drive(False), drive(True)
+    assert none == [0, 0] and two == 3 and hits == (5 if ahead else 0)
+    assert beside_ahead - beside < 16 << 20
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_requested_logits_rows():
     """Further rows asked for (nvllm_request_logits) in calls that a step issued ahead would answer or overwrite."""
     cfg = C.tiny_llama(hidden=1032)  # the head's products of few rows are split along k: another step's slices are elsewhere
