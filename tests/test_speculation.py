@@ -80,9 +80,9 @@ def test_arrivals_discard_one_step_each():
         run.close()
 
 
-def test_recurrent_state_is_not_stepped_ahead():
-    """Calls that a step issued ahead would not match (another token, another batch), on a model whose steps update state in
-    place: the same with speculation asked for as without."""
+def test_recurrent_state_of_steps_that_are_not_asked_for():
+    """Calls that a step issued ahead does not match (another token, another batch), on a model whose steps update state in
+    place: the same with steps issued ahead, whose state is put back, as without."""
     cfg, w = zozonex.random_weights(zozonex.mixed_model(), 7)
     prompts = [W.random_prompt(cfg.vocab_size, 9 + 4 * i, 40 + i).tolist() for i in range(3)]
 
@@ -111,7 +111,7 @@ def test_recurrent_state_is_not_stepped_ahead():
 @pytest.mark.parametrize("family", ["zozonex", "lazovik", "sutuvik", "sozurax", "defilorn"])
 def test_recurrent_state_goes_back(family):
     """Steps issued ahead on models whose steps update state in place: taken where they match; where the next call has another
-    token, batch, order or slots, or is a prompt or a repetition, the state they changed is put back."""
+    token, batch, order or slots, or is a prompt, the state they changed is put back."""
     m = importlib.import_module("test_" + family)
     cfg, w = m.random_weights(m.mixed_model(), 7)
     prompts = [W.random_prompt(cfg.vocab_size, 9 + 4 * i, 40 + i).tolist() for i in range(4)]
@@ -157,6 +157,59 @@ def test_recurrent_state_goes_back(family):
     for (a, la), (b, lb) in zip(want, got):
         np.testing.assert_array_equal(a, b)
         np.testing.assert_array_equal(la, lb)
+
+
+@pytest.mark.parametrize("family", ["zozonex", "lazovik", "sutuvik", "sozurax", "defilorn"])
+def test_recurrent_state_in_repeated_and_resident_steps(family):
+    """A repetition of a prompt step (rerun) puts the state back that the step in flight behind it changed; run_resident takes the
+    step in flight, and the next call goes on from its state, whether it asks for the step after it or for another token."""
+    m = importlib.import_module("test_" + family)
+    cfg, w = m.random_weights(m.mixed_model(), 7)
+    prompts = [W.random_prompt(cfg.vocab_size, 9 + 4 * i, 40 + i).tolist() for i in range(3)]
+
+    def drive(spec):
+        run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, w.items(), precision=C.PREC_FP32, num_kv_blocks=3, sampling=None, num_state_slots=3)
+        try:
+            run.set_speculation(spec)
+            seqs, outs, issued = [list(p) for p in prompts], [], 0
+
+            def append(tokens):
+                for s, t in zip(seqs, tokens):
+                    s.append(int(t))
+
+            def call(prompt=False):
+                nonlocal issued
+                out, logits = run.run_flat(seqs, prompt, [0] * 3, [[0], [1], [2]], [0.0] * 3, want_logits=True, state_slots=[2, 0, 1])
+                outs.extend((out, logits))
+                # the time of the last step issued is not that of the one asked for
+                issued += run.sync()[1] != run.last_stats.device_ms
+                append(out)
+
+            def resident():
+                run.run_resident()
+                outs.append(run.sync(3)[0].copy())
+                append(outs[-1])
+
+            call(prompt=True)
+            for _ in range(2):
+                run.rerun()
+                outs.append(run.sync(3)[0].copy())
+            for k in range(12):
+                call()
+                if k in (2, 5, 8):
+                    resident()
+                if k == 5:
+                    resident()       # one that is not in flight
+                if k in (5, 8):
+                    seqs[1][-1] = 5  # another token than the one that came out
+            return outs, issued
+        finally:
+            run.close()
+
+    (want, none), (got, issued) = drive(False), drive(True)
+    assert none == 0 and issued >= 5
+    for a, b in zip(want, got):
+        np.testing.assert_array_equal(a, b)
 
 
 @pytest.mark.parametrize("n,ahead", [(31, True), (32, False)])
