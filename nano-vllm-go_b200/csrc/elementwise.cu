@@ -1470,8 +1470,10 @@ cudaError_t launch_sample(cudaStream_t st, const float* logits, int ldl, int V, 
                           const float* temperature, const float* uniforms, int* out_tokens,
                           unsigned long long* amax, int* ticket, int vsplit) {
   if (n <= 0) return cudaSuccess;
-  // a CTA of a large vocabulary: 4096 logits, all its loads in flight (8192 one after another: 16 steps of GPT-2 alone 3800 us, 3763 so)
-  const int chunks = (amax && ticket && vsplit == 0 && V >= 16384) ? min(64, V / 4096) : 1;
+  // A CTA of a large vocabulary: at most 4096 logits up to 262144 of them, all its loads in flight (8192 one after another: 16
+  // steps of GPT-2 alone 3800 us, 3763 so; a few more than 4096, by rounding the CTAs down, cost a step of one to 128 rows of
+  // 32000 / 50257 / 128256 another 0.3 to 1.8 us).
+  const int chunks = (amax && ticket && vsplit == 0 && V >= 16384) ? min(64, ceil_div(V, 4096)) : 1;
   (void)launch_k(sample_kernel, dim3(n, chunks), dim3(chunks > 1 ? 256 : 1024), 0, st, logits, ldl,
                  V, temperature, uniforms, out_tokens, amax, ticket, vsplit, next_trace(7));
   return cudaGetLastError();

@@ -102,6 +102,20 @@ def test_argmax_bit_exact_with_ties():
     assert got[0] == 100 and got[1] == 0 and got[2] == 50256
 
 
+@pytest.mark.parametrize("vocab", [16383, 16384, 16385, 20480, 20484, 32000])
+def test_argmax_of_vocabularies_shared_out(vocab):
+    """From 16384 logits on several CTAs reduce a row (elementwise.cu launch_sample)."""
+    cfg = C.tiny_llama(vocab_size=vocab, num_layers=1)
+    prompts = [W.random_prompt(vocab, 2 + i % 3, i) for i in range(96)]
+    run = nvllm_pkg.sub("runner").CudaModelRunner(cfg, W.random_weights(cfg, 3), precision=C.PREC_FP32, num_kv_blocks=96, sampling=None)
+    try:
+        out, logits = run.run_flat(prompts, True, [0] * 96, [[i] for i in range(96)], [0.0] * 96, want_logits=True)
+    finally:
+        run.close()
+    np.testing.assert_array_equal(out, logits.argmax(1))
+    assert len({int(t) * 4 // vocab for t in out}) == 4  # winners from everywhere
+
+
 # ------------------------------------------------------------------ whole forward pass
 # Prompt seeds of the strict (free-running, identical-token) cases: the first seed >= 4321 whose
 # oracle top-2 margin is >= 2 % of max|logit| on every compared step, for fp32 and bf16-rounded
