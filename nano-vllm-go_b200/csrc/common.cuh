@@ -58,7 +58,10 @@ __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
 // partial sums.  16 decode steps, us before / with the hint: 64 sequences of 640 tokens through four Llama-1B layers 5059 /
 // 4761 (K / V alone: all of it), 128 through routed experts 6261 / 5954, one through GPT-2 3924 / 3686.  K / V that would fit
 // L2 until the next step gain nothing from staying there (GPT-2, one sequence: 3597 / 3620; 64 x 60 tokens through routed
-// experts 5460 / 5148), so all of them go.
+// experts 5460 / 5148), and neither do pages of a prefix that sequences share, though each of them reads those lines in the
+// same step (one step of 64 / 128 sequences on 2048 common tokens and 60 of their own: four Llama-1B layers 272 / 265 and 401 /
+// 381, routed experts 288 / 275 and 402 / 379, two Llama-3B layers 241 / 232 and 354 / 334; of 16 on 4096: 274 / 271), so all of
+// them go.
 __device__ __forceinline__ uint64_t l2_once() {
   uint64_t p;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));

@@ -392,8 +392,9 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         const int odd = lane & 1, pr = lane >> 1;
         uint8_t* stg = epi_stage.act[warp - 2];
         const int j0 = (n0 + q * 32) >> 1;
-        // (a choice of the unit per token keeps a lane's sixteen from overlapping: 64 prompts of 512 through four Llama-1B
-        // layers 10.69 ms so, 10.27 with the choice outside; 64 of 384 through routed experts 4.45 and 4.29)
+        // (a choice of the unit per token keeps a lane's sixteen from overlapping: 64 prompts of 384 through four layers of
+        // routed experts 4.34 ms so, 4.23 with the choice outside; 64 of 512 through four Llama-1B layers 10.4 and 10.1, where
+        // the runs of one side differ by as much)
         auto glu_rows = [&](auto unit) {
 #pragma unroll 1
           for (int c0 = 32 * half; c0 < PR_BT && m0 + c0 < Me; c0 += 64) {

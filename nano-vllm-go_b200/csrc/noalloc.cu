@@ -2,7 +2,7 @@
 // kernel of single-sequence decode) with its fp32 split-K slices in a file-scope device array
 // instead of a cudaMalloc'ed workspace.  For callers that cannot allocate: code under CUDA graph
 // capture, tight serving loops, harnesses that forbid cudaMalloc.  No counterpart in the
-// reference; added at the request of the run's operators.
+// reference.
 //
 //   C[M, N] (fp32) = A[M, K] @ W[N, K]^T     A, W, C are DEVICE pointers the caller owns.
 //

@@ -27,7 +27,8 @@ run.trace_begin(1 << 17)
 for _ in range(2):
     run.run_resident()
 rec = run.trace_end(1 << 17)
-names = {1: "gemm", 2: "norm", 3: "rope_kv", 4: "attn_dec", 46: "gemm_pair", 47: "norm_rows"}
+names = {1: "gemm", 2: "norm", 3: "rope_kv", 4: "attn_dec", 46: "gemm_pair", 47: "norm_rows", 53: "norm_step", 54: "norm_route",
+         55: "state_copy", 56: "copy_out"}
 aux = rec[rec[:, 1] == 9]
 rec = rec[rec[:, 1] != 9]
 seqs = sorted(set(int(x) for x in rec[:, 0]))
