@@ -28,7 +28,7 @@ void free_workspace(nvllm_handle* h) {
                   w.sort.counts, w.sort.offsets, w.sort.cursor, w.sort.sorted_pair, w.sort.pair_row,
                   w.sort.a_rows, w.sort.tile_expert, w.sort.tile_row0, w.sort.tile_rows,
                   w.sort.n_tiles, w.sort.part, w.moe_Y, w.moe_y, w.moe_xs, w.lr_qkw, w.lr_v, w.lr_o, w.att_gate, w.sh_gate, w.mx_in,
-                  w.m2_xbc, w.m2_dtx, w.m2_decay, w.v_first, w.side_g, w.att_split, w.att_split_cnt, w.ml_gates, w.ml_nq, w.state_copy};
+                  w.m2_xbc, w.m2_dtx, w.m2_decay, w.v_first, w.side_g, w.att_split, w.att_split_cnt, w.ml_gates, w.ml_nq};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& r : h->ropes) {
@@ -67,7 +67,7 @@ static void fit_split_room(nvllm_handle* h) {
   h->ws.fit_head = r.head;
 }
 
-int ensure_workspace(nvllm_handle* h, int T, int n) {
+static int make_workspace(nvllm_handle* h, int T, int n) {
   Workspace& w = h->ws;
   if (T <= w.T_cap && n <= w.n_cap) return NVLLM_OK;
   NV_CHECK(h, cudaStreamSynchronize(h->stream));
@@ -233,14 +233,31 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
     WS(w.moe_y, Tc * H * 4);
   }
 #undef WS
-  // last, so that it takes room from nothing else; a handle without it does not issue steps ahead
-  if (h->state_slot_floats && h->n_mamba == 0) {
-    const size_t one = (h->state_slot_floats + 1) * 4;
-    const int seqs = (int)std::min<size_t>(std::min(nc, h->num_state_slots), STATE_COPY / one);
-    if (seqs > 0 && A((void**)&w.state_copy, seqs * one) == cudaSuccess) w.state_copy_seqs = seqs;
-    else (void)cudaGetLastError();
-  }
   return NVLLM_OK;
+}
+int ensure_workspace(nvllm_handle* h, int T, int n) {
+  const int rc = make_workspace(h, T, n);
+  if (rc != NVLLM_ERR_NOMEM || !h->state_copy) return rc;
+  free_state_copy(h);  // the step itself comes before steps issued ahead
+  return make_workspace(h, T, n);
+}
+
+// The room for recurrent state copied aside (run.cu save_state): made once, with the handle.  Without it no step is issued
+// ahead.
+void make_state_copy(nvllm_handle* h) {
+  const size_t one = (h->state_slot_floats + 1) * 4;
+  const int seqs = (int)std::min<size_t>(h->num_state_slots, STATE_COPY / one);
+  if (seqs > 0 && cudaMalloc((void**)&h->state_copy, seqs * one) == cudaSuccess) {
+    h->state_copy_seqs = seqs;
+    return;
+  }
+  (void)cudaGetLastError();
+  h->state_copy = nullptr;
+}
+void free_state_copy(nvllm_handle* h) {
+  if (h->state_copy) cudaFree(h->state_copy);
+  h->state_copy = nullptr;
+  h->state_copy_seqs = h->state_copy_n = 0;
 }
 
 // ------------------------------------------------------------------ profiling

@@ -78,7 +78,7 @@ void layered_free(nvllm_handle* h) {
   h->pos_freq = nullptr;
   F(h->state_pool);
   h->state_pool = nullptr;
-  h->state_copy_n = 0;
+  free_state_copy(h);
   for (auto& r : h->ropes) {
     F(r.inv_freq); F(r.cosT); F(r.sinT);
   }
@@ -644,6 +644,7 @@ int layered_finalize(nvllm_handle* h) {
     NV_CHECK(h, cudaMalloc((void**)&r.inv_freq, (size_t)half * 8));
     NV_CHECK(h, cudaMemcpy(r.inv_freq, f.data(), (size_t)half * 8, cudaMemcpyHostToDevice));
   }
+  if (h->state_slot_floats) make_state_copy(h);
   NV_CHECK(h, cudaStreamSynchronize(h->stream));
   h->finalized = true;
   return NVLLM_OK;

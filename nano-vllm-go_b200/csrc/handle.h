@@ -178,10 +178,6 @@ struct Workspace {
   float* tp_buf = nullptr;   // [T, H] fp32 partial sums handed to the all-reduce (tp > 1)
   const float* logits_final = nullptr;  // where the last step's summed logits live
   int n_cap_out = 0;
-  // models with recurrent state: that of a step's sequences before the step issued ahead, [n][state_slot_floats], then the n
-  // slots; for up to state_copy_seqs of them (run.cu save_state)
-  float* state_copy = nullptr;
-  int state_copy_seqs = 0;
   size_t logits_p_floats = 0;
   float* attn_ws = nullptr;
   size_t attn_ws_floats = 0;
@@ -389,7 +385,10 @@ struct nvllm_handle {
     int misses = 0, skip = 0;  // misses in a row, calls that do not speculate because of them
   } spec_pause[2];             // of steps issued by decode and by prefill calls (run.cu)
   int spec_kind = 0;           // which of them issued the last one
-  int state_copy_n = 0;        // sequences whose recurrent state before the step issued ahead is in ws.state_copy (0: none)
+  // models with recurrent state: that of a step's sequences before the step issued ahead, [n][state_slot_floats], then the n
+  // slots, for up to state_copy_seqs of them (run.cu save_state); how many it holds now (0: none)
+  float* state_copy = nullptr;
+  int state_copy_seqs = 0, state_copy_n = 0;
   std::vector<int32_t> spec_slots;
   std::vector<int32_t> spec_len, spec_nb, spec_bt;  // per-sequence lengths / block tables of the last call
   // device-resident decode state as the host knows it: context length (incl. the token the last
@@ -419,6 +418,8 @@ extern thread_local std::string g_create_error;
 
 void free_workspace(nvllm_handle* h);
 int ensure_workspace(nvllm_handle* h, int T, int n);
+void make_state_copy(nvllm_handle* h);
+void free_state_copy(nvllm_handle* h);
 int forward_step(nvllm_handle* h);  // runs h->lay
 int forward_step_layered(nvllm_handle* h);  // forward_layered.cu
 int layered_set_weight(nvllm_handle* h, const char* name, int dtype, const void* host,

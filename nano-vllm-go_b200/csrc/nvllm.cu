@@ -362,7 +362,7 @@ int nvllm_memory_info(const nvllm_handle* h, uint64_t* weight_bytes, uint64_t* k
   if (!h) return NVLLM_ERR_INVALID;
   if (weight_bytes) *weight_bytes = h->weight_bytes;
   if (kv_bytes) *kv_bytes = h->kv_bytes;
-  if (workspace_bytes) *workspace_bytes = h->ws_bytes;
+  if (workspace_bytes) *workspace_bytes = h->ws_bytes + h->state_copy_seqs * (h->state_slot_floats + 1) * 4;
   return NVLLM_OK;
 }
 

@@ -174,13 +174,13 @@ static int check_waits(nvllm_handle* h) {
 }
 // Recurrent state is updated in place: it is copied aside before a step is issued ahead, and back if that step is not the one
 // asked for.  The copy costs its stream twice per step where the host's turn costs some 80 us, so steps of more state than
-// STATE_COPY are left to the host; its place is part of the workspace, not made between steps.  Decode steps of a delta-rule
+// STATE_COPY are left to the host; its room is made with the handle.  Decode steps of a delta-rule
 // layer (16 heads of 128 x 128; 1.1 MB a sequence) and a window attention layer, us without / with: 4 sequences 160 / 113, 32
 // 201 / 145, 64 260 / 193, 120 360 / 273.  Mamba-2 state that lives in KV blocks is not copied: those models wait for the host.
 static bool save_state(nvllm_handle* h, int n) {
-  if (n > h->ws.state_copy_seqs) return false;
-  if (launch_state_copy(h->stream, n, h->lay.d + h->lay.state_slots, h->state_pool, h->state_slot_floats, h->ws.state_copy,
-                        reinterpret_cast<int*>(h->ws.state_copy + (size_t)n * h->state_slot_floats), false) != cudaSuccess)
+  if (n > h->state_copy_seqs) return false;
+  if (launch_state_copy(h->stream, n, h->lay.d + h->lay.state_slots, h->state_pool, h->state_slot_floats, h->state_copy,
+                        reinterpret_cast<int*>(h->state_copy + (size_t)n * h->state_slot_floats), false) != cudaSuccess)
     return false;
   h->state_copy_n = n;
   return true;
@@ -191,8 +191,8 @@ static int restore_state(nvllm_handle* h) {
   if (n == 0) return NVLLM_OK;
   h->state_copy_n = 0;
   NV_CHECK(h, cudaSetDevice(h->dev));
-  NV_CHECK(h, launch_state_copy(h->stream, n, nullptr, h->state_pool, h->state_slot_floats, h->ws.state_copy,
-                                reinterpret_cast<int*>(h->ws.state_copy + (size_t)n * h->state_slot_floats), true));
+  NV_CHECK(h, launch_state_copy(h->stream, n, nullptr, h->state_pool, h->state_slot_floats, h->state_copy,
+                                reinterpret_cast<int*>(h->state_copy + (size_t)n * h->state_slot_floats), true));
   return NVLLM_OK;
 }
 static void remember_call(nvllm_handle* h, int n, const int32_t* cu_seqlens, const int32_t* block_tables,

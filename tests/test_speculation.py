@@ -215,7 +215,7 @@ def test_recurrent_state_in_repeated_and_resident_steps(family):
 @pytest.mark.parametrize("n,ahead", [(31, True), (32, False)])
 def test_room_for_the_state(n, ahead):
     """4 MB of state a sequence: up to 128 MB are copied aside, a step of more waits for the host.  The room is made with the
-    workspace, not between decode steps, and is part of what memory_info says."""
+    handle, not between decode steps, and is part of what memory_info says."""
     torch = pytest.importorskip("torch")
     z = zozonex
     cfg, w = z.random_weights(z.model([z.layer(z.delta(heads=64, kv_heads=8, dim=128, vdim=128, conv=2), 48),
