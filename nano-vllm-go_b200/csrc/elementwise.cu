@@ -76,8 +76,14 @@ __global__ void embed_kernel(const int* __restrict__ tokens, const int* __restri
 
 // The same for prompts: a warp per row, four neighbouring entries per lane (whole sectors in every access), eight pieces of the
 // row in flight, no block barriers.  Bound by memory.  24 k rows of 2048, bf16 copy and sums of squares: 174 -> 95 us; 18.7 k of
-// 1024 50 -> 23.
-constexpr int EMBED_WARPS = 8, EMBED_MIN_ROWS = 512;
+// 1024 50 -> 23.  A row's chain is eight times as long as in a block of its own, so there have to be enough of them: twelve to
+// an SM, and with sines (fp64, which a warp computes one piece after another) sixty-four.  A block / a warp per row, us:
+//   rows                1024         1536         1792         2048         4096         8192        16000        24000
+//   width  768       2.0 / 4.6    2.5 / 4.5    4.9 / 4.5    6.6 / 4.7   10.7 / 8.5   19.9 / 12.9
+//         2048       5.9 / 9.3    8.9 / 9.7   10.3 / 9.2   11.9 / 9.3   22.9 / 19.8  45.7 / 29.2
+//         4544       7.6 / 8.9   10.8 / 9.1   11.7 / 9.2   14.5 / 10.1  27.5 / 22.6  54.0 / 36.4
+//         2048, sines 6.4 / 14.7  8.9 / 14.9               11.9 / 14.8  22.4 / 31.1  45.5 / 45.0  85.4 / 75.2  130 / 112
+constexpr int EMBED_WARPS = 8, EMBED_MIN_ROWS = 12 * 148, EMBED_MIN_ROWS_SINES = 64 * 148;
 template <typename WT>
 __global__ void __launch_bounds__(32 * EMBED_WARPS) embed_rows_kernel(const int* __restrict__ tokens, const int* __restrict__ positions, int T,
                                                                       const WT* __restrict__ wte, const WT* __restrict__ wpe, int max_pos,
@@ -156,7 +162,7 @@ cudaError_t launch_embed(cudaStream_t st, int wdt, const int* tokens, const int*
                          int H, void* xb, float* ssq, const float* g, const double* pos_freq, void* y) {
   if (T <= 0) return cudaSuccess;
   if ((xb == nullptr) != (ssq == nullptr) || (xb && !g)) return cudaErrorInvalidValue;
-  if (T >= EMBED_MIN_ROWS && H % 8 == 0) {  // (fewer rows: a block each is the shorter way)
+  if (T >= (pos_freq ? EMBED_MIN_ROWS_SINES : EMBED_MIN_ROWS) && H % 8 == 0) {
     const dim3 grid(ceil_div(T, EMBED_WARPS)), block(32 * EMBED_WARPS);
     return wdt == DT_F32 ? launch_k(embed_rows_kernel<float>, grid, block, 0, st, tokens, positions, T, (const float*)wte, (const float*)wpe,
                                     max_pos, mult, x, H, (bf16*)xb, ssq, g, pos_freq, (float*)y, next_trace(5))
