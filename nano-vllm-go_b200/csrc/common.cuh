@@ -74,6 +74,14 @@ __device__ __forceinline__ uint4 ld_once16(const void* p) {
                : "l"(p), "l"(l2_once()));
   return v;
 }
+// The same as ordinary lines, for fp32 weights: the policy's registers are what the widest kernels that read those (six rows,
+// four weight rows to a warp: 128 registers) do not have.  With them half the CTAs are on an SM: a step of one / six sequences
+// through four Llama-1B layers in fp32 375 / 607 us so, 426 / 801 with the policy, and nothing gained by it elsewhere.
+__device__ __forceinline__ uint4 ld_stream16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 // streaming variant for weights read exactly once (do not pollute the caches)
 __device__ __forceinline__ void load8_stream(const bf16* p, float (&v)[8]) {
   const uint4 r = ld_once16(p);
@@ -86,7 +94,7 @@ __device__ __forceinline__ void load8_stream(const bf16* p, float (&v)[8]) {
   }
 }
 __device__ __forceinline__ void load8_stream(const float* p, float (&v)[8]) {
-  const uint4 a = ld_once16(p), b = ld_once16(p + 4);
+  const uint4 a = ld_stream16(p), b = ld_stream16(p + 4);
   v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
   v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
 }

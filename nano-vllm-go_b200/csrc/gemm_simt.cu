@@ -54,8 +54,8 @@ template <> struct Raw8<bf16> {
 template <> struct Raw8<float> {
   uint4 a, b;
   __device__ __forceinline__ void ld(const float* p) {
-    a = ld_once16(p);
-    b = ld_once16(p + 4);
+    a = ld_stream16(p);
+    b = ld_stream16(p + 4);
   }
   __device__ __forceinline__ void cvt(float (&o)[8]) const {
     o[0] = __uint_as_float(a.x); o[1] = __uint_as_float(a.y); o[2] = __uint_as_float(a.z); o[3] = __uint_as_float(a.w);
