@@ -361,7 +361,6 @@ template <int MI>
 __global__ void __launch_bounds__(FG_THREADS)
 gemm_f32_kernel(GemmArgs g, int kc, Trace tr) {
   TRACE_ENTRY(tr);
-  pdl_launch_dependents();
   constexpr int BM = 8 * MI;
   extern __shared__ __align__(16) float fsm[];  // [stage][BM + 64][pitch]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -438,6 +437,13 @@ gemm_f32_kernel(GemmArgs g, int kc, Trace tr) {
       }
     }
   }
+  // The kernels behind this one are let in here and not at its start.  They release each other at once, so that the next
+  // product's CTAs used to come in while these still filled the SMs unevenly, and stayed where they came in: six on one SM,
+  // two on most.  (Between them a norm of a step takes most of an SM's registers, which made it worse.)  Decode steps of
+  // 9, 12, 16 sequences in fp32, us released at the start / here: GPT-2 787 / 576, 785 / 580, 879 / 586; four Llama-1B layers
+  // 581 / 516, 582 / 520, 579 / 527; a delta-rule and a window layer 373 / 294, 424 / 314, 481 / 313.  (Eight blocks of k
+  // earlier 629, 537 and 326 in those of 9.)
+  pdl_launch_dependents();
   float* out = g.out + (size_t)blockIdx.z * g.split_stride;
 #pragma unroll
   for (int i = 0; i < MI; i++) {

@@ -7,7 +7,7 @@ import nvllm_pkg
 
 pytestmark = pytest.mark.gpu
 
-GEMV = 11  # id in the timeline
+GEMV, PRODUCT = 11, 12  # ids in the timeline
 
 
 def timeline(cfg, n):
@@ -40,3 +40,16 @@ def test_ctas_of_a_product_on_an_sm(n, ctas):
     cfg = C.tiny_llama(hidden=1024, ffn_dim=16384, num_layers=1)
     launches = [r for r in timeline(cfg, n) if r[0, 1] == GEMV]
     assert most_on_one_sm(max(launches, key=len)) >= ctas
+
+
+@pytest.mark.parametrize("n", [9, 16])
+def test_the_kernel_behind_a_product_comes_late(n):
+    """CTAs that come in while a product's own still fill the SMs unevenly stay where they are (gemm_simt.cu)."""
+    launches = timeline(C.tiny_llama(hidden=1024, ffn_dim=16384, num_layers=1), n)
+    seen = 0
+    for rec, behind in zip(launches, launches[1:]):
+        if rec[0, 1] == PRODUCT and len(rec) >= 100:
+            start, end = rec[:, 4].max(), rec[:, 6].max()
+            assert behind[:, 4].min() >= start + (end - start) // 3
+            seen += 1
+    assert seen >= 2
