@@ -564,7 +564,8 @@ int nvllm_set_speculation(nvllm_handle* h, int enabled);
 /* GetVocabSize / GetModelConfig (purego/generic_runner.go:184-196). */
 int nvllm_get_config(const nvllm_handle* h, nvllm_config* out);
 
-/* Bytes of HBM the handle holds: weights, KV pool, workspaces. */
+/* Bytes of HBM the handle holds: weights, KV pool (recurrent state included), workspaces (with the room that recurrent
+ * state is copied aside to; 128 MB at most). */
 int nvllm_memory_info(const nvllm_handle* h, uint64_t* weight_bytes,
                       uint64_t* kv_bytes, uint64_t* workspace_bytes);
 
