@@ -242,12 +242,14 @@ int ensure_workspace(nvllm_handle* h, int T, int n) {
   return make_workspace(h, T, n);
 }
 
-// The room for recurrent state copied aside (run.cu save_state): made once, with the handle.  Without it no step is issued
-// ahead.
+// The room for recurrent state copied aside (run.cu save_state): made once, with the handle, where as much again stays free
+// for what calls allocate.  Without it no step is issued ahead.
 void make_state_copy(nvllm_handle* h) {
   const size_t one = (h->state_slot_floats + 1) * 4;
   const int seqs = (int)std::min<size_t>(h->num_state_slots, STATE_COPY / one);
-  if (seqs > 0 && cudaMalloc((void**)&h->state_copy, seqs * one) == cudaSuccess) {
+  size_t room = 0, all = 0;
+  if (seqs > 0 && cudaMemGetInfo(&room, &all) == cudaSuccess && room >= seqs * one + STATE_COPY &&
+      cudaMalloc((void**)&h->state_copy, seqs * one) == cudaSuccess) {
     h->state_copy_seqs = seqs;
     return;
   }
